@@ -77,34 +77,77 @@ struct SweepParams {
 // unfused in the reference's order) and the box test; surviving (point,
 // transform) pairs are compacted into Q / gidx / kidx (batch order:
 // arbitrary).
-__global__ void activate_chunk_kernel(const double* __restrict__ GV, int64_t nG,
-                                      const double* __restrict__ S,
-                                      const double* __restrict__ T, int K, SweepParams sp,
-                                      const unsigned long long* __restrict__ mm,
-                                      double* __restrict__ Q, int32_t* __restrict__ gidx,
-                                      int32_t* __restrict__ kidx, unsigned* __restrict__ cnt) {
+//
+// Bound by the FP64 pipe when every pair takes the FP64 motion (27 FP64
+// operations; 64 poses x 580k points: 1.74 ms, 1.02 ms this way).  Most pairs
+// fall outside the box, so the motion is first taken in FP32: the coordinates' rounding and
+// the FP32 operations move each component by less than 10 u per term
+// |A| (|g| + |t|), u = 2^-24; a pair farther outside than 1e-6 (16 u) of that
+// sum is rejected, any other (NaN included) is decided in FP64 as before.
+// Survivors take their places with one atomic per warp and transform.
+__global__ void __launch_bounds__(256) activate_chunk_kernel(
+    const double* __restrict__ GV, int64_t nG, const double* __restrict__ S,
+    const double* __restrict__ T, int K, SweepParams sp,
+    const unsigned long long* __restrict__ mm, double* __restrict__ Q,
+    int32_t* __restrict__ gidx, int32_t* __restrict__ kidx, unsigned* __restrict__ cnt) {
+  __shared__ float s_A[16 * 12];
+  for (int i = threadIdx.x; i < K * 12; i += blockDim.x) s_A[i] = (float)T[i];
+  __syncthreads();
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (g >= nG) return;
-  const double sg = S[g];
-  if (sp.finite_iso && sg == sg && sg < sp.skip_below) return;
-  const double x = GV[g * 3], y = GV[g * 3 + 1], z = GV[g * 3 + 2];
+  const int lane = threadIdx.x & 31;
+  bool alive = g < nG;
+  double x = 0, y = 0, z = 0;
+  if (alive) {
+    const double sg = S[g];
+    alive = !(sp.finite_iso && sg == sg && sg < sp.skip_below);
+    x = GV[g * 3];
+    y = GV[g * 3 + 1];
+    z = GV[g * 3 + 2];
+  }
+  if (!__any_sync(0xffffffffu, alive)) return;
+  const float fx = (float)x, fy = (float)y, fz = (float)z;
   double lo[3], hi[3];
+  float flo[3], fhi[3];
   for (int j = 0; j < 3; ++j) {
     lo[j] = __dsub_rn(from_ordered_bits(mm[j]), sp.ext);
     hi[j] = __dadd_rn(from_ordered_bits(mm[3 + j]), sp.ext);
+    flo[j] = __double2float_rd(lo[j]);
+    fhi[j] = __double2float_ru(hi[j]);
   }
   for (int k = 0; k < K; ++k) {
-    const double* A = T + 12 * k;
-    const double d0 = __dsub_rn(x, A[3]), d1 = __dsub_rn(y, A[7]), d2 = __dsub_rn(z, A[11]);
-    double gv[3];
-    bool inside = true;
-    for (int j = 0; j < 3; ++j) {
-      gv[j] = __dadd_rn(__dadd_rn(__dmul_rn(d0, A[j]), __dmul_rn(d1, A[4 + j])),
-                        __dmul_rn(d2, A[8 + j]));
-      inside &= lo[j] <= gv[j] && gv[j] <= hi[j];
+    bool maybe = alive;
+    if (sp.finite_iso && alive) {
+      const float* A = s_A + 12 * k;
+      const float d0 = fx - A[3], d1 = fy - A[7], d2 = fz - A[11];
+      const float m0 = fabsf(fx) + fabsf(A[3]), m1 = fabsf(fy) + fabsf(A[7]),
+                  m2 = fabsf(fz) + fabsf(A[11]);
+      for (int j = 0; j < 3; ++j) {
+        const float v = fmaf(d2, A[8 + j], fmaf(d1, A[4 + j], d0 * A[j]));
+        const float e =
+            1e-6f * fmaf(m2, fabsf(A[8 + j]), fmaf(m1, fabsf(A[4 + j]), m0 * fabsf(A[j]))) + 1e-37f;
+        if (v + e < flo[j] || v - e > fhi[j]) maybe = false;
+      }
     }
-    if (sp.finite_iso && !inside) continue;
-    const unsigned i = atomicAdd(cnt, 1u);
+    if (!__any_sync(0xffffffffu, maybe)) continue;
+    double gv[3] = {0, 0, 0};
+    if (maybe) {
+      const double* A = T + 12 * k;
+      const double d0 = __dsub_rn(x, A[3]), d1 = __dsub_rn(y, A[7]), d2 = __dsub_rn(z, A[11]);
+      bool inside = true;
+      for (int j = 0; j < 3; ++j) {
+        gv[j] = __dadd_rn(__dadd_rn(__dmul_rn(d0, A[j]), __dmul_rn(d1, A[4 + j])),
+                          __dmul_rn(d2, A[8 + j]));
+        inside &= lo[j] <= gv[j] && gv[j] <= hi[j];
+      }
+      if (sp.finite_iso && !inside) maybe = false;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, maybe);
+    if (!m) continue;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(cnt, (unsigned)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (!maybe) continue;
+    const unsigned i = base + __popc(m & ((1u << lane) - 1u));
     Q[(int64_t)i * 3] = gv[0];
     Q[(int64_t)i * 3 + 1] = gv[1];
     Q[(int64_t)i * 3 + 2] = gv[2];
