@@ -180,3 +180,28 @@ def test_squared_distance_random_soup_with_skinny_triangles(cuda):
     Dr, Ir, Cr = O.squared_distance(V, F, P)
     assert np.all(_close2(D, Dr))
     assert np.all(_close2(_tri_dist2(V, F, P, I), D))
+
+
+@pytest.mark.parametrize("nq", [1, 31, 33, 400])
+@pytest.mark.parametrize("subdiv", [0, 2, 4])
+def test_queries_equally_far_from_everything(cuda, subdiv, nq):
+    """Queries at and around a sphere's centre reach nearly every triangle:
+    the searches a thread hands over to a whole warp.  The surface has
+    exactly tied triangles (subdiv 0: the icosahedron), a bounded search and
+    float32 queries included."""
+    V, F = synth.icosphere(subdiv)
+    rng = np.random.default_rng(31)
+    Q = rng.normal(size=(nq, 3)) * 10.0 ** rng.uniform(-9, -1, (nq, 1))
+    Q[0] = 0
+    bvh = G.FastWindingNumberBVH(V, F, tree="binned")
+    for q in (Q, Q.astype(np.float32)):
+        D, I, Cp = bvh.squared_distance(q)
+        Dr, Ir, Cr = O.squared_distance(V, F, q.astype(np.float64))
+        assert _close2(D, Dr).all()
+        assert (np.abs(((q - Cp) ** 2).sum(1) - D) <= 1e-14).all()
+        assert ((I >= 0) & (I < F.shape[0])).all()
+    # nothing below the bound: the reference's "not found"
+    D, I, _ = bvh.squared_distance(Q, up_sqr_d=0.25)
+    Dr, _, _ = O.squared_distance(V, F, Q, 0.25)
+    assert np.array_equal(D == 0.25, Dr == 0.25) and (I[D == 0.25] == -1).all()
+    bvh.close()
