@@ -467,23 +467,73 @@ __global__ void __launch_bounds__(128, 8) soup_eval_mixed_kernel(EvalParams prm,
   }
 }
 
-// Plain FP64 walk (also used, over a list, to re-evaluate threshold queries).
+// Plain FP64 walk.
 template <typename QT, typename WT>
-__global__ void __launch_bounds__(128) soup_eval_fp64_kernel(EvalParams prm, const QT* __restrict__ Q,
+__global__ void __launch_bounds__(128) soup_eval_fp64_kernel(EvalParams prm,
+                                                             const QT* __restrict__ Q,
+                                                             const int32_t* __restrict__ perm,
+                                                             int64_t nQ, WT* __restrict__ W) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const bool valid = i < nQ;
+  int64_t qi = 0;
+  double qx = 0, qy = 0, qz = 0;
+  if (valid) soupwalk::read_query(Q, perm, (const int32_t*)nullptr, i, qi, qx, qy, qz);
+  __shared__ soupwalk::Fp64Queue fp64_q[4];
+  const double acc = soupwalk::walk_fp64(prm, valid, qx, qy, qz, fp64_q[threadIdx.x >> 5]);
+  if (valid) W[qi] = (WT)(acc * kInv4Pi);
+}
+
+// The same two evaluations with T lanes per query (soup_walk.cuh, team
+// walks), for batches too small to fill the GPU with 32 queries per warp.
+template <typename QT, typename WT, int T, int kTree>
+__global__ void __launch_bounds__(128, 7) soup_team_mixed_kernel(
+    EvalParams prm, const QT* __restrict__ Q, const int32_t* __restrict__ perm, int64_t nQ,
+    WT* __restrict__ W, int32_t* __restrict__ refine_list, unsigned* __restrict__ refine_count) {
+  __shared__ soupwalk::NearQueue near_q[4];
+  __shared__ int2 s_stack[4][soupwalk::kTeamStack];
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / T;
+  const bool valid = i < nQ;
+  int64_t qi = 0;
+  double qx = 0, qy = 0, qz = 0;
+  if (valid) soupwalk::read_query(Q, perm, (const int32_t*)nullptr, i, qi, qx, qy, qz);
+  float acc;
+  double acc64;
+  soupwalk::walk_mixed_team<T, kTree>(prm, valid, qx, qy, qz, acc, acc64,
+                                      near_q[threadIdx.x >> 5], s_stack[threadIdx.x >> 5]);
+  if (!valid || (threadIdx.x & (T - 1))) return;
+  const double w = soupwalk::mixed_result(acc, acc64);
+  W[qi] = (WT)w;
+  if (fabs(w - 0.5) <= kBand) {
+    const unsigned s = atomicAdd(refine_count, 1u);
+    refine_list[s] = (int32_t)qi;
+  }
+}
+
+template <typename QT, typename WT, int T>
+__global__ void __launch_bounds__(128) soup_team_fp64_kernel(EvalParams prm,
+                                                             const QT* __restrict__ Q,
                                                              const int32_t* __restrict__ perm,
                                                              const int32_t* __restrict__ list,
                                                              const unsigned* __restrict__ list_count,
                                                              int64_t nQ, WT* __restrict__ W) {
-  const int64_t n = list ? (int64_t)*list_count : nQ;
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (list && blockIdx.x * (int64_t)blockDim.x >= n) return;  // whole warp idle
-  const bool valid = i < n;
-  int64_t qi = 0;
-  double qx = 0, qy = 0, qz = 0;
-  if (valid) soupwalk::read_query(Q, perm, list, i, qi, qx, qy, qz);
   __shared__ soupwalk::Fp64Queue fp64_q[4];
-  const double acc = soupwalk::walk_fp64(prm, valid, qx, qy, qz, fp64_q[threadIdx.x >> 5]);
-  if (valid) W[qi] = (WT)(acc * kInv4Pi);
+  __shared__ int2 s_stack[4][soupwalk::kTeamStack];
+  const int64_t n = list ? (int64_t)*list_count : nQ;
+  const int64_t per_warp = 32 / T;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t w0 = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+       w0 * per_warp < n; w0 += warps) {
+    const int64_t i = w0 * per_warp + (threadIdx.x & 31) / T;
+    const bool valid = i < n;
+    int64_t qi = 0;
+    double qx = 0, qy = 0, qz = 0;
+    if (valid) soupwalk::read_query(Q, perm, list, i, qi, qx, qy, qz);
+    const double acc = soupwalk::walk_fp64_team<T>(prm, valid, qx, qy, qz,
+                                                   fp64_q[threadIdx.x >> 5],
+                                                   s_stack[threadIdx.x >> 5]);
+    if (valid && !(threadIdx.x & (T - 1))) W[qi] = (WT)(acc * kInv4Pi);
+    __syncwarp();
+  }
 }
 
 __global__ void moments_bounded_kernel(const SoupNodeD* __restrict__ nd, int64_t n,
@@ -626,6 +676,23 @@ void soup_build(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t* F,
 }
 
 // ------------------------------------------------------------------- eval --
+// Lanes per query.  Teams win while 32 queries per warp leave the GPU waiting
+// for its longest walks; the warp-coherent walk reads each record once per
+// warp and wins once there are queries enough, the later the more slots the
+// tree has (sparser queries share fewer of them).  Measured crossings, mixed:
+// 1.9k slots ~100k queries, 30k ~200k, 122k ~400k, 1.95M ~1.6M; plain FP64,
+// whose terms are evaluated 32 at a time either way, somewhat earlier.
+// us per call with 32 / 8 / 4 / 1 lanes, mixed, 1.95M slots: 1,000 queries
+// 41 / 60 / 97 / 908; 60k 355 / 264 / 288 / 1344; 600k 2202 / 1060 / 973 /
+// 1480; 2M - / 2968 / 2577 / 2335.  FP64: 1,000 120 / 237 / 376 / 2582;
+// 60k 1868 / 1940 / 2294 / 5309; 200k 5746 / 5408 / 5914 / 7485.
+static int team_size(int64_t nQ, int64_t slots, int precision) {
+  const double cross = 65536.0 + 1024.0 * std::sqrt((double)slots);
+  if (precision == GWN_MIXED)
+    return nQ <= 4096 ? 32 : (double)nQ > cross ? 1 : nQ <= 200000 ? 8 : 4;
+  return nQ <= 60000 && (double)nQ <= 0.75 * cross ? 32 : (double)nQ > 0.75 * cross ? 1 : 8;
+}
+
 template <typename QT, typename WT>
 static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int64_t nQ, void* Wv,
                         int precision, cudaStream_t st) {
@@ -658,6 +725,9 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
   }
   const int32_t* perm = qo.active ? qo.perm.get() : nullptr;
   const unsigned grid = (unsigned)((nQ + 127) / 128);
+  const int team = team_size(nQ, s.nnodes, precision);
+  auto team_grid = [&](int t) { return (unsigned)((nQ * t + 127) / 128); };
+  const bool ref = prm.ref32 != 0;
   if (precision == GWN_MIXED) {
     DevBuf<int32_t> list((size_t)nQ, st);
     DevBuf<unsigned> count(1, st);
@@ -666,22 +736,39 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
       PhaseTimer ph("walk", st);
       // the tree kind is fixed per launch: the reference tree's instance
       // carries no FP64 re-check code
-      auto kernel = prm.ref32 ? soup_eval_mixed_kernel<QT, WT, false, GWN_TREE_REFERENCE>
-                              : soup_eval_mixed_kernel<QT, WT, false, GWN_TREE_BINNED>;
-      launch_kernel(kernel, grid, 128, 0, st, prm, Q, perm, nQ, W, list.get(), count.get(),
-                    (unsigned long long*)nullptr);
+      if (team == 1) {
+        auto kernel = ref ? soup_eval_mixed_kernel<QT, WT, false, GWN_TREE_REFERENCE>
+                          : soup_eval_mixed_kernel<QT, WT, false, GWN_TREE_BINNED>;
+        launch_kernel(kernel, grid, 128, 0, st, prm, Q, perm, nQ, W, list.get(), count.get(),
+                      (unsigned long long*)nullptr);
+      } else {
+        auto kernel = team == 32 ? (ref ? soup_team_mixed_kernel<QT, WT, 32, GWN_TREE_REFERENCE>
+                                        : soup_team_mixed_kernel<QT, WT, 32, GWN_TREE_BINNED>)
+                      : team == 8 ? (ref ? soup_team_mixed_kernel<QT, WT, 8, GWN_TREE_REFERENCE>
+                                         : soup_team_mixed_kernel<QT, WT, 8, GWN_TREE_BINNED>)
+                                  : (ref ? soup_team_mixed_kernel<QT, WT, 4, GWN_TREE_REFERENCE>
+                                         : soup_team_mixed_kernel<QT, WT, 4, GWN_TREE_BINNED>);
+        launch_kernel(kernel, team_grid(team), 128, 0, st, prm, Q, perm, nQ, W, list.get(),
+                      count.get());
+      }
     }
-    GWN_CUDA(cudaGetLastError());
     {
+      // a few queries near the threshold, anywhere: a warp each
       PhaseTimer ph("refine", st);
-      launch_kernel(soup_eval_fp64_kernel<QT, WT>, grid, 128, 0, st, prm, Q, nullptr, list.get(),
-                                                          count.get(), nQ, W);
+      const unsigned rgrid = (unsigned)std::min<int64_t>((nQ + 3) / 4, 8 * num_sms());
+      launch_kernel(soup_team_fp64_kernel<QT, WT, 32>, rgrid, 128, 0, st, prm, Q,
+                    (const int32_t*)nullptr, (const int32_t*)list.get(),
+                    (const unsigned*)count.get(), nQ, W);
     }
-    GWN_CUDA(cudaGetLastError());
   } else {
     PhaseTimer ph("walk", st);
-    launch_kernel(soup_eval_fp64_kernel<QT, WT>, grid, 128, 0, st, prm, Q, perm, nullptr, nullptr, nQ, W);
-    GWN_CUDA(cudaGetLastError());
+    if (team == 1) {
+      launch_kernel(soup_eval_fp64_kernel<QT, WT>, grid, 128, 0, st, prm, Q, perm, nQ, W);
+    } else {
+      auto kernel = team == 32 ? soup_team_fp64_kernel<QT, WT, 32> : soup_team_fp64_kernel<QT, WT, 8>;
+      launch_kernel(kernel, team_grid(team), 128, 0, st, prm, Q, perm, (const int32_t*)nullptr,
+                    (const unsigned*)nullptr, nQ, W);
+    }
   }
 }
 

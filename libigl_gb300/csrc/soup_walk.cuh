@@ -506,6 +506,246 @@ __device__ __forceinline__ double walk_fp64(const EvalParams& prm, bool valid, d
   return acc;
 }
 
+// ------------------------------------------------------------ team walks --
+// Small batches.  The warp-coherent walk needs about 150 dependent steps (a
+// node record's latency each) per warp however few queries there are, and
+// more when 32 neighbouring queries are far apart, so a batch that does not
+// fill the GPU is bound by that chain.  Here T lanes share one query: an item
+// is a range of pre-order slots [c, e) that its lane walks without a stack
+// (an opened node moves to c + 1, any other to its link); a lane that opens
+// a node with siblings after it leaves them as a new item on the team's
+// stack in shared memory, from which idle lanes take the newest.  A full
+// stack only means that the lane keeps the siblings itself.  Items go to
+// lanes in lane order, so the terms each lane adds, and the butterfly sum of
+// the lanes at the end, depend on the query alone.
+// The slots visited and the terms are the warp-coherent walk's; their order
+// of summation is not.
+constexpr int kTeamStack = 128;  // items per warp, shared by its 32 / T teams
+
+template <int T>
+struct Team {
+  int2* stk;          // this team's items
+  unsigned mask, lt;  // lanes of the team; lanes below this one
+  int c = 0, e = 0, sp = 0;
+  static constexpr int kCap = kTeamStack * T / 32;
+
+  __device__ __forceinline__ Team(int2* warp_stack, bool valid, int nnodes) {
+    const int lane = threadIdx.x & 31;
+    stk = warp_stack + (lane / T) * kCap;
+    mask = T == 32 ? 0xffffffffu : ((1u << (T & 31)) - 1u) << (lane & ~(T - 1));
+    lt = (1u << lane) - 1u;
+    if (valid && (lane & (T - 1)) == 0) {
+      c = nnodes > 1 ? 1 : 0;  // an internal root is always opened
+      e = nnodes;
+    }
+  }
+  // Idle lanes take items; false once no lane of the warp has work.
+  __device__ __forceinline__ bool take() {
+    __syncwarp();
+    const unsigned idle = __ballot_sync(0xffffffffu, c >= e) & mask;
+    const int rank = __popc(idle & lt);
+    if (c >= e && rank < sp) {
+      const int2 it = stk[sp - 1 - rank];
+      c = it.x;
+      e = it.y;
+    }
+    sp -= min(sp, __popc(idle));
+    __syncwarp();
+    return __any_sync(0xffffffffu, c < e);
+  }
+  // Moves past the current slot: into it (open) or to `next`, the slot after
+  // its subtree.
+  __device__ __forceinline__ void advance(bool act, bool open, int next) {
+    const bool push = act && open && next < e;
+    const unsigned m = __ballot_sync(0xffffffffu, push) & mask;
+    const bool room = sp + __popc(m) <= kCap;
+    if (act) {
+      if (push && room) {
+        stk[sp + __popc(m & lt)] = make_int2(next, e);
+        e = next;
+      }
+      c = open ? c + 1 : next;
+    }
+    if (room) sp += __popc(m);
+  }
+};
+
+template <typename V>
+__device__ __forceinline__ V team_sum(V v, int T) {
+  for (int o = T >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// walk_mixed for teams of T lanes (every lane of a team passes the team's
+// query); every lane returns the query's sums.
+template <int T, int kTree>
+__device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, bool valid, double qx,
+                                                double qy, double qz, float& acc, double& acc64,
+                                                NearQueue& nq, int2* warp_stack) {
+  const int lane = threadIdx.x & 31;
+  nq.q[lane][0] = qx;
+  nq.q[lane][1] = qy;
+  nq.q[lane][2] = qz;
+  const unsigned lt_mask = (1u << lane) - 1u, full = 0xffffffffu;
+  int nqueued = 0;    // warp-uniform
+  unsigned mine = 0;  // this lane's queue positions
+  const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
+  const float S = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + prm.cmax;
+  const float sigma = guard_sigma(S);
+  acc = 0.f;
+  acc64 = 0.0;
+  Team<T> team(warp_stack, valid, prm.nnodes);
+  while (team.take()) {
+    const bool act = team.c < team.e;
+    bool open = false, want64 = false;
+    int next = 0, slot64 = 0;
+    if (act) {
+      const SoupNodeF* r = prm.nf + team.c;
+      float4 a, rb, rc, rd, re, rf;
+      ldg256(&r->a, a, rb);
+      ldg256(&r->c, rc, rd);
+      ldg256(&r->e, re, rf);
+      const int link = __float_as_int(rf.w);
+      const bool leaf = link < 0;
+      next = leaf ? team.c + 1 : link;
+      const float dx = fx - a.x, dy = fy - a.y, dz = fz - a.z;
+      float r2;
+      bool near;
+      if (kTree == GWN_TREE_REFERENCE) {  // ref_open32
+        r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+        near = r2 <= __fmul_rn(a.w, prm.beta2f);
+      } else {
+        r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const float thr = a.w * prm.beta2f;
+        near = r2 <= thr;
+        if (in_guard_band(r2, thr, sigma)) {
+          const SoupNodeD* r64 = prm.nd + team.c;
+          near = open_test64(nq.q[lane][0], nq.q[lane][1], nq.q[lane][2], r64->P[0], r64->P[1],
+                             r64->P[2], r64->maxP2, prm.beta2d);
+        }
+      }
+      if (!near) {
+        const float om = far_field32(rb, rc, rd, re, rf, dx, dy, dz, r2, prm.order);
+        if (isfinite(om)) acc += om;
+        else near = true;
+      }
+      if (near) {
+        if (leaf) {
+          const int slot = ~link;
+          const float rad = sqrtf(a.w) + prm.eps;
+          if (r2 <= rad * rad * 1.0001f) {
+            want64 = true;
+            slot64 = slot;
+          } else {
+            const float4 t0 = __ldg(&prm.tf[(int64_t)slot * 3]);
+            const float4 t1 = __ldg(&prm.tf[(int64_t)slot * 3 + 1]);
+            const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
+            acc += tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx, t1.x - fy,
+                                          t1.y - fz, t1.z - fx, t1.w - fy, t2.x - fz);
+          }
+        } else {
+          open = true;
+        }
+      }
+    }
+    const unsigned m64 = __ballot_sync(full, want64);
+    if (m64) {
+      const int k = __popc(m64);
+      if (nqueued + k > 32) {
+        flush_near64(prm.td, nq, nqueued, mine, acc64);
+        nqueued = 0;
+        mine = 0;
+      }
+      if (want64) {
+        const int pos = nqueued + __popc(m64 & lt_mask);
+        nq.e[pos] = make_int2(slot64, lane);
+        mine |= 1u << pos;
+      }
+      nqueued += k;
+    }
+    team.advance(act, open, next);
+  }
+  if (nqueued) flush_near64(prm.td, nq, nqueued, mine, acc64);
+  acc = team_sum(acc, T);
+  acc64 = team_sum(acc64, T);
+}
+
+// walk_fp64 for teams of T lanes.
+template <int T>
+__device__ __forceinline__ double walk_fp64_team(const EvalParams& prm, bool valid, double qx,
+                                                 double qy, double qz, Fp64Queue& fq,
+                                                 int2* warp_stack) {
+  const int lane = threadIdx.x & 31;
+  fq.q[lane][0] = qx;
+  fq.q[lane][1] = qy;
+  fq.q[lane][2] = qz;
+  const unsigned lt_mask = (1u << lane) - 1u, full = 0xffffffffu;
+  double acc = 0.0;
+  int nq = 0;         // warp-uniform
+  unsigned mine = 0;  // this lane's queue positions
+  Team<T> team(warp_stack, valid, prm.nnodes);
+  while (team.take()) {
+    const bool act = team.c < team.e;
+    bool open = false, push = false;
+    int next = 0, term = 0;
+    double value = 0.0;
+    if (act) {
+      const SoupNodeD* r = prm.nd + team.c;
+      const long long link = r->link;
+      const bool leaf = link < 0;
+      next = leaf ? team.c + 1 : (int)link;
+      bool near = prm.ref32 ? ref_open32((float)qx, (float)qy, (float)qz,
+                                         __ldg(&prm.nf[team.c].a), prm.beta2f)
+                            : open_test64(qx, qy, qz, r->P[0], r->P[1], r->P[2], r->maxP2,
+                                          prm.beta2d);
+      if (!near) {
+        const double dx = qx - r->P[0], dy = qy - r->P[1], dz = qz - r->P[2];
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (prm.fp64_queue && r2 >= 1e-100) {
+          push = true;
+          term = team.c;
+        } else {
+          const double om = far_field<double>(load_far(r), dx, dy, dz, r2, prm.order);
+          if (isfinite(om)) {
+            push = true;
+            term = kQueuedValue;
+            value = om;
+          } else {
+            near = true;
+          }
+        }
+      }
+      if (near) {
+        if (leaf) {
+          push = true;
+          term = (int)link;  // ~slot
+        } else {
+          open = true;
+        }
+      }
+    }
+    const unsigned m = __ballot_sync(full, push);
+    if (m) {
+      const int k = __popc(m);
+      if (nq + k > 32) {
+        flush_fp64(prm, fq, nq, mine, acc);
+        nq = 0;
+        mine = 0;
+      }
+      if (push) {
+        const int pos = nq + __popc(m & lt_mask);
+        fq.e[pos] = make_int2(term, lane);
+        if (term == kQueuedValue) fq.v[pos] = value;
+        mine |= 1u << pos;
+      }
+      nq += k;
+    }
+    team.advance(act, open, next);
+  }
+  if (nq) flush_fp64(prm, fq, nq, mine, acc);
+  return team_sum(acc, T);
+}
+
 // Plain FP64 walk of one query by one thread, no warp cooperation (for
 // sparse re-evaluation lists whose lanes may belong to different meshes).
 // Visits the same nodes and adds the same terms, in the same order, as

@@ -220,3 +220,33 @@ def test_tree_builder_corner_cases(cuda):
     Ff = np.concatenate([np.stack([a, a + 30, a + 1], 1), np.stack([a + 1, a + 30, a + 31], 1)])
     _check_tree(np.ascontiguousarray(Vf), np.ascontiguousarray(Ff, dtype=np.int32), Q * 0.8 + 0.3)
 
+
+
+@pytest.mark.parametrize("tree", ["reference", "binned"])
+@pytest.mark.parametrize("shape", ["sphere", "nested"])
+def test_lanes_per_query_do_not_change_the_result(cuda, tree, shape):
+    """Small batches share a query between the lanes of a team, large ones walk
+    32 queries per warp: the same queries in batches on either side of each
+    rule's edge.  The terms are the same and their sum runs in another order,
+    so FP32 sums differ by at most about 150 terms x 2^-24 x the terms' total
+    of a few turns (3e-5), FP64 sums by 1e-12.  "nested" puts triangles at
+    2^-k, a deep unbalanced tree whose teams run out of stack."""
+    if shape == "sphere":
+        V, F = synth.icosphere(3)
+    else:
+        k = 2.0 ** -np.arange(120.0)
+        V = (k[:, None, None] * np.array([[1, 0, 0], [1.4, 0, 0.1], [1, 0.4, 0]])).reshape(-1, 3)
+        F = np.arange(V.shape[0], dtype=np.int32).reshape(-1, 3)
+    rng = np.random.default_rng(41)
+    n = 260_000  # past the warp-coherent rule for these trees
+    Q = rng.uniform(-1.3, 1.3, (n, 3))
+    Q[: n // 2] *= 10.0 ** rng.uniform(-6, 0, (n // 2, 1))
+    bvh = G.FastWindingNumberBVH(V, F, tree=tree)
+    for prec, tol in (("mixed", 3e-5), ("fp64", 1e-12)):
+        W = bvh.eval(Q, 2.0, prec)
+        for m in (1, 31, 33, 4096, 4097, 8191, 60_000, 60_001, 70_000):
+            w = bvh.eval(Q[:m], 2.0, prec)
+            assert np.array_equal(np.isfinite(w), np.isfinite(W[:m])), (prec, m)
+            assert np.abs(w - W[:m]).max() <= tol, (prec, m)
+            assert np.array_equal(w, bvh.eval(Q[:m], 2.0, prec)), (prec, m)
+    bvh.close()
