@@ -66,8 +66,10 @@ constexpr int kSpans = 16;
 constexpr int kSplits = kSpans - 1;
 constexpr uint32_t kMinFraction = 16;
 constexpr uint32_t kSmallMax = 2 * kSpans;  // exhaustive / sorted splits
-constexpr uint32_t kMedMax = 1024;           // one CTA per split
+constexpr uint32_t kSub = 1024;              // subtrees built by one CTA, splits by one warp
+constexpr uint32_t kCtaMax = 32768;          // splits by one CTA
 constexpr uint32_t kChunk = 1024;            // positions per CTA in GPU-wide passes
+constexpr uint32_t kSubRef = 0xc0000000u;    // child that is a subtree (above 30-bit items)
 constexpr uint32_t kTerm = 0x80000000u;      // tape entry holding a box index
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr double kNearFrac = 1e-3;
@@ -155,18 +157,25 @@ __device__ __forceinline__ Box keys_box(const uint32_t* k) {
   return b;
 }
 
-// One node of the tree under construction (build order: depth by depth).
+// One node above the subtrees (numbered depth by depth).
 struct RNode {
   uint32_t start, n;  // its boxes: idx[start .. start + n)
   Box all;            // the box its parent's split handed down
   uint32_t cut[5];    // sub-ranges after the splits made so far
   Box sub[4];
   float area[4];
-  int32_t nsub, choice;
-  uint32_t child[4];  // item (triangle id), kInternal | node, kEmpty
+  int32_t choice;
+  uint32_t child[4];  // item (triangle id), kInternal | node, kSubRef | subtree
   // the split of the current round
   uint32_t t_start, t_n, t_mid;
   Box t_box, t_out[2];
+};
+
+// Counters of the build; the fields before ntop are zeroed for every depth.
+struct BuildCounts {
+  uint32_t lists[3][3];  // per round: parts for a warp, a CTA, the whole GPU
+  uint32_t max_n;        // the largest node of the next depth
+  uint32_t ntop, nsub, nodes, max_depth, unbounded;
 };
 
 // --------------------------------------------------------------- boxes --
@@ -243,251 +252,119 @@ __global__ void compact_kernel(const uint32_t* __restrict__ keep, const uint32_t
   }
 }
 
-__global__ void root_init_kernel(RNode* nodes, uint32_t m, const uint32_t* __restrict__ root_keys) {
-  RNode& r = nodes[0];
-  r.start = 0;
-  r.n = m;
-  r.all = keys_box(root_keys);
-  r.nsub = 1;
-  r.choice = 0;
-}
+__global__ void keys_init_kernel(uint32_t* keys) { keys_init(keys); }
 
-// ------------------------------------------------------ split: <= 32 boxes --
-// One split of n <= 32 boxes (FWNFS.h:5350-5585) on a local copy of the
-// indices; returns the cut (boxes [0, mid) go left).
-__device__ void split_small(const Box& all, uint32_t* id, uint32_t n, const Box* __restrict__ tb,
-                            uint32_t& mid, Box& o0, Box& o1) {
-  if (n == 2) {
-    o0 = tb[id[0]];
-    o1 = tb[id[1]];
-    mid = 1;
-    return;
+// ------------------------------------------------ one split by one warp --
+// Splits of at most kSub boxes run in one warp on shared memory: boxes by
+// local index (bx: lo xyz, hi xyz), their current order in perm.  A serial
+// thread per split (insertion sort, three-way partition) was bound by its
+// dependent shared- and local-memory accesses: 4.8 ms of split kernels for
+// 1.3M triangles, most of it one thread per CTA partitioning.
+struct SplitMem {
+  const float* bx;  // [6][stride]
+  int stride;
+  uint16_t *perm, *tmp, *tape_e, *tape_g;  // by position
+};
+struct SplitScratch {  // one per warp
+  uint32_t cnt[kSpans];
+  uint32_t keys[kSpans][6];
+  Box sub[4];
+  float area[4];
+  uint32_t cut[5];
+};
+constexpr unsigned kFull = 0xffffffffu;
+constexpr uint16_t kTerm16 = 0x8000u;
+
+__device__ __forceinline__ Box mem_box(const SplitMem& m, uint32_t e) {
+  Box b;
+  for (int a = 0; a < 3; ++a) {
+    b.lo[a] = m.bx[a * m.stride + e];
+    b.hi[a] = m.bx[(3 + a) * m.stride + e];
   }
-  if (n <= 6) {  // every 2-partition with box 0 on side 0
-    Box lb[6];
-    for (uint32_t b = 0; b < n; ++b) lb[b] = tb[id[b]];
-    const uint32_t lim = 1u << (n - 1);
-    uint32_t best = kNone;
-    float best_h = 0.f;
-    for (uint32_t bits = 1; bits < lim; ++bits) {
-      Box s0 = lb[0], s1;
-      box_empty(s1);
-      uint32_t c0 = 1, c1 = 0;
-      for (uint32_t b = 0; b + 1 < n; ++b) {
-        if ((bits >> b) & 1u) {
-          box_add(s1, lb[b + 1]);
-          ++c1;
-        } else {
-          box_add(s0, lb[b + 1]);
-          ++c0;
-        }
-      }
-      const float h = half_area(s0) * (float)c0 + half_area(s1) * (float)c1;
-      if (best == kNone || h < best_h) {
-        best = bits;
-        best_h = h;
-        o0 = s0;
-        o1 = s1;
-      }
+  return b;
+}
+__device__ __forceinline__ float mem_centre2(const SplitMem& m, uint32_t e, int axis) {
+  return m.bx[axis * m.stride + e] + m.bx[(3 + axis) * m.stride + e];
+}
+__device__ __forceinline__ Box shfl_box(const Box& b, int src) {
+  Box r;
+  for (int a = 0; a < 3; ++a) {
+    r.lo[a] = __shfl_sync(kFull, b.lo[a], src);
+    r.hi[a] = __shfl_sync(kFull, b.hi[a], src);
+  }
+  return r;
+}
+// Inclusive scans of boxes over the lanes (from lane 0 up / from lane 31 down).
+__device__ __forceinline__ Box scan_box_up(Box b) {
+  const int lane = threadIdx.x & 31;
+  for (int o = 1; o < 32; o <<= 1) {
+    Box t;
+    for (int a = 0; a < 3; ++a) {
+      t.lo[a] = __shfl_up_sync(kFull, b.lo[a], o);
+      t.hi[a] = __shfl_up_sync(kFull, b.hi[a], o);
     }
-    uint32_t rest[5];
-    for (uint32_t b = 0; b + 1 < n; ++b) rest[b] = id[b + 1];
-    uint32_t w = 1;
-    for (uint32_t b = 0; b + 1 < n; ++b)
-      if (!((best >> b) & 1u)) id[w++] = rest[b];
-    mid = w;
-    for (uint32_t b = 0; b + 1 < n; ++b)
-      if ((best >> b) & 1u) id[w++] = rest[b];
-    return;
+    if (lane >= o) box_add(b, t);
   }
-  float len;
-  const int axis = longest_axis(all, len);
-  if (!(len > 0.f)) {  // a single point or NaN: an arbitrary split
-    mid = n / 2;
-    o0 = all;
-    o1 = all;
-    return;
-  }
-  // stable sort by centre (the reference's chunked insertion sort + merges
-  // is a stable sort), then sweep
-  float c[kSmallMax];
-  for (uint32_t i = 0; i < n; ++i) c[i] = centre2(tb[id[i]], axis);
-  for (uint32_t i = 1; i < n; ++i) {
-    const float v = c[i];
-    const uint32_t e = id[i];
-    uint32_t j = i;
-    while (j > 0 && v < c[j - 1]) {
-      c[j] = c[j - 1];
-      id[j] = id[j - 1];
-      --j;
+  return b;
+}
+__device__ __forceinline__ Box scan_box_down(Box b) {
+  const int lane = threadIdx.x & 31;
+  for (int o = 1; o < 32; o <<= 1) {
+    Box t;
+    for (int a = 0; a < 3; ++a) {
+      t.lo[a] = __shfl_down_sync(kFull, b.lo[a], o);
+      t.hi[a] = __shfl_down_sync(kFull, b.hi[a], o);
     }
-    c[j] = v;
-    id[j] = e;
+    if (lane + o < 32) box_add(b, t);
   }
-  const uint32_t ns = n - 1;
-  // right boxes as the reference accumulates them: starting from box ns-1,
-  // so the last box never enters (FWNFS.h:5560-5565)
-  Box R[kSmallMax - 1];
-  Box acc = tb[id[ns - 1]];
-  R[ns - 1] = acc;
-  for (uint32_t i = ns - 1; i > 0; --i) {
-    box_add(acc, tb[id[i]]);
-    R[i - 1] = acc;
-  }
-  Box L = tb[id[0]];
-  uint32_t best = 0;
-  float best_h = half_area(L) + half_area(R[0]) * (float)(n - 1);
-  Box bestL = L;
-  for (uint32_t s = 1; s < ns; ++s) {
-    box_add(L, tb[id[s]]);
-    const float h = half_area(L) * (float)(s + 1) + half_area(R[s]) * (float)(n - (s + 1));
-    if (h < best_h) {
-      best = s;
-      best_h = h;
-      bestL = L;
-    }
-  }
-  mid = best + 1;
-  o0 = bestL;
-  o1 = R[best];
+  return b;
+}
+// Lane of the serial rule "start from lane 0, take a later one when strictly
+// smaller": the first smallest value, or lane 0 if its value is NaN.
+__device__ __forceinline__ int first_smallest(float h, bool valid) {
+  const int lane = threadIdx.x & 31;
+  uint32_t k = (valid && h == h) ? fkey(h) : 0xffffffffu;
+  if (lane == 0 && !(h == h)) k = 0u;
+  const uint32_t best = __reduce_min_sync(kFull, k);
+  return __ffs(__ballot_sync(kFull, k == best)) - 1;
 }
 
-__global__ void split_small_kernel(RNode* __restrict__ nodes, const uint32_t* __restrict__ list,
-                                   uint32_t count, uint32_t* __restrict__ idx,
-                                   const Box* __restrict__ tb) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  RNode& N = nodes[list[k]];
-  const uint32_t s = N.t_start, n = N.t_n;
-  uint32_t id[kSmallMax];
-  for (uint32_t i = 0; i < n; ++i) id[i] = idx[s + i];
-  uint32_t mid;
-  Box o0, o1;
-  split_small(N.t_box, id, n, tb, mid, o0, o1);
-  for (uint32_t i = 0; i < n; ++i) idx[s + i] = id[i];
-  N.t_mid = s + mid;
-  N.t_out[0] = o0;
-  N.t_out[1] = o1;
-}
-
-// ------------------------------------------- the sequential partition --
-// partitionByCentre on arrays of (index, centre) pairs, positions [lo, hi):
-// returns the first position >= pivot and the first > pivot.
-__device__ void partition_seq(uint32_t* id, float* c, uint32_t lo, uint32_t hi, float pivot,
-                              uint32_t& ps, uint32_t& pe) {
-  uint32_t s = lo, e = lo;
-  for (uint32_t p = lo; p < hi; ++p) {
-    const float v = c[p];
-    if (v < pivot) {
-      if (p != s) {
-        const uint32_t ti = id[p];
-        if (s == e) {
-          id[p] = id[s];
-          c[p] = c[s];
-        } else {
-          id[p] = id[e];
-          c[p] = c[e];
-          id[e] = id[s];
-          c[e] = c[s];
-        }
-        id[s] = ti;
-        c[s] = v;
-      }
-      ++s;
-      ++e;
-    } else if (v == pivot) {
-      if (p != e) {
-        const uint32_t ti = id[p];
-        id[p] = id[e];
-        c[p] = c[e];
-        id[e] = ti;
-        c[e] = v;
-      }
-      ++e;
-    }
-  }
-  ps = s;
-  pe = e;
-}
-
-// Median of three centres as nthElement picks its pivot (FWNFS.h:5852-5870).
-__device__ __forceinline__ float median3(float a, float b, float c) {
-  float p0 = a, p1 = b, p2 = c, t;
-  if (p0 < p1) { t = p0; p0 = p1; p1 = t; }
-  if (p0 < p2) { t = p0; p0 = p2; p2 = t; }
-  if (p1 < p2) { t = p1; p1 = p2; p2 = t; }
-  return p1;
-}
-
-// Each step narrows [lo, hi) by at least the pivot's own box, so at most
-// hi - lo steps run; the bound only guards against a hang.
-__device__ bool nth_seq(uint32_t* id, float* c, uint32_t lo, uint32_t hi, uint32_t nth) {
-  for (uint32_t step = 0, limit = hi - lo + 1; step < limit; ++step) {
-    const float pv = median3(c[lo], c[lo + (hi - lo) / 2], c[hi - 1]);
-    uint32_t ps, pe;
-    partition_seq(id, c, lo, hi, pv, ps, pe);
-    if (nth < ps) hi = ps;
-    else if (nth < pe) return true;
-    else lo = pe;
-    if (hi <= lo + 1) return true;
-  }
-  return false;
-}
-
-// Span statistics -> chosen span (or -1 when none keeps 1/16 of the boxes on
-// each side, FWNFS.h:5684-5706), with the left / right boxes of that span.
+// Span statistics (16 spans of counts and box keys) -> the chosen span, or -1
+// when none keeps 1/16 of the boxes on each side (FWNFS.h:5684-5706), with
+// the left / right boxes of that span.  Lane i holds span i.
 __device__ int choose_span(const uint32_t* cnt, const uint32_t (*keys)[6], uint32_t n, Box& Lb,
                            Box& Rb, uint32_t& left_count, uint32_t& lc0, uint32_t& lc14) {
-  Box span[kSpans];
-  for (int i = 0; i < kSpans; ++i) {
-    if (cnt[i]) {
-      for (int a = 0; a < 3; ++a) {
-        span[i].lo[a] = fkey_inv(keys[i][a]);
-        span[i].hi[a] = fkey_inv(keys[i][3 + a]);
-      }
-    } else {
-      box_empty(span[i]);
-    }
+  const int lane = threadIdx.x & 31;
+  Box b;
+  box_empty(b);
+  uint32_t lc = 0;
+  if (lane < kSpans && cnt[lane]) {
+    lc = cnt[lane];
+    b = keys_box(keys[lane]);
   }
-  Box L[kSplits], R[kSplits];
-  uint32_t lc[kSplits];
-  Box acc = span[0];
-  L[0] = acc;
-  for (int i = 1; i < kSplits; ++i) {
-    box_add(acc, span[i]);
-    L[i] = acc;
+  const Box L = scan_box_up(b);
+  Box R = scan_box_down(b);
+  for (int a = 0; a < 3; ++a) {  // the spans after this lane's
+    R.lo[a] = __shfl_down_sync(kFull, R.lo[a], 1);
+    R.hi[a] = __shfl_down_sync(kFull, R.hi[a], 1);
   }
-  acc = span[kSpans - 1];
-  R[kSplits - 1] = acc;
-  for (int i = kSplits - 1; i > 0; --i) {
-    box_add(acc, span[i]);
-    R[i - 1] = acc;
-  }
-  uint32_t run = cnt[0];
-  lc[0] = run;
-  for (int i = 1; i < kSplits; ++i) {
-    run += cnt[i];
-    lc[i] = run;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, lc, o);
+    if (lane >= o) lc += t;
   }
   const uint32_t min_count = n / kMinFraction;
   const uint32_t max_count = (uint32_t)(((uint64_t)(kMinFraction - 1) * n) / kMinFraction);
-  float smallest = INFINITY;
-  int si = -1;
-  for (int i = 0; i < kSplits; ++i) {
-    if (lc[i] < min_count || lc[i] > max_count) continue;
-    const float h = (float)lc[i] * half_area(L[i]) + (float)(n - lc[i]) * half_area(R[i]);
-    if (h < smallest) {
-      smallest = h;
-      si = i;
-    }
-  }
-  lc0 = lc[0];
-  lc14 = lc[kSplits - 1];
-  if (si >= 0) {
-    Lb = L[si];
-    Rb = R[si];
-    left_count = lc[si];
-  }
+  const float h = (float)lc * half_area(L) + (float)(n - lc) * half_area(R);
+  const bool ok = lane < kSplits && lc >= min_count && lc <= max_count && h < INFINITY;
+  const uint32_t k = ok ? fkey(h) : 0xffffffffu;
+  const uint32_t best = __reduce_min_sync(kFull, k);
+  lc0 = __shfl_sync(kFull, lc, 0);
+  lc14 = __shfl_sync(kFull, lc, kSplits - 1);
+  if (best == 0xffffffffu) return -1;
+  const int si = __ffs(__ballot_sync(kFull, k == best)) - 1;
+  Lb = shfl_box(L, si);
+  Rb = shfl_box(R, si);
+  left_count = __shfl_sync(kFull, lc, si);
   return si;
 }
 
@@ -500,26 +377,636 @@ __device__ __forceinline__ uint32_t nth_target(uint32_t n, uint32_t lc0, uint32_
   return n / 2;
 }
 
-// --------------------------------------------- split: 33..1024 boxes --
-__global__ void __launch_bounds__(256) split_medium_kernel(RNode* __restrict__ nodes,
-                                                           const uint32_t* __restrict__ list,
-                                                           uint32_t* __restrict__ idx,
-                                                           const Box* __restrict__ tb,
-                                                           unsigned* __restrict__ status) {
-  __shared__ uint32_t s_id[kMedMax];
-  __shared__ float s_c[kMedMax];
-  __shared__ uint32_t s_cnt[kSpans];
-  __shared__ uint32_t s_keys[kSpans][6];
-  __shared__ uint32_t s_bk[2][6];
-  __shared__ uint32_t s_mid;
-  __shared__ int s_need;
-  const int tid = threadIdx.x;
+// Median of three centres as nthElement picks its pivot (FWNFS.h:5852-5870).
+__device__ __forceinline__ float median3(float a, float b, float c) {
+  float p0 = a, p1 = b, p2 = c, t;
+  if (p0 < p1) { t = p0; p0 = p1; p1 = t; }
+  if (p0 < p2) { t = p0; p0 = p2; p2 = t; }
+  if (p1 < p2) { t = p1; p1 = p2; p2 = t; }
+  return p1;
+}
+
+// Prefix state of the partition's tapes: boxes below / equal to the pivot so
+// far, and the counts at the first equal / first upper box.
+struct TapeState {
+  uint32_t nL = 0, nE = 0, firstE = kNone, firstG = kNone, L_atE = 0, LE_atG = 0;
+};
+// One lane's box (class k: 0 below, 1 equal, 2 above, 3 none) of 32 at job
+// position rel: advances the state and returns what the box writes: its
+// place below the pivot (L), its tape entries.
+struct TapeOps {
+  uint32_t L, te, tg, rotE, rotG;
+  bool afterE, afterG;
+};
+__device__ __forceinline__ TapeOps tape_step(TapeState& s, int k, uint32_t rel0) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const unsigned mL = __ballot_sync(kFull, k == 0), mE = __ballot_sync(kFull, k == 1),
+                 mG = __ballot_sync(kFull, k == 2);
+  if (s.firstE == kNone && mE) {
+    const int f = __ffs(mE) - 1;
+    s.firstE = rel0 + f;
+    s.L_atE = s.nL + __popc(mL & ((1u << f) - 1u));
+  }
+  if (s.firstG == kNone && mG) {
+    const int f = __ffs(mG) - 1;
+    s.firstG = rel0 + f;
+    s.LE_atG = s.nL + s.nE + __popc((mL | mE) & ((1u << f) - 1u));
+  }
+  TapeOps o;
+  const uint32_t rel = rel0 + lane;
+  o.L = s.nL + __popc(mL & lt);
+  const uint32_t E = s.nE + __popc(mE & lt), G = rel - o.L - E;
+  o.afterE = s.firstE != kNone && rel > s.firstE;
+  o.afterG = s.firstG != kNone && rel > s.firstG;
+  o.rotE = o.afterE ? o.L - s.L_atE : 0u;
+  o.rotG = o.afterG ? (o.L + E) - s.LE_atG : 0u;
+  o.te = E + o.rotE;
+  o.tg = G + o.rotG;
+  s.nL += __popc(mL);
+  s.nE += __popc(mE);
+  return o;
+}
+
+// partitionByCentre of positions [lo, hi) about the pivot (see the file
+// comment: the queues' tapes), by one warp in shared memory.
+__device__ void warp_partition(const SplitMem& m, int axis, uint32_t lo, uint32_t hi, float pivot,
+                               uint32_t& ps, uint32_t& pe) {
+  const int lane = threadIdx.x & 31;
+  TapeState s;
+  for (uint32_t base = lo; base < hi; base += 32) {
+    const uint32_t p = base + lane;
+    uint16_t e = 0;
+    int k = 3;
+    if (p < hi) {
+      e = m.perm[p];
+      const float c = mem_centre2(m, e, axis);
+      k = c < pivot ? 0 : (c == pivot ? 1 : 2);
+    }
+    const TapeOps o = tape_step(s, k, base - lo);
+    if (k == 0) {
+      m.tmp[lo + o.L] = e;
+      if (o.afterE) m.tape_e[lo + o.te] = (uint16_t)o.rotE;
+      if (o.afterG) m.tape_g[lo + o.tg] = (uint16_t)o.rotG;
+    } else if (k == 1) {
+      m.tape_e[lo + o.te] = kTerm16 | e;
+      if (o.afterG) m.tape_g[lo + o.tg] = (uint16_t)o.rotG;
+    } else if (k == 2) {
+      m.tape_g[lo + o.tg] = kTerm16 | e;
+    }
+  }
+  __syncwarp();
+  const uint32_t RE = s.firstE != kNone ? s.nL - s.L_atE : 0u;
+  const uint32_t RG = s.firstG != kNone ? s.nL + s.nE - s.LE_atG : 0u;
+  for (uint32_t rel = lane; rel < hi - lo; rel += 32) {
+    uint16_t v;
+    if (rel < s.nL) {
+      v = m.tmp[lo + rel];
+    } else {
+      const bool eq = rel < s.nL + s.nE;
+      const uint16_t* tape = (eq ? m.tape_e : m.tape_g) + lo;
+      v = tape[eq ? RE + (rel - s.nL) : RG + (rel - s.nL - s.nE)];
+      while (!(v & kTerm16)) v = tape[v];  // each copy refers to an earlier entry
+    }
+    m.perm[lo + rel] = v & (kTerm16 - 1);
+  }
+  __syncwarp();
+  ps = lo + s.nL;
+  pe = ps + s.nE;
+}
+
+// One split of the boxes at positions [s, s + n) (FWNFS.h:5350-5800); box
+// `all` is the range's; the cut is [s, mid), [mid, s + n).  Every lane gets
+// the results.
+__device__ void warp_split(const SplitMem& m, SplitScratch& sc, uint32_t s, uint32_t n,
+                           const Box& all, uint32_t& mid, Box& o0, Box& o1, unsigned* status) {
+  const int lane = threadIdx.x & 31;
+  if (n == 2) {
+    o0 = mem_box(m, m.perm[s]);
+    o1 = mem_box(m, m.perm[s + 1]);
+    mid = s + 1;
+    return;
+  }
+  if (n <= 6) {  // every 2-partition with box 0 on side 0, one per lane
+    const uint32_t bits = lane + 1;
+    const bool valid = bits < (1u << (n - 1));
+    Box s0 = mem_box(m, m.perm[s]), s1;
+    box_empty(s1);
+    uint32_t c0 = 1, c1 = 0;
+    for (uint32_t b = 0; b + 1 < n; ++b) {
+      const Box x = mem_box(m, m.perm[s + b + 1]);
+      if ((bits >> b) & 1u) {
+        box_add(s1, x);
+        ++c1;
+      } else {
+        box_add(s0, x);
+        ++c0;
+      }
+    }
+    const float h = half_area(s0) * (float)c0 + half_area(s1) * (float)c1;
+    const int w = first_smallest(h, valid);
+    o0 = shfl_box(s0, w);
+    o1 = shfl_box(s1, w);
+    const uint32_t best = (uint32_t)w + 1, zeros = (n - 1) - __popc(best);
+    mid = s + 1 + zeros;
+    uint16_t e = 0;
+    uint32_t to = 0;
+    const bool move = lane >= 1 && (uint32_t)lane < n;
+    if (move) {
+      e = m.perm[s + lane];
+      const uint32_t below = (1u << (lane - 1)) - 1u;
+      to = ((best >> (lane - 1)) & 1u) ? 1 + zeros + __popc(best & below)
+                                       : 1 + __popc(~best & below);
+    }
+    __syncwarp();
+    if (move) m.perm[s + to] = e;
+    __syncwarp();
+    return;
+  }
+  float len;
+  const int axis = longest_axis(all, len);
+  if (!(len > 0.f)) {  // a single point or NaN: an arbitrary split
+    mid = s + n / 2;
+    o0 = all;
+    o1 = all;
+    return;
+  }
+  if (n <= kSmallMax) {
+    // stable sort by centre (the reference's chunked insertion sort + merges
+    // is a stable sort), one box per lane, then the sweep by scans
+    const bool in = (uint32_t)lane < n;
+    const uint16_t e = in ? m.perm[s + lane] : 0;
+    const float c = in ? mem_centre2(m, e, axis) : 0.f;
+    uint32_t rank = 0;
+    for (uint32_t j = 0; j < n; ++j) {
+      const float cj = __shfl_sync(kFull, c, j);
+      if (cj < c || (cj == c && j < (uint32_t)lane)) ++rank;
+    }
+    __syncwarp();
+    if (in) m.perm[s + rank] = e;
+    __syncwarp();
+    const uint32_t ns = n - 1;
+    Box b, r;
+    box_empty(b);
+    box_empty(r);
+    if (in) b = mem_box(m, m.perm[s + lane]);
+    const Box L = scan_box_up(b);
+    // right boxes as the reference accumulates them: starting from box ns-1,
+    // so the last box never enters (FWNFS.h:5560-5565)
+    if ((uint32_t)lane < ns) r = b;
+    Box R = scan_box_down(r);
+    Box R1;
+    for (int a = 0; a < 3; ++a) {
+      R1.lo[a] = __shfl_down_sync(kFull, R.lo[a], 1);
+      R1.hi[a] = __shfl_down_sync(kFull, R.hi[a], 1);
+    }
+    if ((uint32_t)lane + 1 < ns) R = R1;  // lane ns-1 keeps box ns-1
+    const float h = half_area(L) * (float)(lane + 1) + half_area(R) * (float)(n - (lane + 1));
+    const int w = first_smallest(h, (uint32_t)lane < ns);
+    mid = s + w + 1;
+    o0 = shfl_box(L, w);
+    o1 = shfl_box(R, w);
+    return;
+  }
+  // spans
+  for (int i = lane; i < kSpans; i += 32) {
+    sc.cnt[i] = 0;
+    keys_init(sc.keys[i]);
+  }
+  __syncwarp();
+  const float min2 = 2.0f * all.lo[axis];
+  const float scale = (0.5f * (float)kSpans) / len;
+  for (uint32_t p = s + lane; p < s + n; p += 32) {
+    const Box b = mem_box(m, m.perm[p]);
+    const int si = span_of(centre2(b, axis), min2, scale);
+    atomicAdd(&sc.cnt[si], 1u);
+    keys_add(sc.keys[si], b);
+  }
+  __syncwarp();
+  uint32_t lcs = 0, lc0, lc14, ps, pe;
+  const int si = choose_span(sc.cnt, sc.keys, n, o0, o1, lcs, lc0, lc14);
+  if (si >= 0) {
+    const float pivot = min2 + (float)(si + 1) * len / (float)(kSpans / 2);
+    warp_partition(m, axis, s, s + n, pivot, ps, pe);
+    mid = s + lcs;
+    if (mid >= ps && mid <= pe) return;
+    mid = mid < ps ? ps : pe;
+    if (mid == s) ++mid;
+    else if (mid == s + n) --mid;
+  } else {
+    // nthElement: each step narrows [lo, hi) by at least the pivot's own
+    // box; the bound only guards against a hang
+    mid = s + nth_target(n, lc0, lc14);
+    uint32_t lo = s, hi = s + n;
+    bool done = false;
+    for (uint32_t step = 0; step <= n && !done; ++step) {
+      const float pv = median3(mem_centre2(m, m.perm[lo], axis),
+                               mem_centre2(m, m.perm[lo + (hi - lo) / 2], axis),
+                               mem_centre2(m, m.perm[hi - 1], axis));
+      __syncwarp();
+      warp_partition(m, axis, lo, hi, pv, ps, pe);
+      if (mid < ps) hi = ps;
+      else if (mid < pe) done = true;
+      else lo = pe;
+      if (hi <= lo + 1) done = true;
+    }
+    if (!done && lane == 0) atomicOr(status, kStatusInternal);
+  }
+  // the cut moved off the span's, or came from nthElement: the sides' boxes
+  uint32_t k0[6], k1[6];
+  keys_init(k0);
+  keys_init(k1);
+  for (uint32_t p = s + lane; p < s + n; p += 32) {
+    const Box b = mem_box(m, m.perm[p]);
+    uint32_t* k = p < mid ? k0 : k1;
+    for (int a = 0; a < 3; ++a) {
+      k[a] = min(k[a], fkey(b.lo[a]));
+      k[3 + a] = max(k[3 + a], fkey(b.hi[a]));
+    }
+  }
+  for (int a = 0; a < 3; ++a) {
+    k0[a] = __reduce_min_sync(kFull, k0[a]);
+    k1[a] = __reduce_min_sync(kFull, k1[a]);
+    k0[3 + a] = __reduce_max_sync(kFull, k0[3 + a]);
+    k1[3 + a] = __reduce_max_sync(kFull, k1[3 + a]);
+  }
+  o0 = keys_box(k0);
+  o1 = keys_box(k1);
+}
+
+// The part a node splits in rounds 1 and 2: the largest area x count, the
+// first on ties.
+__device__ __forceinline__ int choose_part(const uint32_t* cut, const float* area, int nsub) {
+  int choice = -1;
+  float best = 0.f;
+  for (int i = 0; i < nsub; ++i) {
+    const uint32_t c = cut[i + 1] - cut[i];
+    if (c > 1) {
+      const float h = area[i] * (float)c;
+      if (choice < 0 || h > best) {
+        choice = i;
+        best = h;
+      }
+    }
+  }
+  return choice;
+}
+// Part c of nsub becomes two, cut at mid with boxes o0, o1.
+__device__ __forceinline__ void insert_cut(uint32_t* cut, Box* sub, float* area, int nsub, int c,
+                                           uint32_t mid, const Box& o0, const Box& o1) {
+  for (int i = nsub; i > c; --i) cut[i + 1] = cut[i];
+  for (int i = nsub - 1; i > c; --i) {
+    sub[i + 1] = sub[i];
+    area[i + 1] = area[i];
+  }
+  cut[c + 1] = mid;
+  sub[c] = o0;
+  sub[c + 1] = o1;
+  area[c] = half_area(o0);
+  area[c + 1] = half_area(o1);
+}
+
+// ------------------------------------------------------------- subtrees --
+// A subtree of at most kSub boxes: the boxes idx[start .. start + n).
+struct SubRoot {
+  uint32_t start, n, depth;
+  Box all;
+};
+// What the subtree kernel leaves per subtree node, at [start + local id]
+// (local ids breadth-first; a subtree of n boxes has at most n - 1 nodes):
+// the children (kSubNode | local id, local box index, kSubNone) and the
+// node's depth-first number, slot and first leaf slot relative to the
+// subtree's root, and the slots and items below it.
+struct SubNode {
+  uint16_t child[4];
+  uint16_t pre, slot, item, nslots, nitems, pad;
+};
+constexpr uint16_t kSubNode = 0x8000u, kSubNone = 0xffffu;
+struct SubTotals {
+  uint32_t nodes, slots, levels;
+};
+struct SubList {  // a node of the current depth with more than 4 boxes
+  uint16_t s, n, id, pad;
+  Box all;
+};
+constexpr int kSubWarps = 8;
+constexpr int kSubListCap = kSub / 5 + 1;
+struct SubShared {
+  union {
+    float bx[6][kSub];
+    struct {
+      uint16_t nodes[kSub], slots[kSub], items[kSub], pre[kSub], slot[kSub], item[kSub];
+    } z;
+  };
+  uint16_t perm[kSub], tmp[kSub], tape_e[kSub], tape_g[kSub];
+  uint16_t child[kSub][4];
+  uint16_t lev[kSub + 2];  // depth d: local ids [lev[d], lev[d + 1])
+  SplitScratch sc[kSubWarps];
+  SubList list[2][kSubListCap];
+  uint32_t nodes, take, next;
+};
+
+// Builds the whole subtree below each root in shared memory, one CTA per
+// subtree: depth by depth, a warp per node, the node's three splits one after
+// the other (multiSplit).  In place of one launch per depth, round and size
+// class with host reads between them (82k triangles: 400 launches and 80
+// blocking reads, 5.7 ms).
+__global__ void __launch_bounds__(kSubWarps * 32) subtree_kernel(
+    const SubRoot* __restrict__ roots, uint32_t nroots, const uint32_t* __restrict__ idx,
+    const Box* __restrict__ tb, SubNode* __restrict__ out,
+    uint16_t* __restrict__ lev_out, SubTotals* __restrict__ totals, unsigned* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  SubShared& S = *reinterpret_cast<SubShared*>(s_raw);
+  if (blockIdx.x >= nroots) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const SubRoot root = roots[blockIdx.x];
+  for (uint32_t i = tid; i < root.n; i += blockDim.x) {
+    const Box b = tb[idx[root.start + i]];
+    for (int a = 0; a < 3; ++a) {
+      S.bx[a][i] = b.lo[a];
+      S.bx[3 + a][i] = b.hi[a];
+    }
+    S.perm[i] = (uint16_t)i;
+  }
+  if (tid == 0) {
+    S.nodes = 1;
+    S.lev[0] = 0;
+    S.lev[1] = 1;
+    if (root.n <= 4) {
+      for (uint32_t i = 0; i < 4; ++i) S.child[0][i] = i < root.n ? (uint16_t)i : kSubNone;
+    } else {
+      S.list[0][0] = SubList{0, (uint16_t)root.n, 0, 0, root.all};
+    }
+  }
+  const SplitMem mem{&S.bx[0][0], (int)kSub, S.perm, S.tmp, S.tape_e, S.tape_g};
+  SplitScratch& sc = S.sc[warp];
+  uint32_t ncur = root.n <= 4 ? 0 : 1;
+  uint32_t depths = 1;
+  int cur = 0;
+  while (ncur > 0) {
+    if (tid == 0) S.take = S.next = 0;
+    __syncthreads();
+    for (;;) {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(&S.take, 1u);
+      k = __shfl_sync(kFull, k, 0);
+      if (k >= ncur) break;
+      const SubList N = S.list[cur][k];
+      if (lane == 0) {
+        sc.cut[0] = N.s;
+        sc.cut[1] = (uint32_t)N.s + N.n;
+      }
+      __syncwarp();
+      for (int round = 0; round < 3; ++round) {
+        const int c = round == 0 ? 0 : choose_part(sc.cut, sc.area, round + 1);
+        const uint32_t s = sc.cut[c], n = sc.cut[c + 1] - s;
+        const Box all = round == 0 ? N.all : sc.sub[c];
+        uint32_t mid;
+        Box o0, o1;
+        warp_split(mem, sc, s, n, all, mid, o0, o1, status);
+        __syncwarp();
+        if (lane == 0) insert_cut(sc.cut, sc.sub, sc.area, round + 1, c, mid, o0, o1);
+        __syncwarp();
+      }
+      // children: lane i takes part i
+      const uint32_t s = lane < 4 ? sc.cut[lane] : 0, n = lane < 4 ? sc.cut[lane + 1] - s : 1;
+      const unsigned inner = __ballot_sync(kFull, n > 1);
+      uint32_t id = 0;
+      if (lane == 0) id = atomicAdd(&S.nodes, (uint32_t)__popc(inner));
+      id = __shfl_sync(kFull, id, 0) + __popc(inner & ((1u << lane) - 1u));
+      if (lane < 4) {
+        S.child[N.id][lane] = n > 1 ? (uint16_t)(kSubNode | id) : S.perm[s];
+        if (n > 4) {
+          S.list[cur ^ 1][atomicAdd(&S.next, 1u)] =
+              SubList{(uint16_t)s, (uint16_t)n, (uint16_t)id, 0, sc.sub[lane]};
+        } else if (n > 1) {
+          for (uint32_t i = 0; i < 4; ++i) S.child[id][i] = i < n ? S.perm[s + i] : kSubNone;
+        }
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    ncur = S.next;
+    cur ^= 1;
+    const uint32_t made = S.nodes;
+    if (made > S.lev[depths]) ++depths;
+    __syncthreads();
+    if (tid == 0) S.lev[depths] = (uint16_t)made;
+    __syncthreads();
+  }
+  __syncthreads();  // the boxes' memory is reused from here
+  for (uint32_t d = depths; d-- > 0;) {
+    for (uint32_t x = S.lev[d] + tid; x < S.lev[d + 1]; x += blockDim.x) {
+      uint32_t nodes = 1, slots = 1, items = 0;
+      for (int i = 0; i < 4; ++i) {
+        const uint16_t c = S.child[x][i];
+        if (c == kSubNone) continue;
+        if (c & kSubNode) {
+          nodes += S.z.nodes[c & ~kSubNode];
+          slots += S.z.slots[c & ~kSubNode];
+          items += S.z.items[c & ~kSubNode];
+        } else {
+          ++slots;
+          ++items;
+        }
+      }
+      S.z.nodes[x] = (uint16_t)nodes;
+      S.z.slots[x] = (uint16_t)slots;
+      S.z.items[x] = (uint16_t)items;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    S.z.pre[0] = S.z.slot[0] = S.z.item[0] = 0;
+    totals[blockIdx.x] = SubTotals{S.nodes, S.z.slots[0], depths};
+  }
+  __syncthreads();
+  for (uint32_t d = 0; d < depths; ++d) {
+    for (uint32_t x = S.lev[d] + tid; x < S.lev[d + 1]; x += blockDim.x) {
+      uint32_t pre = S.z.pre[x] + 1, slot = S.z.slot[x] + 1, item = S.z.item[x];
+      SubNode o;
+      o.pre = S.z.pre[x];
+      o.slot = S.z.slot[x];
+      o.item = S.z.item[x];
+      o.nslots = S.z.slots[x];
+      o.nitems = S.z.items[x];
+      o.pad = 0;
+      for (int i = 0; i < 4; ++i) {
+        const uint16_t c = S.child[x][i];
+        o.child[i] = c;
+        if (c == kSubNone) continue;
+        if (c & kSubNode) {
+          const uint32_t y = c & ~kSubNode;
+          S.z.pre[y] = (uint16_t)pre;
+          S.z.slot[y] = (uint16_t)slot;
+          S.z.item[y] = (uint16_t)item;
+          pre += S.z.nodes[y];
+          slot += S.z.slots[y];
+          item += S.z.items[y];
+        } else {
+          ++slot;
+          ++item;
+        }
+      }
+      out[root.start + x] = o;
+    }
+    __syncthreads();
+  }
+  for (uint32_t d = tid; d <= depths; d += blockDim.x) lev_out[root.start + d] = S.lev[d];
+}
+// ------------------------------------------------------- the top of the tree --
+// Nodes of more than kSub boxes, one depth at a time.  Their splits run by
+// size: up to kSub boxes in a warp, up to kCtaMax in a CTA, more across the
+// GPU; every kernel reads its task count on the device, so a depth ends with
+// one host read.
+__global__ void __launch_bounds__(32) part_warp_kernel(RNode* __restrict__ nodes,
+                                                       const uint32_t* __restrict__ list,
+                                                       const uint32_t* __restrict__ count,
+                                                       uint32_t* __restrict__ idx,
+                                                       const Box* __restrict__ tb,
+                                                       unsigned* __restrict__ status) {
+  __shared__ float bx[6][kSub];
+  __shared__ uint32_t id[kSub];
+  __shared__ uint16_t perm[kSub], tmp[kSub], tape_e[kSub], tape_g[kSub];
+  __shared__ SplitScratch sc;
+  if (blockIdx.x >= *count) return;
+  const int lane = threadIdx.x;
+  RNode& N = nodes[list[blockIdx.x]];
+  const uint32_t s = N.t_start, n = N.t_n;
+  for (uint32_t i = lane; i < n; i += 32) {
+    id[i] = idx[s + i];
+    const Box b = tb[id[i]];
+    for (int a = 0; a < 3; ++a) {
+      bx[a][i] = b.lo[a];
+      bx[3 + a][i] = b.hi[a];
+    }
+    perm[i] = (uint16_t)i;
+  }
+  __syncwarp();
+  const SplitMem mem{&bx[0][0], (int)kSub, perm, tmp, tape_e, tape_g};
+  const Box all = N.t_box;
+  uint32_t mid;
+  Box o0, o1;
+  warp_split(mem, sc, 0, n, all, mid, o0, o1, status);
+  __syncwarp();
+  for (uint32_t i = lane; i < n; i += 32) idx[s + i] = id[perm[i]];
+  if (lane == 0) {
+    N.t_mid = s + mid;
+    N.t_out[0] = o0;
+    N.t_out[1] = o1;
+  }
+}
+
+// partitionByCentre of positions [lo, hi) by one CTA of 32 warps, centres in
+// cen: each warp counts its segment, the segments' prefixes give every warp
+// its tape state, then the tapes are written and resolved.
+struct CtaPart {
+  uint32_t nL[32], nE[32], fE[32], fG[32], L_atE[32], LE_atG[32];
+};
+__device__ void cta_partition(CtaPart& S, uint32_t* idx, float* cen, uint32_t* tmp,
+                              uint32_t* tape_e, uint32_t* tape_g, uint32_t lo, uint32_t hi,
+                              float pivot, uint32_t& ps, uint32_t& pe) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t jn = hi - lo, seg = (jn + 1023) / 1024 * 32;
+  const uint32_t wlo = min(hi, lo + warp * seg), whi = min(hi, wlo + seg);
+  auto cls = [&](uint32_t p) {
+    if (p >= whi) return 3;
+    const float c = cen[p];
+    return c < pivot ? 0 : (c == pivot ? 1 : 2);
+  };
+  TapeState w;
+  for (uint32_t base = wlo; base < whi; base += 32) tape_step(w, cls(base + lane), base - lo);
+  if (lane == 0) {
+    S.nL[warp] = w.nL;
+    S.nE[warp] = w.nE;
+    S.fE[warp] = w.firstE;
+    S.fG[warp] = w.firstG;
+    S.L_atE[warp] = w.L_atE;
+    S.LE_atG[warp] = w.LE_atG;
+  }
+  __syncthreads();
+  // lane i holds warp i's counts; exclusive prefixes
+  uint32_t aL = S.nL[lane], aE = S.nE[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t tL = __shfl_up_sync(kFull, aL, o), tE = __shfl_up_sync(kFull, aE, o);
+    if (lane >= o) {
+      aL += tL;
+      aE += tE;
+    }
+  }
+  const uint32_t nL = __shfl_sync(kFull, aL, 31), nE = __shfl_sync(kFull, aE, 31);
+  aL -= S.nL[lane];
+  aE -= S.nE[lane];
+  const unsigned hasE = __ballot_sync(kFull, S.fE[lane] != kNone),
+                 hasG = __ballot_sync(kFull, S.fG[lane] != kNone);
+  TapeState t;
+  t.nL = __shfl_sync(kFull, aL, warp);
+  t.nE = __shfl_sync(kFull, aE, warp);
+  if (hasE) {
+    const int f = __ffs(hasE) - 1;
+    t.firstE = S.fE[f];
+    t.L_atE = S.L_atE[f] + __shfl_sync(kFull, aL, f);
+  }
+  if (hasG) {
+    const int f = __ffs(hasG) - 1;
+    t.firstG = S.fG[f];
+    t.LE_atG = S.LE_atG[f] + __shfl_sync(kFull, aL + aE, f);
+  }
+  for (uint32_t base = wlo; base < whi; base += 32) {
+    const uint32_t p = base + lane;
+    const int k = cls(p);
+    const uint32_t e = p < whi ? idx[p] : 0;
+    const TapeOps o = tape_step(t, k, base - lo);
+    if (k == 0) {
+      tmp[lo + o.L] = e;
+      if (o.afterE) tape_e[lo + o.te] = o.rotE;
+      if (o.afterG) tape_g[lo + o.tg] = o.rotG;
+    } else if (k == 1) {
+      tape_e[lo + o.te] = kTerm | e;
+      if (o.afterG) tape_g[lo + o.tg] = o.rotG;
+    } else if (k == 2) {
+      tape_g[lo + o.tg] = kTerm | e;
+    }
+  }
+  __syncthreads();
+  const uint32_t RE = t.firstE != kNone ? nL - t.L_atE : 0u;
+  const uint32_t RG = t.firstG != kNone ? nL + nE - t.LE_atG : 0u;
+  for (uint32_t rel = threadIdx.x; rel < jn; rel += blockDim.x) {
+    uint32_t v;
+    if (rel < nL) {
+      v = tmp[lo + rel];
+    } else {
+      const bool eq = rel < nL + nE;
+      const uint32_t* tape = (eq ? tape_e : tape_g) + lo;
+      v = tape[eq ? RE + (rel - nL) : RG + (rel - nL - nE)];
+      while (!(v & kTerm)) v = tape[v];  // each copy refers to an earlier entry
+    }
+    idx[lo + rel] = v & ~kTerm;
+  }
+  __syncthreads();
+  ps = lo + nL;
+  pe = ps + nE;
+}
+
+__global__ void __launch_bounds__(1024) part_cta_kernel(
+    RNode* nodes, const uint32_t* list, const uint32_t* count, uint32_t* idx, float* cen,
+    uint32_t* tmp, uint32_t* tape_e, uint32_t* tape_g, const Box* __restrict__ tb,
+    unsigned* status) {
+  __shared__ uint32_t s_cnt[32][kSpans];
+  __shared__ uint32_t s_keys[32][kSpans][6];
+  __shared__ CtaPart s_part;
+  __shared__ Box s_L, s_R;
+  __shared__ int s_si;
+  __shared__ uint32_t s_lcs, s_target, s_bk[2][6];
+  if (blockIdx.x >= *count) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   RNode& N = nodes[list[blockIdx.x]];
   const uint32_t s = N.t_start, n = N.t_n;
   const Box B = N.t_box;
   float len;
   const int axis = longest_axis(B, len);
   if (!(len > 0.f)) {
+    __syncthreads();
     if (tid == 0) {
       N.t_mid = s + n / 2;
       N.t_out[0] = B;
@@ -527,289 +1014,384 @@ __global__ void __launch_bounds__(256) split_medium_kernel(RNode* __restrict__ n
     }
     return;
   }
-  if (tid < kSpans) {
-    s_cnt[tid] = 0;
-    keys_init(s_keys[tid]);
+  for (int i = lane; i < kSpans; i += 32) {
+    s_cnt[warp][i] = 0;
+    keys_init(s_keys[warp][i]);
   }
   if (tid < 2) keys_init(s_bk[tid]);
-  __syncthreads();
+  __syncwarp();
   const float min2 = 2.0f * B.lo[axis];
   const float scale = (0.5f * (float)kSpans) / len;
-  for (uint32_t i = tid; i < n; i += blockDim.x) {
-    const uint32_t e = idx[s + i];
-    const Box b = tb[e];
+  for (uint32_t p = s + tid; p < s + n; p += blockDim.x) {
+    const Box b = tb[idx[p]];
     const float c = centre2(b, axis);
-    s_id[i] = e;
-    s_c[i] = c;
+    cen[p] = c;
     const int si = span_of(c, min2, scale);
-    atomicAdd(&s_cnt[si], 1u);
-    keys_add(s_keys[si], b);
+    atomicAdd(&s_cnt[warp][si], 1u);
+    keys_add(s_keys[warp][si], b);
+  }
+  __syncthreads();
+  if (tid < kSpans * 7) {  // the warps' tables into the first
+    const int i = tid / 7, f = tid % 7;
+    if (f == 6) {
+      uint32_t v = 0;
+      for (int w = 0; w < 32; ++w) v += s_cnt[w][i];
+      s_cnt[0][i] = v;
+    } else {
+      uint32_t v = s_keys[0][i][f];
+      for (int w = 1; w < 32; ++w) v = f < 3 ? min(v, s_keys[w][i][f]) : max(v, s_keys[w][i][f]);
+      s_keys[0][i][f] = v;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t lcs = 0, lc0, lc14;
+    Box Lb = B, Rb = B;
+    const int si = choose_span(s_cnt[0], s_keys[0], n, Lb, Rb, lcs, lc0, lc14);
+    if (lane == 0) {
+      s_si = si;
+      s_lcs = lcs;
+      s_target = nth_target(n, lc0, lc14);
+      s_L = Lb;
+      s_R = Rb;
+    }
+  }
+  __syncthreads();
+  uint32_t mid, ps, pe;
+  if (s_si >= 0) {
+    const float pivot = min2 + (float)(s_si + 1) * len / (float)(kSpans / 2);
+    cta_partition(s_part, idx, cen, tmp, tape_e, tape_g, s, s + n, pivot, ps, pe);
+    mid = s + s_lcs;
+    if (mid >= ps && mid <= pe) {
+      if (tid == 0) {
+        N.t_mid = mid;
+        N.t_out[0] = s_L;
+        N.t_out[1] = s_R;
+      }
+      return;
+    }
+    mid = mid < ps ? ps : pe;
+    if (mid == s) ++mid;
+    else if (mid == s + n) --mid;
+  } else {
+    // nthElement, as in warp_split
+    mid = s + s_target;
+    uint32_t lo = s, hi = s + n;
+    bool done = false;
+    for (uint32_t step = 0; step <= n && !done; ++step) {
+      const float pv = median3(cen[lo], cen[lo + (hi - lo) / 2], cen[hi - 1]);
+      __syncthreads();
+      cta_partition(s_part, idx, cen, tmp, tape_e, tape_g, lo, hi, pv, ps, pe);
+      for (uint32_t p = lo + tid; p < hi; p += blockDim.x) cen[p] = centre2(tb[idx[p]], axis);
+      if (mid < ps) hi = ps;
+      else if (mid < pe) done = true;
+      else lo = pe;
+      if (hi <= lo + 1) done = true;
+      __syncthreads();
+    }
+    if (!done && tid == 0) atomicOr(status, kStatusInternal);
+  }
+  // the cut moved off the span's, or came from nthElement: the sides' boxes
+  for (uint32_t p0 = s; p0 < s + n; p0 += blockDim.x) {
+    const uint32_t p = p0 + tid;
+    const bool in = p < s + n;
+    const Box b = in ? tb[idx[p]] : B;
+    for (int side = 0; side < 2; ++side) {
+      const bool mine = in && (p < mid) == (side == 0);
+      for (int a = 0; a < 3; ++a) {
+        const uint32_t l = __reduce_min_sync(kFull, mine ? fkey(b.lo[a]) : 0xffffffffu);
+        const uint32_t h = __reduce_max_sync(kFull, mine ? fkey(b.hi[a]) : 0u);
+        if (lane == 0) {
+          atomicMin(&s_bk[side][a], l);
+          atomicMax(&s_bk[side][3 + a], h);
+        }
+      }
+    }
   }
   __syncthreads();
   if (tid == 0) {
-    Box Lb, Rb;
-    uint32_t lcs = 0, lc0, lc14;
-    const int si = choose_span(s_cnt, s_keys, n, Lb, Rb, lcs, lc0, lc14);
-    uint32_t mid;
-    int need = 1;
-    if (si < 0) {
-      mid = nth_target(n, lc0, lc14);
-      if (!nth_seq(s_id, s_c, 0, n, mid)) atomicOr(status, kStatusInternal);
-    } else {
-      const float pivot = min2 + (float)(si + 1) * len / (float)(kSpans / 2);
-      uint32_t ps, pe;
-      partition_seq(s_id, s_c, 0, n, pivot, ps, pe);
-      mid = lcs;
-      if (mid >= ps && mid <= pe) {
-        need = 0;
-        N.t_out[0] = Lb;
-        N.t_out[1] = Rb;
-      } else {
-        mid = mid < ps ? ps : pe;
-        if (mid == 0) ++mid;
-        else if (mid == n) --mid;
-      }
-    }
-    s_mid = mid;
-    s_need = need;
+    N.t_mid = mid;
+    N.t_out[0] = keys_box(s_bk[0]);
+    N.t_out[1] = keys_box(s_bk[1]);
   }
-  __syncthreads();
-  const uint32_t mid = s_mid;
-  if (s_need) {
-    for (uint32_t i = tid; i < n; i += blockDim.x) keys_add(s_bk[i < mid ? 0 : 1], tb[s_id[i]]);
-    __syncthreads();
-    if (tid == 0) {
-      N.t_out[0] = keys_box(s_bk[0]);
-      N.t_out[1] = keys_box(s_bk[1]);
-    }
-  }
-  for (uint32_t i = tid; i < n; i += blockDim.x) idx[s + i] = s_id[i];
-  if (tid == 0) N.t_mid = s + mid;
 }
 
-// ----------------------------------------------- split: > 1024 boxes --
-enum LMode : int32_t { kLDone = 0, kLSpan = 1, kLNth = 2 };
-
+// ---------------------------------------------- splits across the GPU --
 struct LTask {
-  uint32_t node;
-  uint32_t start, n;
+  uint32_t node, start, n;
   int32_t axis;
-  float len, min2, scale;
+  float len, min2, scale, pivot;
   uint32_t cnt[kSpans];
   uint32_t keys[kSpans][6];
   Box Lb, Rb;
   uint32_t lcs;
-  // the partition job in progress: positions [jlo, jlo + jn) around pivot
-  int32_t mode;
-  uint32_t jlo, jn, nth;
-  float pivot;
-  uint32_t firstE, firstG;    // job-relative, kNone if absent
-  uint32_t nL, nE;            // job totals
-  uint32_t nL_atE, nLE_atG;   // prefix counts at firstE / firstG
+  int32_t live;                        // a span split (else left to the CTA kernel)
+  uint32_t chunk0;                     // its first chunk
+  uint32_t firstE, firstG, nL, nE;     // of the partition, relative to start
+  uint32_t L_atE, LE_atG;              // prefix counts at firstE / firstG
   uint32_t mid;
-  int32_t need;               // sub boxes must be recomputed
+  int32_t need;                        // the sides' boxes must be recomputed
   uint32_t bk[2][6];
 };
 
-// 32-bit chunk: CTA b of a GPU-wide pass works on positions
-// [chunk[b].y, chunk[b].z) of large task chunk[b].x.
-
-__global__ void large_init_kernel(RNode* __restrict__ nodes, const uint32_t* __restrict__ list,
-                                  uint32_t count, LTask* __restrict__ T) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  LTask& t = T[k];
-  const uint32_t x = list[k];
-  RNode& N = nodes[x];
-  t.node = x;
-  t.start = N.t_start;
-  t.n = N.t_n;
-  float len;
-  t.axis = longest_axis(N.t_box, len);
-  t.len = len;
-  t.min2 = 2.0f * N.t_box.lo[t.axis];
-  t.scale = (0.5f * (float)kSpans) / len;
-  for (int i = 0; i < kSpans; ++i) {
-    t.cnt[i] = 0;
-    keys_init(t.keys[i]);
+// Tasks of the list and their chunks of kChunk positions; one CTA.  A task
+// with no longest axis goes to the CTA kernel's list.
+__global__ void wide_init_kernel(const RNode* __restrict__ nodes,
+                                 const uint32_t* __restrict__ list,
+                                 const uint32_t* __restrict__ count, LTask* __restrict__ T,
+                                 int4* __restrict__ chunks, uint32_t* __restrict__ nchunks) {
+  __shared__ uint32_t s_total;
+  const uint32_t n = *count;
+  if (threadIdx.x == 0) s_total = 0;
+  for (uint32_t k0 = 0; k0 < n; k0 += 32) {  // warp 0: tasks and chunk offsets
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const uint32_t k = k0 + threadIdx.x;
+      uint32_t c = 0;
+      if (k < n) {
+        LTask& t = T[k];
+        const RNode& N = nodes[list[k]];
+        t.node = list[k];
+        t.start = N.t_start;
+        t.n = N.t_n;
+        t.axis = longest_axis(N.t_box, t.len);
+        t.min2 = 2.0f * N.t_box.lo[t.axis];
+        t.scale = (0.5f * (float)kSpans) / t.len;
+        for (int i = 0; i < kSpans; ++i) {
+          t.cnt[i] = 0;
+          keys_init(t.keys[i]);
+        }
+        keys_init(t.bk[0]);
+        keys_init(t.bk[1]);
+        t.live = t.len > 0.f;
+        t.firstE = t.firstG = kNone;
+        t.nL = t.nE = t.L_atE = t.LE_atG = 0;
+        t.need = 0;
+        c = (t.n + kChunk - 1) / kChunk;
+      }
+      uint32_t incl = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if ((int)threadIdx.x >= o) incl += v;
+      }
+      if (k < n) T[k].chunk0 = s_total + incl - c;
+      __syncwarp();
+      if (threadIdx.x == 31) s_total += incl;
+    }
   }
-  keys_init(t.bk[0]);
-  keys_init(t.bk[1]);
-  t.need = 0;
-  if (!(len > 0.f)) {
-    t.mode = kLDone;
-    t.mid = t.start + t.n / 2;
-    N.t_out[0] = N.t_box;
-    N.t_out[1] = N.t_box;
-  } else {
-    t.mode = kLSpan;
+  __syncthreads();
+  if (threadIdx.x == 0) *nchunks = s_total;
+  for (uint32_t k = 0; k < n; ++k) {
+    const uint32_t s = T[k].start, len = T[k].n, c0 = T[k].chunk0;
+    for (uint32_t c = threadIdx.x; c * kChunk < len; c += blockDim.x)
+      chunks[c0 + c] = make_int4((int)k, (int)(s + c * kChunk),
+                                 (int)(s + min(len, (c + 1) * kChunk)), 0);
   }
 }
 
-__global__ void __launch_bounds__(256) large_span_kernel(const int4* __restrict__ chunks,
-                                                         LTask* __restrict__ T,
-                                                         const uint32_t* __restrict__ idx,
-                                                         const Box* __restrict__ tb) {
-  __shared__ uint32_t s_cnt[kSpans];
-  __shared__ uint32_t s_keys[kSpans][6];
+__global__ void __launch_bounds__(256) wide_span_kernel(const int4* __restrict__ chunks,
+                                                        const uint32_t* __restrict__ nchunks,
+                                                        LTask* __restrict__ T,
+                                                        const uint32_t* __restrict__ idx,
+                                                        const Box* __restrict__ tb,
+                                                        float* __restrict__ cen) {
+  __shared__ uint32_t s_cnt[8][kSpans];
+  __shared__ uint32_t s_keys[8][kSpans][6];
+  if (blockIdx.x >= *nchunks) return;
   const int4 ch = chunks[blockIdx.x];
   LTask& t = T[ch.x];
-  const int tid = threadIdx.x;
-  if (tid < kSpans) {
-    s_cnt[tid] = 0;
-    keys_init(s_keys[tid]);
+  if (!t.live) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = lane; i < kSpans; i += 32) {
+    s_cnt[warp][i] = 0;
+    keys_init(s_keys[warp][i]);
   }
-  __syncthreads();
+  __syncwarp();
   const int axis = t.axis;
   const float min2 = t.min2, scale = t.scale;
   for (int p = ch.y + tid; p < ch.z; p += blockDim.x) {
     const Box b = tb[idx[p]];
-    const int si = span_of(centre2(b, axis), min2, scale);
-    atomicAdd(&s_cnt[si], 1u);
-    keys_add(s_keys[si], b);
+    const float c = centre2(b, axis);
+    cen[p] = c;
+    const int si = span_of(c, min2, scale);
+    atomicAdd(&s_cnt[warp][si], 1u);
+    keys_add(s_keys[warp][si], b);
   }
   __syncthreads();
-  if (tid < kSpans && s_cnt[tid]) {
-    atomicAdd(&t.cnt[tid], s_cnt[tid]);
-    for (int a = 0; a < 3; ++a) {
-      atomicMin(&t.keys[tid][a], s_keys[tid][a]);
-      atomicMax(&t.keys[tid][3 + a], s_keys[tid][3 + a]);
+  if (tid < kSpans * 7) {
+    const int i = tid / 7, f = tid % 7;
+    uint32_t total = 0;
+    for (int w = 0; w < 8; ++w) total += s_cnt[w][i];
+    if (total) {
+      if (f == 6) {
+        atomicAdd(&t.cnt[i], total);
+      } else {
+        uint32_t v = s_keys[0][i][f];
+        for (int w = 1; w < 8; ++w) v = f < 3 ? min(v, s_keys[w][i][f]) : max(v, s_keys[w][i][f]);
+        if (f < 3) atomicMin(&t.keys[i][f], v);
+        else atomicMax(&t.keys[i][f], v);
+      }
     }
   }
 }
 
-__device__ __forceinline__ float centre_at(const uint32_t* idx, const Box* tb, uint32_t p,
-                                           int axis) {
-  return centre2(tb[idx[p]], axis);
-}
-
-__global__ void large_choose_kernel(LTask* __restrict__ T, uint32_t count,
-                                    const uint32_t* __restrict__ idx, const Box* __restrict__ tb) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  LTask& t = T[k];
-  if (t.mode != kLSpan) return;
-  uint32_t lc0, lc14;
-  const int si = choose_span(t.cnt, t.keys, t.n, t.Lb, t.Rb, t.lcs, lc0, lc14);
-  t.jlo = t.start;
-  t.jn = t.n;
+// One warp per task: the span and pivot; without one, the CTA kernel's list.
+__global__ void wide_choose_kernel(LTask* __restrict__ T, const uint32_t* __restrict__ count,
+                                   uint32_t* __restrict__ cta_list,
+                                   uint32_t* __restrict__ cta_count) {
+  if (blockIdx.x >= *count) return;
+  LTask& t = T[blockIdx.x];
+  const int lane = threadIdx.x;
+  int si = -1;
+  uint32_t lcs = 0, lc0, lc14;
+  Box Lb, Rb;
+  if (t.live) si = choose_span(t.cnt, t.keys, t.n, Lb, Rb, lcs, lc0, lc14);
+  __syncwarp();
+  if (lane != 0) return;
   if (si < 0) {
-    t.mode = kLNth;
-    t.nth = t.start + nth_target(t.n, lc0, lc14);
-    t.pivot = median3(centre_at(idx, tb, t.start, t.axis),
-                      centre_at(idx, tb, t.start + t.n / 2, t.axis),
-                      centre_at(idx, tb, t.start + t.n - 1, t.axis));
-  } else {
-    t.pivot = t.min2 + (float)(si + 1) * t.len / (float)(kSpans / 2);
+    t.live = 0;
+    cta_list[atomicAdd(cta_count, 1u)] = t.node;
+    return;
   }
+  t.Lb = Lb;
+  t.Rb = Rb;
+  t.lcs = lcs;
+  t.pivot = t.min2 + (float)(si + 1) * t.len / (float)(kSpans / 2);
 }
 
-__global__ void part_init_kernel(LTask* __restrict__ T, uint32_t count) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  T[k].firstE = kNone;
-  T[k].firstG = kNone;
-}
-
-// Pass 1: class of every position (0 below, 1 equal, 2 above the pivot),
-// counts per chunk, first equal / first above per job.
-__global__ void __launch_bounds__(256) part_classify_kernel(const int4* __restrict__ chunks,
+// Pass 1: counts of the classes (below, equal, above) per chunk, first equal
+// and first upper box per task.
+__global__ void __launch_bounds__(256) wide_classify_kernel(const int4* __restrict__ chunks,
+                                                            const uint32_t* __restrict__ nchunks,
                                                             LTask* __restrict__ T,
-                                                            const uint32_t* __restrict__ idx,
-                                                            const Box* __restrict__ tb,
-                                                            uint8_t* __restrict__ cls,
-                                                            uint32_t* __restrict__ chunk_cnt) {
-  __shared__ uint32_t s_n[3];
+                                                            const float* __restrict__ cen,
+                                                            uint2* __restrict__ chunk_cnt) {
+  __shared__ uint32_t s_n[2], s_f[2];
+  if (blockIdx.x >= *nchunks) return;
   const int4 ch = chunks[blockIdx.x];
   LTask& t = T[ch.x];
-  const int tid = threadIdx.x;
-  if (tid < 3) s_n[tid] = 0;
+  if (!t.live) return;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < 2) {
+    s_n[tid] = 0;
+    s_f[tid] = kNone;
+  }
   __syncthreads();
-  uint32_t n0 = 0, n1 = 0, n2 = 0, fE = kNone, fG = kNone;
+  const float pivot = t.pivot;
+  uint32_t n0 = 0, n1 = 0, fE = kNone, fG = kNone;
   for (int p = ch.y + tid; p < ch.z; p += blockDim.x) {
-    const float c = centre2(tb[idx[p]], t.axis);
-    const uint8_t k = c < t.pivot ? 0 : (c == t.pivot ? 1 : 2);
-    cls[p] = k;
-    const uint32_t rel = (uint32_t)p - t.jlo;
-    if (k == 0) ++n0;
-    else if (k == 1) {
+    const float c = cen[p];
+    const uint32_t rel = (uint32_t)p - t.start;
+    if (c < pivot) {
+      ++n0;
+    } else if (c == pivot) {
       ++n1;
       fE = min(fE, rel);
     } else {
-      ++n2;
       fG = min(fG, rel);
     }
   }
-  atomicAdd(&s_n[0], n0);
-  atomicAdd(&s_n[1], n1);
-  atomicAdd(&s_n[2], n2);
-  if (fE != kNone) atomicMin(&t.firstE, fE);
-  if (fG != kNone) atomicMin(&t.firstG, fG);
-  __syncthreads();
-  if (tid < 3) chunk_cnt[blockIdx.x * 3 + tid] = s_n[tid];
-}
-
-// Pass 2: per job, the counts before each of its chunks (its chunks are
-// consecutive in the chunk list: jc = (first, count)).
-__global__ void part_chunk_scan_kernel(LTask* __restrict__ T, uint32_t count,
-                                       const int2* __restrict__ jc,
-                                       const uint32_t* __restrict__ chunk_cnt,
-                                       uint32_t* __restrict__ chunk_base) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count || jc[k].y == 0) return;
-  uint32_t a = 0, b = 0, c = 0;
-  for (int i = jc[k].x; i < jc[k].x + jc[k].y; ++i) {
-    chunk_base[i * 3 + 0] = a;
-    chunk_base[i * 3 + 1] = b;
-    chunk_base[i * 3 + 2] = c;
-    a += chunk_cnt[i * 3 + 0];
-    b += chunk_cnt[i * 3 + 1];
-    c += chunk_cnt[i * 3 + 2];
+  n0 = __reduce_add_sync(kFull, n0);
+  n1 = __reduce_add_sync(kFull, n1);
+  fE = __reduce_min_sync(kFull, fE);
+  fG = __reduce_min_sync(kFull, fG);
+  if (lane == 0) {
+    atomicAdd(&s_n[0], n0);
+    atomicAdd(&s_n[1], n1);
+    atomicMin(&s_f[0], fE);
+    atomicMin(&s_f[1], fG);
   }
-  T[k].nL = a;
-  T[k].nE = b;
+  __syncthreads();
+  if (tid == 0) {
+    chunk_cnt[blockIdx.x] = make_uint2(s_n[0], s_n[1]);
+    if (s_f[0] != kNone) atomicMin(&t.firstE, s_f[0]);
+    if (s_f[1] != kNone) atomicMin(&t.firstG, s_f[1]);
+  }
 }
 
-// Pass 3: prefix counts of "below" and "equal" at every position.  Thread t
-// of the CTA owns positions 4t .. 4t+3 of the chunk.
-__global__ void __launch_bounds__(256) part_prefix_kernel(const int4* __restrict__ chunks,
-                                                          LTask* __restrict__ T,
-                                                          const uint8_t* __restrict__ cls,
-                                                          const uint32_t* __restrict__ chunk_base,
-                                                          uint32_t* __restrict__ preL,
-                                                          uint32_t* __restrict__ preE) {
+// Pass 2: one warp per task turns its chunks' counts into the counts before
+// each chunk.
+__global__ void wide_scan_kernel(LTask* __restrict__ T, const uint32_t* __restrict__ count,
+                                 uint2* __restrict__ chunk_cnt) {
+  if (blockIdx.x >= *count) return;
+  LTask& t = T[blockIdx.x];
+  if (!t.live) return;
+  const int lane = threadIdx.x;
+  const uint32_t nc = (t.n + kChunk - 1) / kChunk;
+  uint32_t baseL = 0, baseE = 0;
+  for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
+    const bool in = c0 + lane < nc;
+    const uint2 v = in ? chunk_cnt[t.chunk0 + c0 + lane] : make_uint2(0, 0);
+    uint32_t a = v.x, b = v.y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t ta = __shfl_up_sync(kFull, a, o), tb = __shfl_up_sync(kFull, b, o);
+      if (lane >= o) {
+        a += ta;
+        b += tb;
+      }
+    }
+    if (in) chunk_cnt[t.chunk0 + c0 + lane] = make_uint2(baseL + a - v.x, baseE + b - v.y);
+    baseL += __shfl_sync(kFull, a, 31);
+    baseE += __shfl_sync(kFull, b, 31);
+  }
+  if (lane == 0) {
+    t.nL = baseL;
+    t.nE = baseE;
+  }
+}
+
+// The chunk's prefix counts of "below" and "equal" at the thread's first
+// position (thread t of the CTA owns positions 4t .. 4t+3) and the classes of
+// its positions.
+__device__ __forceinline__ void chunk_prefix(const int4& ch, const float* cen, float pivot,
+                                             uint2 base, uint8_t* k, uint32_t& L, uint32_t& E) {
   __shared__ uint32_t s_warp[8];
-  const int4 ch = chunks[blockIdx.x];
-  LTask& t = T[ch.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int p0 = ch.y + 4 * tid;
-  uint8_t k[4];
   uint32_t own = 0;  // below in the low 16 bits, equal in the high 16
   for (int j = 0; j < 4; ++j) {
     const int p = p0 + j;
-    k[j] = p < ch.z ? cls[p] : 2;
+    k[j] = 2;
+    if (p < ch.z) {
+      const float c = cen[p];
+      k[j] = c < pivot ? 0 : (c == pivot ? 1 : 2);
+    }
     own += k[j] == 0 ? 1u : (k[j] == 1 ? 0x10000u : 0u);
   }
   uint32_t incl = own;
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    const uint32_t v = __shfl_up_sync(kFull, incl, o);
     if (lane >= o) incl += v;
   }
   if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
-  uint32_t wbase = 0;
-  for (int w = 0; w < warp; ++w) wbase += s_warp[w];
-  uint32_t run = wbase + incl - own;
-  uint32_t L = chunk_base[blockIdx.x * 3 + 0] + (run & 0xffffu);
-  uint32_t E = chunk_base[blockIdx.x * 3 + 1] + (run >> 16);
+  uint32_t run = incl - own;
+  for (int w = 0; w < warp; ++w) run += s_warp[w];
+  L = base.x + (run & 0xffffu);
+  E = base.y + (run >> 16);
+}
+
+// Pass 3: the prefix counts at each task's first equal / first upper box.
+__global__ void __launch_bounds__(256) wide_first_kernel(const int4* __restrict__ chunks,
+                                                         const uint32_t* __restrict__ nchunks,
+                                                         LTask* __restrict__ T,
+                                                         const float* __restrict__ cen,
+                                                         const uint2* __restrict__ chunk_base) {
+  if (blockIdx.x >= *nchunks) return;
+  const int4 ch = chunks[blockIdx.x];
+  LTask& t = T[ch.x];
+  if (!t.live) return;
+  const uint32_t r0 = (uint32_t)ch.y - t.start, r1 = (uint32_t)ch.z - t.start;
+  const uint32_t fE = t.firstE, fG = t.firstG;
+  if (!((fE >= r0 && fE < r1) || (fG >= r0 && fG < r1))) return;
+  uint8_t k[4];
+  uint32_t L, E;
+  chunk_prefix(ch, cen, t.pivot, chunk_base[blockIdx.x], k, L, E);
   for (int j = 0; j < 4; ++j) {
-    const int p = p0 + j;
-    if (p >= ch.z) break;
-    preL[p] = L;
-    preE[p] = E;
-    const uint32_t rel = (uint32_t)p - t.jlo;
-    if (rel == t.firstE) t.nL_atE = L;
-    if (rel == t.firstG) t.nLE_atG = L + E;
+    const uint32_t rel = r0 + 4 * threadIdx.x + j;
+    if (rel >= r1) break;
+    if (rel == fE) t.L_atE = L;
+    if (rel == fG) t.LE_atG = L + E;
     if (k[j] == 0) ++L;
     else if (k[j] == 1) ++E;
   }
@@ -817,92 +1399,103 @@ __global__ void __launch_bounds__(256) part_prefix_kernel(const int4* __restrict
 
 // Pass 4: boxes below the pivot go to their place (in tmp); the equal and
 // upper queues' operations are written to their tapes.
-__global__ void __launch_bounds__(256) part_tape_kernel(const int4* __restrict__ chunks,
-                                                        const LTask* __restrict__ T,
-                                                        const uint32_t* __restrict__ idx,
-                                                        const uint8_t* __restrict__ cls,
-                                                        const uint32_t* __restrict__ preL,
-                                                        const uint32_t* __restrict__ preE,
-                                                        uint32_t* __restrict__ tmp,
-                                                        uint32_t* __restrict__ tapeE,
-                                                        uint32_t* __restrict__ tapeG) {
+__global__ void __launch_bounds__(256) wide_tape_kernel(
+    const int4* __restrict__ chunks, const uint32_t* __restrict__ nchunks,
+    const LTask* __restrict__ T, const uint32_t* __restrict__ idx, const float* __restrict__ cen,
+    const uint2* __restrict__ chunk_base, uint32_t* __restrict__ tmp,
+    uint32_t* __restrict__ tape_e, uint32_t* __restrict__ tape_g) {
+  if (blockIdx.x >= *nchunks) return;
   const int4 ch = chunks[blockIdx.x];
   const LTask& t = T[ch.x];
-  const uint32_t jlo = t.jlo, fE = t.firstE, fG = t.firstG;
-  for (int p = ch.y + threadIdx.x; p < ch.z; p += blockDim.x) {
-    const uint32_t rel = (uint32_t)p - jlo;
-    const uint8_t k = cls[p];
-    const uint32_t e = idx[p];
-    const uint32_t L = preL[p], E = preE[p], G = rel - L - E;
+  if (!t.live) return;
+  const uint32_t s = t.start, fE = t.firstE, fG = t.firstG, n = t.n;
+  uint8_t k[4];
+  uint32_t L, E;
+  chunk_prefix(ch, cen, t.pivot, chunk_base[blockIdx.x], k, L, E);
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t p = (uint32_t)ch.y + 4 * threadIdx.x + j;
+    if (p >= (uint32_t)ch.z) break;
+    const uint32_t rel = p - s, e = idx[p], G = rel - L - E;
     const bool afterE = fE != kNone && rel > fE, afterG = fG != kNone && rel > fG;
-    const uint32_t rotE = afterE ? L - t.nL_atE : 0u;
-    const uint32_t rotG = afterG ? (L + E) - t.nLE_atG : 0u;
-    // every tape position is below the job's size (a tape holds at most
-    // one entry per box of the job); the checks only guard the memory
-    const uint32_t te = E + rotE, tg = G + rotG, jn = t.jn;
-    if (k == 0) {
-      if (L < jn) tmp[jlo + L] = e;
-      if (afterE && te < jn) tapeE[jlo + te] = rotE;
-      if (afterG && tg < jn) tapeG[jlo + tg] = rotG;
-    } else if (k == 1) {
-      if (te < jn) tapeE[jlo + te] = kTerm | e;
-      if (afterG && tg < jn) tapeG[jlo + tg] = rotG;
-    } else {
-      if (tg < jn) tapeG[jlo + tg] = kTerm | e;
+    const uint32_t rotE = afterE ? L - t.L_atE : 0u;
+    const uint32_t rotG = afterG ? (L + E) - t.LE_atG : 0u;
+    // every tape position is below the task's size (a tape holds at most
+    // one entry per box of the task); the checks only guard the memory
+    const uint32_t te = E + rotE, tg = G + rotG;
+    if (k[j] == 0) {
+      if (L < n) tmp[s + L] = e;
+      if (afterE && te < n) tape_e[s + te] = rotE;
+      if (afterG && tg < n) tape_g[s + tg] = rotG;
+      ++L;
+    } else if (k[j] == 1) {
+      if (te < n) tape_e[s + te] = kTerm | e;
+      if (afterG && tg < n) tape_g[s + tg] = rotG;
+      ++E;
+    } else if (tg < n) {
+      tape_g[s + tg] = kTerm | e;
     }
   }
 }
 
-// Pass 5 (repeated): one pointer-doubling step on both tapes.
-__global__ void __launch_bounds__(256) part_jump_kernel(const int4* __restrict__ chunks,
-                                                        const LTask* __restrict__ T,
-                                                        uint32_t* __restrict__ tapeE,
-                                                        uint32_t* __restrict__ tapeG) {
+// Pass 5: every tape entry follows its copies back to a box.  All entries
+// walk at once and keep their progress in the tape, so a walk meets entries
+// that are already (partly) resolved: pointer doubling without rounds.  Each
+// step goes to an earlier entry, so a walk ends whatever the others do.
+__global__ void __launch_bounds__(256) wide_resolve_kernel(const int4* __restrict__ chunks,
+                                                           const uint32_t* __restrict__ nchunks,
+                                                           const LTask* __restrict__ T,
+                                                           uint32_t* tape_e, uint32_t* tape_g) {
+  if (blockIdx.x >= *nchunks) return;
   const int4 ch = chunks[blockIdx.x];
   const LTask& t = T[ch.x];
-  const uint32_t jlo = t.jlo;
-  const uint32_t nG = t.jn - t.nL - t.nE;
-  const uint32_t lenE = t.nE + (t.firstE != kNone ? t.nL - t.nL_atE : 0u);
-  const uint32_t lenG = nG + (t.firstG != kNone ? (t.nL + t.nE) - t.nLE_atG : 0u);
+  if (!t.live) return;
+  const uint32_t s = t.start;
+  const uint32_t nG = t.n - t.nL - t.nE;
+  const uint32_t lenE = t.nE + (t.firstE != kNone ? t.nL - t.L_atE : 0u);
+  const uint32_t lenG = nG + (t.firstG != kNone ? (t.nL + t.nE) - t.LE_atG : 0u);
+  auto walk = [&](uint32_t* tape, uint32_t rel) {
+    uint32_t at = rel, v = __ldcg(tape + rel);
+    while (!(v & kTerm) && v < at) {
+      at = v;
+      v = __ldcg(tape + v);
+      __stcg(tape + rel, v);
+    }
+  };
   for (int p = ch.y + threadIdx.x; p < ch.z; p += blockDim.x) {
-    const uint32_t rel = (uint32_t)p - jlo;
-    // a copy always refers to an earlier tape entry (v < rel)
-    if (rel < lenE) {
-      const uint32_t v = tapeE[p];
-      if (!(v & kTerm) && v < rel) tapeE[p] = tapeE[jlo + v];
-    }
-    if (rel < lenG) {
-      const uint32_t v = tapeG[p];
-      if (!(v & kTerm) && v < rel) tapeG[p] = tapeG[jlo + v];
-    }
+    const uint32_t rel = (uint32_t)p - s;
+    if (rel < lenE) walk(tape_e + s, rel);
+    if (rel < lenG) walk(tape_g + s, rel);
   }
 }
 
 // Pass 6: the partitioned order back into idx: below | equal queue | upper
 // queue (each queue = the last k entries of its tape).
-__global__ void __launch_bounds__(256) part_scatter_kernel(const int4* __restrict__ chunks,
+__global__ void __launch_bounds__(256) wide_scatter_kernel(const int4* __restrict__ chunks,
+                                                           const uint32_t* __restrict__ nchunks,
                                                            const LTask* __restrict__ T,
                                                            const uint32_t* __restrict__ tmp,
-                                                           const uint32_t* __restrict__ tapeE,
-                                                           const uint32_t* __restrict__ tapeG,
+                                                           const uint32_t* __restrict__ tape_e,
+                                                           const uint32_t* __restrict__ tape_g,
                                                            uint32_t* __restrict__ idx,
                                                            unsigned* __restrict__ status) {
+  if (blockIdx.x >= *nchunks) return;
   const int4 ch = chunks[blockIdx.x];
   const LTask& t = T[ch.x];
-  const uint32_t jlo = t.jlo;
-  const uint32_t RE = t.firstE != kNone ? t.nL - t.nL_atE : 0u;
-  const uint32_t RG = t.firstG != kNone ? (t.nL + t.nE) - t.nLE_atG : 0u;
+  if (!t.live) return;
+  const uint32_t s = t.start;
+  const uint32_t RE = t.firstE != kNone ? t.nL - t.L_atE : 0u;
+  const uint32_t RG = t.firstG != kNone ? (t.nL + t.nE) - t.LE_atG : 0u;
   for (int p = ch.y + threadIdx.x; p < ch.z; p += blockDim.x) {
-    const uint32_t rel = (uint32_t)p - jlo;
+    const uint32_t rel = (uint32_t)p - s;
     uint32_t v = 0;
     if (rel < t.nL) {
       v = tmp[p] | kTerm;
     } else if (rel < t.nL + t.nE) {
       const uint32_t q = RE + (rel - t.nL);
-      if (q < t.jn) v = tapeE[jlo + q];
+      if (q < t.n) v = tape_e[s + q];
     } else {
       const uint32_t q = RG + (rel - t.nL - t.nE);
-      if (q < t.jn) v = tapeG[jlo + q];
+      if (q < t.n) v = tape_g[s + q];
     }
     if (!(v & kTerm)) {  // an unresolved queue entry: an internal error, never expected
       atomicOr(status, kStatusInternal);
@@ -912,56 +1505,32 @@ __global__ void __launch_bounds__(256) part_scatter_kernel(const int4* __restric
   }
 }
 
-// After a partition: the span split takes its cut, or an nthElement step
-// narrows its range (and picks the next pivot from the new order).
-__global__ void part_update_kernel(LTask* __restrict__ T, uint32_t count,
-                                   const uint32_t* __restrict__ idx, const Box* __restrict__ tb) {
+// After the partition: the cut, and whether it moved off the span's.
+__global__ void wide_cut_kernel(LTask* __restrict__ T, const uint32_t* __restrict__ count) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
+  if (k >= *count || !T[k].live) return;
   LTask& t = T[k];
-  if (t.mode == kLDone) return;
-  const uint32_t ps = t.jlo + t.nL, pe = ps + t.nE;
-  if (t.mode == kLSpan) {
-    uint32_t mid = t.start + t.lcs;
-    t.mode = kLDone;
-    if (mid >= ps && mid <= pe) {
-      t.mid = mid;
-      t.need = 0;
-      return;
-    }
+  const uint32_t ps = t.start + t.nL, pe = ps + t.nE;
+  uint32_t mid = t.start + t.lcs;
+  if (mid < ps || mid > pe) {
     mid = mid < ps ? ps : pe;
     if (mid == t.start) ++mid;
     else if (mid == t.start + t.n) --mid;
-    t.mid = mid;
     t.need = 1;
-    return;
   }
-  // nthElement step
-  uint32_t lo = t.jlo, hi = t.jlo + t.jn;
-  bool done = false;
-  if (t.nth < ps) hi = ps;
-  else if (t.nth < pe) done = true;
-  else lo = pe;
-  if (!done && hi <= lo + 1) done = true;
-  if (done) {
-    t.mode = kLDone;
-    t.mid = t.nth;
-    t.need = 1;
-    return;
-  }
-  t.jlo = lo;
-  t.jn = hi - lo;
-  t.pivot = median3(centre_at(idx, tb, lo, t.axis), centre_at(idx, tb, lo + (hi - lo) / 2, t.axis),
-                    centre_at(idx, tb, hi - 1, t.axis));
+  t.mid = mid;
 }
 
-__global__ void __launch_bounds__(256) large_boxes_kernel(const int4* __restrict__ chunks,
-                                                          LTask* __restrict__ T,
-                                                          const uint32_t* __restrict__ idx,
-                                                          const Box* __restrict__ tb) {
+__global__ void __launch_bounds__(256) wide_boxes_kernel(const int4* __restrict__ chunks,
+                                                         const uint32_t* __restrict__ nchunks,
+                                                         LTask* __restrict__ T,
+                                                         const uint32_t* __restrict__ idx,
+                                                         const Box* __restrict__ tb) {
   __shared__ uint32_t s_bk[2][6];
+  if (blockIdx.x >= *nchunks) return;
   const int4 ch = chunks[blockIdx.x];
   LTask& t = T[ch.x];
+  if (!t.live || !t.need) return;
   const int tid = threadIdx.x;
   if (tid < 2) keys_init(s_bk[tid]);
   __syncthreads();
@@ -975,14 +1544,13 @@ __global__ void __launch_bounds__(256) large_boxes_kernel(const int4* __restrict
   }
 }
 
-__global__ void large_finish_kernel(RNode* __restrict__ nodes, const LTask* __restrict__ T,
-                                    uint32_t count) {
+__global__ void wide_finish_kernel(RNode* __restrict__ nodes, const LTask* __restrict__ T,
+                                   const uint32_t* __restrict__ count) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
+  if (k >= *count || !T[k].live) return;
   const LTask& t = T[k];
   RNode& N = nodes[t.node];
   N.t_mid = t.mid;
-  if (!(t.len > 0.f)) return;  // t_out already the node box
   if (t.need) {
     N.t_out[0] = keys_box(t.bk[0]);
     N.t_out[1] = keys_box(t.bk[1]);
@@ -992,7 +1560,23 @@ __global__ void large_finish_kernel(RNode* __restrict__ nodes, const LTask* __re
   }
 }
 
-// --------------------------------------------------- rounds and levels --
+// The root: a node, or the only subtree when it is small enough.
+__global__ void tree_init_kernel(RNode* nodes, SubRoot* subs, uint32_t m,
+                                 const uint32_t* __restrict__ root_keys, BuildCounts* bc) {
+  BuildCounts c = {};
+  if (m > kSub) {
+    nodes[0].start = 0;
+    nodes[0].n = m;
+    nodes[0].all = keys_box(root_keys);
+    c.ntop = 1;
+  } else {
+    subs[0] = SubRoot{0, m, 0, keys_box(root_keys)};
+    c.nsub = 1;
+  }
+  *bc = c;
+}
+
+// --------------------------------------------------- rounds and depths --
 // The split each node makes this round (multiSplit: round 0 splits the
 // whole range; rounds 1 and 2 the part with the largest area x count,
 // the first on ties), sorted into the three size classes.
@@ -1002,35 +1586,16 @@ __global__ void prepare_round_kernel(RNode* __restrict__ nodes, uint32_t lb, uin
   const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= le) return;
   RNode& N = nodes[x];
-  if (N.n <= 4) return;
-  uint32_t s, n;
-  Box b;
+  const int c = round == 0 ? 0 : choose_part(N.cut, N.area, round + 1);
   if (round == 0) {
-    s = N.start;
-    n = N.n;
-    b = N.all;
-  } else {
-    int choice = -1;
-    float best = 0.f;
-    for (int i = 0; i < N.nsub; ++i) {
-      const uint32_t c = N.cut[i + 1] - N.cut[i];
-      if (c > 1) {
-        const float h = N.area[i] * (float)c;
-        if (choice < 0 || h > best) {
-          choice = i;
-          best = h;
-        }
-      }
-    }
-    N.choice = choice;
-    s = N.cut[choice];
-    n = N.cut[choice + 1] - s;
-    b = N.sub[choice];
+    N.cut[0] = N.start;
+    N.cut[1] = N.start + N.n;
   }
-  N.t_start = s;
-  N.t_n = n;
-  N.t_box = b;
-  const int cat = n <= kSmallMax ? 0 : (n <= kMedMax ? 1 : 2);
+  N.choice = c;
+  N.t_start = N.cut[c];
+  N.t_n = N.cut[c + 1] - N.cut[c];
+  N.t_box = round == 0 ? N.all : N.sub[c];
+  const int cat = N.t_n <= kSub ? 0 : (N.t_n <= kCtaMax ? 1 : 2);
   const uint32_t pos = atomicAdd(&counts[cat], 1u);
   lists[(size_t)cat * cap + pos] = x;
 }
@@ -1040,71 +1605,177 @@ __global__ void finish_round_kernel(RNode* __restrict__ nodes, uint32_t lb, uint
   const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= le) return;
   RNode& N = nodes[x];
-  if (N.n <= 4) return;
-  if (round == 0) {
-    N.cut[0] = N.start;
-    N.cut[1] = N.t_mid;
-    N.cut[2] = N.start + N.n;
-    N.sub[0] = N.t_out[0];
-    N.sub[1] = N.t_out[1];
-    N.area[0] = half_area(N.sub[0]);
-    N.area[1] = half_area(N.sub[1]);
-    N.nsub = 2;
-    return;
-  }
-  const int c = N.choice, ns = N.nsub;
-  for (int i = ns; i > c; --i) N.cut[i + 1] = N.cut[i];
-  for (int i = ns - 1; i > c; --i) {
-    N.sub[i + 1] = N.sub[i];
-    N.area[i + 1] = N.area[i];
-  }
-  N.cut[c + 1] = N.t_mid;
-  N.sub[c] = N.t_out[0];
-  N.sub[c + 1] = N.t_out[1];
-  N.area[c] = half_area(N.sub[c]);
-  N.area[c + 1] = half_area(N.sub[c + 1]);
-  N.nsub = ns + 1;
+  insert_cut(N.cut, N.sub, N.area, round + 1, N.choice, N.t_mid, N.t_out[0], N.t_out[1]);
 }
 
-// Children of a depth: items go into the lanes; every part of two or more
-// boxes becomes a node of the next depth (cnt[] = how many).
-__global__ void count_children_kernel(RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
-                                      const uint32_t* __restrict__ idx, uint32_t* __restrict__ cnt) {
+// Children of a depth: single boxes are items; parts of at most kSub boxes
+// become subtrees, larger ones the nodes of the next depth (numbered from le).
+__global__ void make_children_kernel(RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
+                                     uint32_t depth, const uint32_t* __restrict__ idx,
+                                     SubRoot* __restrict__ subs, BuildCounts* __restrict__ bc) {
   const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= le) return;
   RNode& N = nodes[x];
-  uint32_t k = 0;
-  if (N.n <= 4) {
-    for (uint32_t i = 0; i < 4; ++i) N.child[i] = i < N.n ? idx[N.start + i] : kEmpty;
-  } else {
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t c = N.cut[i + 1] - N.cut[i];
-      if (c == 1) N.child[i] = idx[N.cut[i]];
-      else ++k;
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t s = N.cut[i], c = N.cut[i + 1] - s;
+    if (c == 1) {
+      N.child[i] = idx[s];
+    } else if (c <= kSub) {
+      const uint32_t k = atomicAdd(&bc->nsub, 1u);
+      subs[k] = SubRoot{s, c, depth + 1, N.sub[i]};
+      N.child[i] = kSubRef | k;
+    } else {
+      const uint32_t o = atomicAdd(&bc->ntop, 1u);
+      atomicMax(&bc->max_n, c);
+      N.child[i] = kInternal | o;
+      RNode& C = nodes[o];
+      C.start = s;
+      C.n = c;
+      C.all = N.sub[i];
     }
   }
-  cnt[x - lb] = k;
 }
 
-__global__ void make_children_kernel(RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
-                                     const uint32_t* __restrict__ offs) {
-  const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= le) return;
-  RNode& N = nodes[x];
-  if (N.n <= 4) return;
-  uint32_t o = le + offs[x - lb];
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t c = N.cut[i + 1] - N.cut[i];
-    if (c == 1) continue;
-    N.child[i] = kInternal | o;
-    RNode& C = nodes[o];
-    C.start = N.cut[i];
-    C.n = c;
-    C.all = N.sub[i];
-    C.nsub = 1;
-    C.choice = 0;
-    ++o;
+// Subtree sizes bottom-up and depth-first positions top-down over the nodes
+// above the subtrees (a few thousand at most): one CTA, depth by depth.
+struct Place {
+  uint32_t pre, slot, item;
+};
+__global__ void __launch_bounds__(1024) top_positions_kernel(
+    const RNode* __restrict__ nodes, const uint32_t* __restrict__ lev, int depths,
+    const SubRoot* __restrict__ subs, const SubTotals* __restrict__ totals, uint32_t nsub,
+    Place* size, Place* place, Place* __restrict__ sub_place, BuildCounts* __restrict__ bc) {
+  const int tid = threadIdx.x;
+  uint32_t deepest = (uint32_t)depths;
+  for (uint32_t k = tid; k < nsub; k += blockDim.x)
+    deepest = max(deepest, subs[k].depth + totals[k].levels);
+  atomicMax(&bc->max_depth, deepest);
+  if (depths == 0) {
+    if (tid == 0) {
+      sub_place[0] = Place{0, 0, 0};
+      bc->nodes = totals[0].nodes;
+    }
+    return;
   }
+  auto size_of = [&](uint32_t c) {
+    if ((c & kSubRef) == kSubRef) {
+      const uint32_t k = c & ~kSubRef;
+      return Place{totals[k].nodes, totals[k].slots, subs[k].n};
+    }
+    return (c & kInternal) ? size[c & ~kInternal] : Place{0, 1, 1};
+  };
+  for (int d = depths - 1; d >= 0; --d) {
+    for (uint32_t x = lev[d] + tid; x < lev[d + 1]; x += blockDim.x) {
+      Place z{1, 1, 0};
+      for (int i = 0; i < 4; ++i) {
+        const Place c = size_of(nodes[x].child[i]);
+        z.pre += c.pre;
+        z.slot += c.slot;
+        z.item += c.item;
+      }
+      size[x] = z;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    place[0] = Place{0, 0, 0};
+    bc->nodes = size[0].pre;
+  }
+  __syncthreads();
+  for (int d = 0; d < depths; ++d) {
+    for (uint32_t x = lev[d] + tid; x < lev[d + 1]; x += blockDim.x) {
+      Place p = place[x];
+      ++p.pre;
+      ++p.slot;
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t c = nodes[x].child[i];
+        if ((c & kSubRef) == kSubRef) sub_place[c & ~kSubRef] = p;
+        else if (c & kInternal) place[c & ~kInternal] = p;
+        const Place z = size_of(c);
+        p.pre += z.pre;
+        p.slot += z.slot;
+        p.item += z.item;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Per node in depth-first numbering: the reference's child array, what its
+// merge reads (kid: an item's leaf slot or kInternal | node) and its slot and
+// the slot past its subtree; per item its triangle and slot.
+__global__ void __launch_bounds__(128) sub_emit_kernel(
+    const SubRoot* __restrict__ subs, const SubTotals* __restrict__ totals,
+    const Place* __restrict__ sub_place, const SubNode* __restrict__ sn,
+    const uint32_t* __restrict__ idx, uint4* __restrict__ child, uint4* __restrict__ kid,
+    uint2* __restrict__ slots, int32_t* __restrict__ tri_index, uint32_t* __restrict__ item_slot) {
+  const uint32_t start = subs[blockIdx.x].start;
+  const Place r = sub_place[blockIdx.x];
+  for (uint32_t x = threadIdx.x; x < totals[blockIdx.x].nodes; x += blockDim.x) {
+    const SubNode N = sn[start + x];
+    uint32_t slot = r.slot + N.slot + 1, item = r.item + N.item;
+    uint32_t c[4], q[4];
+    for (int i = 0; i < 4; ++i) {
+      c[i] = q[i] = kEmpty;
+      if (N.child[i] == kSubNone) continue;
+      if (N.child[i] & kSubNode) {
+        const SubNode Y = sn[start + (N.child[i] & ~kSubNode)];
+        c[i] = q[i] = kInternal | (r.pre + Y.pre);
+        slot = r.slot + Y.slot + Y.nslots;
+        item = r.item + Y.item + Y.nitems;
+      } else {
+        c[i] = idx[start + N.child[i]];
+        q[i] = item;
+        tri_index[item] = (int32_t)c[i];
+        item_slot[item] = slot;
+        ++slot;
+        ++item;
+      }
+    }
+    const uint32_t p = r.pre + N.pre;
+    child[p] = make_uint4(c[0], c[1], c[2], c[3]);
+    kid[p] = make_uint4(q[0], q[1], q[2], q[3]);
+    slots[p] = make_uint2(r.slot + N.slot, r.slot + N.slot + N.nslots);
+  }
+}
+
+__global__ void top_emit_kernel(const RNode* __restrict__ nodes, uint32_t n,
+                                const Place* __restrict__ size, const Place* __restrict__ place,
+                                const SubRoot* __restrict__ subs,
+                                const SubTotals* __restrict__ totals,
+                                const Place* __restrict__ sub_place, uint4* __restrict__ child,
+                                uint4* __restrict__ kid, uint2* __restrict__ slots,
+                                int32_t* __restrict__ tri_index,
+                                uint32_t* __restrict__ item_slot) {
+  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  const Place me = place[x];
+  uint32_t slot = me.slot + 1, item = me.item;
+  uint32_t c[4], q[4];
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t y = nodes[x].child[i];
+    if ((y & kSubRef) == kSubRef) {
+      const uint32_t k = y & ~kSubRef;
+      c[i] = q[i] = kInternal | sub_place[k].pre;
+      slot += totals[k].slots;
+      item += subs[k].n;
+    } else if (y & kInternal) {
+      const uint32_t k = y & ~kInternal;
+      c[i] = q[i] = kInternal | place[k].pre;
+      slot += size[k].slot;
+      item += size[k].item;
+    } else {
+      c[i] = y;
+      q[i] = item;
+      tri_index[item] = (int32_t)y;
+      item_slot[item] = slot;
+      ++slot;
+      ++item;
+    }
+  }
+  child[me.pre] = make_uint4(c[0], c[1], c[2], c[3]);
+  kid[me.pre] = make_uint4(q[0], q[1], q[2], q[3]);
+  slots[me.pre] = make_uint2(me.slot, me.slot + size[x].slot);
 }
 
 // ------------------------------------------------------------- moments --
@@ -1243,26 +1914,26 @@ __device__ __forceinline__ T lane_maxP2(const Loc<T>& C) {
 // A node's own data from its children's (the reference's post(),
 // FWNFS.h:6892-7118), in the reference's order of operations.
 template <typename T>
-__device__ void merge_loc(const Loc<T>* ch, int nch, int order, Loc<T>& out) {
+__device__ __forceinline__ void merge_loc(const Loc<T>* const* ch, int nch, int order, Loc<T>& out) {
   zero_loc(out);
   for (int d = 0; d < 3; ++d) {
-    out.N[d] = ch[0].N[d];
-    out.areaP[d] = ch[0].areaP[d];
-    out.lo[d] = ch[0].lo[d];
-    out.hi[d] = ch[0].hi[d];
+    out.N[d] = ch[0]->N[d];
+    out.areaP[d] = ch[0]->areaP[d];
+    out.lo[d] = ch[0]->lo[d];
+    out.hi[d] = ch[0]->hi[d];
   }
-  out.area = ch[0].area;
+  out.area = ch[0]->area;
   for (int i = 1; i < nch; ++i) {
     for (int d = 0; d < 3; ++d) {
-      out.N[d] += ch[i].N[d];
-      out.areaP[d] += ch[i].areaP[d];
+      out.N[d] += ch[i]->N[d];
+      out.areaP[d] += ch[i]->areaP[d];
     }
-    out.area += ch[i].area;
+    out.area += ch[i]->area;
   }
   for (int i = 1; i < nch; ++i)
     for (int d = 0; d < 3; ++d) {
-      out.lo[d] = out.lo[d] < ch[i].lo[d] ? out.lo[d] : ch[i].lo[d];
-      out.hi[d] = out.hi[d] > ch[i].hi[d] ? out.hi[d] : ch[i].hi[d];
+      out.lo[d] = out.lo[d] < ch[i]->lo[d] ? out.lo[d] : ch[i]->lo[d];
+      out.hi[d] = out.hi[d] > ch[i]->hi[d] ? out.hi[d] : ch[i]->hi[d];
     }
   if (out.area > T(0)) {
     const T inv = T(1) / out.area;
@@ -1272,21 +1943,21 @@ __device__ void merge_loc(const Loc<T>* ch, int nch, int order, Loc<T>& out) {
   }
   if (order < 1) return;
   for (int d = 0; d < 3; ++d) {
-    out.Nii[d] = ch[0].Nii[d];
-    out.Niii[d] = ch[0].Niii[d];
+    out.Nii[d] = ch[0]->Nii[d];
+    out.Niii[d] = ch[0]->Niii[d];
   }
-  out.perm = ch[0].perm;
-  for (int k = 0; k < 6; ++k) out.c2[k] = ch[0].c2[k];
+  out.perm = ch[0]->perm;
+  for (int k = 0; k < 6; ++k) out.c2[k] = ch[0]->c2[k];
   for (int i = 1; i < nch; ++i) {
     for (int d = 0; d < 3; ++d) {
-      out.Nii[d] += ch[i].Nii[d];
-      out.Niii[d] += ch[i].Niii[d];
+      out.Nii[d] += ch[i]->Nii[d];
+      out.Niii[d] += ch[i]->Niii[d];
     }
-    out.perm += ch[i].perm;
-    for (int k = 0; k < 6; ++k) out.c2[k] += ch[i].c2[k];
+    out.perm += ch[i]->perm;
+    for (int k = 0; k < 6; ++k) out.c2[k] += ch[i]->c2[k];
   }
   for (int i = 0; i < nch; ++i) {
-    const Loc<T>& C = ch[i];
+    const Loc<T>& C = *ch[i];
     const T dx = C.P[0] - out.P[0], dy = C.P[1] - out.P[1], dz = C.P[2] - out.P[2];
     const T* n = C.N;
     out.Nii[0] += n[0] * dx;
@@ -1314,61 +1985,6 @@ __device__ void merge_loc(const Loc<T>* ch, int nch, int order, Loc<T>& out) {
   }
 }
 
-// Sizes of each node's subtree: nodes, slots (lanes in the walk array) and
-// items; bottom-up, one depth per launch.
-__global__ void sizes_kernel(const RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
-                             uint32_t* __restrict__ nsize, uint32_t* __restrict__ nslots,
-                             uint32_t* __restrict__ nitems) {
-  const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= le) return;
-  uint32_t sz = 1, sl = 1, it = 0;
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t c = nodes[x].child[i];
-    if (c == kEmpty) continue;
-    if (c & kInternal) {
-      const uint32_t y = c & ~kInternal;
-      sz += nsize[y];
-      sl += nslots[y];
-      it += nitems[y];
-    } else {
-      ++sl;
-      ++it;
-    }
-  }
-  nsize[x] = sz;
-  nslots[x] = sl;
-  nitems[x] = it;
-}
-
-// Depth-first positions, top-down: the reference's node number (pre-order,
-// children in lane order), the node's slot in the walk array, the first
-// leaf slot of its subtree.
-__global__ void positions_kernel(const RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
-                                 const uint32_t* __restrict__ nsize,
-                                 const uint32_t* __restrict__ nslots,
-                                 const uint32_t* __restrict__ nitems, uint32_t* __restrict__ pre,
-                                 uint32_t* __restrict__ slot, uint32_t* __restrict__ ibase) {
-  const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= le) return;
-  uint32_t p = pre[x] + 1, sp = slot[x] + 1, ib = ibase[x];
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t c = nodes[x].child[i];
-    if (c == kEmpty) continue;
-    if (c & kInternal) {
-      const uint32_t y = c & ~kInternal;
-      pre[y] = p;
-      p += nsize[y];
-      slot[y] = sp;
-      sp += nslots[y];
-      ibase[y] = ib;
-      ib += nitems[y];
-    } else {
-      ++sp;
-      ++ib;
-    }
-  }
-}
-
 __device__ void load_tri(const double* __restrict__ V, int64_t nV, const int32_t* __restrict__ F,
                          uint32_t f, double* v) {
   for (int c = 0; c < 3; ++c) {
@@ -1378,221 +1994,155 @@ __device__ void load_tri(const double* __restrict__ V, int64_t nV, const int32_t
   }
 }
 
-__device__ void write_records(const Loc<float>& C32, const Loc<double>& C64, long long link,
-                              SoupNodeF* nf, SoupNodeD* nd) {
-  const float m32 = lane_maxP2(C32);
+// The walks' records of a slot.  *bad is set where a moment is not finite or
+// beyond 1e100 in magnitude (gwn_soup_impl::moments_bounded); the bit patterns
+// of non-negative doubles compare as the values do, NaN above all.
+__device__ __forceinline__ void write_record32(const Loc<float>& C, int link, SoupNodeF* nf,
+                                               bool root) {
   SoupNodeF R;
-  R.a = make_float4(C32.P[0], C32.P[1], C32.P[2], m32);
-  {
-    // the reference's FP32 moments (with its FP32 sums of the mixed terms),
-    // packed into the walk's far-field forms
-    double N[3], Nii[3], Niii[3], c2[6];
-    for (int d = 0; d < 3; ++d) {
-      N[d] = C32.N[d];
-      Nii[d] = C32.Nii[d];
-      Niii[d] = C32.Niii[d];
-    }
-    for (int k = 0; k < 6; ++k) c2[k] = C32.c2[k];
-    pack_far32(R, N, Nii, (double)(C32.Nxy + C32.Nyx), (double)(C32.Nyz + C32.Nzy),
-               (double)(C32.Nzx + C32.Nxz), Niii, (double)C32.perm, c2, (int)link);
-  }
-  *nf = R;
-  SoupNodeD D;
+  R.a = make_float4(C.P[0], C.P[1], C.P[2], root ? INFINITY : lane_maxP2(C));
+  // the reference's FP32 moments (with its FP32 sums of the mixed terms),
+  // packed into the walk's far-field forms
+  double N[3], Nii[3], Niii[3], c2[6];
   for (int d = 0; d < 3; ++d) {
-    D.P[d] = C64.P[d];
-    D.N[d] = C64.N[d];
-    D.Nii[d] = C64.Nii[d];
-    D.Niii[d] = C64.Niii[d];
+    N[d] = C.N[d];
+    Nii[d] = C.Nii[d];
+    Niii[d] = C.Niii[d];
   }
-  D.maxP2 = lane_maxP2(C64);
-  D.Nxy_yx = C64.Nxy + C64.Nyx;
-  D.Nyz_zy = C64.Nyz + C64.Nzy;
-  D.Nzx_xz = C64.Nzx + C64.Nxz;
-  D.perm = C64.perm;
-  for (int k = 0; k < 6; ++k) D.c2[k] = C64.c2[k];
+  for (int k = 0; k < 6; ++k) c2[k] = C.c2[k];
+  pack_far32(R, N, Nii, (double)(C.Nxy + C.Nyx), (double)(C.Nyz + C.Nzy),
+             (double)(C.Nzx + C.Nxz), Niii, (double)C.perm, c2, link);
+  *nf = R;
+}
+__device__ __forceinline__ bool beyond(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > __double_as_longlong(1e100);
+}
+__device__ __forceinline__ bool write_record64(const Loc<double>& C, long long link, SoupNodeD* nd,
+                                               bool root) {
+  SoupNodeD D;
+  bool bad = false;
+  for (int d = 0; d < 3; ++d) {
+    D.P[d] = C.P[d];
+    D.N[d] = C.N[d];
+    D.Nii[d] = C.Nii[d];
+    D.Niii[d] = C.Niii[d];
+    bad |= beyond(C.N[d]) || beyond(C.Nii[d]) || beyond(C.Niii[d]);
+  }
+  D.maxP2 = root ? (double)INFINITY : lane_maxP2(C);
+  D.Nxy_yx = C.Nxy + C.Nyx;
+  D.Nyz_zy = C.Nyz + C.Nzy;
+  D.Nzx_xz = C.Nzx + C.Nxz;
+  D.perm = C.perm;
+  bad |= beyond(D.Nxy_yx) || beyond(D.Nyz_zy) || beyond(D.Nzx_xz) || beyond(D.perm);
+  for (int k = 0; k < 6; ++k) {
+    D.c2[k] = C.c2[k];
+    bad |= beyond(C.c2[k]);
+  }
   D.link = link;
   *nd = D;
+  return bad;
 }
 
-// Moments of one depth, bottom-up: each node merges its children's data
-// (items computed here) and writes its lanes' slot records; the root also
-// writes slot 0.
-__global__ void moments_kernel(const RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
-                               const double* __restrict__ V, int64_t nV,
-                               const int32_t* __restrict__ F, int order,
-                               const uint32_t* __restrict__ nslots,
-                               const uint32_t* __restrict__ nitems,
-                               const uint32_t* __restrict__ slot,
-                               const uint32_t* __restrict__ ibase, Loc<float>* __restrict__ L32,
-                               Loc<double>* __restrict__ L64, SoupNodeF* __restrict__ nf,
-                               SoupNodeD* __restrict__ nd, float4* __restrict__ tf,
-                               double* __restrict__ td, int32_t* __restrict__ tri_index) {
-  const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= le) return;
-  Loc<float> c32[4];
-  Loc<double> c64[4];
+// Items: one thread per leaf slot computes the triangle's data in both
+// precisions, its records, and leaves the data for the merges.  (One thread
+// per node did all this for its items and kept up to four children's data in
+// local memory: 4.16 ms for 1.3M triangles.)
+__global__ void __launch_bounds__(128) items_kernel(
+    int64_t m, const int32_t* __restrict__ tri_index, const uint32_t* __restrict__ item_slot,
+    const double* __restrict__ V, int64_t nV, const int32_t* __restrict__ F, int order,
+    Loc<float>* __restrict__ L32, Loc<double>* __restrict__ L64, SoupNodeF* __restrict__ nf,
+    SoupNodeD* __restrict__ nd, float4* __restrict__ tf, double* __restrict__ td,
+    BuildCounts* __restrict__ bc) {
+  const int64_t ib = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (ib >= m) return;
+  const uint32_t sp = item_slot[ib];
+  double v[9];
+  load_tri(V, nV, F, (uint32_t)tri_index[ib], v);
+  {
+    float w[9];
+    for (int k = 0; k < 9; ++k) w[k] = (float)v[k];
+    Loc<float> C;
+    item_loc<float>(w, w + 3, w + 6, order, C);
+    write_record32(C, (int)~ib, nf + sp, false);
+    L32[ib] = C;
+    tf[ib * 3 + 0] = make_float4(w[0], w[1], w[2], w[3]);
+    tf[ib * 3 + 1] = make_float4(w[4], w[5], w[6], w[7]);
+    tf[ib * 3 + 2] = make_float4(w[8], tri_screen_slack(v), 0.f, 0.f);
+  }
+  Loc<double> C;
+  item_loc<double>(v, v + 3, v + 6, order, C);
+  if (write_record64(C, ~ib, nd + sp, false)) bc->unbounded = 1;
+  L64[ib] = C;
+  for (int k = 0; k < 9; ++k) td[ib * 9 + k] = v[k];
+}
+
+// One node p (depth-first number): merges its children's data (items at
+// [0, m), nodes at [m, m + nodes)) and writes its slot's records.
+struct MergeArgs {
+  const uint4* kid;
+  const uint2* slots;
+  uint32_t m;
+  int order;
+  Loc<float>* L32;
+  Loc<double>* L64;
+  SoupNodeF* nf;
+  SoupNodeD* nd;
+  BuildCounts* bc;
+};
+template <typename T>
+__device__ __forceinline__ void merge_node(const MergeArgs& A, uint4 kid, const Loc<T>* L,
+                                           Loc<T>& out) {
+  const uint32_t k[4] = {kid.x, kid.y, kid.z, kid.w};
+  const Loc<T>* ch[4];
   int nch = 0;
-  uint32_t sp = slot[x] + 1, ib = ibase[x];
+#pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t c = nodes[x].child[i];
-    if (c == kEmpty) break;
-    long long link;
-    if (c & kInternal) {
-      const uint32_t y = c & ~kInternal;
-      c32[nch] = L32[y];
-      c64[nch] = L64[y];
-      link = (long long)sp + nslots[y];
-      write_records(c32[nch], c64[nch], link, nf + sp, nd + sp);
-      sp += nslots[y];
-      ib += nitems[y];
-    } else {
-      double v[9];
-      load_tri(V, nV, F, c, v);
-      float w[9];
-      for (int k = 0; k < 9; ++k) w[k] = (float)v[k];
-      item_loc<float>(w, w + 3, w + 6, order, c32[nch]);
-      item_loc<double>(v, v + 3, v + 6, order, c64[nch]);
-      link = ~(long long)ib;
-      write_records(c32[nch], c64[nch], link, nf + sp, nd + sp);
-      for (int k = 0; k < 9; ++k) td[(int64_t)ib * 9 + k] = v[k];
-      tf[(int64_t)ib * 3 + 0] = make_float4(w[0], w[1], w[2], w[3]);
-      tf[(int64_t)ib * 3 + 1] = make_float4(w[4], w[5], w[6], w[7]);
-      tf[(int64_t)ib * 3 + 2] = make_float4(w[8], tri_screen_slack(v), 0.f, 0.f);
-      tri_index[ib] = (int32_t)c;
-      ++sp;
-      ++ib;
-    }
-    ++nch;
+    ch[i] = L;
+    if (k[i] == kEmpty) continue;
+    ch[i] = L + ((k[i] & kInternal) ? A.m + (k[i] & ~kInternal) : k[i]);
+    nch = i + 1;
   }
-  Loc<float> o32;
-  Loc<double> o64;
-  merge_loc(c32, nch, order, o32);
-  merge_loc(c64, nch, order, o64);
-  L32[x] = o32;
-  L64[x] = o64;
-  if (x == 0) {  // the root: slot 0, always opened by the walks
-    write_records(o32, o64, (long long)nslots[0], nf, nd);
-    nf[0].a.w = INFINITY;
-    nd[0].maxP2 = INFINITY;
+  merge_loc(ch, nch, A.order, out);
+}
+__device__ void merge_at(const MergeArgs& A, uint32_t p) {
+  const uint4 kid = A.kid[p];
+  const uint2 sl = A.slots[p];
+  {
+    Loc<float> C;
+    merge_node<float>(A, kid, A.L32, C);
+    A.L32[A.m + p] = C;
+    write_record32(C, (int)sl.y, A.nf + sl.x, p == 0);
+  }
+  Loc<double> C;
+  merge_node<double>(A, kid, A.L64, C);
+  A.L64[A.m + p] = C;
+  if (write_record64(C, (long long)sl.y, A.nd + sl.x, p == 0)) A.bc->unbounded = 1;
+}
+
+// All nodes of a subtree, deepest depth first; one CTA per subtree.
+__global__ void __launch_bounds__(128) sub_merge_kernel(MergeArgs A,
+                                                        const SubRoot* __restrict__ subs,
+                                                        const SubTotals* __restrict__ totals,
+                                                        const Place* __restrict__ sub_place,
+                                                        const SubNode* __restrict__ sn,
+                                                        const uint16_t* __restrict__ lev) {
+  const uint32_t start = subs[blockIdx.x].start, pre = sub_place[blockIdx.x].pre;
+  for (uint32_t d = totals[blockIdx.x].levels; d-- > 0;) {
+    for (uint32_t x = lev[start + d] + threadIdx.x; x < lev[start + d + 1]; x += blockDim.x)
+      merge_at(A, pre + sn[start + x].pre);
+    __syncthreads();
   }
 }
 
-// Reference node array: 4 entries per node in the reference's numbering.
-__global__ void export_tree_kernel(const RNode* __restrict__ nodes, uint32_t nn,
-                                   const uint32_t* __restrict__ pre, uint32_t* __restrict__ out) {
-  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nn) return;
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t c = nodes[x].child[i];
-    out[(size_t)pre[x] * 4 + i] = (c != kEmpty && (c & kInternal)) ? (kInternal | pre[c & ~kInternal]) : c;
-  }
+// One depth of the nodes above the subtrees.
+__global__ void __launch_bounds__(128) top_merge_kernel(MergeArgs A,
+                                                        const Place* __restrict__ place,
+                                                        uint32_t lb, uint32_t le) {
+  const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < le) merge_at(A, place[x].pre);
 }
 
 inline unsigned blocks_for(uint64_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t); }
-
-// Host side of one round's large splits.
-struct LargeRunner {
-  cudaStream_t st;
-  RNode* nodes;
-  uint32_t* idx;
-  uint32_t* tmp;
-  uint32_t* tapeE;
-  uint32_t* tapeG;
-  uint32_t* preL;
-  uint32_t* preE;
-  uint8_t* cls;
-  const Box* tb;
-  unsigned* status;
-
-  void run(const uint32_t* list_dev, uint32_t count) {
-    DevBuf<LTask> T(count, st);
-    launch_kernel(large_init_kernel, blocks_for(count, 64), 64, 0, st, nodes, list_dev, count,
-                  T.get());
-    std::vector<LTask> h(count);
-    GWN_CUDA(cudaMemcpyAsync(h.data(), T.get(), count * sizeof(LTask), cudaMemcpyDeviceToHost, st));
-    GWN_CUDA(cudaStreamSynchronize(st));
-    // span statistics over every task with a real axis
-    {
-      std::vector<int4> ch;
-      for (uint32_t k = 0; k < count; ++k)
-        if (h[k].mode == kLSpan) add_chunks(ch, k, h[k].start, h[k].n);
-      if (!ch.empty()) {
-        DevBuf<int4> dch(ch.size(), st);
-        dch.upload(ch.data(), ch.size(), st);
-        launch_kernel(large_span_kernel, (unsigned)ch.size(), 256, 0, st, (const int4*)dch.get(),
-                      T.get(), (const uint32_t*)idx, tb);
-        launch_kernel(large_choose_kernel, blocks_for(count, 64), 64, 0, st, T.get(), count,
-                      (const uint32_t*)idx, tb);
-        GWN_CUDA(cudaStreamSynchronize(st));
-      }
-    }
-    // partitions until every span split and nthElement is done (each
-    // nthElement step narrows its range, so the count is bounded by its size)
-    for (uint64_t iter = 0;; ++iter) {
-      GWN_REQUIRE(iter < 100000,
-                  "soup_build: the partition loop did not finish");
-      GWN_CUDA(cudaMemcpyAsync(h.data(), T.get(), count * sizeof(LTask), cudaMemcpyDeviceToHost, st));
-      GWN_CUDA(cudaStreamSynchronize(st));
-      std::vector<int4> ch;
-      std::vector<int2> jc(count, make_int2(0, 0));
-      uint32_t maxn = 0;
-      for (uint32_t k = 0; k < count; ++k) {
-        if (h[k].mode == kLDone) continue;
-        jc[k].x = (int)ch.size();
-        add_chunks(ch, k, h[k].jlo, h[k].jn);
-        jc[k].y = (int)ch.size() - jc[k].x;
-        maxn = std::max(maxn, h[k].jn);
-      }
-      if (ch.empty()) break;
-      const unsigned nch = (unsigned)ch.size();
-      DevBuf<int4> dch(nch, st);
-      dch.upload(ch.data(), nch, st);
-      DevBuf<int2> djc(count, st);
-      djc.upload(jc.data(), count, st);
-      DevBuf<uint32_t> ccnt((size_t)nch * 3, st), cbase((size_t)nch * 3, st);
-      const int4* c4 = dch.get();
-      launch_kernel(part_init_kernel, blocks_for(count, 64), 64, 0, st, T.get(), count);
-      launch_kernel(part_classify_kernel, nch, 256, 0, st, c4, T.get(), (const uint32_t*)idx, tb,
-                    cls, ccnt.get());
-      launch_kernel(part_chunk_scan_kernel, blocks_for(count, 64), 64, 0, st, T.get(), count,
-                    (const int2*)djc.get(), (const uint32_t*)ccnt.get(), cbase.get());
-      launch_kernel(part_prefix_kernel, nch, 256, 0, st, c4, T.get(), (const uint8_t*)cls,
-                    (const uint32_t*)cbase.get(), preL, preE);
-      launch_kernel(part_tape_kernel, nch, 256, 0, st, c4, (const LTask*)T.get(),
-                    (const uint32_t*)idx, (const uint8_t*)cls, (const uint32_t*)preL,
-                    (const uint32_t*)preE, tmp, tapeE, tapeG);
-      int rounds = 1;
-      while ((1ull << rounds) < (unsigned long long)maxn + 1) ++rounds;
-      for (int r = 0; r <= rounds; ++r)
-        launch_kernel(part_jump_kernel, nch, 256, 0, st, c4, (const LTask*)T.get(), tapeE, tapeG);
-      launch_kernel(part_scatter_kernel, nch, 256, 0, st, c4, (const LTask*)T.get(),
-                    (const uint32_t*)tmp, (const uint32_t*)tapeE, (const uint32_t*)tapeG, idx,
-                    status);
-      launch_kernel(part_update_kernel, blocks_for(count, 64), 64, 0, st, T.get(), count,
-                    (const uint32_t*)idx, tb);
-    }
-    // sub boxes where the cut moved off the span's (or came from nthElement)
-    {
-      std::vector<int4> ch;
-      for (uint32_t k = 0; k < count; ++k)
-        if (h[k].need) add_chunks(ch, k, h[k].start, h[k].n);
-      if (!ch.empty()) {
-        DevBuf<int4> dch(ch.size(), st);
-        dch.upload(ch.data(), ch.size(), st);
-        launch_kernel(large_boxes_kernel, (unsigned)ch.size(), 256, 0, st,
-                      (const int4*)dch.get(), T.get(), (const uint32_t*)idx, tb);
-      }
-    }
-    launch_kernel(large_finish_kernel, blocks_for(count, 64), 64, 0, st, nodes,
-                  (const LTask*)T.get(), count);
-    GWN_CUDA(cudaStreamSynchronize(st));  // chunk lists live on this stack frame
-  }
-
-  static void add_chunks(std::vector<int4>& ch, uint32_t k, uint32_t lo, uint32_t n) {
-    for (uint32_t b = 0; b < n; b += kChunk)
-      ch.push_back(make_int4((int)k, (int)(lo + b), (int)(lo + std::min(n, b + kChunk)), 0));
-  }
-};
 
 __global__ void iota3_kernel(int32_t* F, int64_t m) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1634,11 +2184,10 @@ void soup_build_ref(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t
     launch_kernel(tri_box_kernel, blocks_for((uint64_t)nF), 256, 0, st, V, nV, F, nF, tb.get(),
                   keep.get(), status.ptr());
     exclusive_scan_u32(keep.get(), pos.get(), nF, st);
-    std::vector<uint32_t> init = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    root_keys.upload(init.data(), 6, st);
+    launch_kernel(keys_init_kernel, 1, 1, 0, st, root_keys.get());
     launch_kernel(compact_kernel, blocks_for((uint64_t)nF), 256, 0, st, (const uint32_t*)keep.get(),
                   (const uint32_t*)pos.get(), nF, (const Box*)tb.get(), idx.get(), root_keys.get());
-    uint32_t last[2];
+    unsigned* last = pinned_words();
     GWN_CUDA(cudaMemcpyAsync(&last[0], pos.get() + (nF - 1), 4, cudaMemcpyDeviceToHost, st));
     GWN_CUDA(cudaMemcpyAsync(&last[1], keep.get() + (nF - 1), 4, cudaMemcpyDeviceToHost, st));
     GWN_CUDA(cudaStreamSynchronize(st));
@@ -1652,79 +2201,132 @@ void soup_build_ref(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t
     for (int d = 0; d < 3; ++d) s.lo[d] = s.hi[d] = 0;
     return;
   }
-  // ---- tree, depth by depth
-  const size_t cap = (size_t)std::max<uint32_t>(m, 1);
-  DevBuf<RNode> nodes(cap, st);
-  DevBuf<uint32_t> tmp(cap, st), tapeE(cap, st), tapeG(cap, st), preL(cap, st), preE(cap, st);
-  DevBuf<uint8_t> cls(cap, st);
-  DevBuf<uint32_t> lists(cap * 3, st), counts(3, st), ccount(cap, st), coffs(cap, st);
-  launch_kernel(root_init_kernel, 1, 1, 0, st, nodes.get(), m, (const uint32_t*)root_keys.get());
-  LargeRunner large{st,        nodes.get(), idx.get(),  tmp.get(),
-                    tapeE.get(), tapeG.get(), preL.get(), preE.get(),
-                    cls.get(),  tb.get(),    status.ptr()};
-  std::vector<uint32_t> level = {0, 1};  // depth d holds nodes [level[d], level[d + 1])
-  uint32_t lb = 0, le = 1;
-  while (true) {
-    const uint32_t nl = le - lb;
-    for (int round = 0; round < 3; ++round) {
-      counts.zero(st);
-      launch_kernel(prepare_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le, round,
-                    lists.get(), (uint32_t)cap, counts.get());
-      uint32_t hc[3];
-      GWN_CUDA(cudaMemcpyAsync(hc, counts.get(), sizeof(hc), cudaMemcpyDeviceToHost, st));
-      GWN_CUDA(cudaStreamSynchronize(st));
-      if (hc[0] + hc[1] + hc[2] == 0) break;  // every node of this depth holds <= 4 items
-      if (hc[0])
-        launch_kernel(split_small_kernel, blocks_for(hc[0], 128), 128, 0, st, nodes.get(),
-                      (const uint32_t*)lists.get(), hc[0], idx.get(), (const Box*)tb.get());
-      if (hc[1])
-        launch_kernel(split_medium_kernel, hc[1], 256, 0, st, nodes.get(),
-                      (const uint32_t*)(lists.get() + cap), idx.get(), (const Box*)tb.get(),
-                      status.ptr());
-      if (hc[2]) large.run(lists.get() + 2 * cap, hc[2]);
-      launch_kernel(finish_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le, round);
-    }
-    launch_kernel(count_children_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
-                  (const uint32_t*)idx.get(), ccount.get());
-    exclusive_scan_u32(ccount.get(), coffs.get(), nl, st);
-    uint32_t lastc[2];
-    GWN_CUDA(cudaMemcpyAsync(&lastc[0], coffs.get() + (nl - 1), 4, cudaMemcpyDeviceToHost, st));
-    GWN_CUDA(cudaMemcpyAsync(&lastc[1], ccount.get() + (nl - 1), 4, cudaMemcpyDeviceToHost, st));
+  // ---- tree: depth by depth down to kSub boxes, then whole subtrees
+  const uint32_t split_max = m / (kSub + 1) + 1;  // parts of more than kSub boxes in a depth
+  const uint32_t wide_max = m / (kCtaMax + 1) + 1;
+  const uint32_t chunk_max = m / kChunk + wide_max;
+  uint32_t node_cap = m > kSub ? 8 * split_max + 64 : 1;
+  DevBuf<RNode> nodes(node_cap, st);
+  DevBuf<uint32_t> lists((size_t)split_max * 3, st);
+  DevBuf<SubRoot> subs((size_t)m / 2 + 1, st);
+  DevBuf<BuildCounts> bc(1, st);
+  BuildCounts* hbc = reinterpret_cast<BuildCounts*>(pinned_words());
+  static_assert(sizeof(BuildCounts) <= 64 * sizeof(unsigned), "pinned words");
+  auto read_counts = [&]() {
+    GWN_CUDA(cudaMemcpyAsync(hbc, bc.get(), sizeof(BuildCounts), cudaMemcpyDeviceToHost, st));
     GWN_CUDA(cudaStreamSynchronize(st));
-    const uint32_t added = lastc[0] + lastc[1];
-    GWN_REQUIRE((size_t)le + added <= cap, "soup_build: tree larger than its bound");
-    if (added == 0) break;
-    launch_kernel(make_children_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
-                  (const uint32_t*)coffs.get());
-    lb = le;
-    le += added;
-    level.push_back(le);
+  };
+  launch_kernel(tree_init_kernel, 1, 1, 0, st, nodes.get(), subs.get(), m,
+                (const uint32_t*)root_keys.get(), bc.get());
+  std::vector<uint32_t> level = {0};  // depth d of the top holds nodes [level[d], level[d + 1])
+  uint32_t nsub = 1;
+  if (m > kSub) {
+    DevBuf<uint32_t> tmp(m, st), tapeE(m, st), tapeG(m, st), nchunks(1, st);
+    DevBuf<float> cen(m, st);
+    DevBuf<LTask> tasks;
+    DevBuf<int4> chunks;
+    DevBuf<uint2> chunk_cnt;
+    if (m > kCtaMax) {
+      tasks.alloc(wide_max, st);
+      chunks.alloc(chunk_max, st);
+      chunk_cnt.alloc(chunk_max, st);
+    }
+    uint32_t lb = 0, le = 1, max_n = m;
+    level.push_back(1);
+    while (le > lb) {
+      const uint32_t nl = le - lb, parts = std::min(nl, split_max);
+      if (le + split_max > node_cap) {
+        const uint32_t cap2 = 2 * node_cap + split_max;
+        DevBuf<RNode> more(cap2, st);
+        GWN_CUDA(cudaMemcpyAsync(more.get(), nodes.get(), (size_t)le * sizeof(RNode),
+                                 cudaMemcpyDeviceToDevice, st));
+        nodes = std::move(more);
+        node_cap = cap2;
+      }
+      GWN_CUDA(cudaMemsetAsync(bc.get(), 0, offsetof(BuildCounts, ntop), st));
+      for (int round = 0; round < 3; ++round) {
+        uint32_t* cnt = bc.get()->lists[round];
+        uint32_t *lw = lists.get(), *lc = lw + split_max, *lg = lc + split_max;
+        launch_kernel(prepare_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le, round,
+                      lists.get(), split_max, cnt);
+        if (max_n > kCtaMax) {
+          const uint32_t *c2 = cnt + 2, *nch = nchunks.get();
+          LTask* T = tasks.get();
+          const int4* ch = chunks.get();
+          const uint32_t nt = std::min(nl, wide_max);
+          launch_kernel(wide_init_kernel, 1, 512, 0, st, (const RNode*)nodes.get(),
+                        (const uint32_t*)lg, c2, T, chunks.get(), nchunks.get());
+          launch_kernel(wide_span_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                        (const uint32_t*)idx.get(), (const Box*)tb.get(), cen.get());
+          launch_kernel(wide_choose_kernel, nt, 32, 0, st, T, c2, lc, cnt + 1);
+          launch_kernel(wide_classify_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                        (const float*)cen.get(), chunk_cnt.get());
+          launch_kernel(wide_scan_kernel, nt, 32, 0, st, T, c2, chunk_cnt.get());
+          launch_kernel(wide_first_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                        (const float*)cen.get(), (const uint2*)chunk_cnt.get());
+          launch_kernel(wide_tape_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                        (const uint32_t*)idx.get(), (const float*)cen.get(),
+                        (const uint2*)chunk_cnt.get(), tmp.get(), tapeE.get(), tapeG.get());
+          launch_kernel(wide_resolve_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                        tapeE.get(), tapeG.get());
+          launch_kernel(wide_scatter_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                        (const uint32_t*)tmp.get(), (const uint32_t*)tapeE.get(),
+                        (const uint32_t*)tapeG.get(), idx.get(), status.ptr());
+          launch_kernel(wide_cut_kernel, blocks_for(nt, 64), 64, 0, st, T, c2);
+          launch_kernel(wide_boxes_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                        (const uint32_t*)idx.get(), (const Box*)tb.get());
+          launch_kernel(wide_finish_kernel, blocks_for(nt, 64), 64, 0, st, nodes.get(),
+                        (const LTask*)T, c2);
+        }
+        launch_kernel(part_cta_kernel, parts, 1024, 0, st, nodes.get(), (const uint32_t*)lc,
+                      (const uint32_t*)(cnt + 1), idx.get(), cen.get(), tmp.get(), tapeE.get(),
+                      tapeG.get(), (const Box*)tb.get(), status.ptr());
+        if (round > 0)  // a whole node has more than kSub boxes
+          launch_kernel(part_warp_kernel, nl, 32, 0, st, nodes.get(), (const uint32_t*)lw,
+                        (const uint32_t*)cnt, idx.get(), (const Box*)tb.get(), status.ptr());
+        launch_kernel(finish_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le, round);
+      }
+      launch_kernel(make_children_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
+                    (uint32_t)level.size() - 2, (const uint32_t*)idx.get(), subs.get(), bc.get());
+      read_counts();
+      if (host_mode) status.check(st, "soup_build");
+      lb = le;
+      le = hbc->ntop;
+      nsub = hbc->nsub;
+      max_n = hbc->max_n;
+      GWN_REQUIRE(le <= node_cap, "soup_build: tree larger than its bound");
+      if (le > lb) level.push_back(le);
+    }
   }
-  const uint32_t nn = le;
-  const int depth = (int)level.size() - 1;  // number of depths
+  const int top_depths = (int)level.size() - 1;
+  const uint32_t ntop = level.back();
+  DevBuf<SubNode> sn(m, st);
+  DevBuf<uint16_t> lev((size_t)m + 1, st);  // a subtree of n > 1 boxes is at most n - 1 deep
+  DevBuf<SubTotals> totals(nsub, st);
+  DevBuf<Place> size(std::max<uint32_t>(ntop, 1), st), place(std::max<uint32_t>(ntop, 1), st),
+      sub_place(nsub, st);
+  DevBuf<uint32_t> dlevel(level.size(), st);
+  dlevel.upload(level.data(), level.size(), st);
+  {
+    static_assert(sizeof(SubShared) <= 100 * 1024, "two CTAs per SM");
+    GWN_CUDA(cudaFuncSetAttribute(subtree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(SubShared)));
+    launch_kernel(subtree_kernel, nsub, kSubWarps * 32, sizeof(SubShared), st,
+                  (const SubRoot*)subs.get(), nsub, (const uint32_t*)idx.get(),
+                  (const Box*)tb.get(), sn.get(), lev.get(), totals.get(), status.ptr());
+  }
+  launch_kernel(top_positions_kernel, 1, 1024, 0, st, (const RNode*)nodes.get(),
+                (const uint32_t*)dlevel.get(), top_depths, (const SubRoot*)subs.get(),
+                (const SubTotals*)totals.get(), nsub, size.get(), place.get(), sub_place.get(),
+                bc.get());
+  read_counts();
   if (host_mode) status.check(st, "soup_build");
-  // ---- sizes (bottom-up) and depth-first positions (top-down)
-  DevBuf<uint32_t> nsize(nn, st), nslots(nn, st), nitems(nn, st), pre(nn, st), slot(nn, st),
-      ibase(nn, st);
-  for (int d = depth - 1; d >= 0; --d)
-    launch_kernel(sizes_kernel, blocks_for(level[d + 1] - level[d]), 256, 0, st,
-                  (const RNode*)nodes.get(), level[d], level[d + 1], nsize.get(), nslots.get(),
-                  nitems.get());
-  GWN_CUDA(cudaMemsetAsync(pre.get(), 0, 4, st));
-  GWN_CUDA(cudaMemsetAsync(slot.get(), 0, 4, st));
-  GWN_CUDA(cudaMemsetAsync(ibase.get(), 0, 4, st));
-  for (int d = 0; d < depth; ++d)
-    launch_kernel(positions_kernel, blocks_for(level[d + 1] - level[d]), 256, 0, st,
-                  (const RNode*)nodes.get(), level[d], level[d + 1], (const uint32_t*)nsize.get(),
-                  (const uint32_t*)nslots.get(), (const uint32_t*)nitems.get(), pre.get(),
-                  slot.get(), ibase.get());
-  uint32_t total_slots = 0;
-  GWN_CUDA(cudaMemcpyAsync(&total_slots, nslots.get(), 4, cudaMemcpyDeviceToHost, st));
-  GWN_CUDA(cudaStreamSynchronize(st));
-  // ---- moments and the walk's slot records
+  const uint32_t nn = hbc->nodes;
+  // ---- moments and the walk's slot records: a slot per node and per item
+  const uint32_t total_slots = nn + m;
   s.nnodes = total_slots;
   s.ref_nodes = nn;
-  s.max_depth = depth;
+  s.max_depth = (int)hbc->max_depth;
   s.tri_index.alloc(m);
   s.nf.alloc(total_slots);
   // the walk reads records with 256-bit loads
@@ -1735,32 +2337,49 @@ void soup_build_ref(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t
   s.td.alloc((size_t)m * 9);
   s.ref_child.alloc((size_t)nn * 4);
   {
-    DevBuf<Loc<float>> L32(nn, st);
-    DevBuf<Loc<double>> L64(nn, st);
-    for (int d = depth - 1; d >= 0; --d)
-      launch_kernel(moments_kernel, blocks_for(level[d + 1] - level[d], 128), 128, 0, st,
-                    (const RNode*)nodes.get(), level[d], level[d + 1], V, nV, F, order,
-                    (const uint32_t*)nslots.get(), (const uint32_t*)nitems.get(),
-                    (const uint32_t*)slot.get(), (const uint32_t*)ibase.get(), L32.get(),
-                    L64.get(), s.nf.get(), s.nd.get(),
-                    s.tf.get(), s.td.get(), s.tri_index.get());
-    launch_kernel(export_tree_kernel, blocks_for(nn), 256, 0, st, (const RNode*)nodes.get(), nn,
-                  (const uint32_t*)pre.get(), s.ref_child.get());
-    Loc<double> root;
-    GWN_CUDA(cudaMemcpyAsync(&root, L64.get(), sizeof(root), cudaMemcpyDeviceToHost, st));
-    GWN_CUDA(cudaStreamSynchronize(st));
+    DevBuf<uint4> kid(nn, st);
+    DevBuf<uint2> slots(nn, st);
+    DevBuf<uint32_t> item_slot(m, st);
+    uint4* child = reinterpret_cast<uint4*>(s.ref_child.get());
+    launch_kernel(sub_emit_kernel, nsub, 128, 0, st, (const SubRoot*)subs.get(),
+                  (const SubTotals*)totals.get(), (const Place*)sub_place.get(),
+                  (const SubNode*)sn.get(), (const uint32_t*)idx.get(), child, kid.get(),
+                  slots.get(), s.tri_index.get(), item_slot.get());
+    if (ntop)
+      launch_kernel(top_emit_kernel, blocks_for(ntop, 128), 128, 0, st, (const RNode*)nodes.get(),
+                    ntop, (const Place*)size.get(), (const Place*)place.get(),
+                    (const SubRoot*)subs.get(), (const SubTotals*)totals.get(),
+                    (const Place*)sub_place.get(), child, kid.get(), slots.get(),
+                    s.tri_index.get(), item_slot.get());
+    DevBuf<Loc<float>> L32((size_t)total_slots, st);
+    DevBuf<Loc<double>> L64((size_t)total_slots, st);
+    launch_kernel(items_kernel, blocks_for(m, 128), 128, 0, st, (int64_t)m,
+                  (const int32_t*)s.tri_index.get(), (const uint32_t*)item_slot.get(), V, nV, F,
+                  order, L32.get(), L64.get(), s.nf.get(), s.nd.get(), s.tf.get(), s.td.get(),
+                  bc.get());
+    const MergeArgs ma{kid.get(), slots.get(), m,           order,   L32.get(),
+                       L64.get(), s.nf.get(),  s.nd.get(), bc.get()};
+    launch_kernel(sub_merge_kernel, nsub, 128, 0, st, ma, (const SubRoot*)subs.get(),
+                  (const SubTotals*)totals.get(), (const Place*)sub_place.get(),
+                  (const SubNode*)sn.get(), (const uint16_t*)lev.get());
+    for (int d = top_depths - 1; d >= 0; --d)
+      launch_kernel(top_merge_kernel, blocks_for(level[d + 1] - level[d], 128), 128, 0, st, ma,
+                    (const Place*)place.get(), level[d], level[d + 1]);
+    double* root = reinterpret_cast<double*>(pinned_words() + 32);
+    GWN_CUDA(cudaMemcpyAsync(root, L64.get() + m, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    read_counts();
+    s.moments_bounded = hbc->unbounded == 0;
     double diag2 = 0, cmax = 0;
-    for (int d = 0; d < 3; ++d) {
-      s.lo[d] = root.lo[d];
-      s.hi[d] = root.hi[d];
-      const double e = root.hi[d] - root.lo[d];
+    for (int d = 0; d < 3; ++d) {  // Loc starts with the box
+      s.lo[d] = root[d];
+      s.hi[d] = root[3 + d];
+      const double e = s.hi[d] - s.lo[d];
       diag2 += e * e;
-      cmax = fmax(cmax, fmax(fabs(root.lo[d]), fabs(root.hi[d])));
+      cmax = fmax(cmax, fmax(fabs(s.lo[d]), fabs(s.hi[d])));
     }
     s.eps = kNearFrac * sqrt(diag2);
     s.cmax = cmax;
   }
-  soup_check_moments(s, st);
   if (host_mode) status.check(st, "soup_build");
   s.bytes = s.nf.bytes() + s.nd.bytes() + s.tf.bytes() + s.td.bytes() + s.tri_index.bytes() +
             s.ref_child.bytes();
