@@ -167,3 +167,18 @@ def test_query_on_a_point_gives_half_dipole(cuda):
     for prec in ("fp64", "mixed"):
         W = G.fast_winding_number_cloud_oneshot(P, Nn, A, Q, 2, 2.0, precision=prec)
         assert np.abs(W - Wref).max() <= 1e-12
+
+
+@pytest.mark.parametrize("gap", [2.0 ** -19, 2.0 ** -21, 2.0 ** -23, 2.0 ** -45, 2.0 ** -70])
+@pytest.mark.parametrize("m", [2, 3, 31, 33, 40])
+def test_octree_close_points(cuda, m, gap):
+    """Clusters of m points `gap` apart in a unit cube: paths that agree in
+    fewer, exactly and more octants than a 21-octant sort key holds, runs of
+    equal keys below and above the length one thread orders, and points too
+    close for the sorted build (2^-70 around the origin)."""
+    rng = np.random.default_rng(m)
+    centre = np.zeros(3) if gap < 2.0 ** -52 else rng.random(3)
+    cluster = centre + rng.random((m, 3)) * gap
+    P = np.concatenate([rng.random((200, 3)), cluster, rng.random((50, 3)) - 0.5])
+    assert_octree_equal(P[rng.permutation(P.shape[0])])
+    assert_octree_equal(cluster)
