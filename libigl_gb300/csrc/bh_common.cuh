@@ -82,6 +82,77 @@ __device__ __forceinline__ bool in_guard_band(float r2, float thr, float sigma) 
   return fabsf(r2 - thr) <= fmaf(2e-5f, r2 + thr, sigma);
 }
 __host__ __device__ inline float guard_sigma(float S) { return 2e-8f * S * S; }
+
+// ------------------------------------------------------------ team walks --
+// Small batches.  The warp-coherent walk needs about 150 dependent steps (a
+// node record's latency each) per warp however few queries there are, and
+// more when 32 neighbouring queries are far apart, so a batch that does not
+// fill the GPU is bound by that chain.  Here T lanes share one query: an item
+// is a range of pre-order slots [c, e) that its lane walks without a stack
+// (an opened node moves to c + 1, any other to its link); a lane that opens
+// a node with siblings after it leaves them as a new item on the team's
+// stack in shared memory, from which idle lanes take the newest.  A full
+// stack only means that the lane keeps the siblings itself.  Items go to
+// lanes in lane order, so the terms each lane adds, and the butterfly sum of
+// the lanes at the end, depend on the query alone.
+// The slots visited and the terms are the warp-coherent walk's; their order
+// of summation is not.
+constexpr int kTeamStack = 128;  // items per warp, shared by its 32 / T teams
+
+struct Team {
+  int2* stk;          // this team's items
+  unsigned mask, lt;  // lanes of the team; lanes below this one
+  int cap;            // of stk
+  int c = 0, e = 0, sp = 0;
+
+  __device__ __forceinline__ Team(int T, int2* warp_stack, bool valid, int nnodes) {
+    const int lane = threadIdx.x & 31;
+    cap = kTeamStack * T / 32;
+    stk = warp_stack + (lane / T) * cap;
+    mask = (0xffffffffu >> (32 - T)) << (lane & ~(T - 1));
+    lt = (1u << lane) - 1u;
+    if (valid && (lane & (T - 1)) == 0) {
+      c = nnodes > 1 ? 1 : 0;  // an internal root is always opened
+      e = nnodes;
+    }
+  }
+  // Idle lanes take items; false once no lane of the warp has work.
+  __device__ __forceinline__ bool take() {
+    __syncwarp();
+    const unsigned idle = __ballot_sync(0xffffffffu, c >= e) & mask;
+    const int rank = __popc(idle & lt);
+    if (c >= e && rank < sp) {
+      const int2 it = stk[sp - 1 - rank];
+      c = it.x;
+      e = it.y;
+    }
+    sp -= min(sp, __popc(idle));
+    __syncwarp();
+    return __any_sync(0xffffffffu, c < e);
+  }
+  // Moves past the current slot: into it (open) or to `next`, the slot after
+  // its subtree.
+  __device__ __forceinline__ void advance(bool act, bool open, int next) {
+    const bool push = act && open && next < e;
+    const unsigned m = __ballot_sync(0xffffffffu, push) & mask;
+    const bool room = sp + __popc(m) <= cap;
+    if (act) {
+      if (push && room) {
+        stk[sp + __popc(m & lt)] = make_int2(next, e);
+        e = next;
+      }
+      c = open ? c + 1 : next;
+    }
+    if (room) sp += __popc(m);
+  }
+};
+
+template <typename V>
+__device__ __forceinline__ V team_sum(V v, int T) {
+  for (int o = T >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 #endif
 
 }  // namespace gwn

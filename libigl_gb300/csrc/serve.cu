@@ -77,6 +77,8 @@ struct __align__(16) ServeReq {
   int32_t nq;
   int32_t q_f64;
   int32_t precision;
+  int32_t ordered;      // OrderedSum (a call of its size shares queries between lanes)
+  int32_t pad[3];
 };
 
 struct __align__(16) ServeHeader {
@@ -214,13 +216,21 @@ __global__ void __launch_bounds__(128, 8) serve_walk_kernel(ServeHeader* __restr
     const EvalParams prm = R.prm;
     double w;
     if (R.precision == GWN_MIXED) {
-      float acc;
       double acc64;
       soupwalk::WalkCounters c;
-      // every served tree is of the default kind (the builder below)
-      soupwalk::walk_mixed<false, GWN_SOUP_TREE_DEFAULT>(prm, valid, qx, qy, qz, acc, acc64, c,
-                                                         warp_q[threadIdx.x >> 5].near);
-      w = soupwalk::mixed_result(acc, acc64);
+      // every served tree is of the default kind (the builder below); the
+      // kind of sum is that of the request's own call
+      if (R.ordered) {
+        soupwalk::OrderedSum acc;
+        soupwalk::walk_mixed<false, GWN_SOUP_TREE_DEFAULT>(prm, valid, qx, qy, qz, acc, acc64, c,
+                                                           warp_q[threadIdx.x >> 5].near);
+        w = soupwalk::mixed_result(acc, acc64);
+      } else {
+        soupwalk::PlainSum acc;
+        soupwalk::walk_mixed<false, GWN_SOUP_TREE_DEFAULT>(prm, valid, qx, qy, qz, acc, acc64, c,
+                                                           warp_q[threadIdx.x >> 5].near);
+        w = soupwalk::mixed_result(acc, acc64);
+      }
       if (valid && fabs(w - 0.5) <= soupwalk::kBand) {
         const unsigned s = atomicAdd(&counters[1], 1u);
         refine[s] = make_int2(r, j);
@@ -680,6 +690,7 @@ bool gwn_server::form_and_launch(SrvSlot& s, std::unique_lock<std::mutex>& lk) {
     d.prm.status = nullptr;
     d.prm.ref32 = t.tree == GWN_TREE_REFERENCE;
     d.prm.fp64_queue = t.moments_bounded;
+    d.ordered = soup_team_size(r->nq, t.nnodes, r->precision) > 1;
     for (int k = 0; k < 3; ++k) {
       // the query box: the mesh box grown by a quarter on each side
       const double e = std::max(t.hi[k] - t.lo[k], 1e-30);

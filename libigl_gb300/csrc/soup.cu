@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(128, 8) soup_eval_mixed_kernel(EvalParams prm,
   double qx = 0, qy = 0, qz = 0;
   if (valid) soupwalk::read_query(Q, perm, (const int32_t*)nullptr, i, qi, qx, qy, qz);
   __shared__ soupwalk::NearQueue near_q[4];
-  float acc;
+  soupwalk::PlainSum acc;
   double acc64;
   soupwalk::WalkCounters c;
   soupwalk::walk_mixed<kStats, kTree>(prm, valid, qx, qy, qz, acc, acc64, c,
@@ -485,20 +485,20 @@ __global__ void __launch_bounds__(128) soup_eval_fp64_kernel(EvalParams prm,
 
 // The same two evaluations with T lanes per query (soup_walk.cuh, team
 // walks), for batches too small to fill the GPU with 32 queries per warp.
-template <typename QT, typename WT, int T, int kTree>
+template <typename QT, typename WT, int kTree>
 __global__ void __launch_bounds__(128, 7) soup_team_mixed_kernel(
-    EvalParams prm, const QT* __restrict__ Q, const int32_t* __restrict__ perm, int64_t nQ,
+    EvalParams prm, int T, const QT* __restrict__ Q, const int32_t* __restrict__ perm, int64_t nQ,
     WT* __restrict__ W, int32_t* __restrict__ refine_list, unsigned* __restrict__ refine_count) {
   __shared__ soupwalk::NearQueue near_q[4];
-  __shared__ int2 s_stack[4][soupwalk::kTeamStack];
+  __shared__ int2 s_stack[4][kTeamStack];
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / T;
   const bool valid = i < nQ;
   int64_t qi = 0;
   double qx = 0, qy = 0, qz = 0;
   if (valid) soupwalk::read_query(Q, perm, (const int32_t*)nullptr, i, qi, qx, qy, qz);
-  float acc;
+  soupwalk::OrderedSum acc;
   double acc64;
-  soupwalk::walk_mixed_team<T, kTree>(prm, valid, qx, qy, qz, acc, acc64,
+  soupwalk::walk_mixed_team<kTree>(prm, T, valid, qx, qy, qz, acc, acc64,
                                       near_q[threadIdx.x >> 5], s_stack[threadIdx.x >> 5]);
   if (!valid || (threadIdx.x & (T - 1))) return;
   const double w = soupwalk::mixed_result(acc, acc64);
@@ -509,15 +509,15 @@ __global__ void __launch_bounds__(128, 7) soup_team_mixed_kernel(
   }
 }
 
-template <typename QT, typename WT, int T>
-__global__ void __launch_bounds__(128) soup_team_fp64_kernel(EvalParams prm,
+template <typename QT, typename WT>
+__global__ void __launch_bounds__(128) soup_team_fp64_kernel(EvalParams prm, int T,
                                                              const QT* __restrict__ Q,
                                                              const int32_t* __restrict__ perm,
                                                              const int32_t* __restrict__ list,
                                                              const unsigned* __restrict__ list_count,
                                                              int64_t nQ, WT* __restrict__ W) {
   __shared__ soupwalk::Fp64Queue fp64_q[4];
-  __shared__ int2 s_stack[4][soupwalk::kTeamStack];
+  __shared__ int2 s_stack[4][kTeamStack];
   const int64_t n = list ? (int64_t)*list_count : nQ;
   const int64_t per_warp = 32 / T;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -528,9 +528,9 @@ __global__ void __launch_bounds__(128) soup_team_fp64_kernel(EvalParams prm,
     int64_t qi = 0;
     double qx = 0, qy = 0, qz = 0;
     if (valid) soupwalk::read_query(Q, perm, list, i, qi, qx, qy, qz);
-    const double acc = soupwalk::walk_fp64_team<T>(prm, valid, qx, qy, qz,
-                                                   fp64_q[threadIdx.x >> 5],
-                                                   s_stack[threadIdx.x >> 5]);
+    const double acc = soupwalk::walk_fp64_team(prm, T, valid, qx, qy, qz,
+                                                fp64_q[threadIdx.x >> 5],
+                                                s_stack[threadIdx.x >> 5]);
     if (valid && !(threadIdx.x & (T - 1))) W[qi] = (WT)(acc * kInv4Pi);
     __syncwarp();
   }
@@ -676,7 +676,7 @@ void soup_build(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t* F,
 }
 
 // ------------------------------------------------------------------- eval --
-// Lanes per query.  Teams win while 32 queries per warp leave the GPU waiting
+// Teams win while 32 queries per warp leave the GPU waiting
 // for its longest walks; the warp-coherent walk reads each record once per
 // warp and wins once there are queries enough, the later the more slots the
 // tree has (sparser queries share fewer of them).  Measured crossings, mixed:
@@ -686,7 +686,7 @@ void soup_build(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t* F,
 // 41 / 60 / 97 / 908; 60k 355 / 264 / 288 / 1344; 600k 2202 / 1060 / 973 /
 // 1480; 2M - / 2968 / 2577 / 2335.  FP64: 1,000 120 / 237 / 376 / 2582;
 // 60k 1868 / 1940 / 2294 / 5309; 200k 5746 / 5408 / 5914 / 7485.
-static int team_size(int64_t nQ, int64_t slots, int precision) {
+int soup_team_size(int64_t nQ, int64_t slots, int precision) {
   const double cross = 65536.0 + 1024.0 * std::sqrt((double)slots);
   if (precision == GWN_MIXED)
     return nQ <= 4096 ? 32 : (double)nQ > cross ? 1 : nQ <= 200000 ? 8 : 4;
@@ -725,7 +725,7 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
   }
   const int32_t* perm = qo.active ? qo.perm.get() : nullptr;
   const unsigned grid = (unsigned)((nQ + 127) / 128);
-  const int team = team_size(nQ, s.nnodes, precision);
+  const int team = soup_team_size(nQ, s.nnodes, precision);
   auto team_grid = [&](int t) { return (unsigned)((nQ * t + 127) / 128); };
   const bool ref = prm.ref32 != 0;
   if (precision == GWN_MIXED) {
@@ -742,13 +742,9 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
         launch_kernel(kernel, grid, 128, 0, st, prm, Q, perm, nQ, W, list.get(), count.get(),
                       (unsigned long long*)nullptr);
       } else {
-        auto kernel = team == 32 ? (ref ? soup_team_mixed_kernel<QT, WT, 32, GWN_TREE_REFERENCE>
-                                        : soup_team_mixed_kernel<QT, WT, 32, GWN_TREE_BINNED>)
-                      : team == 8 ? (ref ? soup_team_mixed_kernel<QT, WT, 8, GWN_TREE_REFERENCE>
-                                         : soup_team_mixed_kernel<QT, WT, 8, GWN_TREE_BINNED>)
-                                  : (ref ? soup_team_mixed_kernel<QT, WT, 4, GWN_TREE_REFERENCE>
-                                         : soup_team_mixed_kernel<QT, WT, 4, GWN_TREE_BINNED>);
-        launch_kernel(kernel, team_grid(team), 128, 0, st, prm, Q, perm, nQ, W, list.get(),
+        auto kernel = ref ? soup_team_mixed_kernel<QT, WT, GWN_TREE_REFERENCE>
+                          : soup_team_mixed_kernel<QT, WT, GWN_TREE_BINNED>;
+        launch_kernel(kernel, team_grid(team), 128, 0, st, prm, team, Q, perm, nQ, W, list.get(),
                       count.get());
       }
     }
@@ -756,7 +752,7 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
       // a few queries near the threshold, anywhere: a warp each
       PhaseTimer ph("refine", st);
       const unsigned rgrid = (unsigned)std::min<int64_t>((nQ + 3) / 4, 8 * num_sms());
-      launch_kernel(soup_team_fp64_kernel<QT, WT, 32>, rgrid, 128, 0, st, prm, Q,
+      launch_kernel(soup_team_fp64_kernel<QT, WT>, rgrid, 128, 0, st, prm, 32, Q,
                     (const int32_t*)nullptr, (const int32_t*)list.get(),
                     (const unsigned*)count.get(), nQ, W);
     }
@@ -765,8 +761,8 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
     if (team == 1) {
       launch_kernel(soup_eval_fp64_kernel<QT, WT>, grid, 128, 0, st, prm, Q, perm, nQ, W);
     } else {
-      auto kernel = team == 32 ? soup_team_fp64_kernel<QT, WT, 32> : soup_team_fp64_kernel<QT, WT, 8>;
-      launch_kernel(kernel, team_grid(team), 128, 0, st, prm, Q, perm, (const int32_t*)nullptr,
+      launch_kernel(soup_team_fp64_kernel<QT, WT>, team_grid(team), 128, 0, st, prm, team, Q, perm,
+                    (const int32_t*)nullptr,
                     (const unsigned*)nullptr, nQ, W);
     }
   }

@@ -241,6 +241,52 @@ __device__ __forceinline__ void flush_near64(const double* __restrict__ td, Near
   __syncwarp();
 }
 
+// A query's FP32 sum.  PlainSum adds in the order of the walk.  OrderedSum's
+// result does not depend on the order of its terms, so that a walk by a team
+// of lanes and a warp-coherent walk of the same query return the same value:
+// every term is split exactly into a multiple of 2^-12 and a rest, the rest
+// rounded to a multiple of 2^-30, and both are summed as integers.  Adding
+// 1.5 * 2^23 units makes a float's low bits that integer.  Five operations
+// more than a plain sum, and a smaller rounding error (2^-31 per term; a
+// plain sum of a few turns loses up to 2^-22 per addition).
+// add() is false for a term outside +-512 (or NaN), which the caller takes in
+// FP64.  fold() carries the small units, which would overflow after 2^14 equal
+// terms; leaf terms, which repeat for repeated triangles, call it.
+struct PlainSum {
+  static constexpr bool kBounded = false;  // refuses only what is not finite
+  float s = 0.f;
+  __device__ __forceinline__ bool add(float v) {
+    if (!isfinite(v)) return false;
+    s += v;
+    return true;
+  }
+  __device__ __forceinline__ void add_leaf(float v, double&) { s += v; }
+};
+struct OrderedSum {
+  static constexpr bool kBounded = true;
+  int hi = 0, lo = 0;  // units of 2^-12 and 2^-30
+  __device__ __forceinline__ bool add(float v) {
+    if (!(fabsf(v) < 512.f)) return false;
+    const float t = __fadd_rn(v, 3072.f);  // 1.5 * 2^11: units of 2^-12
+    const float r = __fsub_rn(v, __fsub_rn(t, 3072.f));
+    const float u = __fadd_rn(r, 0.01171875f);  // 1.5 * 2^-7: units of 2^-30
+    hi += __float_as_int(t) - 0x45400000;
+    lo += __float_as_int(u) - 0x3c400000;
+    return true;
+  }
+  __device__ __forceinline__ void fold() {
+    hi += lo >> 18;
+    lo &= (1 << 18) - 1;
+  }
+  __device__ __forceinline__ void add_leaf(float v, double& acc64) {
+    if (add(v)) fold();
+    else acc64 += (double)v;
+  }
+  __device__ __forceinline__ double value() const {
+    return (double)(((long long)hi << 18) + lo) * 9.31322574615478515625e-10;  // 2^-30
+  }
+};
+
 // Work counters of the instrumented walk (only touched when kStats).
 struct WalkCounters {
   unsigned long long steps = 0, visits = 0, far = 0, exact32 = 0, exact64 = 0, recheck = 0;
@@ -254,9 +300,9 @@ struct WalkCounters {
 // solid-angle sum as an FP32 part and an FP64 part.  kTree: the tree kind
 // (GWN_TREE_REFERENCE / GWN_TREE_BINNED) when known at compile time, -1 to
 // read it from prm.ref32.
-template <bool kStats, int kTree = -1>
+template <bool kStats, int kTree = -1, typename Sum = PlainSum>
 __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, double qx, double qy,
-                                           double qz, float& acc, double& acc64,
+                                           double qz, Sum& acc, double& acc64,
                                            WalkCounters& c, NearQueue& nq) {
   const int lane = threadIdx.x & 31;
   nq.q[lane][0] = qx;
@@ -269,7 +315,7 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
   const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
   const float S = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + prm.cmax;
   const float sigma = guard_sigma(S);
-  acc = 0.f;
+  acc = Sum();
   acc64 = 0.0;
   int resume = valid ? 0 : 0x7fffffff;
   int node = 0;
@@ -315,8 +361,10 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
         if (!near) {
           if (kStats) ++c.far;
           const float om = far_field32(rb, rc, rd, re, rf, dx, dy, dz, r2, prm.order);
-          if (isfinite(om)) {
-            acc += om;
+          if (acc.add(om)) {
+            resume = leaf ? node + 1 : link;
+          } else if (Sum::kBounded && isfinite(om)) {
+            acc64 += (double)om;
             resume = leaf ? node + 1 : link;
           } else {
             near = true;
@@ -335,8 +383,10 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
               const float4 t0 = __ldg(&prm.tf[(int64_t)slot * 3]);
               const float4 t1 = __ldg(&prm.tf[(int64_t)slot * 3 + 1]);
               const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
-              acc += tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx, t1.x - fy,
-                                            t1.y - fz, t1.z - fx, t1.w - fy, t2.x - fz);
+              acc.add_leaf(tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx,
+                                                  t1.x - fy, t1.y - fz, t1.z - fx, t1.w - fy,
+                                                  t2.x - fz),
+                           acc64);
             }
             resume = node + 1;
           } else {
@@ -368,8 +418,11 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
 }
 
 // Winding number from the two parts of walk_mixed.
-__device__ __forceinline__ double mixed_result(float acc, double acc64) {
-  return acc64 != 0.0 ? ((double)acc + acc64) * kInv4Pi : (double)(acc * kInv4PiF);
+__device__ __forceinline__ double mixed_result(const PlainSum& acc, double acc64) {
+  return acc64 != 0.0 ? ((double)acc.s + acc64) * kInv4Pi : (double)(acc.s * kInv4PiF);
+}
+__device__ __forceinline__ double mixed_result(const OrderedSum& acc, double acc64) {
+  return (acc.value() + acc64) * kInv4Pi;
 }
 
 // Per-warp queue of the plain FP64 walk's terms.  The FP64 pipe charges a
@@ -507,81 +560,12 @@ __device__ __forceinline__ double walk_fp64(const EvalParams& prm, bool valid, d
 }
 
 // ------------------------------------------------------------ team walks --
-// Small batches.  The warp-coherent walk needs about 150 dependent steps (a
-// node record's latency each) per warp however few queries there are, and
-// more when 32 neighbouring queries are far apart, so a batch that does not
-// fill the GPU is bound by that chain.  Here T lanes share one query: an item
-// is a range of pre-order slots [c, e) that its lane walks without a stack
-// (an opened node moves to c + 1, any other to its link); a lane that opens
-// a node with siblings after it leaves them as a new item on the team's
-// stack in shared memory, from which idle lanes take the newest.  A full
-// stack only means that the lane keeps the siblings itself.  Items go to
-// lanes in lane order, so the terms each lane adds, and the butterfly sum of
-// the lanes at the end, depend on the query alone.
-// The slots visited and the terms are the warp-coherent walk's; their order
-// of summation is not.
-constexpr int kTeamStack = 128;  // items per warp, shared by its 32 / T teams
-
-template <int T>
-struct Team {
-  int2* stk;          // this team's items
-  unsigned mask, lt;  // lanes of the team; lanes below this one
-  int c = 0, e = 0, sp = 0;
-  static constexpr int kCap = kTeamStack * T / 32;
-
-  __device__ __forceinline__ Team(int2* warp_stack, bool valid, int nnodes) {
-    const int lane = threadIdx.x & 31;
-    stk = warp_stack + (lane / T) * kCap;
-    mask = T == 32 ? 0xffffffffu : ((1u << (T & 31)) - 1u) << (lane & ~(T - 1));
-    lt = (1u << lane) - 1u;
-    if (valid && (lane & (T - 1)) == 0) {
-      c = nnodes > 1 ? 1 : 0;  // an internal root is always opened
-      e = nnodes;
-    }
-  }
-  // Idle lanes take items; false once no lane of the warp has work.
-  __device__ __forceinline__ bool take() {
-    __syncwarp();
-    const unsigned idle = __ballot_sync(0xffffffffu, c >= e) & mask;
-    const int rank = __popc(idle & lt);
-    if (c >= e && rank < sp) {
-      const int2 it = stk[sp - 1 - rank];
-      c = it.x;
-      e = it.y;
-    }
-    sp -= min(sp, __popc(idle));
-    __syncwarp();
-    return __any_sync(0xffffffffu, c < e);
-  }
-  // Moves past the current slot: into it (open) or to `next`, the slot after
-  // its subtree.
-  __device__ __forceinline__ void advance(bool act, bool open, int next) {
-    const bool push = act && open && next < e;
-    const unsigned m = __ballot_sync(0xffffffffu, push) & mask;
-    const bool room = sp + __popc(m) <= kCap;
-    if (act) {
-      if (push && room) {
-        stk[sp + __popc(m & lt)] = make_int2(next, e);
-        e = next;
-      }
-      c = open ? c + 1 : next;
-    }
-    if (room) sp += __popc(m);
-  }
-};
-
-template <typename V>
-__device__ __forceinline__ V team_sum(V v, int T) {
-  for (int o = T >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// walk_mixed for teams of T lanes (every lane of a team passes the team's
-// query); every lane returns the query's sums.
-template <int T, int kTree>
-__device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, bool valid, double qx,
-                                                double qy, double qz, float& acc, double& acc64,
-                                                NearQueue& nq, int2* warp_stack) {
+// walk_mixed for teams of T lanes, T a power of two from 2 to 32 (every lane
+// of a team passes the team's query); every lane returns the query's sums.
+template <int kTree>
+__device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, int T, bool valid,
+                                                double qx, double qy, double qz, OrderedSum& acc,
+                                                double& acc64, NearQueue& nq, int2* warp_stack) {
   const int lane = threadIdx.x & 31;
   nq.q[lane][0] = qx;
   nq.q[lane][1] = qy;
@@ -592,9 +576,9 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, bool vali
   const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
   const float S = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + prm.cmax;
   const float sigma = guard_sigma(S);
-  acc = 0.f;
+  acc = OrderedSum();
   acc64 = 0.0;
-  Team<T> team(warp_stack, valid, prm.nnodes);
+  Team team(T, warp_stack, valid, prm.nnodes);
   while (team.take()) {
     const bool act = team.c < team.e;
     bool open = false, want64 = false;
@@ -626,8 +610,10 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, bool vali
       }
       if (!near) {
         const float om = far_field32(rb, rc, rd, re, rf, dx, dy, dz, r2, prm.order);
-        if (isfinite(om)) acc += om;
-        else near = true;
+        if (!acc.add(om)) {
+          if (isfinite(om)) acc64 += (double)om;
+          else near = true;
+        }
       }
       if (near) {
         if (leaf) {
@@ -640,8 +626,10 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, bool vali
             const float4 t0 = __ldg(&prm.tf[(int64_t)slot * 3]);
             const float4 t1 = __ldg(&prm.tf[(int64_t)slot * 3 + 1]);
             const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
-            acc += tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx, t1.x - fy,
-                                          t1.y - fz, t1.z - fx, t1.w - fy, t2.x - fz);
+            acc.add_leaf(tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx,
+                                                t1.x - fy, t1.y - fz, t1.z - fx, t1.w - fy,
+                                                t2.x - fz),
+                         acc64);
           }
         } else {
           open = true;
@@ -666,14 +654,15 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, bool vali
     team.advance(act, open, next);
   }
   if (nqueued) flush_near64(prm.td, nq, nqueued, mine, acc64);
-  acc = team_sum(acc, T);
+  acc.fold();
+  acc.hi = team_sum(acc.hi, T);
+  acc.lo = team_sum(acc.lo, T);
   acc64 = team_sum(acc64, T);
 }
 
 // walk_fp64 for teams of T lanes.
-template <int T>
-__device__ __forceinline__ double walk_fp64_team(const EvalParams& prm, bool valid, double qx,
-                                                 double qy, double qz, Fp64Queue& fq,
+__device__ __forceinline__ double walk_fp64_team(const EvalParams& prm, int T, bool valid,
+                                                 double qx, double qy, double qz, Fp64Queue& fq,
                                                  int2* warp_stack) {
   const int lane = threadIdx.x & 31;
   fq.q[lane][0] = qx;
@@ -683,7 +672,7 @@ __device__ __forceinline__ double walk_fp64_team(const EvalParams& prm, bool val
   double acc = 0.0;
   int nq = 0;         // warp-uniform
   unsigned mine = 0;  // this lane's queue positions
-  Team<T> team(warp_stack, valid, prm.nnodes);
+  Team team(T, warp_stack, valid, prm.nnodes);
   while (team.take()) {
     const bool act = team.c < team.e;
     bool open = false, push = false;
