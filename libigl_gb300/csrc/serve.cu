@@ -116,51 +116,62 @@ __device__ __forceinline__ uint32_t morton_cell7(double v, float lo, float inv) 
   return (uint32_t)min(max(c, 0), 127);
 }
 
+// Bound by the reads of the pinned host stage.  A warp takes 32 key positions
+// (of one request: padded sizes are multiples of 32) and reads their queries,
+// contiguous from a 16-byte boundary, as 16-byte words; one query per thread
+// and coordinate took 12-byte strides over the link (2.2M float32 queries:
+// 298 us of stage kernels).
 __global__ void __launch_bounds__(256) serve_stage_kernel(const ServeHeader* __restrict__ dh,
                                                           const ServeReq* __restrict__ dreq,
                                                           const unsigned char* hstage,
                                                           double* __restrict__ dq,
                                                           uint32_t* __restrict__ keys,
                                                           int32_t* __restrict__ vals) {
+  __shared__ uint4 s_raw[8][48];
   const uint32_t na = dh->n_aligned;
   const int nreq = (int)dh->nreq;
-  for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
-    int lo = 0, hi = nreq - 1;  // last request with aoff <= a
+  const int lane = threadIdx.x & 31;
+  uint4* raw = s_raw[threadIdx.x >> 5];
+  for (uint32_t a0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; a0 < na;
+       a0 += gridDim.x * blockDim.x) {
+    int lo = 0, hi = nreq - 1;  // last request with aoff <= a0
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (dreq[mid].aoff <= (int)a) lo = mid;
+      if (dreq[mid].aoff <= (int)a0) lo = mid;
       else hi = mid - 1;
     }
     const ServeReq& R = dreq[lo];
-    const int j = (int)a - R.aoff;
+    const int j0 = (int)a0 - R.aoff;
+    const int cnt = max(0, min(32, R.nq - j0));
+    const int size = R.q_f64 ? 24 : 12;
+    const volatile uint4* src =
+        reinterpret_cast<const volatile uint4*>(hstage + R.q_byte_off + (int64_t)j0 * size);
+    // the stage pads every request to 16 bytes
+    for (int v = lane; v < (cnt * size + 15) / 16; v += 32) {
+      uint4 w;
+      asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                   : "l"(src + v));
+      raw[v] = w;
+    }
+    __syncwarp();
+    auto coord = [&](int k) {
+      return R.q_f64 ? reinterpret_cast<const double*>(raw)[k]
+                     : (double)reinterpret_cast<const float*>(raw)[k];
+    };
+    double* d = dq + 3 * (R.out_off + j0);
+    for (int k = lane; k < 3 * cnt; k += 32) d[k] = coord(k);
     uint32_t key = (uint32_t)lo << 24;
-    if (j < R.nq) {
-      double x, y, z;
-      if (R.q_f64) {
-        const volatile double* p =
-            reinterpret_cast<const volatile double*>(hstage + R.q_byte_off) + 3 * (int64_t)j;
-        x = p[0];
-        y = p[1];
-        z = p[2];
-      } else {
-        const volatile float* p =
-            reinterpret_cast<const volatile float*>(hstage + R.q_byte_off) + 3 * (int64_t)j;
-        x = (double)p[0];
-        y = (double)p[1];
-        z = (double)p[2];
-      }
-      double* d = dq + 3 * (R.out_off + j);
-      d[0] = x;
-      d[1] = y;
-      d[2] = z;
-      key |= spread10(morton_cell7(x, R.lo[0], R.inv[0])) |
-             (spread10(morton_cell7(y, R.lo[1], R.inv[1])) << 1) |
-             (spread10(morton_cell7(z, R.lo[2], R.inv[2])) << 2);
+    if (lane < cnt) {
+      key |= spread10(morton_cell7(coord(3 * lane), R.lo[0], R.inv[0])) |
+             (spread10(morton_cell7(coord(3 * lane + 1), R.lo[1], R.inv[1])) << 1) |
+             (spread10(morton_cell7(coord(3 * lane + 2), R.lo[2], R.inv[2])) << 2);
     } else {
       key |= 1u << 23;  // padding lanes sort after the request's queries
     }
-    keys[a] = key;
-    vals[a] = (int32_t)a;
+    keys[a0 + lane] = key;
+    vals[a0 + lane] = (int32_t)(a0 + lane);
+    __syncwarp();
   }
 }
 
