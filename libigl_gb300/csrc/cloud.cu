@@ -855,50 +855,49 @@ __global__ void __launch_bounds__(128) cloud_eval_fp64_kernel(CloudEvalParams pr
 }
 
 // FP64 re-evaluation of the listed queries (results within the band of
-// 0.5), one warp per query: the lanes share the query's walk (the listed
-// queries lie anywhere on the surface, so a warp of 32 of them would walk
-// the union of 32 walks); a leaf's dipoles are split over the lanes, a far
-// cell's expansion is evaluated by one lane, and the lanes' sums are added
-// at the end.
+// 0.5), one warp per query, its lanes a team (bh_common.cuh): the listed
+// queries lie anywhere on the surface, so 32 of them would walk the union of
+// 32 walks, and one node at a time a query's walk is a chain of about a
+// thousand FP64 tests (2M points, 230 queries: 1335 us that way).
 template <typename QT, typename WT>
-__global__ void __launch_bounds__(128) cloud_refine_warp_kernel(CloudEvalParams prm,
-                                                                const QT* __restrict__ Q,
-                                                                const int32_t* __restrict__ list,
-                                                                const unsigned* __restrict__ count,
-                                                                WT* __restrict__ W) {
+__global__ void __launch_bounds__(128) cloud_refine_kernel(CloudEvalParams prm,
+                                                           const QT* __restrict__ Q,
+                                                           const int32_t* __restrict__ list,
+                                                           const unsigned* __restrict__ count,
+                                                           WT* __restrict__ W) {
+  __shared__ int2 s_stack[4][kTeamStack];
   const unsigned n = *count;
-  const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < (int64_t)n;
        w += nwarps) {
     const int64_t qi = list[w];
     const double qx = (double)Q[qi * 3], qy = (double)Q[qi * 3 + 1], qz = (double)Q[qi * 3 + 2];
     double acc = 0.0;
-    int node = 0;
-    while (node < prm.nnodes) {
-      const CloudNodeD* r = prm.nd + node;
-      const int4 l = r->l;
-      if (l.w) {
-        for (int j = lane; j < l.z; j += 32) {
-          const double* pd = prm.pd + ((int64_t)l.y + j) * 6;
-          acc += dipole64(pd[0] - qx, pd[1] - qy, pd[2] - qz, pd[3], pd[4], pd[5]);
+    Team team(32, s_stack[threadIdx.x >> 5], true, prm.nnodes);
+    while (team.take()) {
+      const bool act = team.c < team.e;
+      bool open = false;
+      int next = 0;
+      if (act) {
+        const CloudNodeD* r = prm.nd + team.c;
+        const int4 l = r->l;
+        next = l.x;
+        if (l.w) {
+          for (int j = 0; j < l.z; ++j) {
+            const double* pd = prm.pd + ((int64_t)l.y + j) * 6;
+            acc += dipole64(pd[0] - qx, pd[1] - qy, pd[2] - qz, pd[3], pd[4], pd[5]);
+          }
+        } else if (far64(qx, qy, qz, r->cm, r->r, prm.beta)) {
+          acc += expansion_packed64(r->pk, __dsub_rn(r->cm[0], qx), __dsub_rn(r->cm[1], qy),
+                                    __dsub_rn(r->cm[2], qz), prm.num_terms);
+        } else {
+          open = true;
         }
-        node = l.x;
-      } else if (node == 0) {
-        node = 1;
-      } else if (far64(qx, qy, qz, r->cm, r->r, prm.beta)) {
-        if (lane == 0) {
-          const double lx = __dsub_rn(r->cm[0], qx), ly = __dsub_rn(r->cm[1], qy),
-                       lz = __dsub_rn(r->cm[2], qz);
-          acc += expansion_packed64(r->pk, lx, ly, lz, prm.num_terms);
-        }
-        node = l.x;
-      } else {
-        node = node + 1;
       }
+      team.advance(act, open, next);
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) W[qi] = (WT)acc;
+    acc = team_sum(acc, 32);
+    if ((threadIdx.x & 31) == 0) W[qi] = (WT)acc;
   }
 }
 
@@ -1304,7 +1303,7 @@ static void cloud_eval_t(const gwn_cloud_impl& c, double beta, const void* Qv, i
     GWN_CUDA(cudaGetLastError());
     {
       PhaseTimer ph("refine", st);
-      launch_kernel(cloud_refine_warp_kernel<QT, WT>, (unsigned)(num_sms() * 8), 128, 0, st, prm,
+      launch_kernel(cloud_refine_kernel<QT, WT>, (unsigned)(num_sms() * 8), 128, 0, st, prm,
                     Q, (const int32_t*)list.get(), (const unsigned*)count.get(), W);
     }
     GWN_CUDA(cudaGetLastError());
