@@ -110,6 +110,79 @@ cudaMemPool_t device_pool() {
   return g_pools[d];
 }
 
+namespace {
+// A device's handle memory: the pool and the stream its allocations and
+// releases are ordered on (nothing else runs there).  Kept for the process.
+struct HandlePool {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;
+};
+std::vector<HandlePool> g_handle_pools;  // per device
+
+HandlePool handle_pool(int d) {
+  std::lock_guard<std::mutex> lk(g_dev_mutex);
+  if ((int)g_handle_pools.size() <= d) g_handle_pools.resize(d + 1);
+  HandlePool& h = g_handle_pools[d];
+  if (!h.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = d;
+    size_t free_b = 0, total = 0;
+    GWN_CUDA(cudaMemGetInfo(&free_b, &total));
+    uint64_t keep = total / 16;
+    cudaMemPool_t pool = nullptr;
+    GWN_CUDA(cudaMemPoolCreate(&pool, &props));
+    GWN_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    if (!h.stream) GWN_CUDA(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
+    h.pool = pool;
+  }
+  return h;
+}
+}  // namespace
+
+void* handle_alloc(size_t bytes, int* device) {
+  const int d = current_device();
+  const HandlePool h = handle_pool(d);
+  void* p = nullptr;
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, h.pool, h.stream);
+  if (e == cudaErrorMemoryAllocation) {  // give back what the pools keep, once
+    cudaGetLastError();
+    GWN_CUDA(cudaDeviceSynchronize());
+    cudaMemPoolTrimTo(h.pool, 0);
+    cudaMemPoolTrimTo(device_pool(), 0);
+    e = cudaMallocFromPoolAsync(&p, bytes, h.pool, h.stream);
+  }
+  GWN_CUDA(e);
+  const cudaError_t w = cudaStreamSynchronize(h.stream);
+  if (w != cudaSuccess) {
+    cudaFreeAsync(p, h.stream);
+    GWN_CUDA(w);
+  }
+  *device = d;
+  return p;
+}
+
+void handle_free(void* p, int device) noexcept {
+  int cur = device;
+  if (cudaGetDevice(&cur) != cudaSuccess) cudaGetLastError();
+  if (cur != device) cudaSetDevice(device);
+  // a release must not overtake a stream that still reads the memory; where
+  // the device cannot be waited for (a capture in progress) it stays allocated,
+  // as with cudaFree
+  if (cudaDeviceSynchronize() == cudaSuccess) {
+    cudaStream_t st = nullptr;
+    {
+      std::lock_guard<std::mutex> lk(g_dev_mutex);
+      if ((int)g_handle_pools.size() > device) st = g_handle_pools[device].stream;
+    }
+    cudaFreeAsync(p, st);
+  } else {
+    cudaGetLastError();
+  }
+  if (cur != device) cudaSetDevice(cur);
+}
 
 int num_sms() {
   const int d = current_device();

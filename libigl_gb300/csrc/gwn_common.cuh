@@ -118,11 +118,21 @@ class DevBuf {
   cudaStream_t stream_ = nullptr;
 };
 
-// Persistent device allocation owned by a handle (cudaMalloc / cudaFree), so
-// its lifetime does not depend on any caller stream.  A structure that lives
-// for one call only can take its memory stream-ordered instead (ordered()
-// before alloc: cudaMallocFromPoolAsync / cudaFreeAsync on that stream), so
-// that neither the allocation nor the release synchronizes the device.
+// Device memory of handles, from a second pool per device that keeps up to
+// 1/16 of the device's memory mapped between handles (cudaMalloc and cudaFree
+// map and unmap it each time: 18 buffers of a 2M-point cloud 4.7 ms a call, 6
+// of an 81k-triangle soup 0.7 ms).  The memory is usable on every stream when
+// handle_alloc returns; handle_free waits for the device first, as cudaFree
+// does, so nothing that still runs can use it.  Both work from any thread and
+// with any device current.
+void* handle_alloc(size_t bytes, int* device);
+void handle_free(void* p, int device) noexcept;
+
+// Persistent device allocation owned by a handle, so its lifetime does not
+// depend on any caller stream.  A structure that lives for one call only can
+// take its memory stream-ordered instead (ordered() before alloc:
+// cudaMallocFromPoolAsync / cudaFreeAsync on that stream), so that neither the
+// allocation nor the release synchronizes the device.
 template <typename T>
 class DevMem {
  public:
@@ -144,14 +154,14 @@ class DevMem {
       GWN_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p_), n * sizeof(T), device_pool(),
                                        stream_));
     else
-      GWN_CUDA(cudaMalloc(reinterpret_cast<void**>(&p_), n * sizeof(T)));
+      p_ = static_cast<T*>(handle_alloc(n * sizeof(T), &device_));
   }
   void release() {
     if (p_) {
       if (ordered_)
         cudaFreeAsync(p_, stream_);
       else
-        cudaFree(p_);
+        handle_free(p_, device_);
     }
     p_ = nullptr;
     n_ = 0;
@@ -164,6 +174,7 @@ class DevMem {
   T* p_ = nullptr;
   size_t n_ = 0;
   bool ordered_ = false;
+  int device_ = 0;
   cudaStream_t stream_ = nullptr;
 };
 
