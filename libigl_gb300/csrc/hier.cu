@@ -54,7 +54,8 @@ namespace gwn {
 namespace {
 
 constexpr int kT = 256;
-constexpr int kMaxSplit = 8;  // subtrees walked in parallel when queries are few
+constexpr int kMaxSplit = 32;  // subtrees walked in parallel when queries are few (a lane of frontier_kernel each)
+constexpr int kWalk = 64;      // threads per CTA of the walks
 constexpr double kNearFrac = 1e-3;
 constexpr double kBand = 1e-3;
 constexpr double kInv2Pi = 0.15915494309189533577;
@@ -601,8 +602,36 @@ __device__ __forceinline__ void flush_hier64(const double* __restrict__ tris64,
   __syncwarp();
 }
 
+// The nodes above subtree y0 (at most log2(kMaxSplit)), root first.  A lane
+// outside one of their boxes takes that node's cap in place of everything
+// below it, in the leftmost of the subtrees below (first: every step from the
+// node down to y0 goes left), as the whole-tree walk would; the others add
+// nothing.
+struct Above {
+  int node[8], n = 0;
+  unsigned left = 0;  // bit i: the step down from node[i] goes left
+
+  __device__ __forceinline__ Above(const NodeH* nodes, int y0) {
+    int x = 0;
+    while (x != y0 && n < 8) {
+      node[n] = x;
+      const int l = x + 1;
+      const int meta = __float_as_int(nodes[l].hi.w);
+      const int l_end = meta <= -2 ? l + 1 : __float_as_int(nodes[l].lo.w);
+      const bool go_left = y0 < l_end;
+      if (go_left) left |= 1u << n;
+      ++n;
+      x = go_left ? l : l_end;
+    }
+  }
+  __device__ __forceinline__ bool first(int i) const {
+    const unsigned m = ((1u << n) - 1u) & ~((1u << i) - 1u);
+    return (left & m) == m;
+  }
+};
+
 template <typename QT>
-__global__ void __launch_bounds__(kT, 4) hier_walk_kernel(HierDev H, const QT* __restrict__ Q,
+__global__ void __launch_bounds__(kWalk, 16) hier_walk_kernel(HierDev H, const QT* __restrict__ Q,
                                                        int64_t nQ,
                                                        const int32_t* __restrict__ perm,
                                                        double cx, double cy, double cz,
@@ -635,7 +664,7 @@ __global__ void __launch_bounds__(kT, 4) hier_walk_kernel(HierDev H, const QT* _
   }
   Sum32 acc;
   double acc64 = 0.0;
-  __shared__ HierQueue hqs[kT / 32];
+  __shared__ HierQueue hqs[kWalk / 32];
   HierQueue& hq = hqs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   hq.q[lane][0] = px;
@@ -643,21 +672,23 @@ __global__ void __launch_bounds__(kT, 4) hier_walk_kernel(HierDev H, const QT* _
   hq.q[lane][2] = pz;
   int nqueued = 0;  // warp-uniform
   int resume = valid ? x0 : 0x7fffffff;
-  if (ranges && valid) {
-    // a query outside the root's box takes the root's cap alone (in
-    // subtree 0), as the whole-tree walk does, instead of one cap per subtree
-    const NodeH r0 = H.nodes[0];
-    const int meta0 = __float_as_int(r0.hi.w);
-    if (meta0 >= 0 && (qh.x < r0.lo.x || qh.x > r0.hi.x || qh.y < r0.lo.y || qh.y > r0.hi.y ||
-                       qh.z < r0.lo.z || qh.z > r0.hi.z)) {
-      if (blockIdx.y == 0) {
-        const int cn = H.capn[0];
-        for (int k = 0; k < cn; ++k) {
-          const TriH t = H.caps[meta0 + k];
-          acc.add(trih_term32(t, rel_a(t, qh, ql)));
+  if (ranges) {
+    const Above up(H.nodes, x0);
+    for (int i = 0; i < up.n; ++i) {
+      const NodeH nd = H.nodes[up.node[i]];
+      const int meta = __float_as_int(nd.hi.w);
+      if (resume == x0 && meta >= 0 &&
+          (qh.x < nd.lo.x || qh.x > nd.hi.x || qh.y < nd.lo.y || qh.y > nd.hi.y ||
+           qh.z < nd.lo.z || qh.z > nd.hi.z)) {
+        if (up.first(i)) {
+          const int cn = H.capn[up.node[i]];
+          for (int k = 0; k < cn; ++k) {
+            const TriH t = H.caps[meta + k];
+            acc.add(trih_term32(t, rel_a(t, qh, ql)));
+          }
         }
+        resume = 0x7fffffff;
       }
-      resume = 0x7fffffff;
     }
   }
   int x = x0;
@@ -787,7 +818,7 @@ __device__ __forceinline__ void enqueue64(const HierDev& H, Hier64Queue& hq, int
 // node, else its children; leaf and cap triangles in FP64 with the
 // reference's formula (solid_angle.cpp:16-54), through the warp's queue.
 // Same warp walk, subtree split and partial sums as hier_walk_kernel.
-__global__ void __launch_bounds__(kT, 4) hier_walk64_kernel(HierDev H, const double* __restrict__ Q,
+__global__ void __launch_bounds__(kWalk, 16) hier_walk64_kernel(HierDev H, const double* __restrict__ Q,
                                                          int64_t nQ,
                                                          const int32_t* __restrict__ perm,
                                                          double* __restrict__ W,
@@ -806,7 +837,7 @@ __global__ void __launch_bounds__(kT, 4) hier_walk64_kernel(HierDev H, const dou
   const int64_t q = valid ? (perm ? perm[i] : i) : 0;
   const double px = valid ? Q[q * 3] : 0.0, py = valid ? Q[q * 3 + 1] : 0.0,
                pz = valid ? Q[q * 3 + 2] : 0.0;
-  __shared__ Hier64Queue hqs[kT / 32];
+  __shared__ Hier64Queue hqs[kWalk / 32];
   Hier64Queue& hq = hqs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   hq.q[lane][0] = px;
@@ -821,14 +852,16 @@ __global__ void __launch_bounds__(kT, 4) hier_walk64_kernel(HierDev H, const dou
   unsigned mine = 0;  // this lane's queue positions
   int resume = valid ? x0 : 0x7fffffff;
   if (ranges) {
-    // outside the root's box: the root's cap alone, in subtree 0
-    const int meta0 = __float_as_int(H.nodes[0].hi.w);
-    int cnt = 0;
-    if (valid && meta0 >= 0 && outside(0)) {
-      if (blockIdx.y == 0) cnt = H.capn[0];
-      resume = 0x7fffffff;
+    const Above up(H.nodes, x0);
+    for (int i = 0; i < up.n; ++i) {
+      const int y = up.node[i], meta = __float_as_int(H.nodes[y].hi.w);
+      int cnt = 0;
+      if (resume == x0 && meta >= 0 && outside(y)) {
+        if (up.first(i)) cnt = H.capn[y];
+        resume = 0x7fffffff;
+      }
+      if (__any_sync(0xffffffffu, cnt > 0)) enqueue64(H, hq, cnt, meta, nq, mine, acc);
     }
-    enqueue64(H, hq, cnt, meta0, nq, mine, acc);
   }
   int x = x0;
   while (x < x1) {
@@ -871,36 +904,35 @@ __global__ void hier_sum64_kernel(const double* __restrict__ part, int S, int64_
   W[q] = a * kInv2Pi;
 }
 
-// The top of the tree cut into at most S subtrees (breadth first; a leaf
-// above the cut stays whole): ranges of pre-order positions.  One thread.
+// The top of the tree cut into at most S <= 32 subtrees (breadth first; a leaf
+// above the cut stays whole): ranges of pre-order positions.  One warp, a
+// subtree per lane.
 __global__ void frontier_kernel(const NodeH* __restrict__ nodes, int S, int2* __restrict__ ranges,
                                 int* __restrict__ nranges) {
+  __shared__ int s_next[kMaxSplit];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x;
   auto end_of = [&](int y) {
     const int meta = __float_as_int(nodes[y].hi.w);
     return meta <= -2 ? y + 1 : __float_as_int(nodes[y].lo.w);
   };
-  int cur[8], nxt[8];
-  int nc = 1;
-  cur[0] = 0;
-  bool grew = true;
-  while (grew && nc * 2 <= S) {
-    grew = false;
-    int m = 0;
-    for (int i = 0; i < nc; ++i) {
-      const int y = cur[i];
-      if (__float_as_int(nodes[y].hi.w) <= -2) {
-        nxt[m++] = y;
-      } else {
-        nxt[m++] = y + 1;
-        nxt[m++] = end_of(y + 1);
-        grew = true;
-      }
+  int nc = 1, y = 0;
+  while (nc * 2 <= S) {
+    const bool inner = lane < nc && __float_as_int(nodes[y].hi.w) > -2;
+    const unsigned m = __ballot_sync(full, inner);
+    if (!m) break;
+    if (lane < nc) {
+      const int at = lane + __popc(m & ((1u << lane) - 1u));
+      s_next[at] = inner ? y + 1 : y;
+      if (inner) s_next[at + 1] = end_of(y + 1);
     }
-    for (int i = 0; i < m; ++i) cur[i] = nxt[i];
-    nc = m;
+    nc += __popc(m);
+    __syncwarp();
+    if (lane < nc) y = s_next[lane];
+    __syncwarp();
   }
-  for (int i = 0; i < nc; ++i) ranges[i] = make_int2(cur[i], end_of(cur[i]));
-  *nranges = nc;
+  if (lane < nc) ranges[lane] = make_int2(y, end_of(y));
+  if (lane == 0) *nranges = nc;
 }
 
 // W from the subtrees' partial sums (fixed order), and the FP64 re-check list.
@@ -1103,25 +1135,33 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
                   reinterpret_cast<const TriH*>(h.caps.get()),
                   reinterpret_cast<const TriH*>(h.tris.get()), h.tris64.get(), (int)h.nnodes,
                   h.box64.get(), h.caps64.get()};
-  // Too few queries to fill the GPU: each warp of queries walks one of up to
-  // 8 subtrees (blockIdx.y), and the partial sums are added in a fixed order.
+  // Too few queries for six waves of warps: each warp of queries walks one of
+  // up to 32 subtrees (blockIdx.y), and the partial sums are added in a fixed
+  // order.  Warps near the surface walk far longer than the others, and with
+  // the caps above the cut kept (Above) a finer cut adds no work: FP64, 100,000
+  // queries, 81,920 triangles: 33.2 ms with up to 8 subtrees that keep the
+  // root's cap only; 33.5 / 25.8 / 22.8 / 21.4 ms at 1 / 3 / 6 / 12 waves with
+  // all of them; mixed, 300,000 queries, 20,480 triangles 2.70 -> 2.66 / 2.74 /
+  // 2.48 / 2.35 ms, 100,000 queries, 5,120 triangles 1.17 -> 1.26 / 1.07 / 1.09
+  // / 1.15 ms.
   const int64_t warps = (nQ + 31) / 32;
-  const int64_t want = 3 * (int64_t)num_sms() * 32;
+  const int64_t want = 6 * (int64_t)num_sms() * 32;
+  const unsigned wblk = (unsigned)((nQ + kWalk - 1) / kWalk);
   int S = 1;
   while (S < kMaxSplit && warps * S < want) S *= 2;
   const int32_t* perm = qo.active ? qo.perm.get() : nullptr;
   if (precision == GWN_PLAIN_FP64) {
     PhaseTimer ph("hier_walk", st);
     if (S == 1) {
-      launch_kernel(hier_walk64_kernel, nblk(nQ), kT, 0, st, H, Q, nQ, perm, W,
+      launch_kernel(hier_walk64_kernel, wblk, kWalk, 0, st, H, Q, nQ, perm, W,
                     (const int2*)nullptr, (const int*)nullptr, (double*)nullptr);
     } else {
       DevBuf<int2> ranges(kMaxSplit, st);
       DevBuf<int> nranges(1, st);
       DevBuf<double> part((size_t)S * nQ, st);
       part.zero(st);
-      launch_kernel(frontier_kernel, 1, 1, 0, st, H.nodes, S, ranges.get(), nranges.get());
-      launch_kernel(hier_walk64_kernel, dim3(nblk(nQ), S), kT, 0, st, H, Q, nQ, perm, W,
+      launch_kernel(frontier_kernel, 1, 32, 0, st, H.nodes, S, ranges.get(), nranges.get());
+      launch_kernel(hier_walk64_kernel, dim3(wblk, S), kWalk, 0, st, H, Q, nQ, perm, W,
                     (const int2*)ranges.get(), (const int*)nranges.get(), part.get());
       launch_kernel(hier_sum64_kernel, nblk(nQ), kT, 0, st, (const double*)part.get(), S, nQ, W);
     }
@@ -1130,7 +1170,7 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
   {
     PhaseTimer ph("hier_walk", st);
     if (S == 1) {
-      launch_kernel(hier_walk_kernel<double>, nblk(nQ), kT, 0, st, H, Q, nQ,
+      launch_kernel(hier_walk_kernel<double>, wblk, kWalk, 0, st, H, Q, nQ,
                     (const int32_t*)(qo.active ? qo.perm.get() : nullptr), h.c[0], h.c[1],
                     h.c[2], W, redo.get(), nredo.get(), (const int2*)nullptr,
                     (const int*)nullptr, (double*)nullptr);
@@ -1139,8 +1179,8 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
       DevBuf<int> nranges(1, st);
       DevBuf<double> part((size_t)S * nQ, st);
       part.zero(st);
-      launch_kernel(frontier_kernel, 1, 1, 0, st, H.nodes, S, ranges.get(), nranges.get());
-      launch_kernel(hier_walk_kernel<double>, dim3(nblk(nQ), S), kT, 0, st, H, Q, nQ,
+      launch_kernel(frontier_kernel, 1, 32, 0, st, H.nodes, S, ranges.get(), nranges.get());
+      launch_kernel(hier_walk_kernel<double>, dim3(wblk, S), kWalk, 0, st, H, Q, nQ,
                     (const int32_t*)(qo.active ? qo.perm.get() : nullptr), h.c[0], h.c[1],
                     h.c[2], W, redo.get(), nredo.get(), (const int2*)ranges.get(),
                     (const int*)nranges.get(), part.get());

@@ -129,3 +129,20 @@ def test_fp64_hierarchy_matches_cpu_hierarchy_and_all_pairs(cuda):
     assert np.abs(W32.astype(np.float64) - ref).max() <= 1e-6
     Wm32 = G.winding_number(V, F, Q32, precision="mixed")
     assert np.abs(Wm32.astype(np.float64) - ref).max() <= 1e-4
+
+
+@pytest.mark.parametrize("prec,tol", [("mixed", 1e-6), ("fp64", 1e-12)])
+def test_batches_of_every_split_agree(cuda, prec, tol):
+    """Few queries walk up to 32 subtrees in parallel, many walk the whole
+    tree: the same queries in batches on either side of each split, on a mesh
+    with holes (caps at every level) and on one whose top is a single leaf
+    pair.  A split changes only which partial sum a term joins."""
+    rng = np.random.default_rng(71)
+    for V, F in (_meshes()["holes"], _meshes()["messy"]):
+        Q = np.concatenate([_queries(V, 1000, 72), rng.uniform(-6, 6, (1_000_000, 3))])
+        h = G.WindingNumberAABB(V, F)
+        W = h.winding_number(Q, prec)
+        for m in (1, 31, 33, 64, 65, 2000, 40_000, 300_000):
+            w = h.winding_number(Q[:m], prec)
+            assert np.abs(w - W[:m]).max() <= tol, (prec, m)
+        h.close()
