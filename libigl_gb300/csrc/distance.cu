@@ -804,6 +804,10 @@ void closest_launch(const ClosestParams& prm, const QT* Q, const int32_t* perm, 
 
 }  // namespace
 
+// The stack holds at most one entry per level plus one (each pop pushes at
+// most two children).
+bool soup_search_fits(int max_depth) { return max_depth + 2 < kStack; }
+
 void soup_squared_distance(const gwn_soup_impl& s, const void* Q, int q_dtype, int64_t nQ,
                            double up_sqr_d, double* sqrD, int32_t* I, double* C,
                            cudaStream_t st) {
@@ -823,9 +827,7 @@ void soup_squared_distance(const gwn_soup_impl& s, const void* Q, int q_dtype, i
   }
   const int32_t* perm = qo.active ? qo.perm.get() : nullptr;
   PhaseTimer ph("closest", st);
-  // The stack holds at most one entry per level plus one (each pop pushes at
-  // most two children).
-  const bool dfs = s.max_depth + 2 < kStack;
+  const bool dfs = soup_search_fits(s.max_depth);
   if (q_dtype == GWN_F64)
     closest_launch(prm, static_cast<const double*>(Q), perm, nQ, up_sqr_d, sqrD, I, C, dfs, st);
   else
@@ -892,7 +894,8 @@ void signed_distance_run(const double* P, int64_t nP, const double* V, int64_t n
   const double up_sqr_d = std::pow(max_abs, 2.0);
   const double low_sqr_d = std::pow(std::fmax(max_abs - (upper_bound - lower_bound), 0.0), 2.0);
   gwn_soup_impl tree;
-  soup_build(tree, V, nV, F, nF, 2, true, st);
+  // only the fast winding number's sign walks the moments
+  soup_build(tree, V, nV, F, nF, 2, true, st, sign_type != GWN_SD_FAST_WINDING_NUMBER);
   DevBuf<double> sqrD((size_t)nP, st);
   soup_squared_distance(tree, P, GWN_F64, nP, up_sqr_d, sqrD.get(), I, C, st);
   DevBuf<double> W;

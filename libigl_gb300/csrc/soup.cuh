@@ -133,8 +133,12 @@ void soup_tree_build(const double* V, int64_t nV, const int32_t* F, int32_t* val
                      const double* clo, const double* chi, int32_t* left, int32_t* right,
                      int32_t* parent, cudaStream_t st);
 
+// search_only: what soup_squared_distance reads alone (no moments, no walk
+// records), where the tree's depth allows it.
 void soup_build(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t* F, int64_t nF,
-                int order, bool host_mode, cudaStream_t st);
+                int order, bool host_mode, cudaStream_t st, bool search_only = false);
+// Whether the depth-first search's stack holds a tree of this depth.
+bool soup_search_fits(int max_depth);
 // The reference's own 4-wide tree and FP32 moments (soup_ref.cu); fills the
 // same walk records (slot 0 the root, then every child lane depth-first),
 // without the closest-point search nodes.

@@ -347,7 +347,7 @@ void swept_volume_run(const double* V, int64_t nV, const int32_t* F, int64_t nF,
                           precision == GWN_MIXED;
     {
       PhaseTimer ph("build", st);
-      soup_build(tree, V, nV, F, nF, 2, true, st);
+      soup_build(tree, V, nV, F, nF, 2, true, st, sign_type != GWN_SD_FAST_WINDING_NUMBER);
       if (sign_type == GWN_SD_PSEUDONORMAL) pseudonormal_precompute(V, nV, F, nF, pn, st);
       if (use_hier) hier_build(V, nV, F, nF, hier, sticky_status_word(), st, true);
     }
