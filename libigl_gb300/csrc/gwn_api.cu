@@ -473,10 +473,16 @@ void gwn_soup_free(gwn_soup* soup) { delete soup; }
 int gwn_soup_export(const gwn_soup* soup, double* nodes, int32_t* tri_index) {
   return guarded("gwn_soup_export", [&] {
     GWN_REQUIRE(soup != nullptr, "soup handle is null");
-    static_assert(sizeof(SoupNodeD) == 24 * sizeof(double), "node record layout");
     const gwn_soup_impl& s = soup->impl;
-    if (nodes && s.nnodes)
+    if (nodes && s.nnodes) {
       GWN_CUDA(cudaMemcpy(nodes, s.nd.get(), s.nd.bytes(), cudaMemcpyDeviceToHost));
+      for (int64_t i = 0; i < s.nnodes; ++i) {  // the records hold packed forms
+        SoupNodeD D;
+        std::memcpy(&D, nodes + i * 24, sizeof(D));
+        unpack_far64(D, nodes + i * 24 + 4);
+        std::memcpy(nodes + i * 24 + 23, &D.link, sizeof(D.link));
+      }
+    }
     if (tri_index && s.n)
       GWN_CUDA(cudaMemcpy(tri_index, s.tri_index.get(), s.tri_index.bytes(),
                           cudaMemcpyDeviceToHost));

@@ -449,21 +449,13 @@ __global__ void emit_kernel(const BuildM* __restrict__ M, const int32_t* __restr
   D.P[1] = m.P[1];
   D.P[2] = m.P[2];
   D.maxP2 = maxP2;
-  for (int d = 0; d < 3; ++d) {
-    D.N[d] = m.N[d];
-    D.Nii[d] = m.Nii[d];
-    D.Niii[d] = m.Niii[d];
-  }
-  D.Nxy_yx = m.Nxy + m.Nyx;
-  D.Nyz_zy = m.Nyz + m.Nzy;
-  D.Nzx_xz = m.Nzx + m.Nxz;
-  D.perm = m.perm;
-  for (int k = 0; k < 6; ++k) D.c2[k] = m.c2[k];
+  const double xy = m.Nxy + m.Nyx, yz = m.Nyz + m.Nzy, zx = m.Nzx + m.Nxz;
+  pack_far64(D, m.N, m.Nii, xy, yz, zx, m.Niii, m.perm, m.c2);
   D.link = link;
   nd[p] = D;
   SoupNodeF Fr;
   Fr.a = make_float4((float)D.P[0], (float)D.P[1], (float)D.P[2], (float)maxP2);
-  pack_far32(Fr, D.N, D.Nii, D.Nxy_yx, D.Nyz_zy, D.Nzx_xz, D.Niii, D.perm, D.c2, (int)link);
+  pack_far32(Fr, m.N, m.Nii, xy, yz, zx, m.Niii, m.perm, m.c2, (int)link);
   nf[p] = Fr;
   if (leaf) {
     const int32_t f = sorted_tri[slot];
@@ -590,7 +582,7 @@ __global__ void moments_bounded_kernel(const SoupNodeD* __restrict__ nd, int64_t
   const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   bool bad = false;
   if (x < n) {
-    const double* m = nd[x].N;  // N .. c2: the 19 moments after P, maxP2
+    const double* m = nd[x].N;  // N .. L: the 19 values after P, maxP2
     for (int k = 0; k < 19; ++k) bad |= !(fabs(m[k]) <= 1e100);
   }
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(unbounded, 1u);
@@ -608,9 +600,8 @@ __global__ void fill_zero_kernel(WT* w, int64_t n) {
 void soup_check_moments(gwn_soup_impl& s, cudaStream_t st) {
   s.moments_bounded = true;
   if (s.nnodes == 0) return;
-  static_assert(offsetof(SoupNodeD, c2) + 6 * sizeof(double) - offsetof(SoupNodeD, N) ==
-                    19 * sizeof(double),
-                "the 19 moments are contiguous");
+  static_assert(offsetof(SoupNodeD, link) - offsetof(SoupNodeD, N) == 19 * sizeof(double),
+                "the 19 values are contiguous");
   DevBuf<unsigned> flag(1, st);
   flag.zero(st);
   launch_kernel(moments_bounded_kernel, (unsigned)((s.nnodes + 255) / 256), 256, 0, st,

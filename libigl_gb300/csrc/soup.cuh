@@ -56,14 +56,68 @@ __host__ __device__ inline void pack_far32(SoupNodeF& R, const double N[3], cons
                     (float)(-7.5 * perm), lf);
 }
 
-// 192-byte FP64 node record (plain FP64 walk, FP64 re-checks).
+// 192-byte FP64 node record (plain FP64 walk, FP64 re-checks): the same forms
+// in FP64.  The quadratic form has no trace and the cubic form no Laplacian
+// (both brackets are harmonic), so A_zz = -(A_xx + A_yy), K_xzz = -(3 K_xxx +
+// K_xyy), K_yzz = -(3 K_yyy + K_xxy) and K_zzz = -(K_xxz + K_yyz) / 3 are not
+// stored; S and L, the parts of the moments that the forms do not hold, are
+// kept for gwn_soup_export.
 struct __align__(16) SoupNodeD {
   double P[3], maxP2;
-  double N[3], Nii[3];
-  double Nxy_yx, Nyz_zy, Nzx_xz;
-  double Niii[3], perm, c2[6];
+  double N[3];
+  double A[5];  // xx yy xy xz yz
+  double K[7];  // xxx yyy xxy xxz xyy yyz xyz
+  double S, L[3];
   long long link;
 };
+static_assert(sizeof(SoupNodeD) == 24 * sizeof(double), "node record layout");
+
+__host__ __device__ inline void pack_far64(SoupNodeD& D, const double N[3], const double Nii[3],
+                                           double Nxy_yx, double Nyz_zy, double Nzx_xz,
+                                           const double Niii[3], double perm, const double c2[6]) {
+  D.S = Nii[0] + Nii[1] + Nii[2];
+  D.L[0] = 3 * Niii[0] + (c2[3] + c2[4]);
+  D.L[1] = 3 * Niii[1] + (c2[5] + c2[0]);
+  D.L[2] = 3 * Niii[2] + (c2[1] + c2[2]);
+  for (int d = 0; d < 3; ++d) D.N[d] = N[d];
+  D.A[0] = D.S - 3 * Nii[0];
+  D.A[1] = D.S - 3 * Nii[1];
+  D.A[2] = -3 * Nxy_yx;
+  D.A[3] = -3 * Nzx_xz;
+  D.A[4] = -3 * Nyz_zy;
+  D.K[0] = 1.5 * D.L[0] - 7.5 * Niii[0];
+  D.K[1] = 1.5 * D.L[1] - 7.5 * Niii[1];
+  D.K[2] = 1.5 * D.L[1] - 7.5 * c2[0];
+  D.K[3] = 1.5 * D.L[2] - 7.5 * c2[1];
+  D.K[4] = 1.5 * D.L[0] - 7.5 * c2[3];
+  D.K[5] = 1.5 * D.L[2] - 7.5 * c2[2];
+  D.K[6] = -7.5 * perm;
+}
+
+// The moments of a record, m = {N, Nii, Nxy_yx, Nyz_zy, Nzx_xz, Niii, perm,
+// c2}: 19 values.
+inline void unpack_far64(const SoupNodeD& D, double m[19]) {
+  for (int d = 0; d < 3; ++d) m[d] = D.N[d];
+  m[3] = (D.S - D.A[0]) / 3;
+  m[4] = (D.S - D.A[1]) / 3;
+  m[5] = (D.S + (D.A[0] + D.A[1])) / 3;
+  m[6] = -D.A[2] / 3;
+  m[7] = -D.A[4] / 3;
+  m[8] = -D.A[3] / 3;
+  const double Kzzz = -(D.K[3] + D.K[5]) / 3, Kxzz = -(3 * D.K[0] + D.K[4]),
+               Kyzz = -(3 * D.K[1] + D.K[2]);
+  auto u = [](double L, double K) { return (1.5 * L - K) / 7.5; };
+  m[9] = u(D.L[0], D.K[0]);
+  m[10] = u(D.L[1], D.K[1]);
+  m[11] = u(D.L[2], Kzzz);
+  m[12] = -D.K[6] / 7.5;
+  m[13] = u(D.L[1], D.K[2]);
+  m[14] = u(D.L[2], D.K[3]);
+  m[15] = u(D.L[2], D.K[5]);
+  m[16] = u(D.L[0], D.K[4]);
+  m[17] = u(D.L[0], Kxzz);
+  m[18] = u(D.L[1], Kyzz);
+}
 
 #ifdef __CUDACC__
 // Error slack of the FP32 closest-point screen for one triangle (v: three

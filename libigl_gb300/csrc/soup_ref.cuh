@@ -336,7 +336,7 @@ __device__ __forceinline__ void write_record(const MomentArgs& A, const Loc<floa
   A.nf[slot] = R;
 }
 
-// Sets bc->unbounded where a moment is not finite or beyond 1e100 in magnitude
+// Sets bc->unbounded where a value is not finite or beyond 1e100 in magnitude
 // (gwn_soup_impl::moments_bounded); the bit patterns of non-negative doubles
 // compare as the values do, NaN above all.
 __device__ __forceinline__ bool beyond(double x) {
@@ -345,24 +345,13 @@ __device__ __forceinline__ bool beyond(double x) {
 __device__ __forceinline__ void write_record(const MomentArgs& A, const Loc<double>& C,
                                              uint32_t slot, int link, bool root) {
   SoupNodeD D;
-  bool bad = false;
-  for (int d = 0; d < 3; ++d) {
-    D.P[d] = C.P[d];
-    D.N[d] = C.N[d];
-    D.Nii[d] = C.Nii[d];
-    D.Niii[d] = C.Niii[d];
-    bad |= beyond(C.N[d]) || beyond(C.Nii[d]) || beyond(C.Niii[d]);
-  }
+  for (int d = 0; d < 3; ++d) D.P[d] = C.P[d];
   D.maxP2 = root ? (double)INFINITY : lane_maxP2(C);
-  D.Nxy_yx = C.Nxy + C.Nyx;
-  D.Nyz_zy = C.Nyz + C.Nzy;
-  D.Nzx_xz = C.Nzx + C.Nxz;
-  D.perm = C.perm;
-  bad |= beyond(D.Nxy_yx) || beyond(D.Nyz_zy) || beyond(D.Nzx_xz) || beyond(D.perm);
-  for (int k = 0; k < 6; ++k) {
-    D.c2[k] = C.c2[k];
-    bad |= beyond(C.c2[k]);
-  }
+  pack_far64(D, C.N, C.Nii, C.Nxy + C.Nyx, C.Nyz + C.Nzy, C.Nzx + C.Nxz, C.Niii, C.perm, C.c2);
+  bool bad = beyond(D.S);
+  for (int d = 0; d < 3; ++d) bad |= beyond(D.N[d]) || beyond(D.L[d]);
+  for (int k = 0; k < 5; ++k) bad |= beyond(D.A[k]);
+  for (int k = 0; k < 7; ++k) bad |= beyond(D.K[k]);
   D.link = link;
   A.nd[slot] = D;
   if (bad) A.bc->unbounded = 1;

@@ -24,42 +24,31 @@ constexpr double kBand = 1e-3;  // |W - 0.5| band re-evaluated in plain FP64
 constexpr float kInv4PiF = 0.079577471545947667884f;
 constexpr double kInv4Pi = 0.079577471545947667884;
 
-// Far field of one node about its average point, FWNFS.h:7195-7251, with
-// (dx,dy,dz) = q - P and r2 = |q - P|^2: the reference's expression, in FP64
-// on the FP64 records (the FP32 walk evaluates the packed forms of
-// pack_far32 instead, far_field32 below).
-template <typename T>
-struct Far {
-  T N[3], Nii[3], Nxy_yx, Nyz_zy, Nzx_xz, Niii[3], perm, c2[6];
-};
-
-template <typename T>
-__device__ __forceinline__ T far_field(const Far<T>& m, T dx, T dy, T dz, T r2, int order) {
-  // m2 = 1/|q-P|^2, m1 = sqrt(m2), as the reference
-  const T m2 = T(1) / r2;
-  const T m1 = g_sqrt(m2);
-  const T qx = dx * m1, qy = dy * m1, qz = dz * m1;
-  T omega = -m2 * (qx * m.N[0] + qy * m.N[1] + qz * m.N[2]);
-  if (order >= 1) {
-    const T q2x = qx * qx, q2y = qy * qy, q2z = qz * qz;
-    const T m3 = m2 * m1;
-    omega += m3 * (m.Nii[0] + m.Nii[1] + m.Nii[2] -
-                   T(3) * (q2x * m.Nii[0] + q2y * m.Nii[1] + q2z * m.Nii[2] + qx * qy * m.Nxy_yx +
-                           qx * qz * m.Nzx_xz + qy * qz * m.Nyz_zy));
-    if (order >= 2) {
-      const T q3x = q2x * qx, q3y = q2y * qy, q3z = q2z * qz;
-      const T m4 = m2 * m2;
-      const T t0x = m.c2[3] + m.c2[4], t0y = m.c2[5] + m.c2[0], t0z = m.c2[1] + m.c2[2];
-      const T t1x = qy * m.c2[0] + qz * m.c2[1];
-      const T t1y = qz * m.c2[2] + qx * m.c2[3];
-      const T t1z = qx * m.c2[4] + qy * m.c2[5];
-      omega += m4 * (T(1.5) * (qx * (T(3) * m.Niii[0] + t0x) + qy * (T(3) * m.Niii[1] + t0y) +
-                               qz * (T(3) * m.Niii[2] + t0z)) -
-                     T(7.5) * (q3x * m.Niii[0] + q3y * m.Niii[1] + q3z * m.Niii[2] +
-                               qx * qy * qz * m.perm + q2x * t1x + q2y * t1y + q2z * t1z));
-    }
+// FP64 far field of a packed record (pack_far64), FWNFS.h:7195-7251, (dx,dy,dz)
+// = q - P, r2 = |q - P|^2: the FP32 walk's forms.  Bound by the FP64 pipe; in
+// place of the reference's expression on the moments (a division, a square
+// root and about 60 operations) one reciprocal square root and about 35.
+__device__ __forceinline__ double far_field64(const SoupNodeD* r, double dx, double dy, double dz,
+                                              double r2, int order) {
+  const double2* v = reinterpret_cast<const double2*>(r);
+  const double2 n01 = __ldg(v + 2), n2a = __ldg(v + 3);
+  const double m1 = rsqrt(r2), m2 = m1 * m1;
+  const double qx = dx * m1, qy = dy * m1, qz = dz * m1;
+  const double lin = qx * n01.x + qy * n01.y + qz * n2a.x;
+  if (order == 0) return -m2 * lin;
+  const double2 a12 = __ldg(v + 4), a34 = __ldg(v + 5);  // yy xy | xz yz
+  const double x2 = qx * qx, y2 = qy * qy, z2 = qz * qz, yz = qy * qz;
+  double s = qx * (n2a.y * qx + a12.y * qy + a34.x * qz) + a12.x * y2 - (n2a.y + a12.x) * z2 +
+             a34.y * yz;
+  if (order >= 2) {
+    // xxx yyy | xxy xxz | xyy yyz | xyz S
+    const double2 k01 = __ldg(v + 6), k23 = __ldg(v + 7), k45 = __ldg(v + 8), k6 = __ldg(v + 9);
+    const double kx = k01.x * x2 + k45.x * y2 - (3 * k01.x + k45.x) * z2 + k6.x * yz;
+    const double ky = k23.x * x2 + k01.y * y2 - (3 * k01.y + k23.x) * z2;
+    const double kz = k23.y * x2 + k45.y * y2 - (k23.y + k45.y) * (1.0 / 3.0) * z2;
+    s += m1 * (qx * kx + qy * ky + qz * kz);
   }
-  return omega;
+  return m2 * (m1 * s - lin);
 }
 
 // Exact triangle solid angle, FWNFS.h:6070-6110 (normalised corner vectors).
@@ -90,6 +79,34 @@ __device__ __forceinline__ T tri_solid_angle(T ax, T ay, T az, T bx, T by, T bz,
   return T(2) * g_atan2(num, den);
 }
 
+// The plain FP64 walk's triangle term: the unnormalised form of
+// solid_angle_vos64 below, angle included in FP64, with the normalised form's
+// zeros (a corner at q, coinciding corners, a zero determinant).  Nine
+// divisions fewer; corners so far or near that the products of three lengths
+// would leave the range take the normalised form.
+__device__ __forceinline__ double tri_solid_angle64(const double* __restrict__ t, double qx,
+                                                    double qy, double qz) {
+  const double ax = t[0] - qx, ay = t[1] - qy, az = t[2] - qz;
+  const double bx = t[3] - qx, by = t[4] - qy, bz = t[5] - qz;
+  const double cx = t[6] - qx, cy = t[7] - qy, cz = t[8] - qz;
+  const double la2 = ax * ax + ay * ay + az * az;
+  const double lb2 = bx * bx + by * by + bz * bz;
+  const double lc2 = cx * cx + cy * cy + cz * cz;
+  // all three squares within 2^+-600, by their exponents (never negative)
+  const int ha = __double2hiint(la2), hb = __double2hiint(lb2), hc = __double2hiint(lc2);
+  if (min(ha, min(hb, hc)) < (1023 - 600) << 20 || max(ha, max(hb, hc)) > (1023 + 600) << 20)
+    return tri_solid_angle<double>(ax, ay, az, bx, by, bz, cx, cy, cz);
+  if ((ax == bx && ay == by && az == bz) || (ax == cx && ay == cy && az == cz) ||
+      (bx == cx && by == cy && bz == cz))
+    return 0.0;
+  const double det = ax * (by * cz - bz * cy) + ay * (bz * cx - bx * cz) + az * (bx * cy - by * cx);
+  if (det == 0.0) return 0.0;
+  const double la = sqrt(la2), lb = sqrt(lb2), lc = sqrt(lc2);
+  const double den = la * lb * lc + (ax * bx + ay * by + az * bz) * lc +
+                     (ax * cx + ay * cy + az * cz) * lb + (bx * cx + by * cy + bz * cz) * la;
+  return 2.0 * atan2(det, den);
+}
+
 // FP32 far field of a packed record (pack_far32; b..f its float4s): omega = m2 (m1 (A(q) +
 // m1 K(q)) - q.N) with q = (x - P) m1, (dx,dy,dz) = x - P, r2 = |x - P|^2.
 __device__ __forceinline__ float far_field32(float4 b, float4 c, float4 d, float4 e, float4 f,
@@ -109,21 +126,6 @@ __device__ __forceinline__ float far_field32(float4 b, float4 c, float4 d, float
     s = fmaf(m1, fmaf(qx, kx, fmaf(qy, ky, qz * kz)), a);
   }
   return m2 * fmaf(m1, s, -lin);
-}
-
-__device__ __forceinline__ Far<double> load_far(const SoupNodeD* r) {
-  Far<double> m;
-  for (int d = 0; d < 3; ++d) {
-    m.N[d] = r->N[d];
-    m.Nii[d] = r->Nii[d];
-    m.Niii[d] = r->Niii[d];
-  }
-  m.Nxy_yx = r->Nxy_yx;
-  m.Nyz_zy = r->Nyz_zy;
-  m.Nzx_xz = r->Nzx_xz;
-  m.perm = r->perm;
-  for (int k = 0; k < 6; ++k) m.c2[k] = r->c2[k];
-  return m;
 }
 
 // Query i of a launch (through the spatial order perm, or a re-evaluation
@@ -457,11 +459,10 @@ __device__ __forceinline__ void flush_fp64(const EvalParams& prm, Fp64Queue& fq,
         const SoupNodeD* r = prm.nd + e.x;
         const double dx = qx - r->P[0], dy = qy - r->P[1], dz = qz - r->P[2];
         const double r2 = dx * dx + dy * dy + dz * dz;
-        v = far_field<double>(load_far(r), dx, dy, dz, r2, prm.order);
+        v = far_field64(r, dx, dy, dz, r2, prm.order);
       } else {
         const double* t = prm.td + (int64_t)(~e.x) * 9;
-        v = tri_solid_angle<double>(t[0] - qx, t[1] - qy, t[2] - qz, t[3] - qx, t[4] - qy,
-                                    t[5] - qz, t[6] - qx, t[7] - qy, t[8] - qz);
+        v = tri_solid_angle64(t, qx, qy, qz);
       }
       fq.v[lane] = v;
     }
@@ -513,7 +514,7 @@ __device__ __forceinline__ double walk_fp64(const EvalParams& prm, bool valid, d
             term = node;
             resume = leaf ? node + 1 : (int)link;
           } else {
-            const double om = far_field<double>(load_far(r), dx, dy, dz, r2, prm.order);
+            const double om = far_field64(r, dx, dy, dz, r2, prm.order);
             if (isfinite(om)) {
               push = true;
               term = kQueuedValue;
@@ -694,7 +695,7 @@ __device__ __forceinline__ double walk_fp64_team(const EvalParams& prm, int T, b
           push = true;
           term = team.c;
         } else {
-          const double om = far_field<double>(load_far(r), dx, dy, dz, r2, prm.order);
+          const double om = far_field64(r, dx, dy, dz, r2, prm.order);
           if (isfinite(om)) {
             push = true;
             term = kQueuedValue;
@@ -757,7 +758,7 @@ __device__ inline double walk_fp64_lane(const EvalParams& prm, double qx, double
     const double dx = qx - r->P[0], dy = qy - r->P[1], dz = qz - r->P[2];
     const double r2 = dx * dx + dy * dy + dz * dz;
     if (!near) {
-      const double om = far_field<double>(load_far(r), dx, dy, dz, r2, prm.order);
+      const double om = far_field64(r, dx, dy, dz, r2, prm.order);
       if (isfinite(om)) {
         acc += om;
         node = leaf ? node + 1 : (int)link;
@@ -766,8 +767,7 @@ __device__ inline double walk_fp64_lane(const EvalParams& prm, double qx, double
     }
     if (leaf) {
       const double* t = prm.td + (int64_t)(~link) * 9;
-      acc += tri_solid_angle<double>(t[0] - qx, t[1] - qy, t[2] - qz, t[3] - qx, t[4] - qy,
-                                     t[5] - qz, t[6] - qx, t[7] - qy, t[8] - qz);
+      acc += tri_solid_angle64(t, qx, qy, qz);
     }
     ++node;
   }
