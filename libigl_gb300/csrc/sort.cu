@@ -88,13 +88,20 @@ __global__ void scan_tiles_kernel(const uint32_t* in, uint32_t* out, int64_t n,
 }
 
 // ---------------------------------------------------------------- radix ----
+// A tile is R rounds of 256 elements that its CTA takes one after the other.
+// 16 rounds keep the count table small where the tiles fill the GPU; below
+// kRsFew elements they would not, and a pass is bound by its CTAs' rounds:
+// 15,360 pairs of 64-bit keys, hist + scatter per pass 5.3 + 9.7 us with 16
+// rounds (4 CTAs), 4 rounds (15 CTAs) there.
 constexpr int kRsThreads = 256;
 constexpr int kRsRounds = 16;
+constexpr int kRsFewRounds = 4;
+constexpr int64_t kRsFew = 512 * 1024;
 constexpr int kRsTile = kRsThreads * kRsRounds;
 
 // n_dev (optional): the element count is min(n, *n_dev), read on the device,
 // so that a captured graph can sort batches of varying size.
-template <typename K>
+template <typename K, int R = kRsRounds>
 __global__ void __launch_bounds__(kRsThreads) rs_hist_kernel(const K* __restrict__ keys,
                                                              int64_t n, int shift,
                                                              uint32_t* __restrict__ counts,
@@ -104,9 +111,9 @@ __global__ void __launch_bounds__(kRsThreads) rs_hist_kernel(const K* __restrict
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
-  const int64_t base = blockIdx.x * (int64_t)kRsTile;
+  const int64_t base = blockIdx.x * (int64_t)(R * kRsThreads);
 #pragma unroll 4
-  for (int r = 0; r < kRsRounds; ++r) {
+  for (int r = 0; r < R; ++r) {
     const int64_t i = base + (int64_t)r * kRsThreads + threadIdx.x;
     if (i < n) atomicAdd(&h[(uint32_t)(keys[i] >> shift) & 255u], 1u);
   }
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(kRsThreads) rs_hist_kernel(const K* __restrict
   counts[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-template <typename K>
+template <typename K, int R = kRsRounds>
 __global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(
     const K* __restrict__ kin, const int32_t* __restrict__ vin, K* __restrict__ kout,
     int32_t* __restrict__ vout, int64_t n, int shift, const uint32_t* __restrict__ offsets,
@@ -125,8 +132,8 @@ __global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   s_base[tid] = offsets[(int64_t)tid * ntiles + blockIdx.x];
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const int64_t base = blockIdx.x * (int64_t)kRsTile;
-  for (int r = 0; r < kRsRounds; ++r) {
+  const int64_t base = blockIdx.x * (int64_t)(R * kRsThreads);
+  for (int r = 0; r < R; ++r) {
     const int64_t i = base + (int64_t)r * kRsThreads + tid;
     const bool valid = i < n;
     K k = 0;
@@ -225,17 +232,21 @@ void radix_sort_pairs(K* keys, int32_t* vals, K* keys_tmp, int32_t* vals_tmp, in
                       int begin_bit, int end_bit, cudaStream_t st) {
   if (n <= 1 || end_bit <= begin_bit) return;
   GWN_REQUIRE(n < (int64_t(1) << 32), "radix sort: at most 2^32-1 elements");
-  const int ntiles = (int)((n + kRsTile - 1) / kRsTile);
+  const bool few = n < kRsFew;
+  const int tile = kRsThreads * (few ? kRsFewRounds : kRsRounds);
+  const int ntiles = (int)((n + tile - 1) / tile);
+  auto hist = few ? rs_hist_kernel<K, kRsFewRounds> : rs_hist_kernel<K, kRsRounds>;
+  auto scatter = few ? rs_scatter_kernel<K, kRsFewRounds> : rs_scatter_kernel<K, kRsRounds>;
   DevBuf<uint32_t> counts((size_t)ntiles * 256, st);
   K* ka = keys;
   int32_t* va = vals;
   K* kb = keys_tmp;
   int32_t* vb = vals_tmp;
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
-    launch_kernel(rs_hist_kernel<K>, ntiles, kRsThreads, 0, st, ka, n, shift, counts.get(), ntiles,
+    launch_kernel(hist, ntiles, kRsThreads, 0, st, ka, n, shift, counts.get(), ntiles,
                   (const uint32_t*)nullptr);
     exclusive_scan_u32(counts.get(), counts.get(), (int64_t)ntiles * 256, st);
-    launch_kernel(rs_scatter_kernel<K>, ntiles, kRsThreads, 0, st, ka, va, kb, vb, n, shift,
+    launch_kernel(scatter, ntiles, kRsThreads, 0, st, ka, va, kb, vb, n, shift,
                   counts.get(), ntiles, (const uint32_t*)nullptr);
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -265,10 +276,10 @@ void radix_sort_pairs_devn(uint32_t* keys, int32_t* vals, uint32_t* keys_tmp, in
   uint32_t* kb = keys_tmp;
   int32_t* vb = vals_tmp;
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
-    launch_kernel(rs_hist_kernel<uint32_t>, ntiles, kRsThreads, 0, st, ka, cap, shift, counts,
+    launch_kernel(rs_hist_kernel<uint32_t, kRsRounds>, ntiles, kRsThreads, 0, st, ka, cap, shift, counts,
                   ntiles, n_dev);
     exclusive_scan_u32(counts, counts, (int64_t)ntiles * 256, st, scan_scratch);
-    launch_kernel(rs_scatter_kernel<uint32_t>, ntiles, kRsThreads, 0, st, ka, va, kb, vb, cap,
+    launch_kernel(rs_scatter_kernel<uint32_t, kRsRounds>, ntiles, kRsThreads, 0, st, ka, va, kb, vb, cap,
                   shift, counts, ntiles, n_dev);
     std::swap(ka, kb);
     std::swap(va, vb);
