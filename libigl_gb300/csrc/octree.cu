@@ -404,61 +404,76 @@ __global__ void final_layout_kernel(int64_t ncells, const double* __restrict__ c
 // p are those of the depths cpl[p] + 1 .. cpl[p + 1]: listed p by p, that is
 // depth-first pre-order, the order of the ids.  A cell's end and its children
 // are found by searching the sorted keys.
-// The key holds 21 octants; runs of equal keys (points closer than 2^-21 of
-// the root cube) are ordered by their deeper octants, one thread per run.  A
-// run of more than kTieRun points, or points that share kTieDepth octants
-// (identical ones above all), leave the whole build to the level loop below,
-// which follows them to depth 30000.
+// The key holds 10, 16 or 21 octants (4, 6 or 8 sort passes, by the point
+// count); runs of equal keys are ordered by their deeper octants, one thread
+// per run.  A run of more than kTieRun points takes the longest key; with that,
+// or where points share kTieDepth octants (identical ones above all), the whole
+// build is left to the level loop below, which follows them to depth 30000.
 // In place of about 20 launches, 6 scans and a host read per level, over every
-// point: 2M points 7.0 -> 1.5 ms.
+// point: 2M points 7.0 -> 2.6 ms.
 constexpr int kKeyDepth = 21;
 constexpr int kTieDepth = 64;
 constexpr int kTieRun = 32;
+
+// By depth: the cell width and the step from a centre to its children's, as
+// the reference halves them.
+struct Widths {
+  double w[kTieDepth + 2], step[kTieDepth + 2];
+};
+__global__ void widths_kernel(const double* __restrict__ rw, Widths* __restrict__ t) {
+  double w = *rw;
+  for (int d = 0; d < kTieDepth + 2; ++d) {
+    const double h = __dmul_rn(w, 0.5);
+    t->w[d] = w;
+    t->step[d] = __dmul_rn(h, 0.5);
+    w = h;
+  }
+}
 
 struct PathTotals {
   unsigned long long nindices;
   uint32_t ninternal, max_cpl, deep;
 };
 
-// The octant walk of one point: centre and width as the reference halves them.
+// The octant walk of one point: the centre of its cell.
 struct Walk {
-  double c[3], w;
+  double c[3];
   __device__ __forceinline__ int octant(const double* p) const {
     return (p[0] >= c[0] ? 1 : 0) + (p[1] >= c[1] ? 2 : 0) + (p[2] >= c[2] ? 4 : 0);
   }
-  __device__ __forceinline__ void descend(int o) {
-    const double h = __dmul_rn(w, 0.5), hh = __dmul_rn(h, 0.5);
-    c[0] = __dadd_rn(c[0], (o & 1) ? hh : -hh);
-    c[1] = __dadd_rn(c[1], (o & 2) ? hh : -hh);
-    c[2] = __dadd_rn(c[2], (o & 4) ? hh : -hh);
-    w = h;
+  __device__ __forceinline__ void descend(int o, double step) {
+    c[0] = __dadd_rn(c[0], (o & 1) ? step : -step);
+    c[1] = __dadd_rn(c[1], (o & 2) ? step : -step);
+    c[2] = __dadd_rn(c[2], (o & 4) ? step : -step);
   }
 };
 
+// Keys of kd octants.
 __global__ void path_keys_kernel(const double* __restrict__ P, int64_t n,
-                                 const double* __restrict__ rc, const double* __restrict__ rw,
-                                 unsigned long long* __restrict__ key, int32_t* __restrict__ val) {
+                                 const double* __restrict__ rc, const Widths* __restrict__ t,
+                                 int kd, unsigned long long* __restrict__ key,
+                                 int32_t* __restrict__ val) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double p[3] = {P[i * 3], P[i * 3 + 1], P[i * 3 + 2]};
-  Walk w{{rc[0], rc[1], rc[2]}, *rw};
+  Walk w{{rc[0], rc[1], rc[2]}};
   unsigned long long k = 0;
-  for (int d = 0; d < kKeyDepth; ++d) {
+  for (int d = 0; d < kd; ++d) {
     const int o = w.octant(p);
     k = k << 3 | (unsigned)o;
-    w.descend(o);
+    w.descend(o, t->step[d]);
   }
   key[i] = k;
   val[i] = (int32_t)i;
 }
 
-// Octants that points a and b share beyond the first `from` (which they
-// share), up to kTieDepth; less: a's path is the smaller one.
-__device__ int shared_octants(const double* P, int32_t a, int32_t b, const double* rc, double rw,
-                              bool& less) {
+// Octants that points a and b share, up to kTieDepth; less: a's path is the
+// smaller one.
+__device__ int shared_octants(const double* P, int32_t a, int32_t b, const double* rc,
+                              const Widths* t, bool& less) {
   const double pa[3] = {P[(int64_t)a * 3], P[(int64_t)a * 3 + 1], P[(int64_t)a * 3 + 2]};
   const double pb[3] = {P[(int64_t)b * 3], P[(int64_t)b * 3 + 1], P[(int64_t)b * 3 + 2]};
-  Walk w{{rc[0], rc[1], rc[2]}, rw};
+  Walk w{{rc[0], rc[1], rc[2]}};
   less = false;
   for (int d = 0; d < kTieDepth; ++d) {
     const int oa = w.octant(pa), ob = w.octant(pb);
@@ -466,14 +481,14 @@ __device__ int shared_octants(const double* P, int32_t a, int32_t b, const doubl
       less = oa < ob;
       return d;
     }
-    w.descend(oa);
+    w.descend(oa, t->step[d]);
   }
   return kTieDepth;
 }
 
 // Runs of equal keys, ordered by the octants past the key: one thread per run.
 __global__ void tie_runs_kernel(const double* __restrict__ P, int64_t n,
-                                const double* __restrict__ rc, const double* __restrict__ rw,
+                                const double* __restrict__ rc, const Widths* __restrict__ t,
                                 const unsigned long long* __restrict__ key, int32_t* val,
                                 PathTotals* __restrict__ tot) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -489,7 +504,7 @@ __global__ void tie_runs_kernel(const double* __restrict__ P, int64_t n,
     int64_t j = i;
     while (j > p) {
       bool less;
-      if (shared_octants(P, v, val[j - 1], rc, *rw, less) == kTieDepth) tot->deep = 1;
+      if (shared_octants(P, v, val[j - 1], rc, t, less) == kTieDepth) tot->deep = 1;
       if (!less) break;
       val[j] = val[j - 1];
       --j;
@@ -501,7 +516,7 @@ __global__ void tie_runs_kernel(const double* __restrict__ P, int64_t n,
 // cpl[p] and, per point, how many internal cells start at it.
 __global__ void __launch_bounds__(256) cpl_kernel(const double* __restrict__ P, int64_t n,
                                                   const double* __restrict__ rc,
-                                                  const double* __restrict__ rw,
+                                                  const Widths* __restrict__ t, int kd,
                                                   const unsigned long long* __restrict__ key,
                                                   const int32_t* __restrict__ val,
                                                   int8_t* __restrict__ cpl,
@@ -511,9 +526,9 @@ __global__ void __launch_bounds__(256) cpl_kernel(const double* __restrict__ P, 
   auto shared = [&](int64_t q) {  // octants shared by the sorted points q - 1 and q
     if (q <= 0 || q >= n) return -1;
     const unsigned long long x = key[q - 1] ^ key[q];
-    if (x) return (__clzll((long long)x) - 1) / 3;
+    if (x) return (__clzll((long long)x) - (64 - 3 * kd)) / 3;
     bool less;
-    const int d = shared_octants(P, val[q - 1], val[q], rc, *rw, less);
+    const int d = shared_octants(P, val[q - 1], val[q], rc, t, less);
     if (d == kTieDepth) tot->deep = 1;
     return d;
   };
@@ -534,12 +549,12 @@ __global__ void __launch_bounds__(256) cpl_kernel(const double* __restrict__ P, 
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long t = 0;
+    unsigned long long sum = 0;
     for (int w = 0; w < 8; ++w) {
-      t += s[w];
+      sum += s[w];
       mx = max(mx, m[w]);
     }
-    atomicAdd(&tot->nindices, t);
+    atomicAdd(&tot->nindices, sum);
     if (mx > tot->max_cpl) atomicMax(&tot->max_cpl, mx);
   }
 }
@@ -567,7 +582,7 @@ __global__ void list_cells_kernel(const int8_t* __restrict__ cpl, const uint32_t
 // [p, e), child o's those whose octant at this depth is o.
 __global__ void __launch_bounds__(256) cells_kernel(
     const double* __restrict__ P, int64_t n, const double* __restrict__ rc,
-    const double* __restrict__ rw, const unsigned long long* __restrict__ key,
+    const Widths* __restrict__ t, int kd, const unsigned long long* __restrict__ key,
     const int32_t* __restrict__ val, const int8_t* __restrict__ cpl,
     const uint32_t* __restrict__ base, uint32_t ninternal, const int32_t* __restrict__ cell_first,
     const int8_t* __restrict__ cell_depth, double* __restrict__ cn, double* __restrict__ cw,
@@ -583,15 +598,14 @@ __global__ void __launch_bounds__(256) cells_kernel(
   const int32_t pt = live ? val[p] : 0;
   // centre: lane o follows axis o mod 3 down the path of the cell's first point
   const int axis = o % 3;
-  double c = rc[axis], w = *rw;
+  double c = rc[axis];
   const double x = P[(int64_t)pt * 3 + axis];
   const int dmax = __reduce_max_sync(full, d);
   for (int l = 0; l < dmax; ++l) {
     if (l < d) {
-      const bool up = l < kKeyDepth ? (kp >> (60 - 3 * l + axis)) & 1ull : x >= c;
-      const double h = __dmul_rn(w, 0.5), hh = __dmul_rn(h, 0.5);
-      c = __dadd_rn(c, up ? hh : -hh);
-      w = h;
+      const bool up = l < kd ? (kp >> (3 * (kd - 1 - l) + axis)) & 1ull : x >= c;
+      const double step = t->step[l];
+      c = __dadd_rn(c, up ? step : -step);
     }
   }
   double cc[3];
@@ -599,11 +613,11 @@ __global__ void __launch_bounds__(256) cells_kernel(
   // end of the cell: the first position past p that leaves its path
   int64_t e = n, lb = p;
   if (live) {
-    if (d > kKeyDepth) {
+    if (d > kd) {
       e = p + 1;
       while (e < n && cpl[e] >= d) ++e;
     } else if (d > 0) {
-      const int sh = 63 - 3 * d;
+      const int sh = 3 * (kd - d);
       const unsigned long long top = kp >> sh;
       int64_t step = 1, a = p, b = p + 1;  // a inside, b the first known outside
       while (b < n && (key[b] >> sh) == top) {
@@ -620,7 +634,7 @@ __global__ void __launch_bounds__(256) cells_kernel(
       e = b;
     }
     // first point of the cell with octant >= o
-    if (d >= kKeyDepth) {
+    if (d >= kd) {
       while (lb < e) {
         const int32_t q = val[lb];
         const int oq = (P[(int64_t)q * 3] >= cc[0] ? 1 : 0) +
@@ -630,7 +644,7 @@ __global__ void __launch_bounds__(256) cells_kernel(
         ++lb;
       }
     } else if (o > 0) {
-      const int sh = 60 - 3 * d;
+      const int sh = 3 * (kd - 1 - d);
       int64_t a = p - 1, b = e;  // octant(a) < o <= octant(b)
       while (b - a > 1) {
         const int64_t m = (a + b) >> 1;
@@ -644,11 +658,11 @@ __global__ void __launch_bounds__(256) cells_kernel(
   if (!live) return;
   const int64_t cnt = (o == 7 ? e : up) - lb;
   const int64_t id = 1 + 8 * r + o;
-  const double h = __dmul_rn(w, 0.5), hh = __dmul_rn(h, 0.5);
+  const double hh = t->step[d];
   cn[id * 3 + 0] = __dadd_rn(cc[0], (o & 1) ? hh : -hh);
   cn[id * 3 + 1] = __dadd_rn(cc[1], (o & 2) ? hh : -hh);
   cn[id * 3 + 2] = __dadd_rn(cc[2], (o & 4) ? hh : -hh);
-  cw[id] = h;
+  cw[id] = t->w[d + 1];
   start[id] = lb;
   count[id] = (int32_t)cnt;
   depth[id] = d + 1;
@@ -665,7 +679,7 @@ __global__ void __launch_bounds__(256) cells_kernel(
     cn[0] = rc[0];
     cn[1] = rc[1];
     cn[2] = rc[2];
-    cw[0] = *rw;
+    cw[0] = t->w[0];
     start[0] = 0;
     count[0] = (int32_t)n;
     depth[0] = 0;
@@ -782,22 +796,33 @@ static bool octree_build_paths(gwn_octree_impl& t, const double* dP, int64_t n, 
   DevBuf<int8_t> cpl(N, st);
   DevBuf<uint32_t> starts(N, st), base(N, st);
   DevBuf<PathTotals> tot(1, st);
-  tot.zero(st);
-  launch_kernel(path_keys_kernel, blocks(n), 256, 0, st, dP, n, rc, rw, key.get(), val.get());
-  radix_sort_pairs<unsigned long long>(key.get(), val.get(), key_tmp.get(), val_tmp.get(), n, 0,
-                                       3 * kKeyDepth, st);
-  launch_kernel(tie_runs_kernel, blocks(n), 256, 0, st, dP, n, rc, rw,
-                (const unsigned long long*)key.get(), val.get(), tot.get());
-  launch_kernel(cpl_kernel, blocks(n), 256, 0, st, dP, n, rc, rw,
-                (const unsigned long long*)key.get(), (const int32_t*)val.get(), cpl.get(),
-                starts.get(), tot.get());
-  exclusive_scan_u32(starts.get(), base.get(), n, st);
-  launch_kernel(path_totals_kernel, 1, 1, 0, st, (const uint32_t*)base.get(),
-                (const uint32_t*)(starts.get() + (n - 1)), n, tot.get());
+  DevBuf<Widths> widths(1, st);
   PathTotals* h = reinterpret_cast<PathTotals*>(pinned_words());
-  GWN_CUDA(cudaMemcpyAsync(h, tot.get(), sizeof(PathTotals), cudaMemcpyDeviceToHost, st));
-  GWN_CUDA(cudaStreamSynchronize(st));
-  if (h->deep) return false;
+  const Widths* wt = widths.get();
+  launch_kernel(widths_kernel, 1, 1, 0, st, rw, widths.get());
+  // Octants per key: points spread over a surface share about log2(n) / 2, so
+  // 10 (four passes) and 16 (six) leave few equal keys to 4096 and 16M points.
+  int kd = n <= 4096 ? 10 : (n <= (int64_t(16) << 20) ? 16 : kKeyDepth);
+  for (;;) {
+    tot.zero(st);
+    launch_kernel(path_keys_kernel, blocks(n), 256, 0, st, dP, n, rc, wt, kd, key.get(),
+                  val.get());
+    radix_sort_pairs<unsigned long long>(key.get(), val.get(), key_tmp.get(), val_tmp.get(), n, 0,
+                                         3 * kd, st);
+    launch_kernel(tie_runs_kernel, blocks(n), 256, 0, st, dP, n, rc, wt,
+                  (const unsigned long long*)key.get(), val.get(), tot.get());
+    launch_kernel(cpl_kernel, blocks(n), 256, 0, st, dP, n, rc, wt, kd,
+                  (const unsigned long long*)key.get(), (const int32_t*)val.get(), cpl.get(),
+                  starts.get(), tot.get());
+    exclusive_scan_u32(starts.get(), base.get(), n, st);
+    launch_kernel(path_totals_kernel, 1, 1, 0, st, (const uint32_t*)base.get(),
+                  (const uint32_t*)(starts.get() + (n - 1)), n, tot.get());
+    GWN_CUDA(cudaMemcpyAsync(h, tot.get(), sizeof(PathTotals), cudaMemcpyDeviceToHost, st));
+    GWN_CUDA(cudaStreamSynchronize(st));
+    if (!h->deep) break;
+    if (kd == kKeyDepth) return false;
+    kd = kKeyDepth;
+  }
   const uint32_t ni = h->ninternal;
   t.ncells = 1 + 8 * (int64_t)ni;
   GWN_REQUIRE(t.ncells < (int64_t(1) << 31), "octree has more than 2^31 cells");
@@ -814,7 +839,7 @@ static bool octree_build_paths(gwn_octree_impl& t, const double* dP, int64_t n, 
   DevBuf<int8_t> cell_depth(ni, st);
   launch_kernel(list_cells_kernel, blocks(n), 256, 0, st, (const int8_t*)cpl.get(),
                 (const uint32_t*)base.get(), n, ni, cell_first.get(), cell_depth.get());
-  launch_kernel(cells_kernel, blocks((int64_t)ni * 8), 256, 0, st, dP, n, rc, rw,
+  launch_kernel(cells_kernel, blocks((int64_t)ni * 8), 256, 0, st, dP, n, rc, wt, kd,
                 (const unsigned long long*)key.get(), (const int32_t*)val.get(),
                 (const int8_t*)cpl.get(), (const uint32_t*)base.get(), ni,
                 (const int32_t*)cell_first.get(), (const int8_t*)cell_depth.get(), t.cn.get(),
