@@ -164,7 +164,51 @@ __global__ void empty_cells_kernel(const int32_t* __restrict__ count, int64_t nc
   area[c] = 0.0;
 }
 
-// Pass 2: max |p - CM| and the order-1/2 moments about CM (1 + 36 doubles).
+// Order-1 / order-2 moments of points about CM, and the largest |p - CM|^2
+// (the root of the largest square is the largest root).  The order-2 tensor is
+// symmetric in its first two indices: 6 x 3 sums, each product formed once,
+// 48 FP64 operations per point in place of 84 (the FP64 pipe bounds both
+// passes: 2M points, large cells 2.31 ms, small cells 1.30 ms).
+template <int NT>
+struct CellSums {
+  static constexpr int kSums = NT == 39 ? 27 : (NT == 12 ? 9 : 0);
+  double mx2 = 0;
+  double s[kSums > 0 ? kSums : 1] = {};
+
+  __device__ __forceinline__ void add(double a, const double* pt, const double* n) {
+    mx2 = fmax(mx2, __dadd_rn(__dadd_rn(__dmul_rn(pt[0], pt[0]), __dmul_rn(pt[1], pt[1])),
+                              __dmul_rn(pt[2], pt[2])));
+    if (NT < 12) return;
+    const double ap[3] = {a * pt[0], a * pt[1], a * pt[2]};
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+#pragma unroll
+      for (int u = 0; u < 3; ++u) s[u + 3 * v] += ap[u] * n[v];
+    if (NT < 39) return;
+    int i = 9;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double h = 0.5 * pt[k];
+#pragma unroll
+      for (int u = k; u < 3; ++u) {
+        const double m = h * ap[u];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) s[i++] += m * n[v];
+      }
+    }
+  }
+};
+// Column of the reference's EC row (after its first three) -> index into
+// CellSums::s.
+__host__ __device__ __forceinline__ int sum_of_term(int t) {
+  if (t < 9) return t;
+  const int k = (t - 9) / 9, u = (t - 9) % 3, v = (t - 9) % 9 / 3;
+  const int a = k < u ? k : u, b = k < u ? u : k;
+  return 9 + 3 * (a == 0 ? b : a + b + 1) + v;
+}
+
+// Pass 2: max |p - CM|^2 and the order-1/2 moments about CM (kPart doubles).
+constexpr int kPart = 28;
 template <int NT>
 __global__ void pass2_kernel(CsrView v, const int32_t* __restrict__ chunk_cell,
                              const unsigned* __restrict__ chunk_base, int64_t nchunks,
@@ -179,46 +223,24 @@ __global__ void pass2_kernel(CsrView v, const int32_t* __restrict__ chunk_cell,
   const int64_t s = v.start[c] + off;
   const int32_t cnt = (int32_t)min((int64_t)kChunk, (int64_t)v.count[c] - off);
   const double cm[3] = {CM[c * 3], CM[c * 3 + 1], CM[c * 3 + 2]};
-  double mx = 0;
-  double acc[NT > 3 ? NT - 3 : 1];
-#pragma unroll
-  for (int k = 0; k < NT - 3; ++k) acc[k] = 0;
+  CellSums<NT> sums;
   for (int j = lane; j < cnt; j += 32) {
     const int64_t p = v.idx[s + j];
-    const double a = A[p];
     double pt[3], n[3];
     for (int d = 0; d < 3; ++d) {
       pt[d] = P[p * 3 + d] - cm[d];
       n[d] = N[p * 3 + d];
     }
-    const double nrm = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(pt[0], pt[0]), __dmul_rn(pt[1], pt[1])),
-                                      __dmul_rn(pt[2], pt[2])));
-    mx = fmax(mx, nrm);
-    if (NT >= 12) {
-#pragma unroll
-      for (int vv = 0; vv < 3; ++vv)
-#pragma unroll
-        for (int u = 0; u < 3; ++u) acc[u + 3 * vv] += (a * pt[u]) * n[vv];
-    }
-    if (NT == 39) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double h = 0.5 * pt[k];
-#pragma unroll
-        for (int vv = 0; vv < 3; ++vv)
-#pragma unroll
-          for (int u = 0; u < 3; ++u) acc[9 + 9 * k + u + 3 * vv] += h * ((a * pt[u]) * n[vv]);
-      }
-    }
+    sums.add(A[p], pt, n);
   }
-  mx = warp_max(mx);
+  const double mx2 = warp_max(sums.mx2);
 #pragma unroll
-  for (int k = 0; k < NT - 3; ++k) acc[k] = warp_sum(acc[k]);
+  for (int k = 0; k < sums.kSums; ++k) sums.s[k] = warp_sum(sums.s[k]);
   if (lane == 0) {
-    double* o = part + w * 37;
-    o[0] = mx;
+    double* o = part + w * kPart;
+    o[0] = mx2;
 #pragma unroll
-    for (int k = 0; k < NT - 3; ++k) o[1 + k] = acc[k];
+    for (int k = 0; k < sums.kSums; ++k) o[1 + k] = sums.s[k];
   }
 }
 
@@ -232,15 +254,27 @@ __global__ void combine2_kernel(const int32_t* __restrict__ chunk_cell,
   if (w >= nchunks) return;
   const int32_t c = chunk_cell[w];
   if ((unsigned)w != chunk_base[c]) return;  // not the cell's first chunk
-  double mx = 0;
-  for (unsigned j = lane; j < nch[c]; j += 32) mx = fmax(mx, part[(chunk_base[c] + j) * 37]);
-  mx = warp_max(mx);
-  if (lane == 0) R[c] = mx;
-  for (int k = 3; k < num_terms; ++k) {
-    double s = 0;
-    for (unsigned j = lane; j < nch[c]; j += 32) s += part[(chunk_base[c] + j) * 37 + (k - 2)];
-    s = warp_sum(s);
-    if (lane == 0) EC[c * num_terms + k] = s;
+  const double* first = part + (int64_t)chunk_base[c] * kPart;
+  double mx2 = 0;
+  for (unsigned j = lane; j < nch[c]; j += 32) mx2 = fmax(mx2, first[(int64_t)j * kPart]);
+  mx2 = warp_max(mx2);
+  if (lane == 0) R[c] = sqrt(mx2);
+  // a lane per sum; chunks j, j + 1 .. j + 7 in partial sums of their own, so
+  // that the largest cells' thousands of chunks are not one chain of loads
+  const int nsums = num_terms == 39 ? 27 : (num_terms == 12 ? 9 : 0);
+  double s = 0;
+  if (lane < nsums) {
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const unsigned nc = nch[c];
+    for (unsigned j = 0; j < nc; j += 8)
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (j + k < nc) acc[k] += first[(int64_t)(j + k) * kPart + 1 + lane];
+    for (int k = 0; k < 8; ++k) s += acc[k];
+  }
+  for (int k = lane; k < ((num_terms - 3 + 31) & ~31); k += 32) {
+    const double t = __shfl_sync(0xffffffffu, s, k < num_terms - 3 ? sum_of_term(k) : 0);
+    if (k < num_terms - 3) EC[c * num_terms + 3 + k] = t;
   }
 }
 
@@ -255,7 +289,8 @@ __device__ __forceinline__ void small_cell_moments(CsrView v, int64_t c, int32_t
                                                         double* __restrict__ CM,
                                                         double* __restrict__ R,
                                                         double* __restrict__ area,
-                                                        double* __restrict__ row) {
+                                                        double* __restrict__ first,
+                                                        CellSums<NT>& sums) {
   const int64_t s0 = v.start[c];
   double s[7] = {0, 0, 0, 0, 0, 0, 0};
   for (int j = 0; j < cnt; ++j) {
@@ -272,43 +307,18 @@ __device__ __forceinline__ void small_cell_moments(CsrView v, int64_t c, int32_t
   for (int d = 0; d < 3; ++d) {
     cm[d] = s[1 + d] / s[0];
     CM[c * 3 + d] = cm[d];
-    row[d] = s[4 + d];
+    first[d] = s[4 + d];
   }
-  double mx = 0;
-  double acc[NT > 3 ? NT - 3 : 1];
-#pragma unroll
-  for (int k = 0; k < NT - 3; ++k) acc[k] = 0;
   for (int j = 0; j < cnt; ++j) {
     const int64_t p = v.idx[s0 + j];
-    const double a = A[p];
     double pt[3], n[3];
     for (int d = 0; d < 3; ++d) {
       pt[d] = P[p * 3 + d] - cm[d];
       n[d] = N[p * 3 + d];
     }
-    const double nrm = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(pt[0], pt[0]), __dmul_rn(pt[1], pt[1])),
-                                      __dmul_rn(pt[2], pt[2])));
-    mx = fmax(mx, nrm);
-    if (NT >= 12) {
-#pragma unroll
-      for (int vv = 0; vv < 3; ++vv)
-#pragma unroll
-        for (int u = 0; u < 3; ++u) acc[u + 3 * vv] += (a * pt[u]) * n[vv];
-    }
-    if (NT == 39) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double h = 0.5 * pt[k];
-#pragma unroll
-        for (int vv = 0; vv < 3; ++vv)
-#pragma unroll
-          for (int u = 0; u < 3; ++u) acc[9 + 9 * k + u + 3 * vv] += h * ((a * pt[u]) * n[vv]);
-      }
-    }
+    sums.add(A[p], pt, n);
   }
-  R[c] = mx;
-#pragma unroll
-  for (int k = 0; k < NT - 3; ++k) row[3 + k] = acc[k];
+  R[c] = sqrt(sums.mx2);
 }
 
 // Small non-empty cells grouped by point count (a counting sort on
@@ -390,7 +400,10 @@ __global__ void __launch_bounds__(128) small_cells_kernel(CsrView v, const int32
                                                           double* __restrict__ R,
                                                           double* __restrict__ EC,
                                                           double* __restrict__ area) {
-  __shared__ double rows[4][32 * NT];
+  // half a warp's rows at a time: more shared memory would leave little L1 for
+  // the points, which every level's cells read again (2M points: 2.10 ms with
+  // 32 rows, 5 CTAs per SM)
+  __shared__ double rows[4][16 * NT];
   __shared__ int32_t cells[4][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t i0 = (blockIdx.x * (int64_t)blockDim.x) + warp * 32;  // first entry of the warp
@@ -398,13 +411,23 @@ __global__ void __launch_bounds__(128) small_cells_kernel(CsrView v, const int32
   const int64_t i = i0 + lane;
   const int32_t c = i < n ? list[i] : -1;
   cells[warp][lane] = c;
-  if (c >= 0)
-    small_cell_moments<NT>(v, c, v.count[c], P, N, A, CM, R, area, rows[warp] + lane * NT);
-  __syncwarp();
+  double first[3] = {0, 0, 0};
+  CellSums<NT> sums;
+  if (c >= 0) small_cell_moments<NT>(v, c, v.count[c], P, N, A, CM, R, area, first, sums);
   const int nrows = n - i0 < 32 ? (int)(n - i0) : 32;
-  for (int r = 0; r < nrows; ++r) {
-    double* out = EC + (int64_t)cells[warp][r] * NT;
-    for (int e = lane; e < NT; e += 32) out[e] = rows[warp][r * NT + e];
+  for (int half = 0; half < 32 && half < nrows; half += 16) {
+    __syncwarp();
+    if (lane >= half && lane < half + 16) {
+      double* row = rows[warp] + (lane - half) * NT;
+      for (int d = 0; d < 3; ++d) row[d] = first[d];
+#pragma unroll
+      for (int k = 0; k < NT - 3; ++k) row[3 + k] = sums.s[sum_of_term(k)];
+    }
+    __syncwarp();
+    for (int r = half; r < min(half + 16, nrows); ++r) {
+      double* out = EC + (int64_t)cells[warp][r] * NT;
+      for (int e = lane; e < NT; e += 32) out[e] = rows[warp][(r - half) * NT + e];
+    }
   }
 }
 
@@ -478,7 +501,9 @@ __global__ void emit_nodes_kernel(LayoutIn in, CloudNodeF* __restrict__ nf,
   CloudNodeD D;
   for (int d = 0; d < 3; ++d) D.cm[d] = in.CM[(int64_t)c * 3 + d];
   D.r = in.R[c];
-  {
+  if (leaf) {  // the walks take a leaf's points, never its expansion
+    for (int k = 0; k < 15; ++k) D.pk[k] = 0.0;
+  } else {
     double ec[39];
     for (int k = 0; k < 39; ++k) ec[k] = k < in.num_terms ? in.EC[(int64_t)c * in.num_terms + k] : 0.0;
     pack_cloud(ec, in.num_terms, D.pk);
@@ -608,9 +633,9 @@ __device__ __forceinline__ void read_q(const QT* Q, const int32_t* perm, const i
 // its own values by its bit mask of queue positions, in queue order, which
 // is its walk order.  The mixed walk queues its FP64 near-field terms here,
 // the plain FP64 walk every term.  The lanes' FP64 queries live here too
-// (read only at FP64 re-checks and flushes), and the mixed walk runs 8
-// blocks of 128 threads per SM (64 registers; with the division-free FP32
-// terms, 18.2 -> 17.4 ms for C3's 8M queries against 6).
+// (read only at FP64 re-checks and flushes), and the mixed walk runs 7
+// blocks of 128 threads per SM (72 registers): 2M points, 8M queries with 8 / 7
+// / 6 / 5 blocks 7.84 / 7.24 / 7.81 / 8.88 ms (with 8, spills took 72% of L1).
 struct CloudNearQueue {
   int2 e[32];
   double q[32][3];  // each lane's FP64 query
@@ -700,7 +725,7 @@ __device__ __forceinline__ void queue_points64(const CloudEvalParams& prm, Cloud
 }
 
 template <typename QT, typename WT>
-__global__ void __launch_bounds__(128, 8) cloud_eval_mixed_kernel(CloudEvalParams prm, const QT* __restrict__ Q,
+__global__ void __launch_bounds__(128, 7) cloud_eval_mixed_kernel(CloudEvalParams prm, const QT* __restrict__ Q,
                                                                const int32_t* __restrict__ perm,
                                                                int64_t nQ, WT* __restrict__ W,
                                                                int32_t* __restrict__ refine_list,
@@ -976,7 +1001,7 @@ void precompute(gwn_cloud_impl& c, const CsrView& v, int64_t ncells, const doubl
   const int64_t nchunks = (int64_t)last_n + last_b;
   DevBuf<int32_t> chunk_cell((size_t)std::max<int64_t>(nchunks, 1), st);
   launch_kernel(chunk_fill_kernel, blocks(ncells), 256, 0, st, nch.get(), cbase.get(), ncells, chunk_cell.get());
-  DevBuf<double> part((size_t)std::max<int64_t>(nchunks, 1) * 37, st);
+  DevBuf<double> part((size_t)std::max<int64_t>(nchunks, 1) * kPart, st);
   if (nchunks)
     launch_kernel(pass1_kernel, blocks(nchunks * 32), 256, 0, st, v, chunk_cell.get(), cbase.get(), nchunks, P,
                                                       N, A, part.get());
@@ -1116,15 +1141,15 @@ void cloud_build(gwn_cloud_impl& c, const gwn_octree_impl& t, const double* N, c
     throw Error(GWN_ERR_INTERNAL, "cloud records are not 32-byte aligned");
   c.nd.alloc((size_t)std::max<int64_t>(nnodes, 1));
   finish_extent(c, st);
-  LayoutIn in{val.get(), nullptr, nullptr, key.get(), nnodes, t.start.get(), t.count.get(), t.ch.get(),
-              t.depth.get(), c.CM.get(), c.R.get(), c.EC.get(), c.num_terms, c.area.get(), c.eps,
-              c.cmax};
-  if (nnodes) launch_kernel(emit_nodes_kernel, blocks(nnodes), 256, 0, st, in, c.nf.get(), c.nd.get());
   c.pf.alloc((size_t)std::max<int64_t>(n, 1) * 2);
   c.pd.alloc((size_t)std::max<int64_t>(n, 1) * 6);
   if (n)
     launch_kernel(emit_points_kernel, blocks(n), 256, 0, st, t.perm.get(), n, c.P.get(), c.AN.get(),
                   c.eps, c.cmax, c.pf.get(), c.pd.get());
+  LayoutIn in{val.get(), nullptr, nullptr, key.get(), nnodes, t.start.get(), t.count.get(), t.ch.get(),
+              t.depth.get(), c.CM.get(), c.R.get(), c.EC.get(), c.num_terms, c.area.get(), c.eps,
+              c.cmax};
+  if (nnodes) launch_kernel(emit_nodes_kernel, blocks(nnodes), 256, 0, st, in, c.nf.get(), c.nd.get());
   c.bytes += c.nf.bytes() + c.nd.bytes() + c.pf.bytes() + c.pd.bytes();
 }
 
