@@ -4,10 +4,13 @@
 // point-cloud winding number its areas A from a raw scan
 // (copyleft/cgal/fast_winding_number.cpp:30-38).
 //
-// A warp takes 32 points: their kept neighbours' mean and scatter matrix
-// point by point (lane j holds neighbours j, j + 32, ...), the 3 x 3
-// eigenproblems lane by lane (one point each), then point by point the
-// plane and the triangulation.  GB300 runs FP64 far slower than FP32, so
+// A warp takes 32 points: the kept neighbours' mean and scatter matrix and the
+// 3 x 3 eigenproblems lane by lane (one point each), then point by point the
+// plane and the triangulation, whose triangles are queued and valued 32 at a
+// time.  The FP64 pipe bounds the kernel and charges a warp instruction the
+// same for 1 or 32 lanes: with the sums of each point over the warp (45
+// additions of shuffles for 21 neighbours) and its half dozen triangles alone,
+// 200,000 points took 3.27 ms.  GB300 runs FP64 far slower than FP32, so
 // the hull's orientation tests run in FP32 with an error bound and fall
 // back to FP64 only where the sign is not certain.  Per point, as the
 // reference:
@@ -52,17 +55,13 @@ namespace {
 constexpr int kWarps = 4;  // points per CTA
 
 struct PaShared {
-  double p[kPointAreasMaxK][3];  // kept neighbours, in order
   double u[kPointAreasMaxK], w[kPointAreasMaxK];    // plane coordinates
   double su[kPointAreasMaxK], sw[kPointAreasMaxK];  // images under inversion about vertex 0
   float fu[kPointAreasMaxK], fw[kPointAreasMaxK];   // the images rounded to FP32
   unsigned char ok[kPointAreasMaxK];                // image usable (distinct, not vertex 0)
+  double tri[32][6];  // queued triangles: vertex 0 and the two others in the plane
+  double share[32];   // their shares
 };
-
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // Eigen-decomposition of the symmetric 3 x 3 matrix a (cyclic Jacobi);
 // returns eigenvalues d and eigenvectors as the columns of v, sorted by
@@ -144,37 +143,43 @@ __device__ __forceinline__ double orient(double ax, double ay, double bx, double
   return (bx - ax) * (cy - ay) - (by - ay) * (cx - ax);
 }
 
-// Kept neighbours of point i into S.p (the reference's normal filter);
-// returns their number (-1 when an index lies outside P).  Warp-uniform.
-__device__ int gather_kept(const double* __restrict__ P, int64_t nP, const int32_t* __restrict__ row,
-                           int k, const double* __restrict__ N, PaShared& S) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
+// A bit per neighbour.
+struct Kept {
+  static_assert(kPointAreasMaxK <= 128, "two words");
+  unsigned long long lo = 0, hi = 0;
+  __device__ __forceinline__ void set(int j) {
+    if (j < 64) lo |= 1ull << j;
+    else hi |= 1ull << (j - 64);
+  }
+  __device__ __forceinline__ bool has(int j) const {
+    return ((j < 64 ? lo >> j : hi >> (j - 64)) & 1ull) != 0;
+  }
+  __device__ __forceinline__ int before(int j) const {  // kept ones below j
+    return j < 64 ? __popcll(lo & ((1ull << j) - 1ull))
+                  : __popcll(lo) + __popcll(hi & ((1ull << (j - 64)) - 1ull));
+  }
+  __device__ __forceinline__ int count() const { return __popcll(lo) + __popcll(hi); }
+};
+
+// Neighbours of a point (row) that the reference's normal filter keeps, and
+// their number (-1 when an index lies outside P).  One point per lane.
+__device__ int kept_neighbours(int64_t nP, const int32_t* __restrict__ row, int k,
+                               const double* __restrict__ N, Kept& kept) {
   const int32_t i0 = row[0];
   if (i0 < 0 || i0 >= nP) return -1;
   const double n0x = N[(int64_t)i0 * 3], n0y = N[(int64_t)i0 * 3 + 1], n0z = N[(int64_t)i0 * 3 + 2];
-  int m = 0;
-  bool any_bad = false;
-  for (int j0 = 0; j0 < k; j0 += 32) {
-    const int j = j0 + lane;
-    const int32_t idx = j < k ? row[j] : -1;
-    const bool bad = j < k && (idx < 0 || idx >= nP);
-    bool keep = j < k && !bad;
-    if (keep && k > 1) {
-      const double* nj = N + (int64_t)idx * 3;
-      keep = n0x * nj[0] + n0y * nj[1] + n0z * nj[2] > 0;
+  bool bad = false;
+#pragma unroll 4
+  for (int j = 0; j < k; ++j) {
+    const int32_t idx = row[j];
+    if (idx < 0 || idx >= nP) {
+      bad = true;
+      continue;
     }
-    any_bad |= __any_sync(full, bad);
-    const unsigned b = __ballot_sync(full, keep);
-    if (keep) {
-      const int pos = m + __popc(b & lt);
-      for (int d = 0; d < 3; ++d) S.p[pos][d] = P[(int64_t)idx * 3 + d];
-    }
-    m += __popc(b);
+    const double* nj = N + (int64_t)idx * 3;
+    if (k == 1 || n0x * nj[0] + n0y * nj[1] + n0z * nj[2] > 0) kept.set(j);
   }
-  __syncwarp();
-  return any_bad ? -1 : m;
+  return bad ? -1 : kept.count();
 }
 
 // Sign of orient(a, b, c) for the images: FP32 when its error bound
@@ -201,41 +206,33 @@ __global__ void __launch_bounds__(32 * kWarps) point_areas_kernel(
   const int64_t nwarps = (int64_t)gridDim.x * kWarps;
   for (int64_t base = ((int64_t)blockIdx.x * kWarps + wib) * 32; base < nP; base += nwarps * 32) {
     const int np = (int)(nP - base < 32 ? nP - base : 32);
-    // ---- stage A, point by point: kept count, mean and scatter matrix;
-    // lane t keeps point base + t's
+    // ---- stage A, lane per point: kept neighbours, mean and scatter matrix
     int my_m = 0;
+    Kept my_kept;
     double my_mean[3] = {0, 0, 0}, my_c[6] = {0, 0, 0, 0, 0, 0};
-    for (int t = 0; t < np; ++t) {
-      const int m = gather_kept(P, nP, I + (base + t) * k, k, N, S);
-      if (m <= 2) {
-        if (lane == t) my_m = m;
-        __syncwarp();
-        continue;
+    if (lane < np) {
+      const int32_t* row = I + (base + lane) * k;
+      my_m = kept_neighbours(nP, row, k, N, my_kept);
+      if (my_m > 2) {
+        auto each = [&](auto&& f) {
+#pragma unroll 4
+          for (int j = 0; j < k; ++j)
+            if (my_kept.has(j)) f(P + (int64_t)row[j] * 3);
+        };
+        each([&](const double* p) {
+          for (int d = 0; d < 3; ++d) my_mean[d] += p[d];
+        });
+        for (int d = 0; d < 3; ++d) my_mean[d] /= my_m;
+        each([&](const double* p) {
+          const double x = p[0] - my_mean[0], y = p[1] - my_mean[1], z = p[2] - my_mean[2];
+          my_c[0] += x * x;
+          my_c[1] += x * y;
+          my_c[2] += x * z;
+          my_c[3] += y * y;
+          my_c[4] += y * z;
+          my_c[5] += z * z;
+        });
       }
-      double s0 = 0, s1 = 0, s2 = 0;
-      for (int j = lane; j < m; j += 32) {
-        s0 += S.p[j][0];
-        s1 += S.p[j][1];
-        s2 += S.p[j][2];
-      }
-      const double mean[3] = {warp_sum(s0) / m, warp_sum(s1) / m, warp_sum(s2) / m};
-      double c[6] = {0, 0, 0, 0, 0, 0};
-      for (int j = lane; j < m; j += 32) {
-        const double x = S.p[j][0] - mean[0], y = S.p[j][1] - mean[1], z = S.p[j][2] - mean[2];
-        c[0] += x * x;
-        c[1] += x * y;
-        c[2] += x * z;
-        c[3] += y * y;
-        c[4] += y * z;
-        c[5] += z * z;
-      }
-      for (int q = 0; q < 6; ++q) c[q] = warp_sum(c[q]);
-      if (lane == t) {
-        my_m = m;
-        for (int d = 0; d < 3; ++d) my_mean[d] = mean[d];
-        for (int q = 0; q < 6; ++q) my_c[q] = c[q];
-      }
-      __syncwarp();
     }
     // ---- stage B, lane per point: principal directions, T, A for the
     // degenerate cases
@@ -264,7 +261,25 @@ __global__ void __launch_bounds__(32 * kWarps) point_areas_kernel(
         for (int d = 0; d < 3; ++d) T[i * 3 + d] = t[d];
       }
     }
-    // ---- stage C, point by point: plane, Delaunay star, area
+    // ---- stage C, point by point: plane, Delaunay star; lane t adds the
+    // shares of point t's triangles in the order they were found
+    double my_area = 0.0;
+    int queued = 0;     // triangles in the queue (warp-uniform)
+    unsigned mine = 0;  // queue positions of this lane's point
+    auto flush = [&]() {
+      __syncwarp();
+      if (lane < queued) {
+        const double* q = S.tri[lane];
+        S.share[lane] = voronoi_share(q[0], q[1], q[2], q[3], q[4], q[5]);
+      }
+      __syncwarp();
+      while (mine) {
+        my_area += S.share[__ffs(mine) - 1];
+        mine &= mine - 1;
+      }
+      queued = 0;
+      __syncwarp();
+    };
     for (int t = 0; t < np; ++t) {
       const int m = __shfl_sync(0xffffffffu, my_m, t);
       if (m <= 2) continue;
@@ -274,11 +289,16 @@ __global__ void __launch_bounds__(32 * kWarps) point_areas_kernel(
         e1[d] = __shfl_sync(0xffffffffu, V[d][0], t);
         e2[d] = __shfl_sync(0xffffffffu, V[d][1], t);
       }
-      gather_kept(P, nP, I + (base + t) * k, k, N, S);
-      for (int j = lane; j < m; j += 32) {
-        const double x = S.p[j][0] - mean[0], y = S.p[j][1] - mean[1], z = S.p[j][2] - mean[2];
-        S.u[j] = x * e1[0] + y * e1[1] + z * e1[2];
-        S.w[j] = x * e2[0] + y * e2[1] + z * e2[2];
+      Kept kept;
+      kept.lo = __shfl_sync(0xffffffffu, my_kept.lo, t);
+      kept.hi = __shfl_sync(0xffffffffu, my_kept.hi, t);
+      for (int j = lane; j < k; j += 32) {
+        if (!kept.has(j)) continue;
+        const double* p = P + (int64_t)I[(base + t) * k + j] * 3;
+        const double x = p[0] - mean[0], y = p[1] - mean[1], z = p[2] - mean[2];
+        const int at = kept.before(j);
+        S.u[at] = x * e1[0] + y * e1[1] + z * e1[2];
+        S.w[at] = x * e2[0] + y * e2[1] + z * e2[2];
       }
       __syncwarp();
       const double u0 = S.u[0], w0 = S.w[0];
@@ -299,41 +319,53 @@ __global__ void __launch_bounds__(32 * kWarps) point_areas_kernel(
         S.fw[j] = (float)(qy * inv);
       }
       __syncwarp();
-      double acc = 0.0;
-      for (int j = lane; j < m; j += 32) {
-        if (!S.ok[j]) continue;
+      for (int j0 = 0; j0 < m; j0 += 32) {
+        const int j = j0 + lane;
         int c = -1;
-        for (int l = 1; l < m; ++l) {  // most clockwise image seen from j
-          if (l == j || !S.ok[l]) continue;
-          if (c < 0) {
-            c = l;
-            continue;
+        bool tri = j < m && S.ok[j];
+        if (tri) {
+          for (int l = 1; l < m; ++l) {  // most clockwise image seen from j
+            if (l == j || !S.ok[l]) continue;
+            if (c < 0) {
+              c = l;
+              continue;
+            }
+            const int o = orient_sign(S, j, c, l);
+            if (o < 0) {
+              c = l;
+            } else if (o == 0) {  // collinear: the farther one
+              const double dc = (S.su[c] - S.su[j]) * (S.su[c] - S.su[j]) +
+                                (S.sw[c] - S.sw[j]) * (S.sw[c] - S.sw[j]);
+              const double dl = (S.su[l] - S.su[j]) * (S.su[l] - S.su[j]) +
+                                (S.sw[l] - S.sw[j]) * (S.sw[l] - S.sw[j]);
+              if (dl > dc) c = l;
+            }
           }
-          const int o = orient_sign(S, j, c, l);
-          if (o < 0) {
-            c = l;
-          } else if (o == 0) {  // collinear: the farther one
-            const double dc = (S.su[c] - S.su[j]) * (S.su[c] - S.su[j]) +
-                              (S.sw[c] - S.sw[j]) * (S.sw[c] - S.sw[j]);
-            const double dl = (S.su[l] - S.su[j]) * (S.su[l] - S.su[j]) +
-                              (S.sw[l] - S.sw[j]) * (S.sw[l] - S.sw[j]);
-            if (dl > dc) c = l;
-          }
+          tri = c >= 0;
+          for (int l = 1; tri && l < m; ++l)  // no image strictly right of j -> c
+            if (S.ok[l] && l != j && l != c && orient_sign(S, j, c, l) < 0) tri = false;
+          // vertex 0 (the origin of the images) strictly left of j -> c
+          if (tri) tri = orient(S.su[j], S.sw[j], S.su[c], S.sw[c], 0.0, 0.0) > 0;
         }
-        if (c < 0) continue;
-        bool edge = true;  // no image strictly right of j -> c
-        for (int l = 1; edge && l < m; ++l)
-          if (S.ok[l] && l != j && l != c && orient_sign(S, j, c, l) < 0) edge = false;
-        if (!edge) continue;
-        // vertex 0 (the origin of the images) strictly left of j -> c
-        const double o0 = orient(S.su[j], S.sw[j], S.su[c], S.sw[c], 0.0, 0.0);
-        if (!(o0 > 0)) continue;
-        acc += voronoi_share(u0, w0, S.u[j], S.w[j], S.u[c], S.w[c]);
+        const unsigned b = __ballot_sync(0xffffffffu, tri);
+        const int n = __popc(b);
+        if (queued + n > 32) flush();
+        if (tri) {
+          double* q = S.tri[queued + __popc(b & ((1u << lane) - 1u))];
+          q[0] = u0;
+          q[1] = w0;
+          q[2] = S.u[j];
+          q[3] = S.w[j];
+          q[4] = S.u[c];
+          q[5] = S.w[c];
+        }
+        if (lane == t && n) mine |= (n == 32 ? 0xffffffffu : ((1u << n) - 1u)) << queued;
+        queued += n;
       }
-      const double area = warp_sum(acc);
-      if (lane == 0) A[base + t] = isfinite(area) ? area : 0.0;
       __syncwarp();
     }
+    flush();
+    if (lane < np && my_m > 2) A[base + lane] = isfinite(my_area) ? my_area : 0.0;
   }
 }
 
