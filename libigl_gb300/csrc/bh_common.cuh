@@ -31,9 +31,44 @@ __host__ __device__ inline unsigned long long spread21(unsigned long long x) {
   return x;
 }
 
-// Query ordering for warp coherence: 30-bit Morton key of each query inside
-// a box (lo, inv_extent), sorted; the traversal then reads queries through
-// the returned permutation.
+// Position of cell (x, y, z) of a grid of 2^b cells per axis along the Hilbert
+// curve, as 3 b bits: Skilling's transposition of the coordinates ("Programming
+// the Hilbert curve", 2004), interleaved.  Its leading bits are the position on
+// the coarser grids' curves.
+template <int b>
+__host__ __device__ inline uint32_t hilbert3(uint32_t x, uint32_t y, uint32_t z) {
+  for (uint32_t q = 1u << (b - 1); q > 1; q >>= 1) {
+    const uint32_t p = q - 1;
+    if (x & q) x ^= p;
+    uint32_t t = (x ^ y) & p;
+    if (y & q) {
+      x ^= p;
+    } else {
+      x ^= t;
+      y ^= t;
+    }
+    t = (x ^ z) & p;
+    if (z & q) {
+      x ^= p;
+    } else {
+      x ^= t;
+      z ^= t;
+    }
+  }
+  y ^= x;
+  z ^= y;
+  uint32_t t = 0;
+  for (uint32_t q = 1u << (b - 1); q > 1; q >>= 1)
+    if (z & q) t ^= q - 1;
+  x ^= t;
+  y ^= t;
+  z ^= t;
+  return (spread10(x) << 2) | (spread10(y) << 1) | spread10(z);
+}
+
+// Query ordering for warp coherence: position of each query's cell along a
+// Hilbert curve through a box (lo, inv_extent), sorted; the traversal then
+// reads queries through the returned permutation.
 struct QueryOrder {
   DevBuf<int32_t> perm;
   bool active = false;

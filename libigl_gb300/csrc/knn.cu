@@ -320,7 +320,7 @@ static void knn_t(const gwn_octree_impl& tree, const QT* Q, int64_t nQ, int64_t 
                 (const int32_t*)tree.count.get(), tree.ncells, box.get());
   KnnTree t{box.get(), tree.ch.get(), tree.start.get(), tree.count.get(), tree.perm.get(),
             tree.P.get(), tree.n, (float)cmax};
-  // queries grouped by Morton cell of the root cube, so neighbouring threads
+  // queries along a curve through the root cube, so that neighbouring threads
   // walk the same cells
   double root[4];
   GWN_CUDA(cudaMemcpyAsync(root, tree.cn.get(), 3 * sizeof(double), cudaMemcpyDeviceToHost, st));

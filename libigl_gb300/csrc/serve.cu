@@ -23,7 +23,7 @@
 //              query box, offsets) from pinned host memory;
 //     stage    copy the queries from the pinned host stage into the device
 //              (FP64) and give each a 32-bit key: request index (8 bits),
-//              padding flag, 21-bit Morton code in its mesh's box; each
+//              padding flag, 21-bit Hilbert position in its mesh's box; each
 //              request's queries are padded to a multiple of 32 so that a
 //              warp never spans two requests;
 //     sort     stable radix sort of the keys (4 passes, batch size read on
@@ -70,7 +70,7 @@ constexpr int kBuilders = 4;   // tree builder threads (and streams) per server
 
 struct __align__(16) ServeReq {
   EvalParams prm;     // the request's tree and beta
-  float lo[3], inv[3];  // Morton box of the mesh
+  float lo[3], inv[3];  // ordering box of the mesh
   int64_t q_byte_off;   // queries: byte offset in the host stage
   int64_t out_off;      // first result / device query index (dense)
   int32_t aoff;         // first key position (multiple of 32)
@@ -110,7 +110,7 @@ __global__ void serve_desc_kernel(const uint4* hdesc, uint4* __restrict__ ddesc,
   if (threadIdx.x < 4) counters[threadIdx.x] = 0u;
 }
 
-__device__ __forceinline__ uint32_t morton_cell7(double v, float lo, float inv) {
+__device__ __forceinline__ uint32_t cell7(double v, float lo, float inv) {
   const float t = ((float)v - lo) * inv * 128.f;
   const int c = (int)t;  // NaN -> 0
   return (uint32_t)min(max(c, 0), 127);
@@ -163,9 +163,9 @@ __global__ void __launch_bounds__(256) serve_stage_kernel(const ServeHeader* __r
     for (int k = lane; k < 3 * cnt; k += 32) d[k] = coord(k);
     uint32_t key = (uint32_t)lo << 24;
     if (lane < cnt) {
-      key |= spread10(morton_cell7(coord(3 * lane), R.lo[0], R.inv[0])) |
-             (spread10(morton_cell7(coord(3 * lane + 1), R.lo[1], R.inv[1])) << 1) |
-             (spread10(morton_cell7(coord(3 * lane + 2), R.lo[2], R.inv[2])) << 2);
+      key |= hilbert3<7>(cell7(coord(3 * lane), R.lo[0], R.inv[0]),
+                         cell7(coord(3 * lane + 1), R.lo[1], R.inv[1]),
+                         cell7(coord(3 * lane + 2), R.lo[2], R.inv[2]));
     } else {
       key |= 1u << 23;  // padding lanes sort after the request's queries
     }

@@ -192,8 +192,14 @@ void bucket_order(const uint32_t* keys, int64_t n, uint32_t nbuckets, int32_t* p
   cnt.zero(st);
   const unsigned grid = (unsigned)((n + 255) / 256);
   launch_kernel(bucket_rank_kernel, grid, 256, 0, st, keys, n, cnt.get(), rank.get());
-  exclusive_scan_u32(cnt.get(), cnt.get(), nbuckets, st);
-  launch_kernel(bucket_place_kernel, grid, 256, 0, st, keys, n, cnt.get(), rank.get(), perm);
+  bucket_place(keys, rank.get(), n, cnt.get(), nbuckets, perm, st);
+}
+
+void bucket_place(const uint32_t* keys, const uint32_t* rank, int64_t n, uint32_t* cnt,
+                  uint32_t nbuckets, int32_t* perm, cudaStream_t st) {
+  exclusive_scan_u32(cnt, cnt, nbuckets, st);
+  launch_kernel(bucket_place_kernel, (unsigned)((n + 255) / 256), 256, 0, st, keys, n,
+                (const uint32_t*)cnt, rank, perm);
 }
 
 int64_t scan_scratch_elems(int64_t n) {

@@ -32,6 +32,12 @@ void radix_sort_pairs(K* keys, int32_t* vals, K* keys_tmp, int32_t* vals_tmp, in
 void bucket_order(const uint32_t* keys, int64_t n, uint32_t nbuckets, int32_t* perm,
                   cudaStream_t st);
 
+// Its second half, for a caller whose own kernel counted the buckets: rank[i] =
+// element i's place in its bucket, cnt the buckets' sizes (left as their
+// offsets).
+void bucket_place(const uint32_t* keys, const uint32_t* rank, int64_t n, uint32_t* cnt,
+                  uint32_t nbuckets, int32_t* perm, cudaStream_t st);
+
 // Graph-capturable variant for 32-bit keys: sorts the first min(cap, *n_dev)
 // elements (n_dev is device memory, read when the kernels run) with caller
 // scratch (radix_sort_scratch_elems(cap)); an even number of 8-bit passes,
