@@ -48,6 +48,12 @@ __device__ __forceinline__ D3 daxpy(D3 a, double s, D3 d) {
   return {a.x + s * d.x, a.y + s * d.y, a.z + s * d.z};
 }
 
+// a b - c d without contraction: exactly 0 where a b and c d are the same
+// product, so that a triangle shrunk to a segment has its edges' regions only.
+__device__ __forceinline__ double ddet(double a, double b, double c, double d) {
+  return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d));
+}
+
 __device__ D3 closest_on_triangle(D3 p, D3 a, D3 b, D3 c) {
   const D3 ab = dsub(b, a), ac = dsub(c, a), ap = dsub(p, a);
   const double d1 = ddot(ab, ap), d2 = ddot(ac, ap);
@@ -55,15 +61,15 @@ __device__ D3 closest_on_triangle(D3 p, D3 a, D3 b, D3 c) {
   const D3 bp = dsub(p, b);
   const double d3 = ddot(ab, bp), d4 = ddot(ac, bp);
   if (d3 >= 0.0 && d4 <= d3) return b;
-  const double vc = d1 * d4 - d3 * d2;
+  const double vc = ddet(d1, d4, d3, d2);
   const bool a_is_b = a.x == b.x && a.y == b.y && a.z == b.z;
   if (!a_is_b && vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0) return daxpy(a, d1 / (d1 - d3), ab);
   const D3 cp = dsub(p, c);
   const double d5 = ddot(ab, cp), d6 = ddot(ac, cp);
   if (d6 >= 0.0 && d5 <= d6) return c;
-  const double vb = d5 * d2 - d1 * d6;
+  const double vb = ddet(d5, d2, d1, d6);
   if (vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0) return daxpy(a, d2 / (d2 - d6), ac);
-  const double va = d3 * d6 - d5 * d4;
+  const double va = ddet(d3, d6, d5, d4);
   if (va <= 0.0 && (d4 - d3) >= 0.0 && (d5 - d6) >= 0.0)
     return daxpy(b, (d4 - d3) / ((d4 - d3) + (d5 - d6)), dsub(c, b));
   const double denom = 1.0 / (va + vb + vc);
@@ -78,6 +84,7 @@ struct ClosestParams {
   const int32_t* tri_index;
   int nnodes;
   float cmax;
+  float unit, inv_unit;  // powers of two: cmax * unit in [1, 2) (1 for no or huge extent)
 };
 
 // Stack entries a thread's search may take before a whole warp takes the
@@ -158,30 +165,21 @@ __device__ float dist2_triangle32(float px, float py, float pz, float ax, float 
   return dx * dx + dy * dy + dz * dz;
 }
 
-// FP32 screen of a leaf: true when the triangle is farther than the
-// current best (its FP32 distance minus the triangle's stored slack and the
-// query-rounding slack 1e-6 (S + d) is above the best's upper bound).
-__device__ __forceinline__ bool screened_out(const ClosestParams& prm, int slot, float fx,
-                                             float fy, float fz, float S, float bound) {
-  const float4 t0 = __ldg(&prm.tf[(int64_t)slot * 3]);
-  const float4 t1 = __ldg(&prm.tf[(int64_t)slot * 3 + 1]);
-  const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
-  const float d = sqrtf(dist2_triangle32(fx, fy, fz, t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z,
-                                         t1.w, t2.x));
-  const float lower = d - t2.y - 1e-6f * (S + d);
-  return lower > bound;
-}
-
 // FP32 bounds of the distance from q to a leaf's triangle: its FP32
 // distance minus / plus the triangle's stored slack and the query-rounding
-// slack 1e-6 (S + d).
+// slack 1e-6 (S + d).  The distance is taken in units of the surface's size,
+// because its terms of degree four leave the range of FP32 at coordinates of
+// 1e9 or 1e-9.
 __device__ __forceinline__ void leaf_bounds(const ClosestParams& prm, int slot, float fx, float fy,
                                             float fz, float S, float& lower, float& upper) {
   const float4 t0 = __ldg(&prm.tf[(int64_t)slot * 3]);
   const float4 t1 = __ldg(&prm.tf[(int64_t)slot * 3 + 1]);
   const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
-  const float d = sqrtf(dist2_triangle32(fx, fy, fz, t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z,
-                                         t1.w, t2.x));
+  const float w = prm.unit;
+  const float d = prm.inv_unit *
+                  sqrtf(dist2_triangle32(w * fx, w * fy, w * fz, w * t0.x, w * t0.y, w * t0.z,
+                                         w * t0.w, w * t1.x, w * t1.y, w * t1.z, w * t1.w,
+                                         w * t2.x));
   const float e = t2.y + 1e-6f * (S + d);
   lower = d - e;
   upper = __fadd_ru(d, e);
@@ -820,6 +818,9 @@ void soup_squared_distance(const gwn_soup_impl& s, const void* Q, int q_dtype, i
   prm.tri_index = s.tri_index.get();
   prm.nnodes = (int)s.nnodes;
   prm.cmax = (float)s.cmax;
+  const int exponent = prm.cmax > 0.f && prm.cmax < 1e36f ? std::ilogb(prm.cmax) : 0;
+  prm.unit = std::ldexp(1.f, std::min(-exponent, 120));
+  prm.inv_unit = 1.f / prm.unit;
   QueryOrder qo;
   {
     PhaseTimer ph("order_queries", st);

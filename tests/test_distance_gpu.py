@@ -205,3 +205,47 @@ def test_queries_equally_far_from_everything(cuda, subdiv, nq):
     Dr, _, _ = O.squared_distance(V, F, Q, 0.25)
     assert np.array_equal(D == 0.25, Dr == 0.25) and (I[D == 0.25] == -1).all()
     bvh.close()
+
+
+@pytest.mark.parametrize("nf", [1, 2, 8, 9, 10, 33, 300, 4096, 4097, 9000])
+@pytest.mark.parametrize("kind", ["sphere", "plane", "soup"])
+def test_patches_and_soups_at_any_scale(cuda, nf, kind):
+    """From one triangle to more than any search node's own box is made for;
+    normals of all directions, one shared direction (an axis, its opposite, and
+    a slanted one), and none at all (triangles shrunk to segments and points).
+    The bounds never drop the closest triangle (exact brute-force distance),
+    and scaling everything by a power of two scales the result exactly."""
+    rng = np.random.default_rng([nf, len(kind)])
+    if kind == "soup":
+        A = rng.uniform(-1, 1, (nf, 3))
+        T = A[:, None] + rng.normal(0, 0.1, (nf, 3, 3))
+        T[::5, 2] = T[::5, 1]
+        T[::7] = T[::7, :1]
+    else:
+        n = rng.normal(size=(nf, 3))
+        n /= np.linalg.norm(n, axis=1, keepdims=True)
+        if kind == "plane":
+            n[:] = [[0, 0, 1], [0, 0, -1], [0.48, -0.6, -0.64]][nf % 3]
+        u = np.cross(n, n[:, [1, 2, 0]] + [0.1, 0.2, 0.3])
+        u /= np.linalg.norm(u, axis=1, keepdims=True)
+        w = np.cross(n, u)
+        c = n if kind == "sphere" else rng.uniform(-1, 1, (nf, 1)) * u + rng.uniform(-1, 1, (nf, 1)) * w
+        s = rng.normal(0, 1.5 / np.sqrt(nf), (nf, 3, 2))
+        T = c[:, None] + s[..., :1] * u[:, None] + s[..., 1:] * w[:, None]
+    V = np.ascontiguousarray(T.reshape(-1, 3))
+    F = np.arange(3 * nf, dtype=np.int32).reshape(nf, 3)
+    P = np.concatenate([rng.uniform(-1.5, 1.5, (200, 3)), rng.normal(0, 1e-3, (50, 3)),
+                        V[rng.integers(0, len(V), 100)] + rng.normal(0, 1e-5, (100, 3))])
+    bvh = G.FastWindingNumberBVH(V, F, tree="binned")
+    D, I, C = bvh.squared_distance(P)
+    Dr, _, _ = O.squared_distance(V, F, P)
+    assert _close2(D, Dr).all()
+    bvh.close()
+    for scale in (2.0 ** -30, 2.0 ** 40):
+        bvh = G.FastWindingNumberBVH(V * scale, F, tree="binned")
+        Ds, _, Cs = bvh.squared_distance(P * scale)
+        assert np.array_equal(Ds, D * scale ** 2)
+        bvh.close()
+    # the tree of the signed distance, which holds nothing but the search
+    S, I2, C2 = G.signed_distance(P, V, F, G.SIGNED_DISTANCE_TYPE_UNSIGNED)
+    assert np.array_equal(S, np.sqrt(D)) and np.array_equal(I2, I) and np.array_equal(C2, C)
