@@ -11,13 +11,15 @@
 //
 // The reference builds an AABB tree; here the closest-triangle query uses
 // the soup tree that the fast winding number already has, with an FP32 box
-// per node rounded outward: one thread per query searches depth-first,
-// nearer child first, and prunes a subtree when its box lower bound (minus
-// a slack covering the FP32 rounding of the query and the arithmetic) is at
-// least the distance found so far -- the order of the reference's
-// AABB::squared_distance.  Leaves are evaluated in FP64.  For a tree deeper
-// than the search stack, a warp-coherent walk over the pre-order array
-// (bounding-sphere pruning after a greedy descent) is used instead.
+// per node in a frame of its own (along the mean normal of a patch, or the
+// axes for a large node: soup.cu) rounded outward: one thread per query
+// searches depth-first, nearer child first, and prunes a subtree when its
+// box lower bound (minus a slack covering the FP32 rounding of the query and
+// the arithmetic) is at least the distance found so far -- the order of the
+// reference's AABB::squared_distance, whatever the frames.  Leaves are
+// evaluated in FP64.  For a tree deeper than the search stack, a warp-coherent
+// walk over the pre-order array (bounding-sphere pruning after a greedy
+// descent) is used instead.
 // Triangle distance: the closest point by Voronoi region (Ericson, Real-Time
 // Collision Detection 5.1.5; the reference's region order and its a == b
 // guard), squared distance from the closest point.  A strictly smaller
@@ -88,14 +90,19 @@ struct ClosestParams {
 };
 
 // Stack entries a thread's search may take before a whole warp takes the
-// query over.  Most searches take a few tens, but a query about equally far
-// from much of the surface (near a sphere's centre) takes tens of thousands,
-// and one thread at ~500 cycles an entry then sets the kernel's time.
-// Measured (signed distance, 327,680 triangles, 300,000 queries, whole call;
-// 40.8 ms without the limit): 48 entries 9.4 ms, 96 9.7, 192 10.3, 384 11.0,
-// 768 11.9; the swept volume's bounded searches (64 poses, 20,480 triangles),
-// few of them long: 9.75 ms with 48, 7.93 with 96, 7.85 with 384.
+// query over.  Most searches take about a hundred, but a query about equally
+// far from much of the surface (near a sphere's centre) takes tens of
+// thousands, and one thread at ~500 cycles an entry then sets the kernel's
+// time.  Measured (signed distance, 327,680 triangles, 300,000 queries, whole
+// call): 64 entries 5.8 ms, 96 5.6, 192 5.3; the swept volume's bounded searches
+// (64 poses, 20,480 triangles): 5.6, 5.5 and 5.5 ms.
 constexpr int kThreadVisits = 192;
+// Lanes of a warp that have come to a triangle before it turns to those: a
+// triangle's bounds take about five nodes' time however few lanes need them,
+// and more waiting leaves too few lanes at the nodes.  Signed distance and swept
+// volume as above, searches alone: 1 lane 1.52 and 1.46 ms, 4 1.40 and 1.33, 8
+// 1.44 and 1.33, 16 1.40 and 1.41, 32 1.89 and 1.54.
+constexpr int kLeafLanes = 8;
 constexpr int kLongThreads = 128;
 constexpr int kLongStack = 1024;  // shared-memory stack entries per warp
 
@@ -289,25 +296,41 @@ __global__ void __launch_bounds__(128) closest_kernel(ClosestParams prm, const Q
   C[qi * 3 + 2] = b.c.z;
 }
 
-// Conservative FP32 lower bound of the distance from q to a box (lo, hi):
-// the box is rounded outward to FP32; the query's rounding to FP32 and the
-// FP32 arithmetic move the exterior distance by at most a few u
-// (|q| + |box| + d), covered by the slack 1e-6 (S + d).
-__device__ __forceinline__ float box_lower_bound(const float4 lo, const float4 hi, float fx,
-                                                 float fy, float fz, float S) {
-  const float dx = fmaxf(fmaxf(lo.x - fx, fx - hi.x), 0.f);
-  const float dy = fmaxf(fmaxf(lo.y - fy, fy - hi.y), 0.f);
-  const float dz = fmaxf(fmaxf(lo.z - fz, fz - hi.z), 0.f);
+// A child of a search node and a conservative FP32 lower bound of the distance
+// from q to it: the distance of q's coordinates in the box's frame.  The box
+// was rounded outward when it was made; the rounding of q and of the frame's
+// arithmetic move each coordinate by at most 13 u |q|, that of the differences
+// by 4 u S, which is below 30 u S in all, and the frame's norm and the square
+// root the distance by less than 12 u d: 2e-6 (S + d) covers both.  (A NaN
+// counts as inside, an overflow as distance 0.)
+struct Child {
+  int ref;
+  float lb;
+};
+__device__ __forceinline__ Child search_child(const ClosestParams& prm, int node, int side,
+                                              float fx, float fy, float fz, float S) {
+  float4 lo, hi;
+  ldg256(prm.snode + 4 * (int64_t)node + 2 * side, lo, hi);
+  const float3 q = SearchFrame(hi.w)(fx, fy, fz);
+  const float dx = fmaxf(fmaxf(lo.x - q.x, q.x - hi.x), 0.f);
+  const float dy = fmaxf(fmaxf(lo.y - q.y, q.y - hi.y), 0.f);
+  const float dz = fmaxf(fmaxf(lo.z - q.z, q.z - hi.z), 0.f);
   const float d = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
-  return fmaxf(d - 1e-6f * (S + d), 0.f);
+  return {__float_as_int(lo.w), fmaxf(d - 2e-6f * (S + d), 0.f)};
 }
 
 // Closest triangle by depth-first search over the search nodes, nearer
 // child first, pruned by the children's box lower bounds: the order of
 // igl::AABB::squared_distance (AABB.cpp:1180-1203).  One query per thread;
-// one 64-byte search node per internal visit, leaves go straight to their
-// triangle.  A push beyond the stack (the host picks this kernel only for
-// trees shallower than kStack) is reported instead of written.
+// a 64-byte search node per internal visit, read as two 256-bit words, the
+// nearer child kept out of the stack; leaves go straight to their triangle.
+// What bounds it is the two kinds of visit in a warp, and before that the FP64
+// closest points, which cost a warp the same for one lane as for 32: a candidate
+// that a nearer triangle has ruled out gives its place to the next, so that
+// nearly all of them wait for the end, where the lanes take them together
+// (searches of 2.7 ms with boxes along the normals alone, 1.4 ms with this).
+// A push beyond the stack (the host picks this kernel only for trees shallower
+// than kStack) is reported instead of written.
 template <typename QT>
 __global__ void __launch_bounds__(128) closest_dfs_kernel(ClosestParams prm,
                                                           const QT* __restrict__ Q,
@@ -323,6 +346,7 @@ __global__ void __launch_bounds__(128) closest_dfs_kernel(ClosestParams prm,
   const int64_t qi = perm ? (int64_t)perm[i] : i;
   const D3 q{(double)Q[qi * 3], (double)Q[qi * 3 + 1], (double)Q[qi * 3 + 2]};
   Best b{up_sqr_d, -1, {0, 0, 0}, dist_bound(up_sqr_d)};
+  bool handed = false;
   if (isfinite(q.x) && isfinite(q.y) && isfinite(q.z) && prm.nnodes > 0) {
     const float fx = (float)q.x, fy = (float)q.y, fz = (float)q.z;
     const float S = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + prm.cmax;
@@ -333,77 +357,82 @@ __global__ void __launch_bounds__(128) closest_dfs_kernel(ClosestParams prm,
     // the four candidate slots are full), so every triangle that can be the
     // closest, ties included, is evaluated in FP64 as before.
     float ub = b.bound;
-    int cs0 = 0, cs1 = 0, cs2 = 0, cs3 = 0;
+    int cs0 = -1, cs1 = -1, cs2 = -1, cs3 = -1;
     float cl0 = 0.f, cl1 = 0.f, cl2 = 0.f, cl3 = 0.f;
-    int nc = 0;
     auto flush = [&]() {
-      if (nc > 0 && !(cl0 > ub)) eval_leaf(prm, cs0, q, b);
-      if (nc > 1 && !(cl1 > ub)) eval_leaf(prm, cs1, q, b);
-      if (nc > 2 && !(cl2 > ub)) eval_leaf(prm, cs2, q, b);
-      if (nc > 3 && !(cl3 > ub)) eval_leaf(prm, cs3, q, b);
-      nc = 0;
+      if (cs0 >= 0 && !(cl0 > ub)) eval_leaf(prm, cs0, q, b);
+      if (cs1 >= 0 && !(cl1 > ub)) eval_leaf(prm, cs1, q, b);
+      if (cs2 >= 0 && !(cl2 > ub)) eval_leaf(prm, cs2, q, b);
+      if (cs3 >= 0 && !(cl3 > ub)) eval_leaf(prm, cs3, q, b);
+      cs0 = cs1 = cs2 = cs3 = -1;
       ub = fminf(ub, b.bound);
     };
     int stk_n[kStack];
     float stk_lb[kStack];
-    int sp = 0;
-    stk_n[sp] = prm.nnodes > 1 ? 0 : ~0;  // root: internal node 0, or the only leaf
-    stk_lb[sp] = 0.f;
-    ++sp;
-    int visits = 0;
-    while (sp > 0) {
-      --sp;
-      const int ref = stk_n[sp];
-      const float lb = stk_lb[sp];
-      if (lb > ub) continue;
-      if (++visits > kThreadVisits) {  // a long search: left to a whole warp
-        const unsigned k = atomicAdd(longs.count, 1u);
-        longs.query[k] = (int32_t)qi;
-        longs.ub[k] = ub;
-        return;
+    int sp = 0, visits = 0;
+    constexpr int kDone = INT_MIN;  // no slot has this complement
+    int ref = prm.nnodes > 1 ? 0 : ~0;  // root: internal node 0, or the only leaf
+    auto pop = [&]() {  // the newest entry still within ub
+      ref = kDone;
+      while (sp > 0 && ref == kDone) {
+        --sp;
+        if (!(stk_lb[sp] > ub)) ref = stk_n[sp];
       }
-      if (ref < 0) {
-        float lower, upper;
-        leaf_bounds(prm, ~ref, fx, fy, fz, S, lower, upper);
-        if (!(lower > ub)) {
-          if (nc == 4) flush();
-          if (nc == 0) { cs0 = ~ref; cl0 = lower; }
-          else if (nc == 1) { cs1 = ~ref; cl1 = lower; }
-          else if (nc == 2) { cs2 = ~ref; cl2 = lower; }
-          else { cs3 = ~ref; cl3 = lower; }
-          ++nc;
-          ub = fminf(ub, upper);
+    };
+    const unsigned warp = __activemask();
+    // Lanes that have come to a leaf wait for each other.
+    for (;;) {
+      const unsigned leaves = __ballot_sync(warp, ref < 0 && ref != kDone);
+      const unsigned inner = __ballot_sync(warp, ref >= 0);
+      if ((leaves | inner) == 0) break;
+      if (inner == 0 || __popc(leaves) >= kLeafLanes) {
+        if (ref < 0 && ref != kDone) {
+          float lower, upper;
+          leaf_bounds(prm, ~ref, fx, fy, fz, S, lower, upper);
+          if (!(lower > ub)) {
+            ub = fminf(ub, upper);
+            const bool f0 = cs0 < 0 || cl0 > ub, f1 = cs1 < 0 || cl1 > ub;
+            const bool f2 = cs2 < 0 || cl2 > ub, f3 = cs3 < 0 || cl3 > ub;
+            if (!(f0 || f1 || f2 || f3)) flush();
+            if (f0 || !(f1 || f2 || f3)) { cs0 = ~ref; cl0 = lower; }
+            else if (f1) { cs1 = ~ref; cl1 = lower; }
+            else if (f2) { cs2 = ~ref; cl2 = lower; }
+            else { cs3 = ~ref; cl3 = lower; }
+          }
+          ++visits;
+          pop();
         }
-        continue;
-      }
-      const float4* sn = prm.snode + 4 * (int64_t)ref;
-      const float4 lo_l = __ldg(sn), hi_l = __ldg(sn + 1), lo_r = __ldg(sn + 2),
-                   hi_r = __ldg(sn + 3);
-      const int l = __float_as_int(lo_l.w), r = __float_as_int(hi_l.w);
-      const float lbl = box_lower_bound(lo_l, hi_l, fx, fy, fz, S);
-      const float lbr = box_lower_bound(lo_r, hi_r, fx, fy, fz, S);
-      const bool left_first = lbl <= lbr;
-      const int far_n = left_first ? r : l, near_n = left_first ? l : r;
-      const float far_lb = left_first ? lbr : lbl, near_lb = left_first ? lbl : lbr;
-      if (!(far_lb > ub)) {
-        if (sp == kStack) {
-          atomicOr(status, kStatusBadInput);
-          break;
+      } else if (ref >= 0) {
+        const Child cl = search_child(prm, ref, 0, fx, fy, fz, S);
+        const Child cr = search_child(prm, ref, 1, fx, fy, fz, S);
+        const bool left_first = cl.lb <= cr.lb;
+        const int far_n = left_first ? cr.ref : cl.ref, near_n = left_first ? cl.ref : cr.ref;
+        const float far_lb = left_first ? cr.lb : cl.lb, near_lb = left_first ? cl.lb : cr.lb;
+        if (++visits > kThreadVisits) {  // a long search: left to a whole warp
+          const unsigned k = atomicAdd(longs.count, 1u);
+          longs.query[k] = (int32_t)qi;
+          longs.ub[k] = ub;
+          handed = true;
+          ref = kDone;
+        } else {
+          if (!(far_lb > ub)) {
+            if (sp == kStack) {
+              atomicOr(status, kStatusBadInput);
+              ref = kDone;
+              continue;
+            }
+            stk_n[sp] = far_n;
+            stk_lb[sp] = far_lb;
+            ++sp;
+          }
+          if (!(near_lb > ub))
+            ref = near_n;
+          else
+            pop();
         }
-        stk_n[sp] = far_n;
-        stk_lb[sp] = far_lb;
-        ++sp;
-      }
-      if (!(near_lb > ub)) {
-        if (sp == kStack) {
-          atomicOr(status, kStatusBadInput);
-          break;
-        }
-        stk_n[sp] = near_n;
-        stk_lb[sp] = near_lb;
-        ++sp;
       }
     }
+    if (handed) return;
     flush();
   }
   sqrD[qi] = b.d2;
@@ -496,12 +525,10 @@ __global__ void __launch_bounds__(kLongThreads) closest_long_kernel(
       float near_lb = INFINITY, far_lb = INFINITY;
       bool pn = false, pf = false;
       if (live && ref >= 0) {
-        const float4* sn = prm.snode + 4 * (int64_t)ref;
-        const float4 lo_l = __ldg(sn), hi_l = __ldg(sn + 1), lo_r = __ldg(sn + 2),
-                     hi_r = __ldg(sn + 3);
-        const int l = __float_as_int(lo_l.w), r = __float_as_int(hi_l.w);
-        const float lbl = box_lower_bound(lo_l, hi_l, fx, fy, fz, S);
-        const float lbr = box_lower_bound(lo_r, hi_r, fx, fy, fz, S);
+        const Child cl = search_child(prm, ref, 0, fx, fy, fz, S);
+        const Child cr = search_child(prm, ref, 1, fx, fy, fz, S);
+        const int l = cl.ref, r = cr.ref;
+        const float lbl = cl.lb, lbr = cr.lb;
         const bool left_first = lbl <= lbr;
         far_n = left_first ? r : l;
         near_n = left_first ? l : r;

@@ -146,6 +146,47 @@ __device__ inline float tri_screen_slack(const double* v) {
 }
 #endif
 
+#ifdef __CUDACC__
+// Frame of a search node's box.  With n the unit vector of stereographic
+// coordinates (p, r), p^2 + r^2 <= 1, and k = 2 / (1 + p^2 + r^2):
+//   n = (k p, k r, k - 1), u = (1 - k p^2, -k p r, -k p), w = (-k p r, 1 - k r^2, -k r),
+// so that with g = k (p x + r y + z) the coordinates of (x, y, z) are
+// (x - p g, y - r g, g - z).  p = r = 0 is the frame of the axes.  p and r are
+// held as 16-bit multiples of 2^-15 (exact in FP32).  k is the same FP32 number
+// wherever a frame is read; its relative error e leaves the map's norm at most
+// 1 + 2 e, 5e-7 with the approximate reciprocal.
+struct SearchFrame {
+  float p, r, k;
+  __device__ __forceinline__ explicit SearchFrame(float bits) {
+    const uint32_t b = __float_as_uint(bits);
+    p = fmaf(__uint_as_float(0x4b000000u | (b & 0xffffu)), 0x1p-15f, -257.f);
+    r = fmaf(__uint_as_float(0x4b000000u | (b >> 16)), 0x1p-15f, -257.f);
+    float s = fmaf(p, p, fmaf(r, r, 1.f));
+    asm("rcp.approx.f32 %0, %1;" : "=f"(k) : "f"(s));
+    k *= 2.f;
+  }
+  // Coordinates of a point within 13 u max(|x|, |y|, |z|) each, u = 2^-24.
+  __device__ __forceinline__ float3 operator()(float x, float y, float z) const {
+    const float g = k * fmaf(p, x, fmaf(r, y, z));
+    return make_float3(fmaf(-p, g, x), fmaf(-r, g, y), g - z);
+  }
+  // The bits of the frame whose third axis is nearest to +-n; any n will do.
+  __device__ static float bits_of(float3 n) {
+    const float l = sqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
+    float p = 0.f, r = 0.f;
+    if (l > 0.f && isfinite(l)) {
+      const float q = copysignf(1.f, n.z) / (l + fabsf(n.z));
+      p = n.x * q;
+      r = n.y * q;
+    }
+    auto enc = [](float v) {
+      return (uint32_t)min(max(__float2int_rz(v * 32768.f), -32767), 32767) + 32768u;
+    };
+    return __uint_as_float(enc(p) | (enc(r) << 16));
+  }
+};
+#endif
+
 struct gwn_soup_impl {
   int device = 0;
   int order = 2;
@@ -168,9 +209,9 @@ struct gwn_soup_impl {
   DevMem<double> td;     // 9 doubles per slot
   DevMem<int32_t> tri_index;  // input triangle id per slot
   // Closest-point search nodes, one per internal node of the binary tree in
-  // build order (root 0): 4 float4 = boxes of the two children, rounded
-  // outward to FP32, and the children (internal index, or ~slot for a leaf):
-  //   {lo_l.xyz, left}, {hi_l.xyz, right}, {lo_r.xyz, 0}, {hi_r.xyz, 0}.
+  // build order (root 0): for each of the two children 2 float4, its box in
+  // the frame of SearchFrame and the child (internal index, or ~slot for a
+  // leaf): {lo.xyz, child}, {hi.xyz, frame}.
   DevMem<float4> snode;
   // every FP64 moment finite and within 1e100 in magnitude: then no far
   // field at |q - P|^2 >= 1e-100 can overflow, and the plain FP64 walk may
