@@ -55,6 +55,7 @@ namespace {
 
 constexpr int kT = 256;
 constexpr int kMaxSplit = 32;  // subtrees walked in parallel when queries are few (a lane of frontier_kernel each)
+constexpr int kMaxCoarse = 8;  // subtrees above whose roots only the tree's root has its cap taken
 constexpr int kWalk = 64;      // threads per CTA of the walks
 constexpr double kNearFrac = 1e-3;
 constexpr double kBand = 1e-3;
@@ -606,7 +607,10 @@ __device__ __forceinline__ void flush_hier64(const double* __restrict__ tris64,
 // outside one of their boxes takes that node's cap in place of everything
 // below it, in the leftmost of the subtrees below (first: every step from the
 // node down to y0 goes left), as the whole-tree walk would; the others add
-// nothing.
+// nothing.  Of the nodes above the coarse cut (depth `coarse`) only the root's
+// cap is taken: the error of a cap triangle's term grows with the square of its
+// size over the query's distance from its edges, so the largest caps are the
+// least accurate, and a batch that is split has never used them.
 struct Above {
   int node[8], n = 0;
   unsigned left = 0;  // bit i: the step down from node[i] goes left
@@ -624,6 +628,7 @@ struct Above {
       x = go_left ? l : l_end;
     }
   }
+  __device__ __forceinline__ static bool usable(int i, int coarse) { return i == 0 || i >= coarse; }
   __device__ __forceinline__ bool first(int i) const {
     const unsigned m = ((1u << n) - 1u) & ~((1u << i) - 1u);
     return (left & m) == m;
@@ -640,7 +645,7 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk_kernel(HierDev H, const Q
                                                        uint32_t* __restrict__ nredo,
                                                        const int2* __restrict__ ranges,
                                                        const int* __restrict__ nranges,
-                                                       double* __restrict__ part) {
+                                                       double* __restrict__ part, int coarse) {
   // ranges: walk only the subtree [ranges[y].x, ranges[y].y) of y = blockIdx.y
   // and write the partial sum (solid angle) to part[y * nQ + q]
   int x0 = 0, x1 = H.nnodes;
@@ -677,7 +682,7 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk_kernel(HierDev H, const Q
     for (int i = 0; i < up.n; ++i) {
       const NodeH nd = H.nodes[up.node[i]];
       const int meta = __float_as_int(nd.hi.w);
-      if (resume == x0 && meta >= 0 &&
+      if (Above::usable(i, coarse) && resume == x0 && meta >= 0 &&
           (qh.x < nd.lo.x || qh.x > nd.hi.x || qh.y < nd.lo.y || qh.y > nd.hi.y ||
            qh.z < nd.lo.z || qh.z > nd.hi.z)) {
         if (up.first(i)) {
@@ -824,7 +829,7 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk64_kernel(HierDev H, const
                                                          double* __restrict__ W,
                                                          const int2* __restrict__ ranges,
                                                          const int* __restrict__ nranges,
-                                                         double* __restrict__ part) {
+                                                         double* __restrict__ part, int coarse) {
   int x0 = 0, x1 = H.nnodes;
   if (ranges) {
     if ((int)blockIdx.y >= *nranges) return;
@@ -856,7 +861,7 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk64_kernel(HierDev H, const
     for (int i = 0; i < up.n; ++i) {
       const int y = up.node[i], meta = __float_as_int(H.nodes[y].hi.w);
       int cnt = 0;
-      if (resume == x0 && meta >= 0 && outside(y)) {
+      if (Above::usable(i, coarse) && resume == x0 && meta >= 0 && outside(y)) {
         if (up.first(i)) cnt = H.capn[y];
         resume = 0x7fffffff;
       }
@@ -1138,23 +1143,26 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
   // Too few queries for six waves of warps: each warp of queries walks one of
   // up to 32 subtrees (blockIdx.y), and the partial sums are added in a fixed
   // order.  Warps near the surface walk far longer than the others, and with
-  // the caps above the cut kept (Above) a finer cut adds no work: FP64, 100,000
-  // queries, 81,920 triangles: 33.2 ms with up to 8 subtrees that keep the
-  // root's cap only; 33.5 / 25.8 / 22.8 / 21.4 ms at 1 / 3 / 6 / 12 waves with
-  // all of them; mixed, 300,000 queries, 20,480 triangles 2.70 -> 2.66 / 2.74 /
-  // 2.48 / 2.35 ms, 100,000 queries, 5,120 triangles 1.17 -> 1.26 / 1.07 / 1.09
-  // / 1.15 ms.
+  // the caps above the cut kept (Above) a finer cut adds little work.  FP64,
+  // 50,001 queries, 20,480 triangles: 10.9 ms with up to 8 subtrees at three
+  // waves, 8.4 ms so; mixed, 100,000 queries, 5,120 triangles 1.15 -> 1.00 ms.
+  // Taking every cap above the cut would give 6.7 and 0.97 ms, but in FP64 two
+  // to five times the root mean square error against 64 bits (1.1e-15 to
+  // 2.9e-15 over ten inputs against 3.4e-16 to 1.5e-15).
   const int64_t warps = (nQ + 31) / 32;
   const int64_t want = 6 * (int64_t)num_sms() * 32;
   const unsigned wblk = (unsigned)((nQ + kWalk - 1) / kWalk);
   int S = 1;
   while (S < kMaxSplit && warps * S < want) S *= 2;
+  // depth of the coarse cut, chosen at half the waves
+  int coarse = 0;
+  while ((1 << coarse) < kMaxCoarse && (warps << coarse) * 2 < want) ++coarse;
   const int32_t* perm = qo.active ? qo.perm.get() : nullptr;
   if (precision == GWN_PLAIN_FP64) {
     PhaseTimer ph("hier_walk", st);
     if (S == 1) {
       launch_kernel(hier_walk64_kernel, wblk, kWalk, 0, st, H, Q, nQ, perm, W,
-                    (const int2*)nullptr, (const int*)nullptr, (double*)nullptr);
+                    (const int2*)nullptr, (const int*)nullptr, (double*)nullptr, 0);
     } else {
       DevBuf<int2> ranges(kMaxSplit, st);
       DevBuf<int> nranges(1, st);
@@ -1162,7 +1170,7 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
       part.zero(st);
       launch_kernel(frontier_kernel, 1, 32, 0, st, H.nodes, S, ranges.get(), nranges.get());
       launch_kernel(hier_walk64_kernel, dim3(wblk, S), kWalk, 0, st, H, Q, nQ, perm, W,
-                    (const int2*)ranges.get(), (const int*)nranges.get(), part.get());
+                    (const int2*)ranges.get(), (const int*)nranges.get(), part.get(), coarse);
       launch_kernel(hier_sum64_kernel, nblk(nQ), kT, 0, st, (const double*)part.get(), S, nQ, W);
     }
     return;
@@ -1173,7 +1181,7 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
       launch_kernel(hier_walk_kernel<double>, wblk, kWalk, 0, st, H, Q, nQ,
                     (const int32_t*)(qo.active ? qo.perm.get() : nullptr), h.c[0], h.c[1],
                     h.c[2], W, redo.get(), nredo.get(), (const int2*)nullptr,
-                    (const int*)nullptr, (double*)nullptr);
+                    (const int*)nullptr, (double*)nullptr, 0);
     } else {
       DevBuf<int2> ranges(kMaxSplit, st);
       DevBuf<int> nranges(1, st);
@@ -1183,7 +1191,7 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
       launch_kernel(hier_walk_kernel<double>, dim3(wblk, S), kWalk, 0, st, H, Q, nQ,
                     (const int32_t*)(qo.active ? qo.perm.get() : nullptr), h.c[0], h.c[1],
                     h.c[2], W, redo.get(), nredo.get(), (const int2*)ranges.get(),
-                    (const int*)nranges.get(), part.get());
+                    (const int*)nranges.get(), part.get(), coarse);
       launch_kernel(hier_sum_kernel, nblk(nQ), kT, 0, st, (const double*)part.get(), S, nQ, W,
                     redo.get(), nredo.get());
     }
