@@ -23,8 +23,8 @@
 // Triangle distance: the closest point by Voronoi region (Ericson, Real-Time
 // Collision Detection 5.1.5; the reference's region order and its a == b
 // guard), squared distance from the closest point.  A strictly smaller
-// distance replaces the current one, so in a tie the first triangle reached
-// is kept (the reference's tree reaches its own first).
+// distance replaces the current one, and in a tie the smaller input triangle
+// index wins, whatever the order of the visits.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -92,15 +92,16 @@ struct ClosestParams {
 // Stack entries a thread's search may take before a whole warp takes the
 // query over.  Most searches take about a hundred, but a query about equally
 // far from much of the surface (near a sphere's centre) takes tens of
-// thousands, and one thread at ~500 cycles an entry then sets the kernel's
-// time.  Measured (signed distance, 327,680 triangles, 300,000 queries, whole
-// call): 64 entries 5.8 ms, 96 5.6, 192 5.3; the swept volume's bounded searches
-// (64 poses, 20,480 triangles): 5.6, 5.5 and 5.5 ms.
+// thousands, and one thread then sets the kernel's time.  Kernel times of both
+// searches: signed distance, 327,680 triangles, 300,000 queries: 64 entries
+// 1.96 ms, 96 1.77, 192 1.44 + 0.1 or less; the swept volume's bounded searches
+// (64 poses, 20,480 triangles), thread search alone: 1.30, 1.33 and 1.33 ms.
+// (Both with boxes along the normals up to 4096 triangles.)
 constexpr int kThreadVisits = 192;
-// Lanes of a warp that have come to a triangle before it turns to those: a
-// triangle's bounds take about five nodes' time however few lanes need them,
-// and more waiting leaves too few lanes at the nodes.  Signed distance and swept
-// volume as above, searches alone: 1 lane 1.52 and 1.46 ms, 4 1.40 and 1.33, 8
+// Lanes of a warp that have come to a triangle before it turns to those: the
+// triangle's bounds cost the warp the same however few lanes need them, and more
+// waiting leaves too few lanes at the nodes.  Thread search's kernel time, signed
+// distance and swept volume as above: 1 lane 1.52 and 1.46 ms, 4 1.40 and 1.33, 8
 // 1.44 and 1.33, 16 1.40 and 1.41, 32 1.89 and 1.54.
 constexpr int kLeafLanes = 8;
 constexpr int kLongThreads = 128;
@@ -328,7 +329,9 @@ __device__ __forceinline__ Child search_child(const ClosestParams& prm, int node
 // closest points, which cost a warp the same for one lane as for 32: a candidate
 // that a nearer triangle has ruled out gives its place to the next, so that
 // nearly all of them wait for the end, where the lanes take them together
-// (searches of 2.7 ms with boxes along the normals alone, 1.4 ms with this).
+// (kernel time 2.73 ms with boxes along the normals alone, 1.44 ms with this and
+// the waiting at leaves).  Signed distance as a whole, 300,000 queries and
+// 327,680 triangles: 8.3 -> 5.32 ms; swept volume 6.1 -> 5.35 ms.
 // A push beyond the stack (the host picks this kernel only for trees shallower
 // than kStack) is reported instead of written.
 template <typename QT>

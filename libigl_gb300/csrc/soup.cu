@@ -407,11 +407,12 @@ __global__ void preorder_kernel(const int32_t* __restrict__ left,
 // but the root, written to its parent's record.  A patch of a smooth surface is
 // thin along its normal but, unless that is an axis, its box by axes is as
 // thick as the patch is wide, and a search then keeps every patch whose box
-// reaches into the sphere of the best distance: over a bumpy sphere of 327,680
-// triangles 908 nodes and 267 triangles for each query, against 94 and 9 with
-// boxes along the nodes' mean normals.  That is for nodes of up to
-// kOrientedTris triangles, as larger ones bend too much to gain (searches of
-// 300,000 queries there with 256, 512, 4096: 1.52, 1.39, 1.44 ms; the swept
+// reaches into the sphere of the best distance.  (Counted by a CPU model with
+// median splits, which is not this tree: over a bumpy sphere of 327,680
+// triangles 908 nodes and 267 triangles a query by axes, 94 and 9 with boxes
+// along the nodes' mean normals.)  That is for nodes of up to kOrientedTris
+// triangles, as larger ones bend too much to gain.  Kernel times of the searches
+// there, 300,000 queries, with 256, 512, 4096: 1.52, 1.39, 1.44 ms; the swept
 // volume's over 20,480 triangles 1.29, 1.29, 1.33 ms; all by axes 4.6 and
 // 2.0 ms).  A node's triangles are consecutive slots.  Nodes of up to kThreadTris triangles are computed by
 // one thread, larger ones by the whole warp, whose nodes are spread over the
