@@ -17,19 +17,17 @@
 // centres, split heuristics, boxes and moments are bit for bit the
 // reference's.
 //
-// Tree build (UT_BVH<4>::initNode, FWNFS.h:4918-5047), one depth at a time:
-//   a node of at most 4 boxes holds them as items; a larger node makes the
-//   reference's three binary splits (multiSplit, FWNFS.h:5249-5346: split
-//   all, then twice the part with the largest area x count), all nodes of
-//   the depth split by split.  A split (FWNFS.h:5350-5800) of
-//     <= 32 boxes runs in one thread (2 boxes trivially, <= 6 by trying every
-//           partition, else a stable sort of the centres and a sweep),
-//     <= 1024 boxes in one CTA (span statistics by shared-memory atomics,
-//           the partition done sequentially in shared memory),
-//     more boxes across the GPU: span statistics by chunk, and the
-//           reference's in-place partition reproduced exactly (below).
-//   Span counts and boxes are order-independent (counts, min, max), so
-//   every decision equals the serial code's.
+// Tree build (UT_BVH<4>::initNode, FWNFS.h:4918-5047).  A node of at most 4
+// boxes holds them as items; a larger node makes the reference's three binary
+// splits (multiSplit, FWNFS.h:5249-5346: split all, then twice the part with
+// the largest area x count).
+//   Nodes of more than 1024 boxes (kSub): one depth at a time, split by split
+//     across the depth; by size a split runs in one warp, in one CTA, or by
+//     chunks across the GPU, each with the reference's in-place partition
+//     reproduced exactly (below).
+//   Smaller subtrees: one CTA each, whole, in shared memory, a warp per node.
+// Span counts and boxes are order-independent (counts, min, max), so every
+// decision equals the serial code's.
 //
 // The in-place three-way partition (partitionByCentre, FWNFS.h:5903-5944)
 // keeps the boxes below the pivot in order at the front; the boxes equal to
@@ -38,12 +36,13 @@
 // of a non-empty queue to its back.  The final order of a queue is read off
 // a tape of its operations: an append writes the box, the r-th rotation
 // writes a copy of tape entry r, and the queue is the tape's last k entries.
-// Every box finds its tape positions from prefix counts; the copies are
-// resolved by pointer doubling.  nthElement (FWNFS.h:5847-5900), the
+// Every box finds its tape positions from prefix counts; a copy is followed to
+// the earlier entries it refers to.  nthElement (FWNFS.h:5847-5900), the
 // fallback when no span is balanced enough, repeats such partitions.
 //
 // Moments (UT_SolidAngle::init's per-item data and its post() merge,
-// FWNFS.h:6668-7118): bottom-up one depth at a time; a node's lanes are its
+// FWNFS.h:6668-7118): triangles first, then bottom-up by depth, inside each
+// subtree in one CTA and above them one launch a depth; a node's lanes are its
 // children's data, and its own data is what its parent's lane holds.
 #include <cuda_runtime.h>
 
