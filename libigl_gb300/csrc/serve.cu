@@ -77,7 +77,7 @@ struct __align__(16) ServeReq {
   int32_t nq;
   int32_t q_f64;
   int32_t precision;
-  int32_t ordered;      // OrderedSum (a call of its size shares queries between lanes)
+  int32_t pair;         // PairSum (a call of its size shares queries between lanes)
   int32_t pad[3];
 };
 
@@ -231,11 +231,11 @@ __global__ void __launch_bounds__(128, 8) serve_walk_kernel(ServeHeader* __restr
       soupwalk::WalkCounters c;
       // every served tree is of the default kind (the builder below); the
       // kind of sum is that of the request's own call
-      if (R.ordered) {
-        soupwalk::OrderedSum acc;
+      if (R.pair) {
+        soupwalk::PairSum acc;
         soupwalk::walk_mixed<false, GWN_SOUP_TREE_DEFAULT>(prm, valid, qx, qy, qz, acc, acc64, c,
                                                            warp_q[threadIdx.x >> 5].near);
-        w = soupwalk::mixed_result(acc, acc64);
+        w = soupwalk::mixed_result(acc.value(), acc64);
       } else {
         soupwalk::PlainSum acc;
         soupwalk::walk_mixed<false, GWN_SOUP_TREE_DEFAULT>(prm, valid, qx, qy, qz, acc, acc64, c,
@@ -701,7 +701,7 @@ bool gwn_server::form_and_launch(SrvSlot& s, std::unique_lock<std::mutex>& lk) {
     d.prm.status = nullptr;
     d.prm.ref32 = t.tree == GWN_TREE_REFERENCE;
     d.prm.fp64_queue = t.moments_bounded;
-    d.ordered = soup_team_size(r->nq, t.nnodes, r->precision) > 1;
+    d.pair = soup_team_size(r->nq, t.nnodes, r->precision) > 1;
     for (int k = 0; k < 3; ++k) {
       // the query box: the mesh box grown by a quarter on each side
       const double e = std::max(t.hi[k] - t.lo[k], 1e-30);

@@ -645,8 +645,7 @@ __global__ void __launch_bounds__(128, 7) soup_team_mixed_kernel(
   int64_t qi = 0;
   double qx = 0, qy = 0, qz = 0;
   if (valid) soupwalk::read_query(Q, perm, (const int32_t*)nullptr, i, qi, qx, qy, qz);
-  soupwalk::OrderedSum acc;
-  double acc64;
+  double acc, acc64;
   soupwalk::walk_mixed_team<kTree>(prm, T, valid, qx, qy, qz, acc, acc64,
                                       near_q[threadIdx.x >> 5], s_stack[threadIdx.x >> 5]);
   if (!valid || (threadIdx.x & (T - 1))) return;

@@ -253,9 +253,9 @@ void soup_remap_index(const int32_t* map, int32_t* I, int64_t n, cudaStream_t st
 void soup_walk_stats(const gwn_soup_impl& s, float beta, const double* Q, int64_t nQ,
                      unsigned long long* out7, cudaStream_t st);
 // Lanes that share a query in a call of nQ queries on a tree of `slots` slots
-// (1: 32 queries per warp).  With more than one, the query's FP32 sum does not
-// depend on the order of its terms (soup_walk.cuh, OrderedSum), and a served
-// request of that size takes the same sum.
+// (1: 32 queries per warp).  With more than one, the query's FP32 sum is kept
+// with its rounding error (soup_walk.cuh, PairSum), because the lanes' terms are
+// added in another order, and a served request of that size takes the same sum.
 int soup_team_size(int64_t nQ, int64_t slots, int precision);
 void soup_eval(const gwn_soup_impl& s, float beta, const void* Q, int q_dtype, int64_t nQ,
                void* W, int w_dtype, int precision, cudaStream_t st);

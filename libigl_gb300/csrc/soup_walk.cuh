@@ -243,49 +243,38 @@ __device__ __forceinline__ void flush_near64(const double* __restrict__ td, Near
   __syncwarp();
 }
 
-// A query's FP32 sum.  PlainSum adds in the order of the walk.  OrderedSum's
-// result does not depend on the order of its terms, so that a walk by a team
-// of lanes and a warp-coherent walk of the same query return the same value:
-// every term is split exactly into a multiple of 2^-12 and a rest, the rest
-// rounded to a multiple of 2^-30, and both are summed as integers.  Adding
-// 1.5 * 2^23 units makes a float's low bits that integer.  Five operations
-// more than a plain sum, and a smaller rounding error (2^-31 per term; a
-// plain sum of a few turns loses up to 2^-22 per addition).
-// add() is false for a term outside +-512 (or NaN), which the caller takes in
-// FP64.  fold() carries the small units, which would overflow after 2^14 equal
-// terms; leaf terms, which repeat for repeated triangles, call it.
+// A query's FP32 sum.  PlainSum adds in the order of the walk.  PairSum keeps
+// the rounding error of every addition (Knuth's two-sum) in a second FP32 word
+// and renormalises, so that a walk by a team of lanes and a warp-coherent walk
+// of the same query, which add the same terms in another order, agree to about
+// 1e-14 turns for sums of a turn; it has FP32's range and its relative accuracy
+// for small sums.
+// add() is false for a term that is not finite.
 struct PlainSum {
-  static constexpr bool kBounded = false;  // refuses only what is not finite
   float s = 0.f;
   __device__ __forceinline__ bool add(float v) {
     if (!isfinite(v)) return false;
     s += v;
     return true;
   }
-  __device__ __forceinline__ void add_leaf(float v, double&) { s += v; }
+  __device__ __forceinline__ void add_leaf(float v) { s += v; }
 };
-struct OrderedSum {
-  static constexpr bool kBounded = true;
-  int hi = 0, lo = 0;  // units of 2^-12 and 2^-30
+struct PairSum {
+  float s = 0.f, e = 0.f;
+  __device__ __forceinline__ void add_leaf(float v) {
+    const float t = __fadd_rn(s, v), b = __fsub_rn(t, s);
+    const float r = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(v, b)));
+    s = __fadd_rn(t, r);
+    e = __fsub_rn(r, __fsub_rn(s, t));
+  }
   __device__ __forceinline__ bool add(float v) {
-    if (!(fabsf(v) < 512.f)) return false;
-    const float t = __fadd_rn(v, 3072.f);  // 1.5 * 2^11: units of 2^-12
-    const float r = __fsub_rn(v, __fsub_rn(t, 3072.f));
-    const float u = __fadd_rn(r, 0.01171875f);  // 1.5 * 2^-7: units of 2^-30
-    hi += __float_as_int(t) - 0x45400000;
-    lo += __float_as_int(u) - 0x3c400000;
+    if (!isfinite(v)) return false;
+    add_leaf(v);
     return true;
   }
-  __device__ __forceinline__ void fold() {
-    hi += lo >> 18;
-    lo &= (1 << 18) - 1;
-  }
-  __device__ __forceinline__ void add_leaf(float v, double& acc64) {
-    if (add(v)) fold();
-    else acc64 += (double)v;
-  }
+  // an overflowed s leaves no error word
   __device__ __forceinline__ double value() const {
-    return (double)(((long long)hi << 18) + lo) * 9.31322574615478515625e-10;  // 2^-30
+    return isfinite(s) ? (double)s + (double)e : (double)s;
   }
 };
 
@@ -365,9 +354,6 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
           const float om = far_field32(rb, rc, rd, re, rf, dx, dy, dz, r2, prm.order);
           if (acc.add(om)) {
             resume = leaf ? node + 1 : link;
-          } else if (Sum::kBounded && isfinite(om)) {
-            acc64 += (double)om;
-            resume = leaf ? node + 1 : link;
           } else {
             near = true;
           }
@@ -387,8 +373,7 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
               const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
               acc.add_leaf(tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx,
                                                   t1.x - fy, t1.y - fz, t1.z - fx, t1.w - fy,
-                                                  t2.x - fz),
-                           acc64);
+                                                  t2.x - fz));
             }
             resume = node + 1;
           } else {
@@ -423,8 +408,9 @@ __device__ __forceinline__ void walk_mixed(const EvalParams& prm, bool valid, do
 __device__ __forceinline__ double mixed_result(const PlainSum& acc, double acc64) {
   return acc64 != 0.0 ? ((double)acc.s + acc64) * kInv4Pi : (double)(acc.s * kInv4PiF);
 }
-__device__ __forceinline__ double mixed_result(const OrderedSum& acc, double acc64) {
-  return (acc.value() + acc64) * kInv4Pi;
+// The sums of a query whose terms may have been added by several lanes.
+__device__ __forceinline__ double mixed_result(double acc, double acc64) {
+  return (acc + acc64) * kInv4Pi;
 }
 
 // Per-warp queue of the plain FP64 walk's terms.  The FP64 pipe charges a
@@ -565,7 +551,7 @@ __device__ __forceinline__ double walk_fp64(const EvalParams& prm, bool valid, d
 // of a team passes the team's query); every lane returns the query's sums.
 template <int kTree>
 __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, int T, bool valid,
-                                                double qx, double qy, double qz, OrderedSum& acc,
+                                                double qx, double qy, double qz, double& sum,
                                                 double& acc64, NearQueue& nq, int2* warp_stack) {
   const int lane = threadIdx.x & 31;
   nq.q[lane][0] = qx;
@@ -577,7 +563,7 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, int T, bo
   const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
   const float S = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + prm.cmax;
   const float sigma = guard_sigma(S);
-  acc = OrderedSum();
+  PairSum acc;
   acc64 = 0.0;
   Team team(T, warp_stack, valid, prm.nnodes);
   while (team.take()) {
@@ -611,10 +597,7 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, int T, bo
       }
       if (!near) {
         const float om = far_field32(rb, rc, rd, re, rf, dx, dy, dz, r2, prm.order);
-        if (!acc.add(om)) {
-          if (isfinite(om)) acc64 += (double)om;
-          else near = true;
-        }
+        near = !acc.add(om);
       }
       if (near) {
         if (leaf) {
@@ -629,8 +612,7 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, int T, bo
             const float4 t2 = __ldg(&prm.tf[(int64_t)slot * 3 + 2]);
             acc.add_leaf(tri_solid_angle<float>(t0.x - fx, t0.y - fy, t0.z - fz, t0.w - fx,
                                                 t1.x - fy, t1.y - fz, t1.z - fx, t1.w - fy,
-                                                t2.x - fz),
-                         acc64);
+                                                t2.x - fz));
           }
         } else {
           open = true;
@@ -655,9 +637,7 @@ __device__ __forceinline__ void walk_mixed_team(const EvalParams& prm, int T, bo
     team.advance(act, open, next);
   }
   if (nqueued) flush_near64(prm.td, nq, nqueued, mine, acc64);
-  acc.fold();
-  acc.hi = team_sum(acc.hi, T);
-  acc.lo = team_sum(acc.lo, T);
+  sum = team_sum(acc.value(), T);
   acc64 = team_sum(acc64, T);
 }
 

@@ -201,3 +201,35 @@ def test_cold_build_does_not_block_resident_meshes(cuda):
         bvh = G.FastWindingNumberBVH(Vb, Fb, 2)
         assert np.abs(Wb - bvh.eval(Qb, 2.0, "mixed", out_dtype=np.float64)).max() <= TOL_SAME
         bvh.close()
+
+
+@pytest.mark.gpu
+def test_served_requests_at_large_accuracy_scales(cuda):
+    """A served request walks one lane per query: inside a closed sphere of
+    327,680 triangles a query adds up to 300,000 far terms of one sign at scales
+    of 100 and more.  W is 1 within the mixed walk's 1e-4, as in the direct call;
+    far outside, where W is as small as 1e-9, both keep FP32's accuracy of the
+    value (3e-6) against the plain FP64 walk."""
+    import libigl_gb300 as G
+    V, F = synth.geodesic_sphere(128)
+    rng = np.random.default_rng(8)
+    Q = rng.normal(size=(257, 3))
+    Q *= 0.05 / np.linalg.norm(Q, axis=1, keepdims=True)
+    T = np.array([[0, 2, 1]], np.int32)
+    P = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0]], float)
+    far = np.array([[0.3, 0.2, z] for z in (1e2, 1e3, 1e4)])
+    with G.Server(hbm_budget_bytes=8 << 30, max_batch_queries=1 << 20, slots=2) as S:
+        m, t = S.add_mesh(V, F), S.add_mesh(P, T)
+        bvh = G.FastWindingNumberBVH(V, F, 2)
+        for scale in (2.0, 30.0, 100.0, 200.0, 400.0):
+            W, _ = S.submit(m, Q, scale, "mixed", out_dtype=np.float64).wait(60)
+            assert np.abs(W - 1).max() <= (5e-3 if scale == 2.0 else 1e-4), scale
+            Wd = bvh.eval(Q, scale, "mixed", out_dtype=np.float64)
+            assert np.abs(W - Wd).max() <= 1e-4, scale
+        bvh.close()
+        bvh = G.FastWindingNumberBVH(P, T, 2)
+        W64 = bvh.eval(far, 2.0, "fp64", out_dtype=np.float64)
+        for W in (S.submit(t, far, 2.0, "mixed", out_dtype=np.float64).wait(60)[0],
+                  bvh.eval(far, 2.0, "mixed", out_dtype=np.float64)):
+            assert (np.abs(W - W64) <= 3e-6 * np.abs(W64)).all()
+        bvh.close()

@@ -250,3 +250,61 @@ def test_lanes_per_query_do_not_change_the_result(cuda, tree, shape):
             assert np.abs(w - W[:m]).max() <= tol, (prec, m)
             assert np.array_equal(w, bvh.eval(Q[:m], 2.0, prec)), (prec, m)
     bvh.close()
+
+
+@pytest.mark.parametrize("nq,scales", [(1, (2, 30, 100, 200, 400)), (33, (30, 100, 200, 400)),
+                                       (3000, (100, 200)), (30_000, (60, 100, 200)),
+                                       (210_000, (60, 80, 100, 200))])
+def test_many_small_terms_of_one_sign(cuda, nq, scales):
+    """A closed sphere of 327,680 triangles seen from inside: from a scale of
+    about 100 a query adds up to 300,000 far terms of one sign, each below 1e-4
+    sr.  Up to 3000 queries share a query between 32 lanes, 30,000 between 8,
+    210,000 between 4.  W is 1 to the mixed walk's 1e-4 (at scale 2 to the
+    expansion's 5e-3), and so is the plain FP64 walk's."""
+    V, F = synth.geodesic_sphere(128)
+    rng = np.random.default_rng(3)
+    Q = rng.normal(size=(nq, 3))
+    Q *= 0.05 * rng.uniform(0, 1, (nq, 1)) / np.linalg.norm(Q, axis=1, keepdims=True)
+    bvh = G.FastWindingNumberBVH(V, F, 2)
+    for scale in scales:
+        tol = 5e-3 if scale == 2 else 1e-4
+        W = bvh.eval(Q, scale, "mixed", out_dtype=np.float64)
+        assert np.abs(W - 1).max() <= tol, scale
+        W64 = bvh.eval(Q[:64], scale, "fp64", out_dtype=np.float64)
+        assert np.abs(W64 - 1).max() <= tol, scale
+        assert np.abs(W[:64] - W64).max() <= 1e-4, scale
+    bvh.close()
+
+
+@pytest.mark.parametrize("nq", [1, 32, 5000, 100_000])
+def test_small_sums_keep_their_relative_accuracy(cuda, nq):
+    """One triangle of unit size from 1e2 to 1e6 units away, within 45 degrees
+    of its normal: W down to 1e-14, in FP32 within the about 50 roundings of a
+    far field or a triangle term (50 x 2^-24 = 3e-6 of the value)."""
+    V = np.array([[0.1, 0, 0], [1.1, 0.2, 0], [0.3, 0.9, 0.1]])
+    F = np.array([[0, 1, 2]], np.int32)
+    n = np.cross(V[1] - V[0], V[2] - V[0])
+    rng = np.random.default_rng(5)
+    d = rng.normal(size=(nq, 3))
+    d = 1.5 * n / np.linalg.norm(n) + d / np.linalg.norm(d, axis=1, keepdims=True)
+    d *= 10.0 ** rng.uniform(2, 6, (nq, 1)) / np.linalg.norm(d, axis=1, keepdims=True)
+    bvh = G.FastWindingNumberBVH(V, F, 2)
+    W = bvh.eval(d, 2.0, "mixed", out_dtype=np.float64)
+    W64 = bvh.eval(d, 2.0, "fp64", out_dtype=np.float64)
+    bvh.close()
+    assert (np.abs(W64) > 1e-15).all()
+    assert (np.abs(W - W64) <= 3e-6 * np.abs(W64)).all()
+
+
+def test_coincident_sheets_beyond_forty_thousand_turns(cuda):
+    """An 80-triangle sphere 45,000 times over, queries at its centre, at a scale
+    that opens every triangle and leaves its term in FP32: W = 45,000, 565,000 sr,
+    each term within about 50 roundings."""
+    V, F = synth.icosphere(1)
+    bvh = G.FastWindingNumberBVH(V, np.tile(F, (45_000, 1)), 2)
+    Q = np.array([[0, 0, 0], [1e-3, 2e-3, 0]])
+    W = bvh.eval(Q, 6.0, "mixed", out_dtype=np.float64)
+    W64 = bvh.eval(Q, 6.0, "fp64", out_dtype=np.float64)
+    bvh.close()
+    assert np.abs(W64 - 45_000).max() <= 45_000 * 1e-10
+    assert np.abs(W - 45_000).max() <= 45_000 * 3e-6
