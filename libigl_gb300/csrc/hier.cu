@@ -603,37 +603,29 @@ __device__ __forceinline__ void flush_hier64(const double* __restrict__ tris64,
   __syncwarp();
 }
 
-// The nodes above subtree y0 (at most log2(kMaxSplit)), root first.  A lane
-// outside one of their boxes takes that node's cap in place of everything
-// below it, in the leftmost of the subtrees below (first: every step from the
-// node down to y0 goes left), as the whole-tree walk would; the others add
-// nothing.  Of the nodes above the coarse cut (depth `coarse`) only the root's
-// cap is taken: the error of a cap triangle's term grows with the square of its
-// size over the query's distance from its edges, so the largest caps are the
-// least accurate, and a batch that is split has never used them.
-struct Above {
-  int node[8], n = 0;
-  unsigned left = 0;  // bit i: the step down from node[i] goes left
-
-  __device__ __forceinline__ Above(const NodeH* nodes, int y0) {
-    int x = 0;
-    while (x != y0 && n < 8) {
-      node[n] = x;
-      const int l = x + 1;
-      const int meta = __float_as_int(nodes[l].hi.w);
-      const int l_end = meta <= -2 ? l + 1 : __float_as_int(nodes[l].lo.w);
-      const bool go_left = y0 < l_end;
-      if (go_left) left |= 1u << n;
-      ++n;
-      x = go_left ? l : l_end;
-    }
-  }
-  __device__ __forceinline__ static bool usable(int i, int coarse) { return i == 0 || i >= coarse; }
-  __device__ __forceinline__ bool first(int i) const {
-    const unsigned m = ((1u << n) - 1u) & ~((1u << i) - 1u);
-    return (left & m) == m;
-  }
-};
+// f(node, first) for the nodes above subtree y0 whose caps a split batch takes,
+// root first (up to kMaxSplit / 2 of them: a cut that meets a leaf in every
+// round goes down one level for one subtree more).  A lane outside such a node's
+// box takes its cap in place of everything below it, in the leftmost of the
+// subtrees below, as the whole-tree walk would; the others add nothing.  first:
+// y0 is that leftmost subtree, which in pre-order is as many positions past the
+// node as it is levels below.  Of the nodes above the coarse cut (depth
+// `coarse`) only the root's cap is taken: the error of a cap triangle's term
+// grows with the square of its size over the query's distance from its edges, so
+// the largest caps are the least accurate, and a batch that is split has never
+// used them.
+template <typename Fn>
+__device__ __forceinline__ void each_above(const NodeH* nodes, int y0, int coarse, Fn&& f) {
+  auto towards = [&](int x) {  // the child of x on the path to y0
+    const int l = x + 1, meta = __float_as_int(nodes[l].hi.w);
+    const int l_end = meta <= -2 ? l + 1 : __float_as_int(nodes[l].lo.w);
+    return y0 < l_end ? l : l_end;
+  };
+  int depth = 0;
+  for (int x = 0; x != y0; x = towards(x)) ++depth;
+  for (int x = 0, d = 0; x != y0; x = towards(x), ++d)
+    if (d == 0 || d >= coarse) f(x, y0 - x == depth - d);
+}
 
 template <typename QT>
 __global__ void __launch_bounds__(kWalk, 16) hier_walk_kernel(HierDev H, const QT* __restrict__ Q,
@@ -678,15 +670,14 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk_kernel(HierDev H, const Q
   int nqueued = 0;  // warp-uniform
   int resume = valid ? x0 : 0x7fffffff;
   if (ranges) {
-    const Above up(H.nodes, x0);
-    for (int i = 0; i < up.n; ++i) {
-      const NodeH nd = H.nodes[up.node[i]];
+    each_above(H.nodes, x0, coarse, [&](int y, bool first) {
+      const NodeH nd = H.nodes[y];
       const int meta = __float_as_int(nd.hi.w);
-      if (Above::usable(i, coarse) && resume == x0 && meta >= 0 &&
+      if (resume == x0 && meta >= 0 &&
           (qh.x < nd.lo.x || qh.x > nd.hi.x || qh.y < nd.lo.y || qh.y > nd.hi.y ||
            qh.z < nd.lo.z || qh.z > nd.hi.z)) {
-        if (up.first(i)) {
-          const int cn = H.capn[up.node[i]];
+        if (first) {
+          const int cn = H.capn[y];
           for (int k = 0; k < cn; ++k) {
             const TriH t = H.caps[meta + k];
             acc.add(trih_term32(t, rel_a(t, qh, ql)));
@@ -694,7 +685,7 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk_kernel(HierDev H, const Q
         }
         resume = 0x7fffffff;
       }
-    }
+    });
   }
   int x = x0;
   while (x < x1) {
@@ -857,16 +848,15 @@ __global__ void __launch_bounds__(kWalk, 16) hier_walk64_kernel(HierDev H, const
   unsigned mine = 0;  // this lane's queue positions
   int resume = valid ? x0 : 0x7fffffff;
   if (ranges) {
-    const Above up(H.nodes, x0);
-    for (int i = 0; i < up.n; ++i) {
-      const int y = up.node[i], meta = __float_as_int(H.nodes[y].hi.w);
+    each_above(H.nodes, x0, coarse, [&](int y, bool first) {
+      const int meta = __float_as_int(H.nodes[y].hi.w);
       int cnt = 0;
-      if (Above::usable(i, coarse) && resume == x0 && meta >= 0 && outside(y)) {
-        if (up.first(i)) cnt = H.capn[y];
+      if (resume == x0 && meta >= 0 && outside(y)) {
+        if (first) cnt = H.capn[y];
         resume = 0x7fffffff;
       }
       if (__any_sync(0xffffffffu, cnt > 0)) enqueue64(H, hq, cnt, meta, nq, mine, acc);
-    }
+    });
   }
   int x = x0;
   while (x < x1) {
@@ -1143,7 +1133,7 @@ void hier_eval(const HierTree& h, const double* Q, int64_t nQ, double* W, cudaSt
   // Too few queries for six waves of warps: each warp of queries walks one of
   // up to 32 subtrees (blockIdx.y), and the partial sums are added in a fixed
   // order.  Warps near the surface walk far longer than the others, and with
-  // the caps above the cut kept (Above) a finer cut adds little work.  FP64,
+  // the caps above the cut kept (each_above) a finer cut adds little work.  FP64,
   // 50,001 queries, 20,480 triangles: 10.9 ms with up to 8 subtrees at three
   // waves, 8.4 ms so; mixed, 100,000 queries, 5,120 triangles 1.15 -> 1.00 ms.
   // Taking every cap above the cut would give 6.7 and 0.97 ms, but in FP64 two

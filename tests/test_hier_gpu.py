@@ -172,3 +172,31 @@ def test_split_batches_keep_the_accuracy_of_the_terms(cuda, nu, nq):
         w = torch.atan2(det, den).sum(-1) / (2 * np.pi)
         err.append(w.cpu().numpy() - W[s:s + 2000])
     assert np.quantile(np.abs(np.concatenate(err)), 0.999) <= 64 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("nq", [1, 31, 1000, 50_000])
+@pytest.mark.parametrize("strays", [5, 8, 11, 14])
+def test_single_triangles_at_halving_distances(cuda, strays, nq):
+    """An open patch of 2048 triangles in a corner of the box, and single
+    triangles at halving distances from it: the tree loses one triangle a level
+    there, so that the parallel subtrees of a small batch lie up to 16 levels
+    deep.  Queries outside the root's box, whose cap the whole tree shares, and
+    between the nested boxes, against the all-pairs sum."""
+    g = np.stack(np.meshgrid(np.arange(33.0), np.arange(33.0), indexing="ij"), -1).reshape(-1, 2)
+    V = np.concatenate([g, g @ [[0.3], [0.2]]], 1) / 32 * 2.0 ** -strays
+    i = (33 * np.arange(32)[:, None] + np.arange(32)).reshape(-1)
+    F = np.concatenate([np.stack([i, i + 33, i + 1], 1), np.stack([i + 1, i + 33, i + 34], 1)])
+    k = 2.0 ** -np.arange(strays)[:, None, None]
+    T = k * (1 + np.array([[0, 0, 0], [0.2, 0, 0.05], [0, 0.2, 0.1]]))
+    F = np.concatenate([F, len(V) + np.arange(3 * strays).reshape(-1, 3)]).astype(np.int32)
+    V = np.concatenate([V, T.reshape(-1, 3)])
+    rng = np.random.default_rng([strays, nq])
+    Q = rng.uniform(-0.5, 1.7, (nq, 3))
+    near = rng.normal(size=(nq, 3)) * 2.0 ** rng.uniform(-strays - 2, 1, (nq, 1))
+    Q = np.where(rng.random((nq, 1)) < 0.7, near, Q)
+    W = O.winding_number(V, F, Q)
+    assert nq < 1000 or np.abs(W).max() > 0.1
+    h = G.WindingNumberAABB(V, F)
+    assert np.abs(h.winding_number(Q, "fp64") - W).max() <= 1e-11
+    assert np.abs(h.winding_number(Q, "mixed") - W).max() <= 1e-4
+    h.close()
