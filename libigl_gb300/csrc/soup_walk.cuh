@@ -83,9 +83,17 @@ __device__ __forceinline__ T tri_solid_angle(T ax, T ay, T az, T bx, T by, T bz,
 // solid_angle_vos64 below, angle included in FP64, with the normalised form's
 // zeros (a corner at q, coinciding corners, a zero determinant).  Nine
 // divisions fewer; corners so far or near that the products of three lengths
-// would leave the range take the normalised form.
+// would leave the range take the normalised form.  The determinant of the
+// corners loses (distance / edge)^2 of its digits, where the normalised form
+// loses distance / edge, so beyond about two edges (the mean square edge below
+// a quarter of the mean square distance: sum of l^2 - dot products) it is taken
+// as the corner's product with the edges' normal, which loses neither (rms
+// error at 2, 20, 200 edges: corners 7e-17, 7e-18, 5e-18; normalised 6e-17,
+// 3e-18, 3e-19; edges 6e-17, 9e-19, 1e-20; next to the triangle the corners'
+// is the better one).  Only a walk whose scale beta exceeds 2 opens a triangle
+// from there; the others are spared the test (2% of 300,001 queries' 5.79 ms).
 __device__ __forceinline__ double tri_solid_angle64(const double* __restrict__ t, double qx,
-                                                    double qy, double qz) {
+                                                    double qy, double qz, double beta2) {
   const double ax = t[0] - qx, ay = t[1] - qy, az = t[2] - qz;
   const double bx = t[3] - qx, by = t[4] - qy, bz = t[5] - qz;
   const double cx = t[6] - qx, cy = t[7] - qy, cz = t[8] - qz;
@@ -99,11 +107,19 @@ __device__ __forceinline__ double tri_solid_angle64(const double* __restrict__ t
   if ((ax == bx && ay == by && az == bz) || (ax == cx && ay == cy && az == cz) ||
       (bx == cx && by == cy && bz == cz))
     return 0.0;
-  const double det = ax * (by * cz - bz * cy) + ay * (bz * cx - bx * cz) + az * (bx * cy - by * cx);
+  const double ab = ax * bx + ay * by + az * bz, ac = ax * cx + ay * cy + az * cz,
+               bc = bx * cx + by * cy + bz * cz;
+  double det;
+  if (beta2 > 4.0 && ab + ac + bc > 0.875 * (la2 + lb2 + lc2)) {
+    const double ux = t[3] - t[0], uy = t[4] - t[1], uz = t[5] - t[2];
+    const double vx = t[6] - t[0], vy = t[7] - t[1], vz = t[8] - t[2];
+    det = ax * (uy * vz - uz * vy) + ay * (uz * vx - ux * vz) + az * (ux * vy - uy * vx);
+  } else {
+    det = ax * (by * cz - bz * cy) + ay * (bz * cx - bx * cz) + az * (bx * cy - by * cx);
+  }
   if (det == 0.0) return 0.0;
   const double la = sqrt(la2), lb = sqrt(lb2), lc = sqrt(lc2);
-  const double den = la * lb * lc + (ax * bx + ay * by + az * bz) * lc +
-                     (ax * cx + ay * cy + az * cz) * lb + (bx * cx + by * cy + bz * cz) * la;
+  const double den = la * lb * lc + ab * lc + ac * lb + bc * la;
   return 2.0 * atan2(det, den);
 }
 
@@ -448,7 +464,7 @@ __device__ __forceinline__ void flush_fp64(const EvalParams& prm, Fp64Queue& fq,
         v = far_field64(r, dx, dy, dz, r2, prm.order);
       } else {
         const double* t = prm.td + (int64_t)(~e.x) * 9;
-        v = tri_solid_angle64(t, qx, qy, qz);
+        v = tri_solid_angle64(t, qx, qy, qz, prm.beta2d);
       }
       fq.v[lane] = v;
     }
@@ -747,7 +763,7 @@ __device__ inline double walk_fp64_lane(const EvalParams& prm, double qx, double
     }
     if (leaf) {
       const double* t = prm.td + (int64_t)(~link) * 9;
-      acc += tri_solid_angle64(t, qx, qy, qz);
+      acc += tri_solid_angle64(t, qx, qy, qz, prm.beta2d);
     }
     ++node;
   }

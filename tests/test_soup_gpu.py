@@ -16,6 +16,7 @@ Checks, through the C ABI:
     test allows (tests/include/igl/fast_winding_number.cpp:76).
 """
 import os
+from decimal import Decimal, getcontext
 
 import numpy as np
 import pytest
@@ -308,3 +309,43 @@ def test_coincident_sheets_beyond_forty_thousand_turns(cuda):
     bvh.close()
     assert np.abs(W64 - 45_000).max() <= 45_000 * 1e-10
     assert np.abs(W - 45_000).max() <= 45_000 * 3e-6
+
+
+def _solid_angle_50_digits(T, q):
+    """Solid angle of triangle T from q (van Oosterom and Strackee), for a
+    small angle: the arc tangent by its series."""
+    getcontext().prec = 50
+    a, b, c = ([Decimal(float(x)) - Decimal(float(y)) for x, y in zip(p, q)] for p in T)
+
+    def dot(u, v):
+        return sum((x * y for x, y in zip(u, v)), Decimal(0))
+
+    la, lb, lc = (dot(p, p).sqrt() for p in (a, b, c))
+    det = (a[0] * (b[1] * c[2] - b[2] * c[1]) + a[1] * (b[2] * c[0] - b[0] * c[2])
+           + a[2] * (b[0] * c[1] - b[1] * c[0]))
+    x = det / (la * lb * lc + dot(a, b) * lc + dot(a, c) * lb + dot(b, c) * la)
+    return 2 * sum((x ** (2 * k + 1) * (-1) ** k / (2 * k + 1) for k in range(20)), Decimal(0))
+
+
+@pytest.mark.parametrize("tree", ["reference", "binned"])
+def test_distant_opened_triangles_keep_their_digits(cuda, tree):
+    """A large accuracy scale opens a triangle d/e = 4 to 1e6 edges away: the
+    plain FP64 term is within 4 u e/d sr of the solid angle (u = 2^-53), the
+    rounding of differences of unit vectors e/d apart."""
+    rng = np.random.default_rng(17)
+    F = np.array([[0, 1, 2]], np.int32)
+    for _ in range(20):
+        T = rng.normal(size=(3, 3))
+        e = max(np.linalg.norm(T[i] - T[j]) for i, j in ((0, 1), (1, 2), (2, 0)))
+        n = np.cross(T[1] - T[0], T[2] - T[0])
+        d = rng.normal(size=(30, 3))
+        d = 1.5 * n / np.linalg.norm(n) + d / np.linalg.norm(d, axis=1, keepdims=True)
+        far = 10.0 ** rng.uniform(np.log10(4), 6, (30, 1))
+        Q = T.mean(0) + far * e * d / np.linalg.norm(d, axis=1, keepdims=True)
+        bvh = G.FastWindingNumberBVH(T, F, 2, tree=tree)
+        W = bvh.eval(Q, 1e9, "fp64", out_dtype=np.float64)
+        bvh.close()
+        for q, w, f in zip(Q, W, far[:, 0]):
+            err = abs(float(Decimal(float(w)) * Decimal(4 * np.pi) - _solid_angle_50_digits(T, q)))
+            # 2 u |value|: the factor 1 / 4 pi and its product here
+            assert err <= 2.0 ** -53 * (4 / f + 3 * abs(4 * np.pi * w)), f
