@@ -862,6 +862,23 @@ __global__ void __launch_bounds__(32) part_warp_kernel(RNode* __restrict__ nodes
   }
 }
 
+// Entries first, first + stride, .. below n of a tape follow their copies back to
+// a box.  All entries walk at once and keep their progress in the tape, so a walk
+// meets entries that are already (partly) resolved: pointer doubling without
+// rounds.  Each step goes to an earlier entry, so a walk ends whatever the others
+// do.
+__device__ __forceinline__ void resolve_tape(uint32_t* tape, uint32_t n, uint32_t first,
+                                             uint32_t stride) {
+  for (uint32_t rel = first; rel < n; rel += stride) {
+    uint32_t at = rel, v = __ldcg(tape + rel);
+    while (!(v & kTerm) && v < at) {
+      at = v;
+      v = __ldcg(tape + v);
+      __stcg(tape + rel, v);
+    }
+  }
+}
+
 // partitionByCentre of positions [lo, hi) by one CTA of 32 warps, centres in
 // cen: each warp counts its segment, the segments' prefixes give every warp
 // its tape state, then the tapes are written and resolved.
@@ -936,16 +953,14 @@ __device__ void cta_partition(CtaPart& S, uint32_t* idx, float* cen, uint32_t* t
   __syncthreads();
   const uint32_t RE = t.firstE != kNone ? nL - t.L_atE : 0u;
   const uint32_t RG = t.firstG != kNone ? nL + nE - t.LE_atG : 0u;
+  resolve_tape(tape_e + lo, nE + RE, threadIdx.x, blockDim.x);
+  resolve_tape(tape_g + lo, jn - nL - nE + RG, threadIdx.x, blockDim.x);
+  __syncthreads();
   for (uint32_t rel = threadIdx.x; rel < jn; rel += blockDim.x) {
     uint32_t v;
-    if (rel < nL) {
-      v = tmp[lo + rel];
-    } else {
-      const bool eq = rel < nL + nE;
-      const uint32_t* tape = (eq ? tape_e : tape_g) + lo;
-      v = tape[eq ? RE + (rel - nL) : RG + (rel - nL - nE)];
-      while (!(v & kTerm)) v = tape[v];  // each copy refers to an earlier entry
-    }
+    if (rel < nL) v = tmp[lo + rel];
+    else if (rel < nL + nE) v = __ldcg(tape_e + lo + RE + (rel - nL));
+    else v = __ldcg(tape_g + lo + RG + (rel - nL - nE));
     idx[lo + rel] = v & ~kTerm;
   }
   __syncthreads();
@@ -1402,10 +1417,7 @@ __global__ void __launch_bounds__(256) wide_tape_kernel(
   }
 }
 
-// Pass 5: every tape entry follows its copies back to a box.  All entries
-// walk at once and keep their progress in the tape, so a walk meets entries
-// that are already (partly) resolved: pointer doubling without rounds.  Each
-// step goes to an earlier entry, so a walk ends whatever the others do.
+// Pass 5: the tapes' copies.
 __global__ void __launch_bounds__(256) wide_resolve_kernel(const int4* __restrict__ chunks,
                                                            const uint32_t* __restrict__ nchunks,
                                                            const LTask* __restrict__ T,
@@ -1414,23 +1426,12 @@ __global__ void __launch_bounds__(256) wide_resolve_kernel(const int4* __restric
   const int4 ch = chunks[blockIdx.x];
   const LTask& t = T[ch.x];
   if (!t.live) return;
-  const uint32_t s = t.start;
+  const uint32_t s = t.start, first = (uint32_t)ch.y - s + threadIdx.x, end = (uint32_t)ch.z - s;
   const uint32_t nG = t.n - t.nL - t.nE;
   const uint32_t lenE = t.nE + (t.firstE != kNone ? t.nL - t.L_atE : 0u);
   const uint32_t lenG = nG + (t.firstG != kNone ? (t.nL + t.nE) - t.LE_atG : 0u);
-  auto walk = [&](uint32_t* tape, uint32_t rel) {
-    uint32_t at = rel, v = __ldcg(tape + rel);
-    while (!(v & kTerm) && v < at) {
-      at = v;
-      v = __ldcg(tape + v);
-      __stcg(tape + rel, v);
-    }
-  };
-  for (int p = ch.y + threadIdx.x; p < ch.z; p += blockDim.x) {
-    const uint32_t rel = (uint32_t)p - s;
-    if (rel < lenE) walk(tape_e + s, rel);
-    if (rel < lenG) walk(tape_g + s, rel);
-  }
+  resolve_tape(tape_e + s, min(lenE, end), first, blockDim.x);
+  resolve_tape(tape_g + s, min(lenG, end), first, blockDim.x);
 }
 
 // Pass 6: the partitioned order back into idx: below | equal queue | upper

@@ -21,6 +21,7 @@ FP32 open test (FWNFS.h:7176-7193).  Checked through the C ABI:
     handle equals the binned handle's.
 """
 import os
+import time
 
 import numpy as np
 import pytest
@@ -160,3 +161,55 @@ def test_host_buffers_equal_the_device_call(cuda):
     Wd32 = bvh.eval(torch.from_numpy(Q.astype(np.float32)).cuda(), 2.0,
                     precision="mixed").cpu().numpy()
     assert np.array_equal(Wh32, Wd32)
+
+
+@pytest.mark.parametrize("kind,n", [("far", 40_000), ("far", 330_000), ("scales", 50_000),
+                                    ("scales", 150_000), ("line", 120_000), ("same", 70_000)])
+def test_uneven_trees_equal_the_oracle_tree(cuda, kind, n):
+    """Large nodes without a balanced span: one triangle far away, triangles at
+    sizes and places over five decades, triangles gathered towards one end of a
+    line, and equal ones.  Their cut comes from nthElement over tens of thousands
+    of boxes, whose order of partition decides the whole tree below."""
+    rng = np.random.default_rng([n, len(kind)])
+    if kind == "far":
+        C, s = rng.normal(size=(n, 3)), np.full((n, 1), 0.01)
+        C[n // 2] = [1e4, 0, 0]
+    elif kind == "scales":
+        C = rng.normal(size=(n, 3)) * 10.0 ** rng.uniform(-4, 1, (n, 1))
+        s = 10.0 ** rng.uniform(-5, -1, (n, 1))
+    elif kind == "line":
+        C = np.c_[10.0 ** rng.uniform(-6, 3, n), 1e-3 * rng.normal(size=(n, 2))]
+        s = np.full((n, 1), 1e-4)
+    else:
+        C, s = rng.integers(0, 2, (n, 3)).astype(float), np.full((n, 1), 0.5)
+    D = rng.normal(size=(n, 3, 3))
+    if kind == "same":
+        D[:] = D[0]
+    V = (C[:, None] + s[:, None] * D).reshape(-1, 3)
+    F = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    T = G.FastWindingNumberBVH(V, F, order=2, tree="reference").tree_nodes()
+    To = O.SoupPort(V, F, order=2).tree()
+    assert np.array_equal(T, To)
+
+
+def test_a_far_triangle_costs_the_build_a_few_partitions(cuda):
+    """1.3M triangles and one 10,000 radii away: the root's cut comes from
+    nthElement, some twenty partitions in one CTA: about three times the build
+    of the sphere alone, and seven times with the queues' copies followed one by
+    one."""
+    V, F = synth.geodesic_sphere(256)
+    t = []
+    for far in (False, True):
+        if far:
+            F = np.concatenate([F, len(V) + np.arange(3)[None]]).astype(np.int32)
+            V = np.concatenate([V, [[1e4, 0, 0], [1e4, 1, 0], [1e4, 0, 1]]])
+        v, f = cuda.from_numpy(V).cuda(), cuda.from_numpy(F).cuda()
+        best = float("inf")
+        for k in range(7):
+            cuda.cuda.synchronize()
+            t0 = time.perf_counter()
+            G.FastWindingNumberBVH(v, f).close()
+            if k >= 2:
+                best = min(best, time.perf_counter() - t0)
+        t.append(best)
+    assert t[1] <= 5 * t[0], t
