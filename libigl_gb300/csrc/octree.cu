@@ -404,16 +404,64 @@ __global__ void final_layout_kernel(int64_t ncells, const double* __restrict__ c
 // p are those of the depths cpl[p] + 1 .. cpl[p + 1]: listed p by p, that is
 // depth-first pre-order, the order of the ids.  A cell's end and its children
 // are found by searching the sorted keys.
-// The key holds 10, 16 or 21 octants (4, 6 or 8 sort passes, by the point
-// count); runs of equal keys are ordered by their deeper octants, one thread
-// per run.  A run of more than kTieRun points takes the longest key; with that,
-// or where points share kTieDepth octants (identical ones above all), the whole
-// build is left to the level loop below, which follows them to depth 30000.
+// The key is one word of 10, 16 or 21 octants (4, 6 or 8 sort passes, by the
+// point count) or, where many points share those (a far outlier, points at all
+// scales), three words of 21, sorted last word first.  Runs of equal keys are
+// ordered by their deeper octants, one thread per run of up to kTieRun points.
+// Where points share kTieDepth octants (identical ones above all), or more than
+// kTieRun of them all three words, the whole build is left to the level loop
+// below, which follows them to depth 30000.
 // In place of about 20 launches, 6 scans and a host read per level, over every
-// point: 2M points 7.0 -> 2.6 ms when it came, with longer keys than now.
+// point: 2M points 7.5 -> 1.6 ms.
 constexpr int kKeyDepth = 21;
+constexpr int kKeyWords = 3;
 constexpr int kTieDepth = 64;
 constexpr int kTieRun = 32;
+// A run this long is not expected to be split by the 5 octants that the longest
+// one-word key has more than the shorter one.
+constexpr int kLongRun = 4096;
+
+// A point's key: W words of kd octants.
+template <int W>
+struct PathKeys {
+  unsigned long long* w[W];
+  int kd;
+
+  __device__ __forceinline__ bool equal(int64_t a, int64_t b) const {
+    bool eq = true;
+#pragma unroll
+    for (int i = 0; i < W; ++i) eq = eq && w[i][a] == w[i][b];
+    return eq;
+  }
+};
+// Octant l of a key; whether the first d octants of two keys agree.
+template <int W>
+struct PathKey {
+  unsigned long long w[W];
+  __device__ __forceinline__ PathKey(const PathKeys<W>& k, int64_t p) {
+#pragma unroll
+    for (int i = 0; i < W; ++i) w[i] = k.w[i][p];
+  }
+  __device__ __forceinline__ int octant(int kd, int l) const {
+    unsigned long long v = w[0];
+    if (W > 1) {
+#pragma unroll
+      for (int i = 1; i < W; ++i)
+        if (l >= i * kd) v = w[i];
+      l %= kd;
+    }
+    return (int)((v >> (3 * (kd - 1 - l))) & 7ull);
+  }
+  __device__ __forceinline__ bool agrees(const PathKey& o, int kd, int d) const {
+    bool eq = true;
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const int left = min(max(d - i * kd, 0), kd);  // octants of this word
+      eq = eq && (left == 0 || ((w[i] ^ o.w[i]) >> (3 * (kd - left))) == 0);
+    }
+    return eq;
+  }
+};
 
 // By depth: the cell width and the step from a centre to its children's, as
 // the reference halves them.
@@ -432,7 +480,9 @@ __global__ void widths_kernel(const double* __restrict__ rw, Widths* __restrict_
 
 struct PathTotals {
   unsigned long long nindices;
-  uint32_t ninternal, max_cpl, deep;
+  uint32_t ninternal, max_cpl;
+  uint32_t deep;              // points share kTieDepth octants
+  uint32_t long_run, longer;  // a run of more than kTieRun / kLongRun equal keys
 };
 
 // The octant walk of one point: the centre of its cell.
@@ -448,23 +498,32 @@ struct Walk {
   }
 };
 
-// Keys of kd octants.
+template <int W>
 __global__ void path_keys_kernel(const double* __restrict__ P, int64_t n,
                                  const double* __restrict__ rc, const Widths* __restrict__ t,
-                                 int kd, unsigned long long* __restrict__ key,
-                                 int32_t* __restrict__ val) {
+                                 PathKeys<W> keys, int32_t* __restrict__ val) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double p[3] = {P[i * 3], P[i * 3 + 1], P[i * 3 + 2]};
   Walk w{{rc[0], rc[1], rc[2]}};
-  unsigned long long k = 0;
-  for (int d = 0; d < kd; ++d) {
-    const int o = w.octant(p);
-    k = k << 3 | (unsigned)o;
-    w.descend(o, t->step[d]);
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    unsigned long long k = 0;
+    for (int d = 0; d < keys.kd; ++d) {
+      const int o = w.octant(p);
+      k = k << 3 | (unsigned)o;
+      w.descend(o, t->step[j * keys.kd + d]);
+    }
+    keys.w[j][i] = k;
   }
-  key[i] = k;
   val[i] = (int32_t)i;
+}
+
+__global__ void gather_keys_kernel(const unsigned long long* __restrict__ key,
+                                   const int32_t* __restrict__ val, int64_t n,
+                                   unsigned long long* __restrict__ out) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) out[i] = key[val[i]];
 }
 
 // Octants that points a and b share, up to kTieDepth; less: a's path is the
@@ -487,18 +546,21 @@ __device__ int shared_octants(const double* P, int32_t a, int32_t b, const doubl
 }
 
 // Runs of equal keys, ordered by the octants past the key: one thread per run.
+// Once a run is too long the key will not do, and what has not begun ends here.
+template <int W>
 __global__ void tie_runs_kernel(const double* __restrict__ P, int64_t n,
                                 const double* __restrict__ rc, const Widths* __restrict__ t,
-                                const unsigned long long* __restrict__ key, int32_t* val,
-                                PathTotals* __restrict__ tot) {
+                                PathKeys<W> keys, int32_t* val, PathTotals* tot) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p + 1 >= n || key[p] != key[p + 1] || (p > 0 && key[p - 1] == key[p])) return;
-  int64_t e = p + 2;
-  while (e < n && e - p <= kTieRun && key[e] == key[p]) ++e;
-  if (e - p > kTieRun) {
-    tot->deep = 1;
+  if (p + 1 >= n || !keys.equal(p, p + 1) || (p > 0 && keys.equal(p - 1, p))) return;
+  if (p + kTieRun < n && keys.equal(p, p + kTieRun)) {
+    tot->long_run = 1;
+    if (p + kLongRun < n && keys.equal(p, p + kLongRun)) tot->longer = 1;
     return;
   }
+  if (__ldcg(&tot->long_run)) return;
+  int64_t e = p + 2;
+  while (e < n && keys.equal(p, e)) ++e;
   for (int64_t i = p + 1; i < e; ++i) {  // stable insertion sort
     const int32_t v = val[i];
     int64_t j = i;
@@ -514,19 +576,24 @@ __global__ void tie_runs_kernel(const double* __restrict__ P, int64_t n,
 }
 
 // cpl[p] and, per point, how many internal cells start at it.
+template <int W>
 __global__ void __launch_bounds__(256) cpl_kernel(const double* __restrict__ P, int64_t n,
                                                   const double* __restrict__ rc,
-                                                  const Widths* __restrict__ t, int kd,
-                                                  const unsigned long long* __restrict__ key,
+                                                  const Widths* __restrict__ t,
+                                                  PathKeys<W> keys,
                                                   const int32_t* __restrict__ val,
                                                   int8_t* __restrict__ cpl,
                                                   uint32_t* __restrict__ starts,
                                                   PathTotals* __restrict__ tot) {
+  if (tot->long_run || tot->deep) return;
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   auto shared = [&](int64_t q) {  // octants shared by the sorted points q - 1 and q
     if (q <= 0 || q >= n) return -1;
-    const unsigned long long x = key[q - 1] ^ key[q];
-    if (x) return (__clzll((long long)x) - (64 - 3 * kd)) / 3;
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const unsigned long long x = keys.w[i][q - 1] ^ keys.w[i][q];
+      if (x) return i * keys.kd + (__clzll((long long)x) - (64 - 3 * keys.kd)) / 3;
+    }
     bool less;
     const int d = shared_octants(P, val[q - 1], val[q], rc, t, less);
     if (d == kTieDepth) tot->deep = 1;
@@ -580,10 +647,10 @@ __global__ void list_cells_kernel(const int8_t* __restrict__ cpl, const uint32_t
 
 // Eight lanes per internal cell, one per child: the cell's points are
 // [p, e), child o's those whose octant at this depth is o.
+template <int W>
 __global__ void __launch_bounds__(256) cells_kernel(
     const double* __restrict__ P, int64_t n, const double* __restrict__ rc,
-    const Widths* __restrict__ t, int kd, const unsigned long long* __restrict__ key,
-    const int32_t* __restrict__ val, const int8_t* __restrict__ cpl,
+    const Widths* __restrict__ t, PathKeys<W> keys, const int32_t* __restrict__ val, const int8_t* __restrict__ cpl,
     const uint32_t* __restrict__ base, uint32_t ninternal, const int32_t* __restrict__ cell_first,
     const int8_t* __restrict__ cell_depth, double* __restrict__ cn, double* __restrict__ cw,
     int32_t* __restrict__ ch, int64_t* __restrict__ start, int32_t* __restrict__ count,
@@ -594,7 +661,8 @@ __global__ void __launch_bounds__(256) cells_kernel(
   const bool live = r < ninternal;
   const int64_t p = live ? cell_first[r] : 0;
   const int d = live ? cell_depth[r] : 0;
-  const unsigned long long kp = live ? key[p] : 0;
+  const int kw = keys.kd, kd = W * kw;  // octants per word, of the key
+  const PathKey<W> kp(keys, p);
   const int32_t pt = live ? val[p] : 0;
   // centre: lane o follows axis o mod 3 down the path of the cell's first point
   const int axis = o % 3;
@@ -603,7 +671,7 @@ __global__ void __launch_bounds__(256) cells_kernel(
   const int dmax = __reduce_max_sync(full, d);
   for (int l = 0; l < dmax; ++l) {
     if (l < d) {
-      const bool up = l < kd ? (kp >> (3 * (kd - 1 - l) + axis)) & 1ull : x >= c;
+      const bool up = l < kd ? (kp.octant(kw, l) >> axis) & 1 : x >= c;
       const double step = t->step[l];
       c = __dadd_rn(c, up ? step : -step);
     }
@@ -617,10 +685,9 @@ __global__ void __launch_bounds__(256) cells_kernel(
       e = p + 1;
       while (e < n && cpl[e] >= d) ++e;
     } else if (d > 0) {
-      const int sh = 3 * (kd - d);
-      const unsigned long long top = kp >> sh;
+      auto inside = [&](int64_t m) { return kp.agrees(PathKey<W>(keys, m), kw, d); };
       int64_t step = 1, a = p, b = p + 1;  // a inside, b the first known outside
-      while (b < n && (key[b] >> sh) == top) {
+      while (b < n && inside(b)) {
         a = b;
         step *= 2;
         b = p + step;
@@ -628,7 +695,7 @@ __global__ void __launch_bounds__(256) cells_kernel(
       b = min(b, n);
       while (b - a > 1) {
         const int64_t m = (a + b) >> 1;
-        if ((key[m] >> sh) == top) a = m;
+        if (inside(m)) a = m;
         else b = m;
       }
       e = b;
@@ -644,11 +711,10 @@ __global__ void __launch_bounds__(256) cells_kernel(
         ++lb;
       }
     } else if (o > 0) {
-      const int sh = 3 * (kd - 1 - d);
       int64_t a = p - 1, b = e;  // octant(a) < o <= octant(b)
       while (b - a > 1) {
         const int64_t m = (a + b) >> 1;
-        if ((int)((key[m] >> sh) & 7ull) >= o) b = m;
+        if (PathKey<W>(keys, m).octant(kw, d) >= o) b = m;
         else a = m;
       }
       lb = b;
@@ -787,47 +853,56 @@ int bits_for(uint64_t maxval) {
 
 }  // namespace
 
-// The build from sorted paths; false when the level loop has to do it.
-static bool octree_build_paths(gwn_octree_impl& t, const double* dP, int64_t n, const double* rc,
-                               const double* rw, cudaStream_t st) {
+// One attempt of the build from sorted paths with keys of W words of kd octants:
+// sorts, and fills the tree unless the totals say that the key will not do.
+template <int W>
+static PathTotals octree_try_paths(gwn_octree_impl& t, const double* dP, int64_t n,
+                                   const double* rc, const Widths* wt, int kd, cudaStream_t st) {
+  using Key = unsigned long long;
   const size_t N = (size_t)n;
-  DevBuf<unsigned long long> key(N, st), key_tmp(N, st);
+  DevBuf<Key> sorted(N, st), tmp(N, st), word[W];
   DevBuf<int32_t> val(N, st), val_tmp(N, st);
   DevBuf<int8_t> cpl(N, st);
   DevBuf<uint32_t> starts(N, st), base(N, st);
   DevBuf<PathTotals> tot(1, st);
-  DevBuf<Widths> widths(1, st);
   PathTotals* h = reinterpret_cast<PathTotals*>(pinned_words());
-  const Widths* wt = widths.get();
-  launch_kernel(widths_kernel, 1, 1, 0, st, rw, widths.get());
-  // Octants per key: points spread over a surface share about log2(n) / 2, so
-  // 10 (four passes) and 16 (six) leave few equal keys to 4096 and 16M points.
-  int kd = n <= 4096 ? 10 : (n <= (int64_t(16) << 20) ? 16 : kKeyDepth);
-  for (;;) {
-    tot.zero(st);
-    launch_kernel(path_keys_kernel, blocks(n), 256, 0, st, dP, n, rc, wt, kd, key.get(),
-                  val.get());
-    radix_sort_pairs<unsigned long long>(key.get(), val.get(), key_tmp.get(), val_tmp.get(), n, 0,
-                                         3 * kd, st);
-    launch_kernel(tie_runs_kernel, blocks(n), 256, 0, st, dP, n, rc, wt,
-                  (const unsigned long long*)key.get(), val.get(), tot.get());
-    launch_kernel(cpl_kernel, blocks(n), 256, 0, st, dP, n, rc, wt, kd,
-                  (const unsigned long long*)key.get(), (const int32_t*)val.get(), cpl.get(),
-                  starts.get(), tot.get());
-    exclusive_scan_u32(starts.get(), base.get(), n, st);
-    launch_kernel(path_totals_kernel, 1, 1, 0, st, (const uint32_t*)base.get(),
-                  (const uint32_t*)(starts.get() + (n - 1)), n, tot.get());
-    GWN_CUDA(cudaMemcpyAsync(h, tot.get(), sizeof(PathTotals), cudaMemcpyDeviceToHost, st));
-    GWN_CUDA(cudaStreamSynchronize(st));
-    if (!h->deep) break;
-    if (kd == kKeyDepth) return false;
-    kd = kKeyDepth;
+  tot.zero(st);
+  PathKeys<W> keys;
+  keys.kd = kd;
+  for (int i = 0; i < W; ++i) {  // by point
+    if (W > 1) word[i].alloc(N, st);
+    keys.w[i] = W > 1 ? word[i].get() : sorted.get();
   }
-  const uint32_t ni = h->ninternal;
+  launch_kernel(path_keys_kernel<W>, blocks(n), 256, 0, st, dP, n, rc, wt, keys, val.get());
+  for (int i = W - 1; i >= 0; --i) {  // stable: the last word first
+    if (W > 1)
+      launch_kernel(gather_keys_kernel, blocks(n), 256, 0, st, (const Key*)word[i].get(),
+                    (const int32_t*)val.get(), n, sorted.get());
+    radix_sort_pairs<Key>(sorted.get(), val.get(), tmp.get(), val_tmp.get(), n, 0, 3 * kd, st);
+  }
+  keys.w[0] = sorted.get();
+  for (int i = 1; i < W; ++i) {  // the other words in the sorted order
+    Key* out = i == 1 ? tmp.get() : word[i - 2].get();
+    launch_kernel(gather_keys_kernel, blocks(n), 256, 0, st, (const Key*)word[i].get(),
+                  (const int32_t*)val.get(), n, out);
+    keys.w[i] = out;
+  }
+  launch_kernel(tie_runs_kernel<W>, blocks(n), 256, 0, st, dP, n, rc, wt, keys, val.get(),
+                tot.get());
+  launch_kernel(cpl_kernel<W>, blocks(n), 256, 0, st, dP, n, rc, wt, keys,
+                (const int32_t*)val.get(), cpl.get(), starts.get(), tot.get());
+  exclusive_scan_u32(starts.get(), base.get(), n, st);
+  launch_kernel(path_totals_kernel, 1, 1, 0, st, (const uint32_t*)base.get(),
+                (const uint32_t*)(starts.get() + (n - 1)), n, tot.get());
+  GWN_CUDA(cudaMemcpyAsync(h, tot.get(), sizeof(PathTotals), cudaMemcpyDeviceToHost, st));
+  GWN_CUDA(cudaStreamSynchronize(st));
+  const PathTotals r = *h;
+  if (r.deep || r.long_run) return r;
+  const uint32_t ni = r.ninternal;
   t.ncells = 1 + 8 * (int64_t)ni;
   GWN_REQUIRE(t.ncells < (int64_t(1) << 31), "octree has more than 2^31 cells");
-  t.nindices = (int64_t)h->nindices;
-  t.max_depth = (int32_t)h->max_cpl + 1;
+  t.nindices = (int64_t)r.nindices;
+  t.max_depth = (int32_t)r.max_cpl + 1;
   t.cn.alloc((size_t)t.ncells * 3);
   t.w.alloc((size_t)t.ncells);
   t.ch.alloc((size_t)t.ncells * 8);
@@ -839,14 +914,32 @@ static bool octree_build_paths(gwn_octree_impl& t, const double* dP, int64_t n, 
   DevBuf<int8_t> cell_depth(ni, st);
   launch_kernel(list_cells_kernel, blocks(n), 256, 0, st, (const int8_t*)cpl.get(),
                 (const uint32_t*)base.get(), n, ni, cell_first.get(), cell_depth.get());
-  launch_kernel(cells_kernel, blocks((int64_t)ni * 8), 256, 0, st, dP, n, rc, wt, kd,
-                (const unsigned long long*)key.get(), (const int32_t*)val.get(),
-                (const int8_t*)cpl.get(), (const uint32_t*)base.get(), ni,
-                (const int32_t*)cell_first.get(), (const int8_t*)cell_depth.get(), t.cn.get(),
+  launch_kernel(cells_kernel<W>, blocks((int64_t)ni * 8), 256, 0, st, dP, n, rc, wt, keys,
+                (const int32_t*)val.get(), (const int8_t*)cpl.get(), (const uint32_t*)base.get(),
+                ni, (const int32_t*)cell_first.get(), (const int8_t*)cell_depth.get(), t.cn.get(),
                 t.w.get(), t.ch.get(), t.start.get(), t.count.get(), t.depth.get());
   GWN_CUDA(cudaMemcpyAsync(t.perm.get(), val.get(), N * 4, cudaMemcpyDeviceToDevice, st));
   GWN_CUDA(cudaStreamSynchronize(st));
-  return true;
+  return r;
+}
+
+// The build from sorted paths; false when the level loop has to do it.
+static bool octree_build_paths(gwn_octree_impl& t, const double* dP, int64_t n, const double* rc,
+                               const double* rw, cudaStream_t st) {
+  DevBuf<Widths> widths(1, st);
+  launch_kernel(widths_kernel, 1, 1, 0, st, rw, widths.get());
+  // Octants per key: points spread over a surface share about log2(n) / 2, so
+  // 10 (four passes) and 16 (six) leave few equal keys to 4096 and 16M points.
+  int kd = n <= 4096 ? 10 : (n <= (int64_t(16) << 20) ? 16 : kKeyDepth);
+  for (;;) {
+    const PathTotals r = octree_try_paths<1>(t, dP, n, rc, widths.get(), kd, st);
+    if (r.deep) return false;
+    if (!r.long_run) return true;
+    if (kd == kKeyDepth || r.longer) break;
+    kd = kKeyDepth;
+  }
+  const PathTotals r = octree_try_paths<kKeyWords>(t, dP, n, rc, widths.get(), kKeyDepth, st);
+  return !r.deep && !r.long_run;
 }
 
 void octree_build(gwn_octree_impl& t, const double* P, int64_t n, bool host_mode, cudaStream_t st) {

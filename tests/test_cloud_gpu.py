@@ -3,6 +3,8 @@ expansion precompute and Barnes-Hut evaluation against the FP64 oracle
 (restated include/igl/octree.cpp and fast_winding_number.cpp), through the
 C ABI; the reference's own golden vector
 (tests/include/igl/fast_winding_number.cpp:17-53, 1e-15)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -182,3 +184,41 @@ def test_octree_close_points(cuda, m, gap):
     P = np.concatenate([rng.random((200, 3)), cluster, rng.random((50, 3)) - 0.5])
     assert_octree_equal(P[rng.permutation(P.shape[0])])
     assert_octree_equal(cluster)
+
+
+@pytest.mark.parametrize("reach", [2.0 ** 8, 2.0 ** 14, 2.0 ** 25, 2.0 ** 45, 2.0 ** 70])
+@pytest.mark.parametrize("m", [33, 4096, 4097, 6000])
+def test_octree_far_points(cuda, m, reach):
+    """m points near the origin and one `reach` away, alone and with points at
+    every scale between: runs of equal keys longer than one thread orders, in
+    one-word keys of both lengths, in keys of three words (2^25, 2^45), and
+    beyond those (2^70, the level loop)."""
+    rng = np.random.default_rng([m, int(np.log2(reach))])
+    P = rng.normal(size=(m, 3))
+    P /= np.linalg.norm(P, axis=1, keepdims=True)
+    far = np.array([[reach, -0.3 * reach, 0.1 * reach]])
+    assert_octree_equal(np.concatenate([P, far]))
+    between = rng.normal(size=(500, 3)) * reach ** rng.uniform(0, 1, (500, 1))
+    P = np.concatenate([P, P[:40] * 2.0 ** -30, between, far])
+    assert_octree_equal(P[rng.permutation(P.shape[0])])
+
+
+def test_far_points_do_not_fall_back_to_a_level_at_a_time(cuda):
+    """2M points with one 1e7 away, and half a million at all scales: three-word
+    keys, at most six times the build of as many points in one place (eleven
+    times and more when two attempts were thrown away for the level loop)."""
+    P = synth.torus_cloud(3, 2_000_000)[0]
+    rng = np.random.default_rng(4)
+    scales = rng.normal(size=(500_000, 3)) * 10.0 ** rng.uniform(-6, 3, (500_000, 1))
+    t = []
+    for X in (P, np.concatenate([P, [[1e7, 3e6, 0]]]), P[:500_000], scales):
+        x = cuda.from_numpy(np.ascontiguousarray(X)).cuda()
+        best = float("inf")
+        for k in range(7):
+            cuda.cuda.synchronize()
+            t0 = time.perf_counter()
+            G.Octree(x).close()
+            if k >= 2:
+                best = min(best, time.perf_counter() - t0)
+        t.append(best)
+    assert t[1] <= 6 * t[0] and t[3] <= 12 * t[2], t
