@@ -661,12 +661,36 @@ template <typename QT, typename WT>
 __global__ void __launch_bounds__(128) soup_team_fp64_kernel(EvalParams prm, int T,
                                                              const QT* __restrict__ Q,
                                                              const int32_t* __restrict__ perm,
-                                                             const int32_t* __restrict__ list,
-                                                             const unsigned* __restrict__ list_count,
                                                              int64_t nQ, WT* __restrict__ W) {
   __shared__ soupwalk::Fp64Queue fp64_q[4];
   __shared__ int2 s_stack[4][kTeamStack];
-  const int64_t n = list ? (int64_t)*list_count : nQ;
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / T;
+  const bool valid = i < nQ;
+  int64_t qi = 0;
+  double qx = 0, qy = 0, qz = 0;
+  if (valid) soupwalk::read_query(Q, perm, (const int32_t*)nullptr, i, qi, qx, qy, qz);
+  const double acc = soupwalk::walk_fp64_team(prm, T, valid, qx, qy, qz, fp64_q[threadIdx.x >> 5],
+                                              s_stack[threadIdx.x >> 5]);
+  if (valid && !(threadIdx.x & (T - 1))) W[qi] = (WT)(acc * kInv4Pi);
+}
+
+// FP64 re-evaluation of the listed queries (results within the band of 0.5).
+// They lie along the sheets where the sum is one half: a few next to a closed
+// surface, a large part of the batch near the plane of a half sphere's rim.  Lanes
+// per query by their number; us a call of 32 / 8 / 1 lanes, half spheres of
+// 41,000 and 655,000 triangles: 4,400 listed 165 / 168 / 335, 16,200 343 / 256 /
+// 401, 44,000 871 / 593 / 590, 81,000 1273 / 911 / 853, 220,000 3214 / 1992 / 1585.
+constexpr int64_t kRefine32 = 4096, kRefine8 = 50000;
+template <typename QT, typename WT>
+__global__ void __launch_bounds__(128) soup_refine_kernel(EvalParams prm, const QT* __restrict__ Q,
+                                                          const int32_t* __restrict__ list,
+                                                          const unsigned* __restrict__ count,
+                                                          WT* __restrict__ W) {
+  __shared__ soupwalk::Fp64Queue fp64_q[4];
+  __shared__ int2 s_stack[4][kTeamStack];
+  soupwalk::Fp64Queue& fq = fp64_q[threadIdx.x >> 5];
+  const int64_t n = *count;
+  const int T = n <= kRefine32 ? 32 : n <= kRefine8 ? 8 : 1;
   const int64_t per_warp = 32 / T;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t w0 = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -675,10 +699,10 @@ __global__ void __launch_bounds__(128) soup_team_fp64_kernel(EvalParams prm, int
     const bool valid = i < n;
     int64_t qi = 0;
     double qx = 0, qy = 0, qz = 0;
-    if (valid) soupwalk::read_query(Q, perm, list, i, qi, qx, qy, qz);
-    const double acc = soupwalk::walk_fp64_team(prm, T, valid, qx, qy, qz,
-                                                fp64_q[threadIdx.x >> 5],
-                                                s_stack[threadIdx.x >> 5]);
+    if (valid) soupwalk::read_query(Q, (const int32_t*)nullptr, list, i, qi, qx, qy, qz);
+    const double acc =
+        T == 1 ? soupwalk::walk_fp64(prm, valid, qx, qy, qz, fq)
+               : soupwalk::walk_fp64_team(prm, T, valid, qx, qy, qz, fq, s_stack[threadIdx.x >> 5]);
     if (valid && !(threadIdx.x & (T - 1))) W[qi] = (WT)(acc * kInv4Pi);
     __syncwarp();
   }
@@ -929,12 +953,13 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
       }
     }
     {
-      // a few queries near the threshold, anywhere: a warp each
       PhaseTimer ph("refine", st);
-      const unsigned rgrid = (unsigned)std::min<int64_t>((nQ + 3) / 4, 8 * num_sms());
-      launch_kernel(soup_team_fp64_kernel<QT, WT>, rgrid, 128, 0, st, prm, 32, Q,
-                    (const int32_t*)nullptr, (const int32_t*)list.get(),
-                    (const unsigned*)count.get(), nQ, W);
+      // enough warps for a whole batch of listed queries, 32 to a warp, and for
+      // a few with a warp each; what is beyond the grid is strided
+      const int64_t fill = 8 * (int64_t)num_sms();
+      const int64_t rgrid = std::max(std::min((nQ + 3) / 4, fill), std::min<int64_t>(grid, 8 * fill));
+      launch_kernel(soup_refine_kernel<QT, WT>, (unsigned)rgrid, 128, 0, st, prm, Q,
+                    (const int32_t*)list.get(), (const unsigned*)count.get(), W);
     }
   } else {
     PhaseTimer ph("walk", st);
@@ -942,8 +967,7 @@ static void soup_eval_t(const gwn_soup_impl& s, float beta, const void* Qv, int6
       launch_kernel(soup_eval_fp64_kernel<QT, WT>, grid, 128, 0, st, prm, Q, perm, nQ, W);
     } else {
       launch_kernel(soup_team_fp64_kernel<QT, WT>, team_grid(team), 128, 0, st, prm, team, Q, perm,
-                    (const int32_t*)nullptr,
-                    (const unsigned*)nullptr, nQ, W);
+                    nQ, W);
     }
   }
 }

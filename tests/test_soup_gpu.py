@@ -16,6 +16,7 @@ Checks, through the C ABI:
     test allows (tests/include/igl/fast_winding_number.cpp:76).
 """
 import os
+import time
 from decimal import Decimal, getcontext
 
 import numpy as np
@@ -349,3 +350,60 @@ def test_distant_opened_triangles_keep_their_digits(cuda, tree):
             err = abs(float(Decimal(float(w)) * Decimal(4 * np.pi) - _solid_angle_50_digits(T, q)))
             # 2 u |value|: the factor 1 / 4 pi and its product here
             assert err <= 2.0 ** -53 * (4 / f + 3 * abs(4 * np.pi * w)), f
+
+
+def _best_us(cuda, f, reps=7):
+    """Shortest of a few passes, waited for."""
+    best = float("inf")
+    for k in range(reps + 2):
+        cuda.cuda.synchronize()
+        t = time.perf_counter()
+        f()
+        cuda.cuda.synchronize()
+        if k >= 2:
+            best = min(best, time.perf_counter() - t)
+    return best * 1e6
+
+
+@pytest.mark.parametrize("m", [1, 33, 4096, 4097, 50_000, 50_001, 200_000])
+def test_results_near_one_half_are_the_fp64_walks(cuda, m):
+    """m queries with W within 5e-4 of one half (below the rim of a half sphere)
+    among as many others: all m are evaluated again by the plain FP64 walk, with
+    32, 8 or one lane each by their number, and the sums differ from that
+    walk's own in their order only (1e-12)."""
+    V, F = synth.geodesic_sphere(32)
+    F = np.ascontiguousarray(F[V[F][:, :, 2].mean(1) > 0])
+    bvh = G.FastWindingNumberBVH(V, F, 2)
+    rng = np.random.default_rng(m)
+    a, r = rng.uniform(0, 2 * np.pi, 400_000), 0.9 * np.sqrt(rng.uniform(0, 1, 400_000))
+    Q = np.stack([r * np.cos(a), r * np.sin(a), -2e-3 * rng.uniform(-1, 1, r.size)], 1)
+    W = bvh.eval(Q, 2.0, "fp64", out_dtype=np.float64)
+    Q = Q[np.abs(W - 0.5) <= 5e-4]
+    assert Q.shape[0] > 1000
+    Q = np.tile(Q, (m // Q.shape[0] + 1, 1))[:m]
+    others = rng.uniform(-3, 3, (m, 3)) + [0, 0, 7]
+    B = np.concatenate([Q, others])[rng.permutation(2 * m)]
+    W = bvh.eval(B, 2.0, "mixed", out_dtype=np.float64)
+    W64 = bvh.eval(B, 2.0, "fp64", out_dtype=np.float64)
+    band = np.abs(W64 - 0.5) <= 9e-4
+    assert band.sum() == m
+    assert np.abs(W - W64)[band].max() <= 1e-12
+    bvh.close()
+
+
+def test_a_batch_near_one_half_costs_its_fp64_walk(cuda):
+    """A million queries below the rim of a half sphere of 655,000 triangles, most
+    of them near one half: the mixed call takes about the FP64 walk's time (at
+    most 1.5 times; with 32 lanes for each, more than twice)."""
+    V, F = synth.geodesic_sphere(256)
+    F = np.ascontiguousarray(F[V[F][:, :, 2].mean(1) > 0])
+    bvh = G.FastWindingNumberBVH(V, F, 2)
+    rng = np.random.default_rng(2)
+    n = 1_000_000
+    a, r = rng.uniform(0, 2 * np.pi, n), 0.9 * np.sqrt(rng.uniform(0, 1, n))
+    Q = cuda.from_numpy(np.stack([r * np.cos(a), r * np.sin(a), -1e-4 * rng.random(n)], 1)).cuda()
+    W = bvh.eval(Q, 2.0, "fp64", out_dtype=np.float64)
+    assert float(((W - 0.5).abs() <= 1e-3).double().mean()) > 0.7
+    t = [_best_us(cuda, lambda: bvh.eval(Q, 2.0, p)) for p in ("mixed", "fp64")]
+    bvh.close()
+    assert t[0] <= 1.5 * t[1], t
