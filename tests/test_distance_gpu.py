@@ -12,6 +12,8 @@ from the exact winding number agree to 1e-9; the fast-winding-number sign is
 the reference's soup algorithm on its own tree, so S may differ by
 2 |dW| |S| with |dW| <= 2e-2 (the reference's own test tolerance against the
 exact winding number is 1e-2)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -249,3 +251,55 @@ def test_patches_and_soups_at_any_scale(cuda, nf, kind):
     # the tree of the signed distance, which holds nothing but the search
     S, I2, C2 = G.signed_distance(P, V, F, G.SIGNED_DISTANCE_TYPE_UNSIGNED)
     assert np.array_equal(S, np.sqrt(D)) and np.array_equal(I2, I) and np.array_equal(C2, C)
+
+
+@pytest.mark.parametrize("far", [0.0, 1e3, 1e6, 1e12])
+def test_search_beside_a_far_triangle(cuda, far):
+    """The search's pruning does not widen with the extent of the surface: one
+    triangle far away, queries next to the rest (distances down to 1e-7, the
+    closest triangle as in the exact search) and next to the far one."""
+    V, F = synth.icosphere(4)
+    rng = np.random.default_rng(77)
+    P = np.concatenate([V[rng.integers(0, len(V), 3000)] + 10.0 ** rng.uniform(-7, -1, (3000, 1))
+                        * rng.normal(size=(3000, 3)), rng.uniform(-1.2, 1.2, (500, 3)),
+                        rng.normal(size=(100, 3)) * 1e-9])
+    if far:
+        T = far * np.array([[1, 0, 0], [1, 1e-4, 0], [1, 0, 1e-4]])
+        F = np.concatenate([F, len(V) + np.arange(3, dtype=np.int32)[None]])
+        V = np.concatenate([V, T])
+        P = np.concatenate([P, T.mean(0) + far * 1e-4 * rng.normal(size=(200, 3))])
+    bvh = G.FastWindingNumberBVH(V, F, tree="binned")
+    D, I, C = bvh.squared_distance(P)
+    bvh.close()
+    Dr, Ir, Cr = O.squared_distance(V, F, P)
+    assert _close2(D, Dr).all()
+    assert _close2(_tri_dist2(V, F, P, I), D).all()
+
+
+def test_search_beside_a_far_triangle_takes_no_longer_than_its_bounds_ask(cuda):
+    """300,000 queries near an 82,000-triangle sphere with one triangle 10,000
+    radii away.  The triangles' own FP32 bounds carry a rounding of 1e-6 of that
+    extent, so the search visits more of the sphere than without it: about six
+    times the time; with node bounds that carried it too, fifteen times."""
+    V, F = synth.geodesic_sphere(64)
+    V = synth.sh_deform(V, np.random.default_rng(3))
+    rng = np.random.default_rng(1)
+    Q = cuda.from_numpy(V[rng.integers(0, len(V), 300_000)]
+                        + 1e-3 * rng.normal(size=(300_000, 3))).cuda()
+    t = []
+    for far in (False, True):
+        if far:
+            F = np.concatenate([F, len(V) + np.arange(3)[None]]).astype(np.int32)
+            V = np.concatenate([V, [[1e4, 0, 0], [1e4, 1, 0], [1e4, 0, 1]]])
+        bvh = G.FastWindingNumberBVH(V, F)
+        best = float("inf")
+        for k in range(8):
+            cuda.cuda.synchronize()
+            t0 = time.perf_counter()
+            bvh.squared_distance(Q)
+            cuda.cuda.synchronize()
+            if k >= 2:
+                best = min(best, time.perf_counter() - t0)
+        t.append(best)
+        bvh.close()
+    assert t[1] <= 10 * t[0], t
