@@ -82,6 +82,14 @@ int gwn_version(void);
 #define GWN_STATUS_BAD_INPUT 2u
 int gwn_device_status(unsigned int* flags, int clear);
 
+/* The library keeps device memory that its calls and handles have used for the
+ * next ones: workspaces as much as the largest calls needed, handles up to 1/16
+ * of the device's memory.  The driver takes it for any allocation of the same
+ * process that finds no other; gwn_release_memory gives what is unused on the
+ * current device back for another process.  Waits for the device; not during a
+ * stream capture. */
+int gwn_release_memory(void);
+
 /* Failure-path testing (no counterpart in the reference, which has asserts
  * only).  The next n launches of a kernel that streams triangles through a
  * bounded bulk-copy ring (the exact path's all-pairs sweeps, in

@@ -140,6 +140,12 @@ def device_status(clear: bool = True) -> int:
     return flags.value
 
 
+def release_memory() -> None:
+    """Give the current device back what the library's memory pools keep unused
+    (see gwn_release_memory)."""
+    N.check(N.load().gwn_release_memory())
+
+
 # --------------------------------------------------------------- exact GWN --
 def winding_number(V, F, O, precision="mixed", out_dtype=None):
     """igl::winding_number(V,F,O,W) (include/igl/winding_number.h:35-44).

@@ -35,6 +35,7 @@ SIGNATURES = {
     "gwn_last_error": ([], C.c_char_p),
     "gwn_version": ([], _i),
     "gwn_device_status": ([_p, _i], _i),
+    "gwn_release_memory": ([], _i),
     "gwn_debug_fail_next_waits": ([_i], _i),
     "gwn_winding_number": ([_p, _i64, _i, _p, _i64, _p, _i, _i64, _p, _i, _i, _i, _p], _i),
     "gwn_winding_number_noalloc": ([_p, _i64, _p, _i64, _p, _i64, _p, _p, _p], _i),

@@ -116,6 +116,7 @@ namespace {
 struct HandlePool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
+  uint64_t keep = 0;  // bytes that stay mapped
 };
 std::vector<HandlePool> g_handle_pools;  // per device
 
@@ -131,10 +132,10 @@ HandlePool handle_pool(int d) {
     props.location.id = d;
     size_t free_b = 0, total = 0;
     GWN_CUDA(cudaMemGetInfo(&free_b, &total));
-    uint64_t keep = total / 16;
+    h.keep = total / 16;
     cudaMemPool_t pool = nullptr;
     GWN_CUDA(cudaMemPoolCreate(&pool, &props));
-    GWN_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    GWN_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &h.keep));
     if (!h.stream) GWN_CUDA(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     h.pool = pool;
   }
@@ -172,16 +173,36 @@ void handle_free(void* p, int device) noexcept {
   // the device cannot be waited for (a capture in progress) it stays allocated,
   // as with cudaFree
   if (cudaDeviceSynchronize() == cudaSuccess) {
-    cudaStream_t st = nullptr;
+    HandlePool h;
     {
       std::lock_guard<std::mutex> lk(g_dev_mutex);
-      if ((int)g_handle_pools.size() > device) st = g_handle_pools[device].stream;
+      if ((int)g_handle_pools.size() > device) h = g_handle_pools[device];
     }
-    cudaFreeAsync(p, st);
+    cudaFreeAsync(p, h.stream);
+    // a pool gives back what is beyond its threshold when a stream is waited for
+    uint64_t reserved = 0;
+    if (h.pool &&
+        cudaMemPoolGetAttribute(h.pool, cudaMemPoolAttrReservedMemCurrent, &reserved) ==
+            cudaSuccess &&
+        reserved > h.keep)
+      cudaStreamSynchronize(h.stream);
   } else {
     cudaGetLastError();
   }
   if (cur != device) cudaSetDevice(cur);
+}
+
+void release_pools() {
+  const int d = current_device();
+  cudaMemPool_t ordered = nullptr, handles = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_dev_mutex);
+    if ((int)g_pools.size() > d) ordered = g_pools[d];
+    if ((int)g_handle_pools.size() > d) handles = g_handle_pools[d].pool;
+  }
+  GWN_CUDA(cudaDeviceSynchronize());
+  if (ordered) GWN_CUDA(cudaMemPoolTrimTo(ordered, 0));
+  if (handles) GWN_CUDA(cudaMemPoolTrimTo(handles, 0));
 }
 
 int num_sms() {
@@ -323,6 +344,10 @@ int gwn_device_status(unsigned int* flags, int clear) {
     v |= noalloc_sticky_status(clear != 0);
     if (flags) *flags = v;
   });
+}
+
+int gwn_release_memory(void) {
+  return guarded("gwn_release_memory", [&] { release_pools(); });
 }
 
 int gwn_debug_fail_next_waits(int n) {

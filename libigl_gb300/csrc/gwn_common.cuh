@@ -123,10 +123,16 @@ class DevBuf {
 // map and unmap it each time: 18 buffers of a 2M-point cloud 4.7 ms a call, 6
 // of an 81k-triangle soup 0.7 ms).  The memory is usable on every stream when
 // handle_alloc returns; handle_free waits for the device first, as cudaFree
-// does, so nothing that still runs can use it.  Both work from any thread and
-// with any device current.
+// does, so nothing that still runs can use it, and gives back at once what is
+// beyond that share.  Both work from any thread and with any device current.
+// (An allocation of this process that finds no memory, from whichever pool or
+// cudaMalloc, takes what the pools keep unused: the driver gives it back then.)
 void* handle_alloc(size_t bytes, int* device);
 void handle_free(void* p, int device) noexcept;
+
+// Gives back to the current device what both pools keep unused.  Waits for the
+// device.
+void release_pools();
 
 // Persistent device allocation owned by a handle, so its lifetime does not
 // depend on any caller stream.  A structure that lives for one call only can
