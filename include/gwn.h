@@ -208,6 +208,8 @@ void gwn_soup_free(gwn_soup* soup);
  *   where link (an int64 stored in the last slot's bytes) is >= 0 for an
  *   internal node (index one past its subtree) and ~slot for a leaf;
  * tri_index: num_triangles input-triangle ids, one per leaf slot.
+ * The records are held as the far field's forms: the order-1 and order-2
+ * moments come back within 6 x 2^-53 of the largest of their order.
  * Either pointer may be NULL. */
 int gwn_soup_export(const gwn_soup* soup, double* nodes, int32_t* tri_index);
 

@@ -136,11 +136,16 @@ __device__ void tri_integrals(const T* A, const T* B, const T* C, const T* P, T 
     // operations less on the FP64 pipe that bounds the items: 920 -> 701 us for
     // 1.3M triangles)
     const T inv = T(1) / oac[i];
+    T rest = -ocb[i] * inv;
     t = oab[i] * inv;
+    if (isinf(inv)) {  // an extent below 5.6e-309
+      t = oab[i] / oac[i];
+      rest = -ocb[i] / oac[i];
+    }
     jd = t * oac[j] - oab[j];
     kd = t * oac[k] - oab[k];
     sa = 2 * area * t;
-    sc = 2 * area * (-ocb[i] * inv);
+    sc = 2 * area * rest;
   }
   const T Pai = A[i] - P[i], Pci = C[i] - P[i];
   const T two3 = T(2.0 / 3.0), one3 = T(1.0 / 3.0), half = T(0.5), qtr = T(0.25);

@@ -21,6 +21,7 @@ def test_release_memory(cuda):
     V, F = synth.icosphere(2)
     bvh = G.FastWindingNumberBVH(V, F)
     bvh.eval(V)
+    _make_and_close_a_cloud(cuda, 1000)  # the kernels are loaded
     G.release_memory()
     cuda.cuda.empty_cache()
     before, _ = cuda.cuda.mem_get_info()

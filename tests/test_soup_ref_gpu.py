@@ -213,3 +213,22 @@ def test_a_far_triangle_costs_the_build_a_few_partitions(cuda):
                 best = min(best, time.perf_counter() - t0)
         t.append(best)
     assert t[1] <= 5 * t[0], t
+
+
+@pytest.mark.parametrize("tiny", [0.0, 5e-324, 1e-310, 1e-300])
+def test_moments_of_triangles_with_a_vanishing_extent(cuda, tiny):
+    """An extent whose reciprocal overflows: the FP64 moments are those of the
+    triangle without it, as far as that moves them (less than 1e-15)."""
+    T = np.array([[[0, 0, 0], [1, tiny, 0], [0.25, 0, 1]], [[0, 0, 0], [tiny, 1, 0], [0, 0.25, 1]],
+                  [[1, 0, 0], [0, 1, tiny], [0, 0.25, 0]]])
+    for P in T:
+        flat = np.where(np.abs(P) < 1e-200, 0.0, P)
+        F = np.array([[0, 1, 2]], np.int32)
+        a, b = G.FastWindingNumberBVH(P, F), G.FastWindingNumberBVH(flat, F)
+        M, M0 = a.export()[0], b.export()[0]
+        a.close()
+        b.close()
+        M, M0 = (m.reshape(-1, 24)[:, :23] for m in (M, M0))
+        fin = np.isfinite(M0)
+        assert np.array_equal(np.isfinite(M), fin)
+        assert np.abs(M[fin] - M0[fin]).max() <= 1e-15
