@@ -24,7 +24,8 @@
 //   Nodes of more than 1024 boxes (kSub): one depth at a time, split by split
 //     across the depth; by size a split runs in one warp, in one CTA, or by
 //     chunks across the GPU, each with the reference's in-place partition
-//     reproduced exactly (below).
+//     reproduced exactly (below).  A large node without a balanced span waits
+//     until the others' splits are made (nthElement across the GPU).
 //   Smaller subtrees: one CTA each, whole, in shared memory, a warp per node.
 // Span counts and boxes are order-independent (counts, min, max), so every
 // decision equals the serial code's.
@@ -161,6 +162,8 @@ struct RNode {
   Box sub[4];
   float area[4];
   int32_t choice;
+  uint32_t done;      // splits made; 4: its children are made too
+  uint32_t waiting;   // its split needs nthElement across the GPU
   uint32_t child[4];  // item (triangle id), kInternal | node, kSubRef | subtree
   // the split of the current round
   uint32_t t_start, t_n, t_mid;
@@ -968,6 +971,28 @@ __device__ void cta_partition(CtaPart& S, uint32_t* idx, float* cen, uint32_t* t
   pe = ps + nE;
 }
 
+// nthElement (FWNFS.h:5847-5900) of positions [lo, hi) about position mid by one
+// CTA; false if it did not end, which cannot happen: each step narrows [lo, hi)
+// by at least the pivot's own box, the bound only guards against a hang.
+__device__ bool cta_nth(CtaPart& S, uint32_t* idx, float* cen, uint32_t* tmp, uint32_t* tape_e,
+                        uint32_t* tape_g, const Box* __restrict__ tb, int axis, uint32_t lo,
+                        uint32_t hi, uint32_t mid) {
+  bool done = false;
+  for (uint32_t step = 0, n = hi - lo; step <= n && !done; ++step) {
+    const float pv = median3(cen[lo], cen[lo + (hi - lo) / 2], cen[hi - 1]);
+    __syncthreads();
+    uint32_t ps, pe;
+    cta_partition(S, idx, cen, tmp, tape_e, tape_g, lo, hi, pv, ps, pe);
+    for (uint32_t p = lo + threadIdx.x; p < hi; p += blockDim.x) cen[p] = centre2(tb[idx[p]], axis);
+    if (mid < ps) hi = ps;
+    else if (mid < pe) done = true;
+    else lo = pe;
+    if (hi <= lo + 1) done = true;
+    __syncthreads();
+  }
+  return done;
+}
+
 __global__ void __launch_bounds__(1024) part_cta_kernel(
     RNode* nodes, const uint32_t* list, const uint32_t* count, uint32_t* idx, float* cen,
     uint32_t* tmp, uint32_t* tape_e, uint32_t* tape_g, const Box* __restrict__ tb,
@@ -1054,22 +1079,9 @@ __global__ void __launch_bounds__(1024) part_cta_kernel(
     if (mid == s) ++mid;
     else if (mid == s + n) --mid;
   } else {
-    // nthElement, as in warp_split
     mid = s + s_target;
-    uint32_t lo = s, hi = s + n;
-    bool done = false;
-    for (uint32_t step = 0; step <= n && !done; ++step) {
-      const float pv = median3(cen[lo], cen[lo + (hi - lo) / 2], cen[hi - 1]);
-      __syncthreads();
-      cta_partition(s_part, idx, cen, tmp, tape_e, tape_g, lo, hi, pv, ps, pe);
-      for (uint32_t p = lo + tid; p < hi; p += blockDim.x) cen[p] = centre2(tb[idx[p]], axis);
-      if (mid < ps) hi = ps;
-      else if (mid < pe) done = true;
-      else lo = pe;
-      if (hi <= lo + 1) done = true;
-      __syncthreads();
-    }
-    if (!done && tid == 0) atomicOr(status, kStatusInternal);
+    if (!cta_nth(s_part, idx, cen, tmp, tape_e, tape_g, tb, axis, s, s + n, mid) && tid == 0)
+      atomicOr(status, kStatusInternal);
   }
   // the cut moved off the span's, or came from nthElement: the sides' boxes
   for (uint32_t p0 = s; p0 < s + n; p0 += blockDim.x) {
@@ -1105,7 +1117,8 @@ struct LTask {
   uint32_t keys[kSpans][6];
   Box Lb, Rb;
   uint32_t lcs;
-  int32_t live;                        // a span split (else left to the CTA kernel)
+  int32_t live;                        // takes part in the partition
+  int32_t more;                        // nthElement has not ended
   uint32_t chunk0;                     // its first chunk
   uint32_t firstE, firstG, nL, nE;     // of the partition, relative to start
   uint32_t L_atE, LE_atG;              // prefix counts at firstE / firstG
@@ -1215,22 +1228,31 @@ __global__ void __launch_bounds__(256) wide_span_kernel(const int4* __restrict__
   }
 }
 
-// One warp per task: the span and pivot; without one, the CTA kernel's list.
+// One warp per task: the span and pivot.  Without a longest axis the CTA kernel
+// cuts it anywhere; without a balanced span the node waits for nthElement.
 __global__ void wide_choose_kernel(LTask* __restrict__ T, const uint32_t* __restrict__ count,
                                    uint32_t* __restrict__ cta_list,
-                                   uint32_t* __restrict__ cta_count) {
+                                   uint32_t* __restrict__ cta_count, RNode* __restrict__ nodes,
+                                   uint32_t* __restrict__ waiting, uint32_t* __restrict__ nwaiting) {
   if (blockIdx.x >= *count) return;
   LTask& t = T[blockIdx.x];
   const int lane = threadIdx.x;
   int si = -1;
-  uint32_t lcs = 0, lc0, lc14;
+  uint32_t lcs = 0, lc0 = 0, lc14 = 0;
   Box Lb, Rb;
   if (t.live) si = choose_span(t.cnt, t.keys, t.n, Lb, Rb, lcs, lc0, lc14);
   __syncwarp();
   if (lane != 0) return;
   if (si < 0) {
+    if (t.live) {
+      RNode& N = nodes[t.node];
+      N.waiting = 1;
+      N.t_mid = t.start + nth_target(t.n, lc0, lc14);
+      waiting[atomicAdd(nwaiting, 1u)] = t.node;
+    } else {
+      cta_list[atomicAdd(cta_count, 1u)] = t.node;
+    }
     t.live = 0;
-    cta_list[atomicAdd(cta_count, 1u)] = t.node;
     return;
   }
   t.Lb = Lb;
@@ -1526,6 +1548,131 @@ __global__ void wide_finish_kernel(RNode* __restrict__ nodes, const LTask* __res
   }
 }
 
+// ---------------------------------------- nthElement across the GPU --
+// A large node without a balanced span waits for these: its partitions about
+// medians of three run through the passes above until the range that holds the
+// cut is small enough for a CTA (kCtaMax), all waiting nodes together.  The usual
+// depth has none, and the host learns of them with the depth's counts.  Builds of
+// 1.3M and 12M triangles with one far away 20.3 and 233 ms in one CTA from the
+// start, 8.5 and 46.9 ms so (5.4 and 36.4 without the far one); 12M at sizes and
+// places over five decades 677 and 116 ms.
+__global__ void nth_begin_kernel(const RNode* __restrict__ nodes,
+                                 const uint32_t* __restrict__ waiting, uint32_t n,
+                                 LTask* __restrict__ T) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  LTask& t = T[k];
+  const RNode& N = nodes[waiting[k]];
+  t.node = waiting[k];
+  t.start = N.t_start;
+  t.n = N.t_n;
+  t.mid = N.t_mid;
+  t.axis = longest_axis(N.t_box, t.len);
+  t.more = 1;
+}
+
+// Chunks of the next partitions and their pivots, or of the whole parts (whole:
+// for the sides' boxes); one CTA.
+__global__ void nth_chunks_kernel(const RNode* __restrict__ nodes, uint32_t n, bool whole,
+                                  const float* __restrict__ cen, LTask* __restrict__ T,
+                                  int4* __restrict__ chunks, uint32_t* __restrict__ nchunks) {
+  __shared__ uint32_t s_total;
+  if (threadIdx.x == 0) s_total = 0;
+  for (uint32_t k0 = 0; k0 < n; k0 += 32) {  // warp 0: tasks and chunk offsets
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const uint32_t k = k0 + threadIdx.x;
+      uint32_t c = 0;
+      if (k < n) {
+        LTask& t = T[k];
+        if (whole) {
+          t.start = nodes[t.node].t_start;
+          t.n = nodes[t.node].t_n;
+          t.live = t.need = 1;
+          keys_init(t.bk[0]);
+          keys_init(t.bk[1]);
+        } else {
+          t.live = t.more && t.n > kCtaMax;
+          t.firstE = t.firstG = kNone;
+          t.nL = t.nE = t.L_atE = t.LE_atG = 0;
+          if (t.live)
+            t.pivot = median3(cen[t.start], cen[t.start + t.n / 2], cen[t.start + t.n - 1]);
+        }
+        if (t.live) c = (t.n + kChunk - 1) / kChunk;
+      }
+      uint32_t incl = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if ((int)threadIdx.x >= o) incl += v;
+      }
+      if (k < n) T[k].chunk0 = s_total + incl - c;
+      __syncwarp();
+      if (threadIdx.x == 31) s_total += incl;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *nchunks = s_total;
+  for (uint32_t k = 0; k < n; ++k) {
+    if (!T[k].live) continue;
+    const uint32_t s = T[k].start, len = T[k].n, c0 = T[k].chunk0;
+    for (uint32_t c = threadIdx.x; c * kChunk < len; c += blockDim.x)
+      chunks[c0 + c] = make_int4((int)k, (int)(s + c * kChunk),
+                                 (int)(s + min(len, (c + 1) * kChunk)), 0);
+  }
+}
+
+// The centres in their new order.
+__global__ void __launch_bounds__(256) nth_centres_kernel(const int4* __restrict__ chunks,
+                                                          const uint32_t* __restrict__ nchunks,
+                                                          const LTask* __restrict__ T,
+                                                          const uint32_t* __restrict__ idx,
+                                                          const Box* __restrict__ tb,
+                                                          float* __restrict__ cen) {
+  if (blockIdx.x >= *nchunks) return;
+  const int4 ch = chunks[blockIdx.x];
+  const int axis = T[ch.x].axis;
+  for (int p = ch.y + threadIdx.x; p < ch.z; p += blockDim.x) cen[p] = centre2(tb[idx[p]], axis);
+}
+
+// The range that holds the cut, as in cta_nth.
+__global__ void nth_narrow_kernel(LTask* __restrict__ T, uint32_t n) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n || !T[k].live) return;
+  LTask& t = T[k];
+  uint32_t lo = t.start, hi = t.start + t.n;
+  const uint32_t ps = lo + t.nL, pe = ps + t.nE;
+  if (t.mid < ps) hi = ps;
+  else if (t.mid < pe) t.more = 0;
+  else lo = pe;
+  if (hi <= lo + 1) t.more = 0;
+  t.start = lo;
+  t.n = hi - lo;
+}
+
+// What is left of each, in a CTA.
+__global__ void __launch_bounds__(1024) nth_cta_kernel(const LTask* __restrict__ T, uint32_t* idx,
+                                                       float* cen, uint32_t* tmp, uint32_t* tape_e,
+                                                       uint32_t* tape_g,
+                                                       const Box* __restrict__ tb,
+                                                       unsigned* status) {
+  __shared__ CtaPart s_part;
+  const LTask& t = T[blockIdx.x];
+  if (!t.more) return;
+  if (!cta_nth(s_part, idx, cen, tmp, tape_e, tape_g, tb, t.axis, t.start, t.start + t.n, t.mid) &&
+      threadIdx.x == 0)
+    atomicOr(status, kStatusInternal);
+}
+
+__global__ void nth_end_kernel(RNode* __restrict__ nodes, const uint32_t* __restrict__ waiting,
+                               uint32_t n) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  RNode& N = nodes[waiting[k]];
+  insert_cut(N.cut, N.sub, N.area, N.done + 1, N.choice, N.t_mid, N.t_out[0], N.t_out[1]);
+  ++N.done;
+  N.waiting = 0;
+}
+
 // The root: a node, or the only subtree when it is small enough.
 __global__ void tree_init_kernel(RNode* nodes, SubRoot* subs, uint32_t m,
                                  const uint32_t* __restrict__ root_keys, BuildCounts* bc) {
@@ -1534,6 +1681,7 @@ __global__ void tree_init_kernel(RNode* nodes, SubRoot* subs, uint32_t m,
     nodes[0].start = 0;
     nodes[0].n = m;
     nodes[0].all = keys_box(root_keys);
+    nodes[0].done = nodes[0].waiting = 0;
     c.ntop = 1;
   } else {
     subs[0] = SubRoot{0, m, 0, keys_box(root_keys)};
@@ -1545,13 +1693,16 @@ __global__ void tree_init_kernel(RNode* nodes, SubRoot* subs, uint32_t m,
 // --------------------------------------------------- rounds and depths --
 // The split each node makes this round (multiSplit: round 0 splits the
 // whole range; rounds 1 and 2 the part with the largest area x count,
-// the first on ties), sorted into the three size classes.
+// the first on ties), sorted into the three size classes.  A node that waits for
+// nthElement sits out the rest of the rounds and goes on from there when they
+// run again.
 __global__ void prepare_round_kernel(RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
                                      int round, uint32_t* __restrict__ lists, uint32_t cap,
                                      uint32_t* __restrict__ counts) {
   const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= le) return;
   RNode& N = nodes[x];
+  if (N.done != (uint32_t)round || N.waiting) return;
   const int c = round == 0 ? 0 : choose_part(N.cut, N.area, round + 1);
   if (round == 0) {
     N.cut[0] = N.start;
@@ -1571,10 +1722,12 @@ __global__ void finish_round_kernel(RNode* __restrict__ nodes, uint32_t lb, uint
   const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= le) return;
   RNode& N = nodes[x];
+  if (N.done != (uint32_t)round || N.waiting) return;
   insert_cut(N.cut, N.sub, N.area, round + 1, N.choice, N.t_mid, N.t_out[0], N.t_out[1]);
+  N.done = round + 1;
 }
 
-// Children of a depth: single boxes are items; parts of at most kSub boxes
+// Children of a depth's nodes whose splits are made: single boxes are items; parts of at most kSub boxes
 // become subtrees, larger ones the nodes of the next depth (numbered from le).
 __global__ void make_children_kernel(RNode* __restrict__ nodes, uint32_t lb, uint32_t le,
                                      uint32_t depth, const uint32_t* __restrict__ idx,
@@ -1582,6 +1735,8 @@ __global__ void make_children_kernel(RNode* __restrict__ nodes, uint32_t lb, uin
   const uint32_t x = lb + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= le) return;
   RNode& N = nodes[x];
+  if (N.done != 3) return;
+  N.done = 4;
   for (int i = 0; i < 4; ++i) {
     const uint32_t s = N.cut[i], c = N.cut[i + 1] - s;
     if (c == 1) {
@@ -1598,6 +1753,7 @@ __global__ void make_children_kernel(RNode* __restrict__ nodes, uint32_t lb, uin
       C.start = s;
       C.n = c;
       C.all = N.sub[i];
+      C.done = C.waiting = 0;
     }
   }
 }
@@ -1819,7 +1975,7 @@ void soup_build_ref(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t
   std::vector<uint32_t> level = {0};  // depth d of the top holds nodes [level[d], level[d + 1])
   uint32_t nsub = 1;
   if (m > kSub) {
-    DevBuf<uint32_t> tmp(m, st), tapeE(m, st), tapeG(m, st), nchunks(1, st);
+    DevBuf<uint32_t> tmp(m, st), tapeE(m, st), tapeG(m, st), nchunks(1, st), waiting;
     DevBuf<float> cen(m, st);
     DevBuf<LTask> tasks;
     DevBuf<int4> chunks;
@@ -1828,7 +1984,60 @@ void soup_build_ref(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t
       tasks.alloc(wide_max, st);
       chunks.alloc(chunk_max, st);
       chunk_cnt.alloc(chunk_max, st);
+      waiting.alloc(wide_max, st);
     }
+    const int4* ch = chunks.get();
+    const uint32_t* nch = nchunks.get();
+    LTask* T = tasks.get();
+    // the passes of one partition of all live tasks (of nt; count on the device)
+    auto partition = [&](uint32_t nt, const uint32_t* count) {
+      launch_kernel(wide_classify_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                    (const float*)cen.get(), chunk_cnt.get());
+      launch_kernel(wide_scan_kernel, nt, 32, 0, st, T, count, chunk_cnt.get());
+      launch_kernel(wide_first_kernel, chunk_max, 256, 0, st, ch, nch, T, (const float*)cen.get(),
+                    (const uint2*)chunk_cnt.get());
+      launch_kernel(wide_tape_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                    (const uint32_t*)idx.get(), (const float*)cen.get(),
+                    (const uint2*)chunk_cnt.get(), tmp.get(), tapeE.get(), tapeG.get());
+      launch_kernel(wide_resolve_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                    tapeE.get(), tapeG.get());
+      launch_kernel(wide_scatter_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                    (const uint32_t*)tmp.get(), (const uint32_t*)tapeE.get(),
+                    (const uint32_t*)tapeG.get(), idx.get(), status.ptr());
+    };
+    // the waiting nodes' splits, the host reading every kNthBatch partitions
+    // whether any is still large; after kNthMax they are left to a CTA whatever
+    // their size
+    constexpr int kNthBatch = 4, kNthMax = 64;
+    auto run_waiting = [&](uint32_t n) {
+      const uint32_t* count = &bc.get()->nwaiting;
+      unsigned* left = pinned_words() + 24;
+      const unsigned grid = blocks_for(n, 64);
+      auto make_chunks = [&](bool whole) {
+        launch_kernel(nth_chunks_kernel, 1, 512, 0, st, (const RNode*)nodes.get(), n, whole,
+                      (const float*)cen.get(), T, chunks.get(), nchunks.get());
+      };
+      launch_kernel(nth_begin_kernel, grid, 64, 0, st, (const RNode*)nodes.get(),
+                    (const uint32_t*)waiting.get(), n, T);
+      for (int it = 1; it <= kNthMax; ++it) {
+        make_chunks(false);
+        partition(n, count);
+        launch_kernel(nth_centres_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
+                      (const uint32_t*)idx.get(), (const Box*)tb.get(), cen.get());
+        launch_kernel(nth_narrow_kernel, grid, 64, 0, st, T, n);
+        if (it % kNthBatch) continue;
+        GWN_CUDA(cudaMemcpyAsync(left, nchunks.get(), 4, cudaMemcpyDeviceToHost, st));
+        GWN_CUDA(cudaStreamSynchronize(st));
+        if (*left == 0) break;
+      }
+      launch_kernel(nth_cta_kernel, n, 1024, 0, st, (const LTask*)T, idx.get(), cen.get(),
+                    tmp.get(), tapeE.get(), tapeG.get(), (const Box*)tb.get(), status.ptr());
+      make_chunks(true);
+      launch_kernel(wide_boxes_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                    (const uint32_t*)idx.get(), (const Box*)tb.get());
+      launch_kernel(wide_finish_kernel, grid, 64, 0, st, nodes.get(), (const LTask*)T, count);
+      launch_kernel(nth_end_kernel, grid, 64, 0, st, nodes.get(), (const uint32_t*)waiting.get(), n);
+    };
     uint32_t lb = 0, le = 1, max_n = m;
     level.push_back(1);
     while (le > lb) {
@@ -1842,52 +2051,47 @@ void soup_build_ref(gwn_soup_impl& s, const double* V, int64_t nV, const int32_t
         node_cap = cap2;
       }
       GWN_CUDA(cudaMemsetAsync(bc.get(), 0, offsetof(BuildCounts, ntop), st));
-      for (int round = 0; round < 3; ++round) {
-        uint32_t* cnt = bc.get()->lists[round];
-        uint32_t *lw = lists.get(), *lc = lw + split_max, *lg = lc + split_max;
-        launch_kernel(prepare_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le, round,
-                      lists.get(), split_max, cnt);
-        if (max_n > kCtaMax) {
-          const uint32_t *c2 = cnt + 2, *nch = nchunks.get();
-          LTask* T = tasks.get();
-          const int4* ch = chunks.get();
-          const uint32_t nt = std::min(nl, wide_max);
-          launch_kernel(wide_init_kernel, 1, 512, 0, st, (const RNode*)nodes.get(),
-                        (const uint32_t*)lg, c2, T, chunks.get(), nchunks.get());
-          launch_kernel(wide_span_kernel, chunk_max, 256, 0, st, ch, nch, T,
-                        (const uint32_t*)idx.get(), (const Box*)tb.get(), cen.get());
-          launch_kernel(wide_choose_kernel, nt, 32, 0, st, T, c2, lc, cnt + 1);
-          launch_kernel(wide_classify_kernel, chunk_max, 256, 0, st, ch, nch, T,
-                        (const float*)cen.get(), chunk_cnt.get());
-          launch_kernel(wide_scan_kernel, nt, 32, 0, st, T, c2, chunk_cnt.get());
-          launch_kernel(wide_first_kernel, chunk_max, 256, 0, st, ch, nch, T,
-                        (const float*)cen.get(), (const uint2*)chunk_cnt.get());
-          launch_kernel(wide_tape_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
-                        (const uint32_t*)idx.get(), (const float*)cen.get(),
-                        (const uint2*)chunk_cnt.get(), tmp.get(), tapeE.get(), tapeG.get());
-          launch_kernel(wide_resolve_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
-                        tapeE.get(), tapeG.get());
-          launch_kernel(wide_scatter_kernel, chunk_max, 256, 0, st, ch, nch, (const LTask*)T,
-                        (const uint32_t*)tmp.get(), (const uint32_t*)tapeE.get(),
-                        (const uint32_t*)tapeG.get(), idx.get(), status.ptr());
-          launch_kernel(wide_cut_kernel, blocks_for(nt, 64), 64, 0, st, T, c2);
-          launch_kernel(wide_boxes_kernel, chunk_max, 256, 0, st, ch, nch, T,
-                        (const uint32_t*)idx.get(), (const Box*)tb.get());
-          launch_kernel(wide_finish_kernel, blocks_for(nt, 64), 64, 0, st, nodes.get(),
-                        (const LTask*)T, c2);
+      for (;;) {
+        for (int round = 0; round < 3; ++round) {
+          uint32_t* cnt = bc.get()->lists[round];
+          uint32_t *lw = lists.get(), *lc = lw + split_max, *lg = lc + split_max;
+          launch_kernel(prepare_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
+                        round, lists.get(), split_max, cnt);
+          if (max_n > kCtaMax) {
+            const uint32_t* c2 = cnt + 2;
+            const uint32_t nt = std::min(nl, wide_max);
+            launch_kernel(wide_init_kernel, 1, 512, 0, st, (const RNode*)nodes.get(),
+                          (const uint32_t*)lg, c2, T, chunks.get(), nchunks.get());
+            launch_kernel(wide_span_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                          (const uint32_t*)idx.get(), (const Box*)tb.get(), cen.get());
+            launch_kernel(wide_choose_kernel, nt, 32, 0, st, T, c2, lc, cnt + 1, nodes.get(),
+                          waiting.get(), &bc.get()->nwaiting);
+            partition(nt, c2);
+            launch_kernel(wide_cut_kernel, blocks_for(nt, 64), 64, 0, st, T, c2);
+            launch_kernel(wide_boxes_kernel, chunk_max, 256, 0, st, ch, nch, T,
+                          (const uint32_t*)idx.get(), (const Box*)tb.get());
+            launch_kernel(wide_finish_kernel, blocks_for(nt, 64), 64, 0, st, nodes.get(),
+                          (const LTask*)T, c2);
+          }
+          launch_kernel(part_cta_kernel, parts, 1024, 0, st, nodes.get(), (const uint32_t*)lc,
+                        (const uint32_t*)(cnt + 1), idx.get(), cen.get(), tmp.get(), tapeE.get(),
+                        tapeG.get(), (const Box*)tb.get(), status.ptr());
+          if (round > 0)  // a whole node has more than kSub boxes
+            launch_kernel(part_warp_kernel, nl, 32, 0, st, nodes.get(), (const uint32_t*)lw,
+                          (const uint32_t*)cnt, idx.get(), (const Box*)tb.get(), status.ptr());
+          launch_kernel(finish_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
+                        round);
         }
-        launch_kernel(part_cta_kernel, parts, 1024, 0, st, nodes.get(), (const uint32_t*)lc,
-                      (const uint32_t*)(cnt + 1), idx.get(), cen.get(), tmp.get(), tapeE.get(),
-                      tapeG.get(), (const Box*)tb.get(), status.ptr());
-        if (round > 0)  // a whole node has more than kSub boxes
-          launch_kernel(part_warp_kernel, nl, 32, 0, st, nodes.get(), (const uint32_t*)lw,
-                        (const uint32_t*)cnt, idx.get(), (const Box*)tb.get(), status.ptr());
-        launch_kernel(finish_round_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le, round);
+        launch_kernel(make_children_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
+                      (uint32_t)level.size() - 2, (const uint32_t*)idx.get(), subs.get(),
+                      bc.get());
+        read_counts();
+        if (host_mode) status.check(st, "soup_build");
+        if (hbc->nwaiting == 0) break;
+        // at most three times a depth: every waiting node makes a split here
+        run_waiting(hbc->nwaiting);
+        GWN_CUDA(cudaMemsetAsync(bc.get(), 0, offsetof(BuildCounts, max_n), st));
       }
-      launch_kernel(make_children_kernel, blocks_for(nl), 256, 0, st, nodes.get(), lb, le,
-                    (uint32_t)level.size() - 2, (const uint32_t*)idx.get(), subs.get(), bc.get());
-      read_counts();
-      if (host_mode) status.check(st, "soup_build");
       lb = le;
       le = hbc->ntop;
       nsub = hbc->nsub;

@@ -21,9 +21,11 @@ struct Box {
   float lo[3], hi[3];
 };
 
-// Counters of the build; the fields before ntop are zeroed for every depth.
+// Counters of the build; the fields before ntop are zeroed for every depth, those
+// before max_n each time a depth's rounds run.
 struct BuildCounts {
   uint32_t lists[3][3];  // per round: parts for a warp, a CTA, the whole GPU
+  uint32_t nwaiting;     // nodes that wait for nthElement
   uint32_t max_n;        // the largest node of the next depth
   uint32_t ntop, nsub, nodes, max_depth, unbounded;
 };

@@ -163,10 +163,13 @@ def test_host_buffers_equal_the_device_call(cuda):
     assert np.array_equal(Wh32, Wd32)
 
 
-@pytest.mark.parametrize("kind,n", [("far", 40_000), ("far", 330_000), ("scales", 50_000),
-                                    ("scales", 150_000), ("line", 120_000), ("same", 70_000)])
+@pytest.mark.parametrize("kind,n", [("far", 32_700), ("far", 32_800), ("far", 40_000),
+                                    ("far", 330_000), ("strays", 300_000), ("scales", 50_000),
+                                    ("scales", 150_000), ("scales", 700_000), ("line", 120_000),
+                                    ("same", 70_000)])
 def test_uneven_trees_equal_the_oracle_tree(cuda, kind, n):
-    """Large nodes without a balanced span: one triangle far away, triangles at
+    """Large nodes without a balanced span: one triangle far away, thirty at
+    doubling distances (a waiting node in several rounds of a depth), triangles at
     sizes and places over five decades, triangles gathered towards one end of a
     line, and equal ones.  Their cut comes from nthElement over tens of thousands
     of boxes, whose order of partition decides the whole tree below."""
@@ -174,6 +177,9 @@ def test_uneven_trees_equal_the_oracle_tree(cuda, kind, n):
     if kind == "far":
         C, s = rng.normal(size=(n, 3)), np.full((n, 1), 0.01)
         C[n // 2] = [1e4, 0, 0]
+    elif kind == "strays":
+        C, s = rng.normal(size=(n, 3)), np.full((n, 1), 0.01)
+        C[rng.permutation(n)[:30]] = 2.0 ** np.arange(3, 33)[:, None] * rng.normal(size=(30, 3))
     elif kind == "scales":
         C = rng.normal(size=(n, 3)) * 10.0 ** rng.uniform(-4, 1, (n, 1))
         s = 10.0 ** rng.uniform(-5, -1, (n, 1))
@@ -194,9 +200,9 @@ def test_uneven_trees_equal_the_oracle_tree(cuda, kind, n):
 
 def test_a_far_triangle_costs_the_build_a_few_partitions(cuda):
     """1.3M triangles and one 10,000 radii away: the root's cut comes from
-    nthElement, some twenty partitions in one CTA: about three times the build
-    of the sphere alone, and seven times with the queues' copies followed one by
-    one."""
+    nthElement, some twenty partitions: less than three times the build of the
+    sphere alone, and seven times in one CTA with the queues' copies followed one
+    by one."""
     V, F = synth.geodesic_sphere(256)
     t = []
     for far in (False, True):
