@@ -92,17 +92,18 @@ struct ClosestParams {
 // Stack entries a thread's search may take before a whole warp takes the
 // query over.  Most searches take about a hundred, but a query about equally
 // far from much of the surface (near a sphere's centre) takes tens of
-// thousands, and one thread then sets the kernel's time.  Kernel times of both
-// searches: signed distance, 327,680 triangles, 300,000 queries: 64 entries
-// 1.96 ms, 96 1.77, 192 1.44 + 0.1 or less; the swept volume's bounded searches
-// (64 poses, 20,480 triangles), thread search alone: 1.30, 1.33 and 1.33 ms.
-// (Both with boxes along the normals up to 4096 triangles.)
+// thousands, and one thread then sets the kernel's time.  us a search call (query
+// order included) with 64 / 128 / 192 / 256 / 384 / 768 entries, 300,000 queries in
+// the box: bumpy sphere of 327,680 triangles 2305 / 1836 / 1662 / 1712 / 1985 /
+// 2397; smooth one of 82,000 1705 / 1077 / 1095 / 1274 / 1588 / 2146; 300,000
+// triangles at all scales 1878 / 1618 / 1720 / 1813 / 2110 / 3019; as many
+// anywhere 1285 / 803 / 768 / 781 / 770 / 794; near the surface no difference.
 constexpr int kThreadVisits = 192;
 // Lanes of a warp that have come to a triangle before it turns to those: the
 // triangle's bounds cost the warp the same however few lanes need them, and more
-// waiting leaves too few lanes at the nodes.  Thread search's kernel time, signed
-// distance and swept volume as above: 1 lane 1.52 and 1.46 ms, 4 1.40 and 1.33, 8
-// 1.44 and 1.33, 16 1.40 and 1.41, 32 1.89 and 1.54.
+// waiting leaves too few lanes at the nodes.  The same calls with 4 / 8 / 16 lanes:
+// 1650 / 1662 / 1803, 1024 / 1095 / 1264, 1636 / 1720 / 1875, 749 / 768 / 882 us;
+// beside a far triangle, whose extent widens the leaves' bounds, 7330 / 6241 / 5026.
 constexpr int kLeafLanes = 8;
 constexpr int kLongThreads = 128;
 constexpr int kLongStack = 1024;  // shared-memory stack entries per warp
